@@ -1,0 +1,68 @@
+"""FP64 division, square root and multiplication on the integer pipes
+(bcm_fp64_int.cuh): bit-identical to IEEE arithmetic on the host, whatever
+the error of the hardware seeds, with every operand out of range flagged;
+and, on the GPU, the flux stage on states that take the fall-back to the
+reference's own expressions (tiny, huge, subnormal and non-finite values)."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import oracle as O
+from bcm_cgli_gb300 import api, cases
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fp64") / "check.so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-o", so,
+                    os.path.join(HERE, "fp64_int_check.cpp")], check=True)
+    lib = C.CDLL(so)
+    lib.fp64_int_bad.restype = C.c_long
+    lib.fp64_int_bad.argtypes = [C.c_int, C.c_int, C.c_long, C.c_double]
+    lib.fp64_int_unflagged.restype = C.c_long
+    return lib
+
+
+@pytest.mark.parametrize("op", range(6))
+@pytest.mark.parametrize("kind", range(6))
+def test_results_are_ieee(host, op, kind):
+    # seeds off by up to 2^-22 (twice the FP32 approximations' error bounds)
+    assert host.fp64_int_bad(op, kind, 300000, 2.0 ** -22) == 0
+
+
+def test_out_of_range_is_flagged(host):
+    assert host.fp64_int_unflagged() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [4, 8, 12])
+@pytest.mark.parametrize("viscous", [True, False])
+def test_flux_out_of_range_states(n, viscous):
+    case = cases.random_case(seed=3, n=n, viscous=viscous)
+    r = cases.splitmix_uniform(5, case.U[..., 0].size).reshape(case.U.shape[:-1])
+    U = case.U
+    U[r < 0.06, 1:4] = 0.0
+    U[(r >= 0.06) & (r < 0.1), 3] *= 1e-200
+    U[(r >= 0.1) & (r < 0.13), 2] *= 1e-320
+    U[(r >= 0.13) & (r < 0.132), 0] *= 1e90
+    U[(r >= 0.132) & (r < 0.134), 4] = -U[(r >= 0.132) & (r < 0.134), 4]
+    U[(r >= 0.134) & (r < 0.1345)] = np.inf
+    U[(r >= 0.1345) & (r < 0.135), 1] = np.nan
+    api.reference_config_for(case)
+    a, b = O.State(case), O.State(case)
+    with np.errstate(all="ignore"):
+        O.Port().flux_stage(case, a, 1)
+    api.BCM_Flux_XYZ_Viscous_Runge_kutta(0, case.ncube, 1, case.dT, case.dTau, case.e, case.fws,
+                                         case.csl, case.cube_size, b.U1_, b.U1, b.U1q, b.U1p1,
+                                         b.U1p2, b.Rku1, b.Residual1, b.er)
+    for k in ("U1_", "Rku1", "Residual1", "U1p1"):
+        x, y = getattr(a, k), getattr(b, k)
+        # with mu_L = 0 the oracle still forms its viscous terms, 0 * inf = NaN
+        # beside a non-finite temperature; the inviscid kernel has none
+        bad = np.argwhere(~((x == y) | (np.isnan(x) & (np.isnan(y) | (not viscous)))))
+        assert bad.size == 0, f"{k}: {len(bad)} mismatches, first {bad[:3]}"
