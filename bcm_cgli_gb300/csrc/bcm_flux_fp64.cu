@@ -21,17 +21,30 @@
 //    (then their left/right states are identical bit for bit); only faces
 //    next to non-fluid flags or cube edges get two evaluations;
 //  * divisions and square roots, which were over 40% of the FP64 pipe's
-//    work, run on the integer pipes (bcm_fp64_int.cuh: the same correctly
-//    rounded results, several quotients sharing one reciprocal);
+//    work, and about two thirds of the multiplications run on the integer
+//    pipes (bcm_fp64_int.cuh: the same correctly rounded results, several
+//    quotients sharing one reciprocal);
 //  * factors that are powers of two are exact, so c*x + y with such a c is
 //    one fused multiply-add with the reference's bits, and common factors
 //    are applied once at the end of a sum;
+//  * one CTA of 16 warps per SM, all in the same phase, and loops instead of
+//    unrolled components: the integer sequences are long, and more resident
+//    CTAs or unrolled copies miss the instruction cache (4^3 boxes: 4.1 ms
+//    for seven CTAs of two warps in an SM, 2.1 ms for one CTA of seven boxes;
+//    8^3: 1.95 ms unrolled, 1.84 ms in loops; 0.88 M cells, viscous);
 //  * where an operand is out of the integer routines' range the face, cell
 //    or primitive is redone by the reference's own expressions;
 //  * everything else keeps the reference's expression order, and this
 //    translation unit is compiled with --fmad=false, so every value equals
 //    the reference's (checked against the C oracle in tests/).
+// One launch over 0.88 M viscous cells in 16^3 cubes: 4.95 -> 1.84 ms (5.6 ->
+// 2.1 ns per cell).  What bounds it now: the FP64 pipe is 71% busy, nearly
+// all additions and fused multiply-adds, with four warps per scheduler to
+// hide its latency; moving the remaining products too was slower (their
+// chains are serial).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "bcm_common.cuh"
 #include "bcm_fp64_int.cuh"
@@ -43,24 +56,46 @@ struct Prim {
   double U, V, W, T;  // T = P/(rho*R): the neighbour form (:1734)
 };
 
-template <int T>
-struct FluxSmem {
-  static constexpr int B = T + 2;  // primitive box edge
-  static constexpr int nPrim = B * B * B;
-  static constexpr int nCell = T * T * T;
-  static constexpr int nFace = (T + 1) * T * T;  // faces of one axis
-  // Two views of a face: the plus-side cell's (the minus-side cell's for the
-  // tile's last face), and the minus-side cell's where its reconstruction
-  // order differs; five fluxes for each axis and the pressure of x and z
-  // faces, value-major.
-  static constexpr int nView = 17 * nFace;
-  static constexpr size_t bytes = sizeof(Prim) * nPrim + sizeof(double) * nCell /*Tc*/ +
-                                  2 * sizeof(double) * nView +
-                                  ((3 * nFace + 15) / 16) * 16 /*second view present*/;
+// The tiles of a CTA: `groups` boxes of ti x tj x tk cells, each inside one
+// cube.  Cubes whose edge is a multiple of 8 take one 8^3 box (compile-time
+// sizes); others the best box of divisors of n (flux_shape).
+constexpr int kFluxThreads = 512;
+struct Shape888 {
+  static constexpr int ti = 8, tj = 8, tk = 8, groups = 1;
 };
-// Threads per CTA: 8^3 tiles one per cell.  For 4^3 tiles two warps.
-template <int T>
-__host__ __device__ constexpr int flux_ctas_per_sm() { return T == 8 ? 1 : 7; }
+struct ShapeAny {
+  int ti, tj, tk, groups;
+};
+// Sizes that follow from a shape, and the shared memory of a CTA:
+//  * the faces' values, value-major per axis: five fluxes and the pressure in
+//    the plus-side cell's view (the minus-side cell's for the box's last
+//    face);
+//  * kSecond slots for the minus-side cell's view of faces where its
+//    reconstruction order differs, and each face's slot;
+//  * the primitives and centre temperatures;
+//  * work columns of the face phase (one double per thread and row).
+constexpr int kSecond = 256, kCols = 22;
+template <typename Sh>
+__host__ __device__ inline int box_cells(const Sh &s) { return s.ti * s.tj * s.tk; }
+template <typename Sh>
+__host__ __device__ inline int box_prims(const Sh &s) {
+  return (s.ti + 2) * (s.tj + 2) * (s.tk + 2);
+}
+template <typename Sh>
+__host__ __device__ inline int box_faces(const Sh &s, int ax) {
+  return box_cells(s) + (ax == 0 ? s.tj * s.tk : (ax == 1 ? s.ti * s.tk : s.ti * s.tj));
+}
+template <typename Sh>
+__host__ __device__ inline int box_faces(const Sh &s) {
+  return box_faces(s, 0) + box_faces(s, 1) + box_faces(s, 2);
+}
+template <typename Sh>
+__host__ __device__ inline size_t flux_smem(const Sh &s) {
+  const size_t faces = (size_t)s.groups * box_faces(s);
+  const size_t prims = s.groups * (sizeof(Prim) * box_prims(s) + sizeof(double) * box_cells(s));
+  const size_t cols = sizeof(double) * kCols * kFluxThreads;
+  return 6 * sizeof(double) * (faces + kSecond) + prims + cols + sizeof(uint16_t) * faces + 16;
+}
 
 // Division by a constant.
 #define BCMG_BY(value) \
@@ -161,47 +196,100 @@ __device__ __forceinline__ Prim prim_int(double q0, double q1, double q2, double
   return p;
 }
 
-// The reference's face flux (face_flux), for operands out of range.
-__device__ __noinline__ void face_ref(int ax, const double *ML, const double *MR, double e,
-                                      double *F, double *dP) {
-  if (ax == 0) face_flux<0, double>(ML, MR, e, F, *dP);
-  else if (ax == 1) face_flux<1, double>(ML, MR, e, F, *dP);
-  else face_flux<2, double>(ML, MR, e, F, *dP);
+// One view of a face by the reference's own expressions (recon, face_flux),
+// for operands out of the integer routines' range; it loads the stencil
+// again (values kept for it would spill the common path).
+__device__ __noinline__ void face_ref(int ax, int ord, const double *base, ptrdiff_t stride,
+                                      double e, double *dst, int nf) {
+  double ML[5], MR[5], F[5], dP;
+  auto ld = [&](int d, int v) -> double { return __ldg(base + 5 * stride * d + v); };
+  recon<double>(ord, ld, ML, MR);
+  if (ax == 0) face_flux<0, double>(ML, MR, e, F, dP);
+  else if (ax == 1) face_flux<1, double>(ML, MR, e, F, dP);
+  else face_flux<2, double>(ML, MR, e, F, dP);
+#pragma unroll
+  for (int v = 0; v < 5; ++v) dst[v * nf] = F[v];
+  dst[5 * nf] = dP;
 }
 
-// face_flux (bcm_common.cuh) with the divisions and roots on the integer
-// pipes and exact power-of-two factors folded; the axis is a run-time value
-// (one copy of the code: three unrolled copies miss the instruction cache).
-__device__ __forceinline__ bool face_int(int ax, const double *ML, const double *MR, double e,
-                                         double *F, double &dP) {
-  const double K = BCMG_K, Km1 = BCMG_K - 1;
-  IntFp o;
-  const Recip kL = o.recip(ML[0]), kR = o.recip(MR[0]);
-  double vL[3], vR[3], v[3];
+// A constant factor of a product.
+#define BCMG_TIMES(value) const_factor<__builtin_bit_cast(uint64_t, (double)(value))>()
+
+// recon() (bcm_common.cuh) with the fifth-order products on the integer
+// pipes: the raw values' small-integer multiples and the final 1/60.
+template <typename Ld>
+__device__ __forceinline__ void recon_int(IntFp &o, int ord, Ld ld, double *col) {
+  if (ord != 5) {
+    double ML[5], MR[5];
+    recon<double>(ord, ld, ML, MR);
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    vL[m] = o.div(ML[1 + m], kL);
-    vR[m] = o.div(MR[1 + m], kR);
+    for (int v = 0; v < 5; ++v) {
+      col[2 * v * kFluxThreads] = ML[v];
+      col[(2 * v + 1) * kFluxThreads] = MR[v];
+    }
+    return;
   }
-  const double VVL = vL[0] * vL[0] + vL[1] * vL[1] + vL[2] * vL[2];
-  const double VVR = vR[0] * vR[0] + vR[1] * vR[1] + vR[2] * vR[2];
-  const double rVL = ML[0] * VVL, rVR = MR[0] * VVR;  // twice 0.5 rho VV
-  const double PL = fma64(-0.5, rVL, ML[4]) * Km1, PR = fma64(-0.5, rVR, MR[4]) * Km1;
-  const double HL = fma64(0.5, VVL, o.div(o.div(K * PL, kL), BCMG_BY(BCMG_K - 1)));
-  const double HR = fma64(0.5, VVR, o.div(o.div(K * PR, kR), BCMG_BY(BCMG_K - 1)));
-  const double sL = o.root(ML[0]), sR = o.root(MR[0]);
+#pragma unroll 1
+  for (int v = 0; v < 5; ++v) {
+    const Factor b = o.plain(ld(-2, v)), c = o.plain(ld(-1, v)), d = o.plain(ld(0, v)),
+                 f = o.plain(ld(1, v));
+    const double l = fma64(2.0, ld(-3, v), -o.times<13>(b)) + o.times<47>(c) + o.times<27>(d) -
+                     o.times<3>(f);
+    const double r = fma64(2.0, ld(2, v), -o.times<3>(b) + o.times<27>(c) + o.times<47>(d) -
+                                              o.times<13>(f));
+    col[2 * v * kFluxThreads] = o.mul(BCMG_TIMES(1. / 60), l);
+    col[(2 * v + 1) * kFluxThreads] = o.mul(BCMG_TIMES(1. / 60), r);
+  }
+}
+
+// face_flux (bcm_common.cuh) with the divisions, roots and most products on
+// the integer pipes and exact power-of-two factors folded.  The axis is a
+// run-time value and the sides and components are loops over the thread's
+// work column (rows: 0..9 left and right values in turn; 10..13 and 14..17
+// velocity and enthalpy of the sides; 18..21 their averages): the code has to
+// stay in the instruction cache (unrolled, it was 5% slower and used 200
+// bytes of spills).
+__device__ __forceinline__ void face_int(IntFp &o, int ax, double *col, double e, double *F,
+                                         double &dP) {
+  const double K = BCMG_K;
+  auto at = [&](int row) -> double & { return col[row * kFluxThreads]; };
+  double PL = 0, PR = 0, EL = 0, ER = 0, sL = 0, sR = 0;
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const double r = at(s);
+    const Recip k = o.recip(r);
+    double VV = 0;
+#pragma unroll 1
+    for (int m = 0; m < 3; ++m) {
+      const double v = o.div(at(2 + 2 * m + s), k);
+      at(10 + 4 * s + m) = v;
+      const double vv = o.mul(v, v);
+      VV = m == 0 ? vv : VV + vv;
+    }
+    const double rV = o.mul(r, VV);  // twice 0.5 rho VV
+    const double P = o.mul(BCMG_TIMES(BCMG_K - 1), fma64(-0.5, rV, at(8 + s)));
+    at(13 + 4 * s) = fma64(0.5, VV, o.div(o.div(K * P, k), BCMG_BY(BCMG_K - 1)));
+    PL = PR; PR = P;
+    EL = ER; ER = fma64(0.5, rV, 3.5 * P);
+    sL = sR; sR = o.root(r);
+  }
   const Recip kS = o.recip(sL + sR);
-  const double rho = o.root(ML[0] * MR[0]);
-#pragma unroll
-  for (int m = 0; m < 3; ++m) v[m] = o.div(sL * vL[m] + sR * vR[m], kS);
-  const double VV = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-  const double H = o.div(sL * HL + sR * HR, kS);
-  const double C = fma64(-0.5, VV, H) * Km1;
+  const double rho = o.root(o.mul(at(0), at(1)));
+  double VV = 0;
+#pragma unroll 1
+  for (int m = 0; m < 4; ++m) {
+    const double v = o.div(o.mul(sL, at(10 + m)) + o.mul(sR, at(14 + m)), kS);
+    at(18 + m) = v;
+    if (m < 3) {
+      const double vv = o.mul(v, v);
+      VV = m == 0 ? vv : VV + vv;
+    }
+  }
+  const double H = at(21);
+  const double C = o.mul(BCMG_TIMES(BCMG_K - 1), fma64(-0.5, VV, H));
   const Recip kC = o.recip(C);
   const double beta = o.floor_at(o.div(VV, kC), e);
-  const double un = ax == 0 ? v[0] : (ax == 1 ? v[1] : v[2]);
-  const double unL = ax == 0 ? vL[0] : (ax == 1 ? vL[1] : vL[2]);
-  const double unR = ax == 0 ? vR[0] : (ax == 1 ? vR[1] : vR[2]);
+  const double un = at(18 + ax), unL = at(10 + ax), unR = at(14 + ax);
   const double omb = 1 - beta;
   const double t2 = (1 + beta) * un;  // twice temp
   const double S2 = o.root(fma64(4.0, beta * C, un * un * omb * omb));  // twice Sp
@@ -214,118 +302,109 @@ __device__ __forceinline__ bool face_int(int ax, const double *ML, const double 
   const double deltaU = (fma64(0.5, S2 - x3, -(beta * an))) * temp1 + tS * du;
   const double deltaP = tS * dp + fma64(0.5, x3, fma64(0.5, S2, -an)) * rho * du;
   const double dr = deltaU * rho;
-  double rvL[3], rvR[3];
-#pragma unroll
+  F[0] = o.half((o.mul(at(0), unL) + o.mul(at(1), unR)) - (o.mul(an, at(1) - at(0)) + dr));
+#pragma unroll 1
   for (int m = 0; m < 3; ++m) {
-    rvL[m] = ML[0] * vL[m];
-    rvR[m] = MR[0] * vR[m];
-  }
-  const double mL = ax == 0 ? rvL[0] : (ax == 1 ? rvL[1] : rvL[2]);
-  const double mR = ax == 0 ? rvR[0] : (ax == 1 ? rvR[1] : rvR[2]);
-  F[0] = o.half((mL + mR) - (an * (MR[0] - ML[0]) + dr));
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    double s = rvL[m] * unL, d = an * (MR[1 + m] - ML[1 + m]) + dr * v[m];
-    const double r = rvR[m] * unR;
+    double s = o.mul(unL, o.mul(at(0), at(10 + m)));
+    double d = o.mul(an, at(3 + 2 * m) - at(2 + 2 * m)) + o.mul(dr, at(18 + m));
+    const double r = o.mul(unR, o.mul(at(1), at(14 + m)));
     if (ax == m) {
       s = s + PL + r + PR;
       d = d + deltaP;
     } else {
       s = s + r;
     }
-    F[1 + m] = o.half(s - d);
+    at(18 + m) = o.half(s - d);
   }
-  const double F5 = an * (MR[4] - ML[4]) + dr * H + deltaP * un;
-  F[4] = o.half(unL * fma64(0.5, rVL, 3.5 * PL) + unR * fma64(0.5, rVR, 3.5 * PR) - F5);
+  const double F5 = o.mul(an, at(9) - at(8)) + o.mul(dr, H) + deltaP * un;
+  F[4] = o.half(o.mul(unL, EL) + o.mul(unR, ER) - F5);
   dP = o.half(PL + PR);
-  return o.ok;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) F[1 + m] = at(18 + m);
 }
 
-// visc_face with the divisions and root on the integer pipes.  by2T0 divides
-// by 2 T0, T0p is T0 + 110, invq inv / 4.
-template <int AX, bool FWD>
-__device__ __forceinline__ void visc_int(IntFp &o, double mu_L, const Recip &by2T0, double T0p,
-                                         double Tc, const Prim &c, const Prim &p, double inv,
-                                         double invq, const Prim &a0, const Prim &a1,
-                                         const Prim &a2, const Prim &a3, const Prim &b0,
-                                         const Prim &b1, const Prim &b2, const Prim &b3,
-                                         double *L) {
-  const double Ts = Tc + p.T;
-  const double temp = o.div(Ts, by2T0);
-  const double mu_E = o.div(mu_L * temp * o.root(temp) * T0p, o.recip(fma64(0.5, Ts, 110.)));
-  double gn[4];
-  if (FWD) {
-    gn[0] = (p.U - c.U) * inv; gn[1] = (p.V - c.V) * inv;
-    gn[2] = (p.W - c.W) * inv; gn[3] = (p.T - Tc) * inv;
-  } else {
-    gn[0] = (c.U - p.U) * inv; gn[1] = (c.V - p.V) * inv;
-    gn[2] = (c.W - p.W) * inv; gn[3] = (Tc - p.T) * inv;
-  }
-  double d[3][3];
-  constexpr int TA = AX == 0 ? 1 : 0, TB = AX == 2 ? 1 : 2;
-#pragma unroll
-  for (int m = 0; m < 3; ++m) d[AX][m] = gn[m];
-  d[TA][0] = (a0.U + a1.U - a2.U - a3.U) * invq;
-  d[TA][1] = (a0.V + a1.V - a2.V - a3.V) * invq;
-  d[TA][2] = (a0.W + a1.W - a2.W - a3.W) * invq;
-  d[TB][0] = (b0.U + b1.U - b2.U - b3.U) * invq;
-  d[TB][1] = (b0.V + b1.V - b2.V - b3.V) * invq;
-  d[TB][2] = (b0.W + b1.W - b2.W - b3.W) * invq;
-  const double div = d[0][0] + d[1][1] + d[2][2];
-  double s[3];
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    s[m] = m == AX ? mu_E * fma64(2.0, d[AX][AX], -(2.0 / 3.0 * div))
-                   : mu_E * (d[m][AX] + d[AX][m]);
-    L[m] = s[m];
-  }
-  const double work = (c.U + p.U) * s[0] + (c.V + p.V) * s[1] + (c.W + p.W) * s[2];  // twice
-  L[3] = fma64(0.5, work, o.div(mu_E * BCMG_CV * BCMG_K * gn[3], BCMG_BY(BCMG_PR)));
+// The tile's primitives as [cell][u, v, w, T].
+struct ViscIn {
+  const double *c;  // the cell
+  double mu_L, T0p, inv, invq, Tc;
+  Recip by2T0;
+};
+
+// visc_face with the divisions, root and products on the integer pipes, for
+// the face towards the neighbour at offset sn (doubles, signed: side) of
+// axis ax.  One copy of the code for the six faces of a cell: the axis and
+// side are run-time values (six unrolled copies miss the instruction
+// cache).  sa and sb are the strides of the other axes, lower axis first.
+__device__ __forceinline__ void visc_int(IntFp &o, const ViscIn &z, int ax, bool fwd, int sn,
+                                         int sa, int sb, double *L) {
+  const int ia = ax == 0 ? 1 : 0, ib = ax == 2 ? 1 : 2;
+  const double *c = z.c, *p = c + sn;
+  const double Ts = z.Tc + p[3];
+  const double temp = o.div(Ts, z.by2T0);
+  const Factor fmu = o.factor(
+      o.div(o.mul(o.mul(o.factor(z.mu_L), temp), o.root(temp)) * z.T0p,
+            o.recip(fma64(0.5, Ts, 110.))));
+  const Factor finv = o.factor(z.inv), finvq = o.factor(z.invq);
+  // normal differences, plus side less minus side
+  const double sg = fwd ? 1.0 : -1.0;
+  auto dn = [&](double x, double y) {  // (x - y) forward, (y - x) backward
+    const double d = x - y;
+    return d_make(d_hi(d) ^ (d_hi(sg) & 0x80000000u), d_lo(d));
+  };
+  const double cn = c[ax], ca = c[ia], cb = c[ib], pn = p[ax], pa = p[ia], pb = p[ib];
+  const double gn = o.mul(finv, dn(pn, cn)), ga = o.mul(finv, dn(pa, ca)),
+               gb = o.mul(finv, dn(pb, cb)), gT = o.mul(finv, dn(p[3], z.Tc));
+  // transverse differences of the velocity along ax and of the transverse one
+  auto tr = [&](int st, int comp) {
+    return o.mul(finvq, c[st + comp] + p[st + comp] - c[comp - st] - p[comp - st]);
+  };
+  const double an = tr(sa, ax), aa = tr(sa, ia), bn = tr(sb, ax), bb = tr(sb, ib);
+  // the divergence in x, y, z order
+  const double div = ax == 2 ? aa + bb + gn : gn + aa + bb;
+  const double tn = o.mul(fmu, fma64(2.0, gn, -(2.0 / 3.0 * div)));
+  const double ta = o.mul(fmu, an + ga), tb = o.mul(fmu, bn + gb);
+  const double wn = o.mul(cn + pn, tn), wa = o.mul(ca + pa, ta), wb = o.mul(cb + pb, tb);
+  const double w0 = ax == 0 ? wn : wa, w1 = ax == 0 ? wa : (ax == 1 ? wn : wb),
+               w2 = ax == 2 ? wn : wb;
+  L[0] = ax == 0 ? tn : ta;
+  L[1] = ax == 0 ? ta : (ax == 1 ? tn : tb);
+  L[2] = ax == 2 ? tn : tb;
+  const double heat =
+      o.mul(BCMG_TIMES(BCMG_K), o.mul(fmu, BCMG_CV)) * gT;
+  L[3] = fma64(0.5, w0 + w1 + w2, o.div(heat, BCMG_BY(BCMG_PR)));
 }
 
-// What the cell phase reads and writes of its CTA and cell.
-template <int T>
+// What the cell phase reads of its box and cell.
 struct CellIn {
-  const Prim *prim;
-  const double *F0, *F1;       // face views
-  const unsigned char *two;
-  int mi, mj, mk;
+  const double *c;              // primitives of the cell
+  int si, sj;                   // strides of the box's i and j (doubles; k: 4)
+  // per axis: the values of the backward and forward faces in the cell's view
+  // and the distances between them
+  const double *Fb[3], *Ff[3];
+  int nf[3], nff[3];
   size_t go;                    // cell offset in the state
   int flag;
   double Tc, dx, e, dT, dTau, mu_L, rho0, P0;
 
   __device__ __forceinline__ const Prim &P(int di, int dj, int dk) const {
-    constexpr int B = T + 2;
-    return prim[((mi + 1 + di) * B + (mj + 1 + dj)) * B + (mk + 1 + dk)];
-  }
-  // the cell's backward and forward faces of an axis
-  __device__ __forceinline__ int face(int ax, int step) const {
-    const int fa = (ax == 0 ? mi : (ax == 1 ? mj : mk)) + step;
-    const int p = ax == 0 ? mj : mi, q = ax == 2 ? mj : mk;
-    return (fa * T + p) * T + q;
-  }
-  __device__ __forceinline__ const double *fwd(int ax, int ff) const {
-    return two[ax * (T + 1) * T * T + ff] ? F1 : F0;
+    return *reinterpret_cast<const Prim *>(c + di * si + dj * sj + dk * 4);
   }
 };
 
 // The cell phase by the reference's own expressions (BDF2 source, viscous
 // balance, preconditioner), for operands out of the integer routines' range.
-template <int T, bool VISCOUS>
-__device__ __noinline__ void cell_ref(const FluxArgs &a, const CellIn<T> &z) {
-  constexpr int NF = (T + 1) * T * T;
+template <bool VISCOUS>
+__device__ __noinline__ void cell_ref(const FluxArgs &a, const CellIn &z) {
   const double dx = z.dx, inv = 1. / dx, e = z.e, dT = z.dT, dTau = z.dTau, mu_L = z.mu_L;
   const size_t go = z.go;
   double acc[5], dPdx = 0, dPdz = 0;
   for (int ax = 0; ax < 3; ++ax) {
-    const int fb = z.face(ax, 0), ff = z.face(ax, 1);
-    const double *Fw = z.fwd(ax, ff);
     for (int v = 0; v < 5; ++v) {
-      const double t = (Fw[(5 * ax + v) * NF + ff] - z.F0[(5 * ax + v) * NF + fb]) / dx;
+      const double t = (z.Ff[ax][v * z.nff[ax]] - z.Fb[ax][v * z.nf[ax]]) / dx;
       acc[v] = ax == 0 ? t : acc[v] + t;
     }
-    if (ax == 0) dPdx = Fw[15 * NF + ff] - z.F0[15 * NF + fb];
-    if (ax == 2) dPdz = Fw[16 * NF + ff] - z.F0[16 * NF + fb];
+    if (ax == 0) dPdx = z.Ff[0][5 * z.nff[0]] - z.Fb[0][5 * z.nf[0]];
+    if (ax == 2) dPdz = z.Ff[2][5 * z.nff[2]] - z.Fb[2][5 * z.nf[2]];
   }
   const Prim &c = z.P(0, 0, 0);
   double vF[5] = {0, 0, 0, 0, 0};
@@ -424,9 +503,8 @@ __device__ __noinline__ void cell_ref(const FluxArgs &a, const CellIn<T> &z) {
 // The cell phase with the divisions on the integer pipes and the exact
 // factors 2 and 4 of the preconditioner's rows applied to whole rows.
 // Returns false (and writes nothing) where an operand is out of range.
-template <int T, bool VISCOUS>
-__device__ __forceinline__ bool cell_int(const FluxArgs &a, const CellIn<T> &z) {
-  constexpr int NF = (T + 1) * T * T;
+template <bool VISCOUS>
+__device__ __forceinline__ bool cell_int(const FluxArgs &a, const CellIn &z) {
   IntFp o;
   const double dx = z.dx, e = z.e, dT = z.dT, dTau = z.dTau;
   const size_t go = z.go;
@@ -435,50 +513,47 @@ __device__ __forceinline__ bool cell_int(const FluxArgs &a, const CellIn<T> &z) 
   double acc[5], dPdx = 0, dPdz = 0;
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
-    const int fb = z.face(ax, 0), ff = z.face(ax, 1);
-    const double *Fw = z.fwd(ax, ff);
+    const int nf = z.nf[ax], nff = z.nff[ax];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      const double t = o.div(Fw[(5 * ax + v) * NF + ff] - z.F0[(5 * ax + v) * NF + fb], kdx);
+      const double t = o.div(z.Ff[ax][v * nff] - z.Fb[ax][v * nf], kdx);
       acc[v] = ax == 0 ? t : acc[v] + t;
     }
     if (z.flag != kFluid) {
-      if (ax == 0) dPdx = Fw[15 * NF + ff] - z.F0[15 * NF + fb];
-      if (ax == 2) dPdz = Fw[16 * NF + ff] - z.F0[16 * NF + fb];
+      if (ax == 0) dPdx = z.Ff[0][5 * nff] - z.Fb[0][5 * nf];
+      if (ax == 2) dPdz = z.Ff[2][5 * nff] - z.Fb[2][5 * nf];
     }
   }
   const Prim &c = z.P(0, 0, 0);
   double vF[5] = {0, 0, 0, 0, 0};
   if (VISCOUS) {
-    auto P = [&](int di, int dj, int dk) -> const Prim & { return z.P(di, dj, dk); };
-    const double T0 = o.div(o.div(z.P0, o.recip(z.rho0)), BCMG_BY(BCMG_R)), T0p = T0 + 110.;
-    const Recip by2T0 = o.recip(2 * T0);
-    const double invq = 0.25 * inv, Tc = z.Tc, mu_L = z.mu_L;
-    double Lb[4], Lf[4];
-    visc_int<0, false>(o, mu_L, by2T0, T0p, Tc, c, P(-1, 0, 0), inv, invq, P(0, 1, 0),
-                       P(-1, 1, 0), P(0, -1, 0), P(-1, -1, 0), P(0, 0, 1), P(-1, 0, 1),
-                       P(0, 0, -1), P(-1, 0, -1), Lb);
-    visc_int<0, true>(o, mu_L, by2T0, T0p, Tc, c, P(1, 0, 0), inv, invq, P(0, 1, 0), P(1, 1, 0),
-                      P(0, -1, 0), P(1, -1, 0), P(0, 0, 1), P(1, 0, 1), P(0, 0, -1),
-                      P(1, 0, -1), Lf);
+    static_assert(sizeof(Prim) == 4 * sizeof(double), "u, v, w, T");
+    const double T0 = o.div(o.div(z.P0, o.recip(z.rho0)), BCMG_BY(BCMG_R));
+    ViscIn q;
+    q.c = &c.U;
+    q.mu_L = z.mu_L;
+    q.T0p = T0 + 110.;
+    q.inv = inv;
+    q.invq = 0.25 * inv;
+    q.Tc = z.Tc;
+    q.by2T0 = o.recip(2 * T0);
+#pragma unroll 1
+    for (int ax = 0; ax < 3; ++ax) {
+      const int sn = ax == 0 ? z.si : (ax == 1 ? z.sj : 4);
+      const int sa = ax == 0 ? z.sj : z.si, sb = ax == 2 ? z.sj : 4;
+      double Lb[4], L[4] = {0, 0, 0, 0};
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {
 #pragma unroll
-    for (int v = 1; v < 5; ++v) vF[v] = (Lf[v - 1] - Lb[v - 1]) * inv;
-    visc_int<1, false>(o, mu_L, by2T0, T0p, Tc, c, P(0, -1, 0), inv, invq, P(1, 0, 0),
-                       P(1, -1, 0), P(-1, 0, 0), P(-1, -1, 0), P(0, 0, 1), P(0, -1, 1),
-                       P(0, 0, -1), P(0, -1, -1), Lb);
-    visc_int<1, true>(o, mu_L, by2T0, T0p, Tc, c, P(0, 1, 0), inv, invq, P(1, 0, 0), P(1, 1, 0),
-                      P(-1, 0, 0), P(-1, 1, 0), P(0, 0, 1), P(0, 1, 1), P(0, 0, -1),
-                      P(0, 1, -1), Lf);
+        for (int v = 0; v < 4; ++v) Lb[v] = L[v];
+        visc_int(o, q, ax, side == 1, side == 1 ? sn : -sn, sa, sb, L);
+      }
 #pragma unroll
-    for (int v = 1; v < 5; ++v) vF[v] = vF[v] + (Lf[v - 1] - Lb[v - 1]) * inv;
-    visc_int<2, false>(o, mu_L, by2T0, T0p, Tc, c, P(0, 0, -1), inv, invq, P(1, 0, 0),
-                       P(1, 0, -1), P(-1, 0, 0), P(-1, 0, -1), P(0, 1, 0), P(0, 1, -1),
-                       P(0, -1, 0), P(0, -1, -1), Lb);
-    visc_int<2, true>(o, mu_L, by2T0, T0p, Tc, c, P(0, 0, 1), inv, invq, P(1, 0, 0), P(1, 0, 1),
-                      P(-1, 0, 0), P(-1, 0, 1), P(0, 1, 0), P(0, 1, 1), P(0, -1, 0),
-                      P(0, -1, 1), Lf);
-#pragma unroll
-    for (int v = 1; v < 5; ++v) vF[v] = vF[v] + (Lf[v - 1] - Lb[v - 1]) * inv;
+      for (int v = 1; v < 5; ++v) {
+        const double x = (L[v - 1] - Lb[v - 1]) * inv;
+        vF[v] = ax == 0 ? x : vF[v] + x;
+      }
+    }
   }
   double *rk = a.Rku1 + 5 * go;
   if (z.flag != kFluid) {
@@ -566,135 +641,237 @@ __device__ __forceinline__ bool cell_int(const FluxArgs &a, const CellIn<T> &z) 
   return true;
 }
 
-template <int T, bool VISCOUS>
-__global__ void __launch_bounds__(T *T *T, flux_ctas_per_sm<T>()) k_flux_fp64(FluxArgs a) {
-  using SM = FluxSmem<T>;
-  constexpr int B = SM::B, NF = SM::nFace;
-  constexpr int NT = T * T * T;
+template <bool VISCOUS, typename Sh>
+__global__ void __launch_bounds__(kFluxThreads, 1) k_flux_fp64(FluxArgs a, Sh sh, int nboxes) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Prim *prim = reinterpret_cast<Prim *>(smem_raw);
-  double *Tcs = reinterpret_cast<double *>(prim + SM::nPrim);
-  double *F0 = Tcs + SM::nCell, *F1 = F0 + SM::nView;
-  unsigned char *two = reinterpret_cast<unsigned char *>(F1 + SM::nView);
+  const int nprim = box_prims(sh), ncell = box_cells(sh), nface = box_faces(sh);
+  const int f0 = box_faces(sh, 0), f1 = box_faces(sh, 1);  // x, y faces; the rest z
+  double *const F0 = reinterpret_cast<double *>(smem_raw), *const F1 = F0 + 6 * sh.groups * nface;
+  Prim *const prim = reinterpret_cast<Prim *>(F1 + 6 * kSecond);
+  double *const Tcs = reinterpret_cast<double *>(prim + sh.groups * nprim);
+  double *const cols = Tcs + sh.groups * ncell;
+  int *const nsecond = reinterpret_cast<int *>(cols + kCols * kFluxThreads);
+  uint16_t *const second = reinterpret_cast<uint16_t *>(nsecond + 1);  // 0: none, else slot + 1
 
   const int n = a.ph.n, S = n + 4, nx = n + 1;
-  const int nt = n / T;
+  const int nti = n / sh.ti, ntj = n / sh.tj, ntk = n / sh.tk, boxes = nti * ntj * ntk;
   const int tid = threadIdx.x;
-  const int tiles = nt * nt * nt;
-  const int cube = a.cube0 + blockIdx.x / tiles;
-  if (!case_active(a.bt, cube)) return;  // converged case (uniform per CTA)
-  const int tl = blockIdx.x % tiles;
-  const int bi = 2 + (tl / (nt * nt)) * T, bj = 2 + ((tl / nt) % nt) * T, bk = 2 + (tl % nt) * T;
   const double *__restrict__ U = a.U1_;
   const int *__restrict__ F = a.FWS;
-  const size_t cb = cell_index(S, cube, 0, 0, 0);
-  // Constants of the cube's case (kernel arguments for a single case).
-  double e = a.e, dT = a.dT, dTau = a.dTau, mu_L = a.ph.mu_L, rho0 = a.ph.rho0, P0 = a.ph.P0;
-  if (a.bt.cube_case) {
-    const CaseConst *q = a.bt.cases + __ldg(a.bt.cube_case + cube);
-    e = q->e; dT = q->dT; dTau = q->dTau; mu_L = q->mu_L; rho0 = q->rho0; P0 = q->P0;
-  }
+  // Box g of this CTA: its cube (0: past the last box, or a converged case)
+  // and the first cell of the box.
+  struct Box { int cube, bi, bj, bk; };
+  auto box = [&](int g) -> Box {
+    const int b = blockIdx.x * sh.groups + g;
+    if (b >= nboxes) return {0, 0, 0, 0};
+    const int cube = a.cube0 + b / boxes, tl = b % boxes;
+    if (!case_active(a.bt, cube)) return {0, 0, 0, 0};
+    return {cube, 2 + (tl / (ntj * ntk)) * sh.ti, 2 + ((tl / ntk) % ntj) * sh.tj,
+            2 + (tl % ntk) * sh.tk};
+  };
+  const Box only = box(0);
+  if (sh.groups == 1 && only.cube == 0) return;
+  if (tid == 0) *nsecond = 0;
+  __syncthreads();
+  // The constants of a cube's case (kernel arguments for a single case).
+  const CaseConst *cases = a.bt.cube_case ? a.bt.cases : nullptr;
+  auto case_at = [&](int cube) { return cases + __ldg(a.bt.cube_case + cube); };
 
-  // Phase 1: primitives over the tile plus a one-cell halo (edges included).
-  for (int p = tid; p < SM::nPrim; p += NT) {
-    int li = p / (B * B), lj = (p / B) % B, lk = p % B;
-    const double *q =
-        U + 5 * (cb + ((size_t)(bi - 1 + li) * S + (bj - 1 + lj)) * S + (bk - 1 + lk));
-    double Tc;
-    prim[p] = prim_int(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3), __ldg(q + 4), Tc);
-    if (li >= 1 && li <= T && lj >= 1 && lj <= T && lk >= 1 && lk <= T)
-      Tcs[((li - 1) * T + (lj - 1)) * T + (lk - 1)] = Tc;
-  }
-
-  // Phase 2: inviscid face fluxes of all three axes, one face per thread and
-  // turn (no barrier between axes: 54 warp turns of an 8^3 tile spread over
-  // 16 warps).
-#pragma unroll 1
-  for (int w = tid; w < 3 * NF; w += NT) {
-    const int ax = w / NF, f = w - ax * NF;
-    const int fa = f / (T * T), p = (f / T) % T, q = f % T;
-    int li, lj, lk;  // local index of the + cell of this face (fa may be T)
+  // Face fa (0..extent) of axis ax at in-plane position (p, q), seen from the
+  // cell on its minus or plus side: where its stencil starts and the order.
+  struct Stencil { const double *base; ptrdiff_t stride; int ob, of; };
+  auto stencil = [&](const Box &b, int ax, int fa, int p, int q) -> Stencil {
+    int li, lj, lk;  // local index of the + cell of this face
     if (ax == 0) { li = fa; lj = p; lk = q; }
     else if (ax == 1) { li = p; lj = fa; lk = q; }
     else { li = p; lj = q; lk = fa; }
-    const int g = (ax == 0 ? bi + li : (ax == 1 ? bj + lj : bk + lk));
+    const int gx = (ax == 0 ? b.bi + li : (ax == 1 ? b.bj + lj : b.bk + lk));
     const ptrdiff_t stride = ax == 0 ? (ptrdiff_t)S * S : (ax == 1 ? (ptrdiff_t)S : 1);
-    const size_t c0 = cb + ((size_t)(bi + li) * S + (bj + lj)) * S + (bk + lk);
-    const int fm2 = __ldg(F + c0 - 2 * stride), fm1 = __ldg(F + c0 - stride), f0 = __ldg(F + c0),
+    const size_t c0 = cell_index(S, b.cube, b.bi + li, b.bj + lj, b.bk + lk);
+    const int fm2 = __ldg(F + c0 - 2 * stride), fm1 = __ldg(F + c0 - stride), fc = __ldg(F + c0),
               fp1 = __ldg(F + c0 + stride);
-    const bool needB = fa < T, needF = fa > 0;
-    const int ob = order_backward(g, fm2, fm1, fp1);
-    const int of = order_forward(g, nx, fm2, f0, fp1);
-    const bool second = needB && needF && ob != of;
-    two[w] = second ? 1 : 0;
-    const double *base = U + 5 * c0;
-    auto ld = [&](int d, int v) -> double { return __ldg(base + 5 * stride * d + v); };
+    return {U + 5 * c0, stride, order_backward(gx, fm2, fm1, fp1),
+            order_forward(gx, nx, fm2, fc, fp1)};
+  };
+
+  // Phase 1: inviscid face fluxes of all three axes, one face per thread and
+  // turn (no barrier between axes: the 54 warp turns of an 8^3 box spread
+  // over 16 warps).
 #pragma unroll 1
-    for (int view = 0; view < (second ? 2 : 1); ++view) {
-      double ML[5], MR[5], Fx[5], dP;
-      recon<double>(view == 0 && needB ? ob : of, ld, ML, MR);
-      if (!face_int(ax, ML, MR, e, Fx, dP)) {
-        double a5[5], b5[5], F5[5], d5;
-        for (int v = 0; v < 5; ++v) { a5[v] = ML[v]; b5[v] = MR[v]; }
-        face_ref(ax, a5, b5, e, F5, &d5);
-        for (int v = 0; v < 5; ++v) Fx[v] = F5[v];
-        dP = d5;
+  for (int w = tid; w < sh.groups * nface; w += kFluxThreads) {
+    const int g = sh.groups == 1 ? 0 : w / nface, fw = w - g * nface;
+    const Box b = sh.groups == 1 ? only : box(g);
+    if (b.cube == 0) continue;
+    const int ax = fw < f0 ? 0 : (fw < f0 + f1 ? 1 : 2);
+    const int f = fw - (ax == 0 ? 0 : (ax == 1 ? f0 : f0 + f1));
+    const int nf = ax == 0 ? f0 : (ax == 1 ? f1 : nface - f0 - f1);
+    const int dp = ax == 0 ? sh.tj : sh.ti, dq = ax == 2 ? sh.tj : sh.tk;  // in-plane extents
+    const int fa = f / (dp * dq);
+    const Stencil st = stencil(b, ax, fa, (f / dq) % dp, f % dq);
+    const bool needB = fa < (ax == 0 ? sh.ti : (ax == 1 ? sh.tj : sh.tk)), needF = fa > 0;
+    const int views = needB && needF && st.ob != st.of ? 2 : 1;
+    if (views == 1) second[w] = 0;
+    const double e = cases ? case_at(b.cube)->e : a.e;
+    auto ld = [&](int d, int v) -> double { return __ldg(st.base + 5 * st.stride * d + v); };
+#pragma unroll 1
+    for (int view = 0; view < views; ++view) {
+      double *dst = F0 + 6 * (w - f) + f;
+      int stv = nf;  // distance between a face's values
+      if (view == 1) {
+        const int slot = atomicAdd(nsecond, 1);
+        second[w] = slot < kSecond ? (uint16_t)(slot + 1) : (uint16_t)0xffff;
+        if (slot >= kSecond) break;  // the cell forms its view itself
+        dst = F1 + 6 * slot;
+        stv = 1;
       }
-      double *dst = view == 0 ? F0 : F1;
+      double Fx[5], dP;
+      double *const col = cols + tid;
+      IntFp o;
+      const int ord = view == 0 && needB ? st.ob : st.of;
+      recon_int(o, ord, ld, col);
+      face_int(o, ax, col, e, Fx, dP);
+      if (o.ok) {
 #pragma unroll
-      for (int v = 0; v < 5; ++v) dst[(5 * ax + v) * NF + f] = Fx[v];
-      if (ax != 1) dst[(ax == 0 ? 15 : 16) * NF + f] = dP;
+        for (int v = 0; v < 5; ++v) dst[v * stv] = Fx[v];
+        dst[5 * stv] = dP;
+      } else {
+        face_ref(ax, ord, st.base, st.stride, e, dst, stv);
+      }
     }
+  }
+  // and the primitives over the boxes plus a one-cell halo (edges included),
+  // by the threads that have no face left
+  const int bj2 = sh.tj + 2, bk2 = sh.tk + 2;
+  const int turns = (sh.groups * nface + kFluxThreads - 1) / kFluxThreads;
+  const int done = sh.groups * nface - (turns - 1) * kFluxThreads;  // threads with a last face
+  for (int w = tid >= done ? tid - done : tid + kFluxThreads - done; w < sh.groups * nprim;
+       w += kFluxThreads) {
+    const int g = sh.groups == 1 ? 0 : w / nprim, p = w - g * nprim;
+    const Box b = sh.groups == 1 ? only : box(g);
+    if (b.cube == 0) continue;
+    const int li = p / (bj2 * bk2), lj = (p / bk2) % bj2, lk = p % bk2;
+    const double *q =
+        U + 5 * cell_index(S, b.cube, b.bi - 1 + li, b.bj - 1 + lj, b.bk - 1 + lk);
+    double Tc;
+    prim[w] = prim_int(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3), __ldg(q + 4), Tc);
+    if (li >= 1 && li <= sh.ti && lj >= 1 && lj <= sh.tj && lk >= 1 && lk <= sh.tk)
+      Tcs[g * ncell + ((li - 1) * sh.tj + (lj - 1)) * sh.tk + (lk - 1)] = Tc;
   }
   __syncthreads();
 
-  // Phase 3: the cell's balance, viscous fluxes, source, preconditioner,
+  // Phase 2: the cell's balance, viscous fluxes, source, preconditioner,
   // increment, force integrands.
-  CellIn<T> z;
-  z.prim = prim;
-  z.F0 = F0;
-  z.F1 = F1;
-  z.two = two;
-  z.mi = tid / (T * T);
-  z.mj = (tid / T) % T;
-  z.mk = tid % T;
-  z.go = cb + ((size_t)(bi + z.mi) * S + (bj + z.mj)) * S + (bk + z.mk);
+  if (tid >= sh.groups * ncell) return;
+  const int g = sh.groups == 1 ? 0 : tid / ncell, cell = tid - g * ncell;
+  const Box b = sh.groups == 1 ? only : box(g);
+  if (b.cube == 0) return;
+  const int mi = cell / (sh.tj * sh.tk), mj = (cell / sh.tk) % sh.tj, mk = cell % sh.tk;
+  CellIn z;
+  z.si = 4 * bj2 * bk2;
+  z.sj = 4 * bk2;
+  z.c = &prim[g * nprim].U + (mi + 1) * z.si + (mj + 1) * z.sj + (mk + 1) * 4;
+  z.e = a.e; z.dT = a.dT; z.dTau = a.dTau;
+  z.mu_L = a.ph.mu_L; z.rho0 = a.ph.rho0; z.P0 = a.ph.P0;
+  if (cases) {
+    const CaseConst *q = case_at(b.cube);
+    z.e = q->e; z.dT = q->dT; z.dTau = q->dTau;
+    z.mu_L = q->mu_L; z.rho0 = q->rho0; z.P0 = q->P0;
+  }
+  double own[3][6];  // the cell's view of a forward face that has no slot
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) {
+    const int first = g * nface + (ax == 0 ? 0 : (ax == 1 ? f0 : f0 + f1));  // of the axis
+    const int plane = ax == 0 ? sh.tj * sh.tk : (ax == 1 ? sh.ti * sh.tk : sh.ti * sh.tj);
+    const int p = ax == 0 ? mj : mi, q = ax == 2 ? mj : mk, m = ax == 0 ? mi : (ax == 1 ? mj : mk);
+    const int fb = m * plane + p * (ax == 2 ? sh.tj : sh.tk) + q, ff = fb + plane;
+    z.nf[ax] = ax == 0 ? f0 : (ax == 1 ? f1 : nface - f0 - f1);
+    z.Fb[ax] = F0 + 6 * first + fb;
+    z.Ff[ax] = F0 + 6 * first + ff;
+    z.nff[ax] = z.nf[ax];
+    const int slot = second[first + ff];
+    if (slot != 0) {
+      z.nff[ax] = 1;
+      if (slot != 0xffff) {
+        z.Ff[ax] = F1 + 6 * (slot - 1);
+      } else {
+        const Stencil st = stencil(b, ax, m + 1, p, q);
+        face_ref(ax, st.of, st.base, st.stride, z.e, own[ax], 1);
+        z.Ff[ax] = own[ax];
+      }
+    }
+  }
+  z.go = cell_index(S, b.cube, b.bi + mi, b.bj + mj, b.bk + mk);
   z.flag = __ldg(F + z.go);
-  z.Tc = Tcs[tid];
-  z.dx = a.cube_size[cube] / n;
-  z.e = e; z.dT = dT; z.dTau = dTau; z.mu_L = mu_L; z.rho0 = rho0; z.P0 = P0;
-  if (!cell_int<T, VISCOUS>(a, z)) {
-    const CellIn<T> zr = z;  // (the copy lives in local memory, z in registers)
-    cell_ref<T, VISCOUS>(a, zr);
+  z.Tc = Tcs[g * ncell + cell];
+  z.dx = a.cube_size[b.cube] / n;
+  if (!cell_int<VISCOUS>(a, z)) {
+    const CellIn zr = z;  // (the copy lives in local memory, z in registers)
+    cell_ref<VISCOUS>(a, zr);
   }
 }
 
-template <int T>
-static cudaError_t launch_t(const FluxArgs &a, int ncubes, cudaStream_t s) {
-  const int nt = a.ph.n / T;
-  const size_t smem = FluxSmem<T>::bytes;
-  const unsigned grid = (unsigned)(ncubes * nt * nt * nt);
-  if (grid == 0) return cudaSuccess;
-  cudaError_t e;
-  if (a.ph.mu_L != 0.0) {
-    e = cudaFuncSetAttribute(k_flux_fp64<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return e;
-    k_flux_fp64<T, true><<<grid, T * T * T, smem, s>>>(a);
-  } else {
-    e = cudaFuncSetAttribute(k_flux_fp64<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return e;
-    k_flux_fp64<T, false><<<grid, T * T * T, smem, s>>>(a);
+// The box of a cube edge that is not a multiple of 8: divisors of n, at most
+// 512 cells in all groups together, with the least time per cell by the
+// measured weights of a turn of the 512 threads over faces (0.36), primitives
+// (0.08) and cells (0.95, however many of the threads have one).
+static ShapeAny flux_shape(int n, int tile) {
+  ShapeAny best{4, 4, 4, 1};
+  double score = 0;
+  auto consider = [&](int i, int j, int k) {
+    ShapeAny s{i, j, k, 1};
+    if (box_cells(s) > kFluxThreads || flux_smem(s) > 227 * 1024) return;
+    while ((s.groups + 1) * box_cells(s) <= kFluxThreads) {
+      ++s.groups;
+      if (flux_smem(s) > 227 * 1024) {
+        --s.groups;
+        break;
+      }
+    }
+    const double t =
+        s.groups * (0.36 * box_faces(s) + 0.08 * box_prims(s)) / kFluxThreads + 0.95;
+    const double v = s.groups * box_cells(s) / t;
+    if (v > score * 1.0001) {
+      score = v;
+      best = s;
+    }
+  };
+  if (tile == 4) {
+    consider(4, 4, 4);
+    return best;
   }
+  int d[64], nd = 0;  // divisors of n (at most 256)
+  for (int i = 1; i <= n; ++i)
+    if (n % i == 0) d[nd++] = i;
+  for (int i = 0; i < nd; ++i)
+    for (int j = 0; j < nd; ++j)
+      for (int k = 0; k < nd; ++k) consider(d[i], d[j], d[k]);
+  return best;
+}
+
+template <bool VISCOUS, typename Sh>
+static cudaError_t launch_shape(const FluxArgs &a, const Sh &sh, int ncubes, cudaStream_t s) {
+  const size_t smem = flux_smem(sh);
+  const int n = a.ph.n;
+  const int nboxes = ncubes * (n / sh.ti) * (n / sh.tj) * (n / sh.tk);
+  if (nboxes == 0) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_flux_fp64<VISCOUS, Sh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const unsigned grid = (unsigned)((nboxes + sh.groups - 1) / sh.groups);
+  k_flux_fp64<VISCOUS, Sh><<<grid, kFluxThreads, smem, s>>>(a, sh, nboxes);
   return cudaGetLastError();
 }
 
 // Cubes [a.cube0, a.cube0 + ncubes) of the flat list.
 cudaError_t launch_flux_fp64(const FluxArgs &a, int ncubes, cudaStream_t s) {
   if (a.ph.n % 4 != 0) return cudaErrorInvalidValue;
-  if (flux_tile(a.ph.n, a.tile) == 8) return launch_t<8>(a, ncubes, s);
-  return launch_t<4>(a, ncubes, s);
+  const bool visc = a.ph.mu_L != 0.0;
+  if (flux_tile(a.ph.n, a.tile) == 8) {
+    const Shape888 sh;
+    return visc ? launch_shape<true>(a, sh, ncubes, s) : launch_shape<false>(a, sh, ncubes, s);
+  }
+  const ShapeAny sh = flux_shape(a.ph.n, a.tile);
+  return visc ? launch_shape<true>(a, sh, ncubes, s) : launch_shape<false>(a, sh, ncubes, s);
 }
 
 }  // namespace bcmg

@@ -99,6 +99,20 @@ struct RecipConst {
   }
 };
 
+// A factor of a product: its significand (shifted left by 5 for mul), its
+// exponent and sign words.
+struct Factor {
+  uint32_t m1, m0, e, sign;
+  bool zero;
+};
+// A compile-time factor, given by its bits.
+template <uint64_t bits>
+BCMG_HD Factor const_factor() {
+  constexpr uint64_t m = ((bits & 0xfffffffffffffull) | (1ull << 52)) << 5;
+  return Factor{(uint32_t)(m >> 32), (uint32_t)m, (uint32_t)(bits >> 32) & kExpMask,
+                (uint32_t)(bits >> 32), false};
+}
+
 // The sticky flag and the operations.
 struct IntFp {
   bool ok = true;
@@ -175,27 +189,69 @@ struct IntFp {
     return d_make((uint32_t)(t >> 33) + (((be + 1021u - sh) >> 1) << 20), (uint32_t)(t >> 1));
   }
 
-  // both factors: exact zero or 2^-503 .. 2^505
-  BCMG_HD double mul(double a, double b) {
-    const uint32_t ah = d_hi(a), al = d_lo(a), bh = d_hi(b), bl = d_lo(b);
-    const uint32_t ea = ah & kExpMask, eb = bh & kExpMask;
-    const bool za = ((ah & 0x7fffffffu) | al) == 0, zb = ((bh & 0x7fffffffu) | bl) == 0;
-    ok &= (za | within(ea, 520, 1528)) & (zb | within(eb, 520, 1528));
-    const uint32_t A1 = shl_pair(al, (ah & kFracMask) | kExpOne, 5), A0 = al << 5;
+  // A factor: exact zero or 2^-503 .. 2^505.
+  BCMG_HD Factor factor(double a) {
+    const uint32_t ah = d_hi(a), al = d_lo(a);
+    Factor f;
+    f.e = ah & kExpMask;
+    f.zero = ((ah & 0x7fffffffu) | al) == 0;
+    ok &= f.zero | within(f.e, 520, 1528);
+    f.m1 = shl_pair(al, (ah & kFracMask) | kExpOne, 5);
+    f.m0 = al << 5;
+    f.sign = ah;
+    return f;
+  }
+  // Product with another factor in the same range.
+  BCMG_HD double mul(const Factor &a, double b) {
+    const uint32_t bh = d_hi(b), bl = d_lo(b), eb = bh & kExpMask;
+    const bool zb = ((bh & 0x7fffffffu) | bl) == 0, z = a.zero | zb;
+    ok &= zb | within(eb, 520, 1528);
     const uint32_t B1 = shl_pair(bl, (bh & kFracMask) | kExpOne, 6), B0 = bl << 6;
-    const uint64_t p0 = (uint64_t)A0 * B0;
-    const uint64_t v = mul_wide(A1, B0, mul_wide(A0, B1, p0 >> 32));
-    const uint64_t H = mul_wide(A1, B1, v >> 32);  // bits 64.. of the product: 52 or 53
+    const uint64_t p0 = (uint64_t)a.m0 * B0;
+    const uint64_t v = mul_wide(a.m1, B0, mul_wide(a.m0, B1, p0 >> 32));
+    const uint64_t H = mul_wide(a.m1, B1, v >> 32);  // bits 64.. of the product: 52 or 53
     const uint32_t Hh = (uint32_t)(H >> 32), Hl = (uint32_t)H, vl = (uint32_t)v;
     const uint32_t s = (Hh >> 20) ^ 1u;
     const uint32_t mh = shl_pair(Hl, Hh, s), ml = shl_pair(vl, Hl, s);
     const uint32_t r = (vl << s) | ((uint32_t)p0 != 0u ? 1u : 0u);  // rounding bits, sticky
     const uint64_t m =
         (((uint64_t)mh << 32) | ml) + (r + 0x7fffffffu + (ml & 1u) < r ? 1u : 0u);
-    const uint32_t ex = ea + eb - ((1023u + s) << 20);
-    const bool z = za || zb;
-    return d_make((z ? 0u : (uint32_t)(m >> 32) + ex) | ((ah ^ bh) & 0x80000000u),
+    const uint32_t ex = a.e + eb - ((1023u + s) << 20);
+    return d_make((z ? 0u : (uint32_t)(m >> 32) + ex) | ((a.sign ^ bh) & 0x80000000u),
                   z ? 0u : (uint32_t)m);
+  }
+  BCMG_HD double mul(double a, double b) { return mul(factor(a), b); }
+
+  // A significand for products with small integers: exact zero or
+  // 2^-503 .. 2^505.
+  BCMG_HD Factor plain(double a) {
+    const uint32_t ah = d_hi(a), al = d_lo(a);
+    Factor f;
+    f.e = ah & kExpMask;
+    f.zero = ((ah & 0x7fffffffu) | al) == 0;
+    ok &= f.zero | within(f.e, 520, 1528);
+    f.m1 = (ah & kFracMask) | kExpOne;
+    f.m0 = al;
+    f.sign = ah;
+    return f;
+  }
+  // C a for a small odd integer C: the product has at most 59 bits, so two
+  // 32-bit products hold it.
+  template <int C>
+  BCMG_HD double times(const Factor &a) {
+    constexpr int k = C < 4 ? 1 : (C < 8 ? 2 : (C < 16 ? 3 : (C < 32 ? 4 : 5)));  // 2^k < C
+    static_assert(C > (1 << k) && C < (2 << k), "an odd integer from 3 to 63");
+    const uint64_t p0 = (uint64_t)a.m0 * C;
+    const uint32_t ph = a.m1 * C + (uint32_t)(p0 >> 32), pl = (uint32_t)p0;
+    const uint32_t g = ph >> (21 + k), s = k + g;  // bits beyond the 53rd
+    // round to nearest even at bit s: add half a unit less one, plus the
+    // last kept bit
+    const uint32_t add = ((1u << (k - 1)) << g) - 1u + ((pl >> s) & 1u);
+    const uint64_t t = (((uint64_t)ph << 32) | pl) + add;
+    const uint32_t th = (uint32_t)(t >> 32);
+    const uint32_t hi = (th >> s) + a.e + (s << 20) - kExpOne;
+    return d_make((a.zero ? 0u : hi) | (a.sign & 0x80000000u),
+                  a.zero ? 0u : shr_pair((uint32_t)t, th, s));
   }
 
   // x / 2: exact zero or any normal number from 2^-511

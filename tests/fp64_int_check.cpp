@@ -41,7 +41,8 @@ void operands(int kind, uint64_t &s, int elo, int ehi, double &a, double &b) {
 }
 }  // namespace
 
-// op 0 div, 1 root, 2 mul, 3 half, 4 floor_at, 5 division by constants
+// op 0 div, 1 root, 2 mul, 3 half, 4 floor_at, 5 division by constants,
+// 6 products with constants
 extern "C" long fp64_int_bad(int op, int kind, long count, double seed_err) {
   uint64_t s = 977 * (uint64_t)op + 31 * (uint64_t)kind + 1;
   long bad = 0;
@@ -76,6 +77,14 @@ extern "C" long fp64_int_bad(int op, int kind, long count, double seed_err) {
       b = std::fabs(b);
       x = o.floor_at(a, b);
       y = a > b ? a : b;
+    } else if (op == 6) {
+      operands(kind, s, 520, 1528, a, b);
+      const Factor f = o.plain(a);
+      bad += !same(o.times<3>(f), 3 * a) + !same(o.times<13>(f), 13 * a);
+      bad += !same(o.times<27>(f), 27 * a) + !same(o.times<47>(f), 47 * a);
+      bad += !same(o.times<5>(f), 5 * a) + !same(o.times<63>(f), 63 * a);
+      x = o.mul(const_factor<__builtin_bit_cast(uint64_t, 1. / 60)>(), a);
+      y = 1. / 60 * a;
     } else {
       operands(kind, s, 768, 1280, a, b);
       x = o.div(a, RecipConst<__builtin_bit_cast(uint64_t, 1.4 - 1)>::get());
@@ -100,6 +109,7 @@ extern "C" long fp64_int_unflagged(void) {
     { IntFp o; o.root(v); n += o.ok; }
     { IntFp o; o.mul(v, 1.5); n += o.ok; }
     { IntFp o; o.mul(1.5, v); n += o.ok; }
+    { IntFp o; o.plain(v); n += o.ok; }
     { IntFp o; if (v != L::max()) { o.half(v); n += o.ok; } }
   }
   { IntFp o; o.recip(0.0); n += o.ok; }

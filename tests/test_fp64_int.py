@@ -28,7 +28,7 @@ def host(tmp_path_factory):
     return lib
 
 
-@pytest.mark.parametrize("op", range(6))
+@pytest.mark.parametrize("op", range(7))
 @pytest.mark.parametrize("kind", range(6))
 def test_results_are_ieee(host, op, kind):
     # seeds off by up to 2^-22 (twice the FP32 approximations' error bounds)
