@@ -637,6 +637,7 @@ int case_lusgs(bcmg_case *c, bool full = true) {
     l.partials = c->partials;
     l.bt = c->bt();
     CK(launch_lusgs(l, c->nreal, c->stream));
+    c->launches += lusgs_launches() - 1;
   }
   ++c->launches;
   if (c->batched)

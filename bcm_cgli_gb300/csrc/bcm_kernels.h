@@ -175,6 +175,8 @@ struct LusgsArgs {
   Batch bt;
 };
 cudaError_t launch_lusgs(const LusgsArgs &a, int ncubes, cudaStream_t s);
+// Kernels of one launch_lusgs call.
+int lusgs_launches();
 
 // Split-precision LU-SGS: FP32 sweeps on the FP32 mirror of the state (deltas
 // from the case's reference state), FP64 update and norm sums.
