@@ -26,6 +26,7 @@ UNITS = [
     # FP32 work of the split path: approximate division/sqrt (a few ulp) and
     # flush-to-zero are inside its error budget; the FP64 parts are unaffected.
     ("bcm_flux_split.cu", ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
+    ("bcm_flux_march.cu", ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
     ("bcm_rk.cu", ["--fmad=false"]),
     ("bcm_halo.cu", ["--fmad=false"]),
     ("bcm_capi.cu", ["--fmad=false"]),

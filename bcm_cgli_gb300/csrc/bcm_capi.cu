@@ -249,6 +249,7 @@ struct bcmg_case {
   }
   float *D2 = nullptr;                   // split precision: FP32 of U1 - U1q
   float *inv_dx = nullptr;               // split precision: n / cube_size per cube
+  uint16_t *codes = nullptr;             // split precision: cell codes of FWS
   int *FWS = nullptr;
   double *cube_size = nullptr;
   int *task_cube = nullptr;  // destination cube of each face task
@@ -385,7 +386,7 @@ struct bcmg_case {
     for (auto x : ev) cudaEventDestroy(x);
     ev.clear();
     dfree(U1_); dfree(U1); dfree(U1q); dfree(U1p1); dfree(U1p2); dfree(Rku1); dfree(Residual1);
-    dfree(M); dfree(M2); dfree(mpar); dfree(D2); dfree(inv_dx);
+    dfree(M); dfree(M2); dfree(mpar); dfree(D2); dfree(inv_dx); dfree(codes);
     dfree(FWS); dfree(cube_size); dfree(task_cube); dfree(tasks); dfree(task_cube_p);
     dfree(tasks_p); dfree(push); dfree(task_cube_q); dfree(tasks_q); dfree(bc_cubes);
     dfree(task_cube_r); dfree(tasks_r); dfree(edge_r);
@@ -479,6 +480,7 @@ int case_flux(bcmg_case *c, int RK) {
     sa.Residual1 = c->Residual1;
     sa.bt = c->bt();
     sa.push = RK >= 1 ? c->push_table() : nullptr;
+    sa.codes = c->codes;
     CK(launch_flux_split(sa, c->nreal, c->stream));
   } else {
     CK(launch_flux_fp64(a, c->nreal, c->stream));
@@ -1139,6 +1141,7 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
         ck(dalloc(&c->mpar, 1), "alloc") && ck(cudaMemset(c->mpar, 0, sizeof(int)), "memset") &&
         ck(dalloc(&c->D2, nd), "alloc") && ck(cudaMemset(c->D2, 0, nd * sizeof(float)), "memset") &&
         ck(dalloc(&c->inv_dx, (size_t)d->ncube), "alloc") &&
+        ck(dalloc(&c->codes, c->ncell), "alloc") &&
         ck(cudaMemset(c->M, 0, nd * sizeof(float)), "memset") &&
         ck(cudaMemset(c->M2, 0, nd * sizeof(float)), "memset") &&
         true))
@@ -1226,6 +1229,7 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
                                            cudaMemcpyHostToDevice, s), "copy") &&
                         ck(cudaMemcpyAsync(c->bc_masks, bcm.data(), sizeof(int) * bcm.size(),
                                            cudaMemcpyHostToDevice, s), "copy"))) &&
+       (!c->codes || ck(launch_cell_codes(c->FWS, c->codes, d->n, d->ncube, s), "cell codes")) &&
        ck(cudaStreamSynchronize(s), "sync");
   if (!ok) return fail(BCMG_ERR_CUDA);
   c->nbc = (int)bcc.size();
@@ -2324,6 +2328,7 @@ struct Compat {
   int precision = BCMG_PRECISION_FP64;
   float *M = nullptr, *M2 = nullptr, *D2 = nullptr, *inv_dx = nullptr;
   int *mpar = nullptr;
+  uint16_t *codes = nullptr;  // cell codes of the call's flags
 
   Phys phys() const {
     Phys p;
@@ -2349,7 +2354,7 @@ struct Compat {
     if (nc == ncube && Sx == full_S && U1_) return BCMG_OK;
     dfree(U1_); dfree(U1); dfree(U1q); dfree(U1p1); dfree(U1p2); dfree(Rku1);
     dfree(Residual1); dfree(cube_size); dfree(partials); dfree(er); dfree(FWS);
-    dfree(M); dfree(M2); dfree(D2); dfree(inv_dx); dfree(mpar);
+    dfree(M); dfree(M2); dfree(D2); dfree(inv_dx); dfree(mpar); dfree(codes);
     ncube = nc;
     S = full_S = Sx;
     ncell = (size_t)nc * S * S * S;
@@ -2368,7 +2373,7 @@ struct Compat {
     if (M) return BCMG_OK;
     const size_t nd = ncell * 5;
     CK(dalloc(&M, nd)); CK(dalloc(&M2, nd)); CK(dalloc(&D2, nd));
-    CK(dalloc(&inv_dx, (size_t)ncube)); CK(dalloc(&mpar, 1));
+    CK(dalloc(&inv_dx, (size_t)ncube)); CK(dalloc(&mpar, 1)); CK(dalloc(&codes, ncell));
     CK(cudaMemsetAsync(mpar, 0, sizeof(int), s));
     return BCMG_OK;
   }
@@ -2715,6 +2720,7 @@ void BCM_Flux_XYZ_Viscous_Runge_kutta(int myid, int ncube, int RK, double deltaT
       CK(cudaMemcpyAsync(C.inv_dx, inv.data(), sizeof(float) * ncube, cudaMemcpyHostToDevice, s));
       CK(launch_mirror(C.U1_, C.M, C.M2, ph.n, ncube, ph.rho0, ph.P0, Batch(), s));
       CK(launch_level_diff(C.U1, C.U1q, C.D2, ph.n, ncube, s));
+      CK(launch_cell_codes(C.FWS, C.codes, ph.n, ncube, s));
       FluxSplitArgs sa;
       sa.ph = ph;
       sa.cube0 = 1;
@@ -2745,6 +2751,7 @@ void BCM_Flux_XYZ_Viscous_Runge_kutta(int myid, int ncube, int RK, double deltaT
       sa.form = 1;
       sa.partials = C.partials;
       sa.Residual1 = C.Residual1;
+      sa.codes = C.codes;
       CK(launch_flux_split(sa, ncube - 1, s));
       const long long total = (long long)(ncube - 1) * ph.n * ph.n * ph.n;
       const int blocks = (int)std::min<long long>(152 * 8, (total + 255) / 256);

@@ -95,8 +95,9 @@ struct FluxSplitArgs {
   int RK;              // stage 1..3: the kernel applies the stage update;
                        // 0: it writes the FP32 residual to R32 instead
   float *R32 = nullptr;  // [ncell][5] (RK == 0)
-  int tile = 0;          // tile edge 8 or 4 (0: 8 when n is a multiple of 8, else 4)
-  int form = 0;          // 8^3 tiles: 0 faces one at a time, 1 in packed FP32 pairs
+  int tile = 0;          // 4: 4^3 tiles; else the march where it serves n, or
+                         // 8^3 tiles (4^3 where 8 does not divide n)
+  int form = 0;          // 0 faces one at a time, 1 in packed FP32 pairs
   double *partials;    // [blocks][7] norm/force partial sums (stage 3)
   double *Residual1;
   Batch bt;
@@ -106,7 +107,16 @@ struct FluxSplitArgs {
   // layers copy its high layers (n, n+1); 0 where none.  Updated fluid
   // cells in those layers write their new value there too.
   const int *push = nullptr;
+  // [ncell] reconstruction orders and flags per cell (launch_cell_codes)
+  const uint16_t *codes = nullptr;
 };
+// Cell codes of a flag field (bcm_flux_march.cu).
+cudaError_t launch_cell_codes(const int *FWS, uint16_t *codes, int n, int ncube, cudaStream_t s);
+// The stage as a march along i (bcm_flux_march.cu): whether it serves cubes of
+// edge n, its norm partial blocks, its launch.
+bool flux_march_fits(int n);
+int flux_march_blocks(int n, int ncubes);
+cudaError_t launch_flux_march(const FluxSplitArgs &a, int ncubes, cudaStream_t s);
 // Tile edge a flux launch uses (tile: 0 default, else 8 or 4 when it divides n).
 int flux_tile(int n, int tile);
 // Blocks of one split flux launch over ncubes cubes (one per tile).
