@@ -16,6 +16,20 @@
 //    case (flags do not change while it steps) instead of staged flags.
 // The two planes of a step go through the face arithmetic as packed FP32
 // pairs (PACK), like the tile kernel's two faces per thread.
+//
+// One RK-stage launch, tile kernel -> march (ms): 2,744 cubes of 16^3 1.726 ->
+// 1.367, 512 of 16^3 0.336 -> 0.276, 512 of 24^3 1.094 -> 0.929, 216 of 32^3
+// 1.096 -> 0.855; edges that 8 does not divide took 4^3 tiles: 512 cubes of
+// 12^3 0.361 -> 0.152, 216 of 20^3 0.696 -> 0.277, 125 of 28^3 1.104 -> 0.439.
+// 39% fewer instructions than the tiles at n = 16.  What bounds it now (ncu, n =
+// 16): instruction latency with four warps per scheduler (issue slots 42%
+// active; 128 registers and 107 KB a CTA allow no more), the FP64 pipe 48%
+// busy with the cells' FP64 sums and conversions.  Tried and left out: nine
+// warps of 96 registers with a warp for the far faces (spills: 1.69 ms at
+// 2,744 cubes), loading the next cell's FP64 levels ahead into registers
+// (spills: 1.63), conversions on the integer pipes (1.40), whole cubes per
+// CTA instead of equal shares (1.34 there, but 0.294 at 512 cubes), one CTA
+// of 576 threads for n = 24 (1.11).
 #include <algorithm>
 #include <type_traits>
 
@@ -77,7 +91,7 @@ __device__ __forceinline__ void cp_async16(float *smem_dst, const float *gmem_sr
 
 constexpr int kRing = 7;    // delta planes i-2 .. i+4 of a step (i, i+1)
 constexpr int kPrimRing = 4;  // primitive planes i-1 .. i+2
-constexpr int kChunk = 4;   // planes per norm partial sum (fixed: independent of the launch)
+constexpr int kChunk = 2;   // planes per unit of work and norm partial sum
 
 // Shared-memory layout (floats) for cubes of edge n in tiles of tj rows.  The
 // row pitch is 5 n (mod 32), so the columns of consecutive threads fall into
@@ -101,27 +115,39 @@ struct MarchLayout {
 
 }  // namespace
 
+// Work is counted in chunks of kChunk planes of a tile, tiles in order; CTA b
+// takes chunks [b * each, (b + 1) * each), a march segment per tile it
+// touches, so that every CTA of one wave does the same work whatever the
+// number of cubes.
+template <int NN>
+__host__ __device__ constexpr int march_rows() {
+  return NN == 20 ? 10 : (NN == 24 ? 8 : (NN == 28 ? 7 : (NN == 32 ? 16 : NN)));
+}
 struct MarchShape {
-  int tj, len;  // rows of a tile, planes of a march segment
+  int tj, each, total;  // rows of a tile, chunks per CTA, chunks in all
 };
 
-template <int NN, bool VISCOUS, bool PACK>
-__global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
+template <int NN, bool VISCOUS, bool PACK, bool NORMS>
+__global__ void __launch_bounds__(NN == 32 ? 512 : 256, NN == 32 ? 1 : 2)
     k_flux_march(FluxSplitArgs a, MarchShape sh) {
   extern __shared__ __align__(16) float smem[];
   const int n = NN ? NN : a.ph.n, S = n + 4;
-  const int tj = NN == 8 ? 8 : (NN == 16 ? 16 : (NN == 24 ? 8 : (NN == 32 ? 16 : sh.tj)));
+  const int tj = NN ? march_rows<NN>() : sh.tj;
   const MarchLayout L(n, tj);
   float *const ring = smem;
   PrimF *const prims = reinterpret_cast<PrimF *>(ring + kRing * L.plane);
   float *const flux = reinterpret_cast<float *>(prims + kPrimRing * L.prim_plane);
 
   const int tid = threadIdx.x, NT = blockDim.x;
-  const int tiles = n / tj, segs = n / sh.len;
-  const int cube = a.cube0 + blockIdx.x / (tiles * segs);
-  if (!case_active(a.bt, cube)) return;  // converged case (uniform per CTA)
-  const int part = blockIdx.x % (tiles * segs);
-  const int j0 = 2 + (part / segs) * tj, i0 = 2 + (part % segs) * sh.len, i1 = i0 + sh.len;
+  const int tiles = n / tj, per_tile = n / kChunk;
+  const int u1 = min(sh.total, ((int)blockIdx.x + 1) * sh.each);
+#pragma unroll 1
+  for (int u = (int)blockIdx.x * sh.each, len; u < u1; u += len) {
+  const int tile = u / per_tile, chunk = u - tile * per_tile;
+  len = min(per_tile - chunk, u1 - u);
+  const int cube = a.cube0 + tile / tiles;
+  if (!case_active(a.bt, cube)) continue;  // converged case (uniform per CTA)
+  const int j0 = 2 + (tile % tiles) * tj, i0 = 2 + chunk * kChunk, i1 = i0 + len * kChunk;
   const SplitConst z = split_const(a, cube);
   const float inv = a.inv_dx[cube];
   // Mirror buffers: read the current one; stages 1..3 write the other one.
@@ -132,17 +158,10 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
   const int SS = S * S;
   const int jlo = j0 - 3 < 0 ? 0 : j0 - 3, jhi = j0 + tj + 3 > S ? S : j0 + tj + 3;
 
-  // Column of this thread: a cell's (j, k), or (past the cells) one of the
-  // tile's far faces: y faces beyond the last row, then z faces beyond k.
-  const int ncol = tj * n, ncol32 = (ncol + 31) & ~31;
+  // Column of this thread (idle threads stay on a valid cell).
+  const int ncol = tj * n;
   const bool is_cell = tid < ncol;
-  const int ex = tid - ncol32;  // far face
-  const bool far_y = ex >= 0 && ex < n, far_z = ex >= n && ex < n + tj;
-  int jl = 0, kl = 0;  // (idle threads stay on a valid cell)
-  if (is_cell) { jl = tid / n; kl = tid - jl * n; }
-  if (far_y) { jl = tj; kl = ex; }
-  if (far_z) { jl = ex - n; kl = n; }
-  const bool do_y = is_cell || far_y, do_z = is_cell || far_z;
+  const int jl = is_cell ? tid / n : 0, kl = is_cell ? tid - (tid / n) * n : 0;
   const int col = (j0 + jl - jlo) * L.pitch + 5 * (kl + 2);  // in a ring plane
   const int prow = (jl + 1) * L.prim_row + kl + 1;           // in a primitive plane
   const size_t go0 = cb + (size_t)(j0 + jl) * S + (kl + 2);  // cell offset of plane 0
@@ -227,7 +246,8 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
     __syncthreads();
   }
 
-  double s5[7] = {0, 0, 0, 0, 0, 0, 0};
+  double s5[8] = {0, 0, 0, 0, 0, 0, 0, 0}, s8 = 0;
+  unsigned c0 = code_at(i0), c1 = code_at(i0 + 1), c2 = code_at(i0 + 2);
 #pragma unroll 1
   for (int i = i0; i < i1; i += 2) {
     // Ring offsets of planes i-2 .. i+4.
@@ -251,7 +271,6 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
     make_prims(i + 2);
     // Faces of the two planes (lanes .x and .y): low y and z faces of planes
     // i, i + 1 into shared memory, i-faces above planes i, i + 1 in registers.
-    const unsigned c0 = code_at(i), c1 = code_at(i + 1);
     auto pair = [&](auto ax_, const float *b0, const float *b1, int stride, int o0, int o1,
                     float *d0, float *d1, int nf) {
       constexpr int AX = decltype(ax_)::value;
@@ -289,24 +308,45 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
     };
     const float *const p0 = ring + off[2] + col, *const p1 = ring + off[3] + col;
     float *const g0 = flux, *const g1 = flux + L.flux;
-    if (do_y) {
-      const int f = jl * n + kl;
-      pair(std::integral_constant<int, 1>(), p0, p1, L.pitch,
-           far_y ? code_fwd(c0, 1) : code_back(c0, 1), far_y ? code_fwd(c1, 1) : code_back(c1, 1),
-           g0 + f, g1 + f, L.fy);
-    }
-    if (do_z) {
-      const int f = 5 * L.fy + jl * (n + 1) + kl;
-      pair(std::integral_constant<int, 2>(), p0, p1, 5,
-           far_z ? code_fwd(c0, 2) : code_back(c0, 2), far_z ? code_fwd(c1, 2) : code_back(c1, 2),
-           g0 + f, g1 + f, L.fz);
+    // The column's own faces; then the tile's far faces (y beyond the last
+    // row, z beyond the last k), whose turn goes round the warps.
+    const int ex = tid - 32 * ((i >> 1) % (NT / 32)) ;
+    const int far = ex >= 0 ? ex : ex + NT;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      int j = jl, k = kl;
+      if (pass == 1) {
+        if (far >= n + tj) break;
+        j = far < n ? tj : far - n;
+        k = far < n ? far : n;
+      }
+      const int dj = (j - jl), dk = (k - kl);
+      const float *const b0 = p0 + dj * L.pitch + 5 * dk, *const b1 = p1 + dj * L.pitch + 5 * dk;
+      unsigned e0 = c0, e1 = c1;
+      if (pass == 1) {
+        const ptrdiff_t o = (ptrdiff_t)(go0 + (size_t)i * SS) + dj * S + dk;
+        e0 = __ldg(a.codes + o);
+        e1 = __ldg(a.codes + o + SS);
+      }
+      if (pass == 0 ? is_cell : far < n) {
+        const int f = j * n + k;
+        const bool end = pass == 1 && j0 + tj == n + 2;  // the cube's last y face
+        pair(std::integral_constant<int, 1>(), b0, b1, L.pitch,
+             end ? code_fwd(e0, 1) : code_back(e0, 1), end ? code_fwd(e1, 1) : code_back(e1, 1),
+             g0 + f, g1 + f, L.fy);
+      }
+      if (pass == 0 ? is_cell : far >= n) {
+        const int f = 5 * L.fy + j * (n + 1) + k;
+        pair(std::integral_constant<int, 2>(), b0, b1, 5,
+             pass ? code_fwd(e0, 2) : code_back(e0, 2), pass ? code_fwd(e1, 2) : code_back(e1, 2),
+             g0 + f, g1 + f, L.fz);
+      }
     }
     float Fa[6], Fb[6];     // i-faces above planes i and i + 1
     float own[2][6];        // the minus-side cell's view where it differs (rare)
     unsigned second = 0;
     if (is_cell) {
-      const bool last = i + 2 == i1;  // the segment's last face: seen from its minus side
-      const unsigned c2 = code_at(i + 2);
+      const bool last = i + 2 == n + 2;  // the cube's last face: seen from its minus side
       const float *const c = ring + col;
       float MLa[5], MRa[5], MLb[5], MRb[5];
       auto lda = [&](int d, int v) -> float { return c[off[3 + d] + v]; };
@@ -344,11 +384,23 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
       }
     }
     __syncthreads();  // fluxes and primitives complete; planes i-2, i-1 are free
-    load_plane(i + 5);
-    load_plane(i + 6);
+    if (i + 2 < i1) {
+      load_plane(i + 5);
+      load_plane(i + 6);
+    }
+    unsigned c3 = 0, c4 = 0;  // the next step's codes
+    if (i + 2 < i1) {
+      c3 = code_at(i + 3);
+      c4 = code_at(i + 4);
+    }
     if (is_cell) {
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {
+        SplitLevels lv;
+        float src[5];
+        split_load(a, go0 + (size_t)(i + q) * SS, lv);
+        split_source(lv, src);
+
         const int p = i + q;
         const unsigned cc = q == 0 ? c0 : c1;
         const float *const g = q == 0 ? g0 : g1;
@@ -363,7 +415,7 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
             for (int v = 0; v < 6; ++v) Ff[v] = own[q][v];
           }
 #pragma unroll
-          for (int v = 0; v < 5; ++v) acc[v] = (Ff[v] - Fx[v]) * inv;
+          for (int v = 0; v < 5; ++v) acc[v] = __fmul_rn(Ff[v] - Fx[v], inv);
           dPdx = Ff[5] - Fx[5];
         }
         {
@@ -374,17 +426,14 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
             Fbv[v] = lo[v * L.fy];
             Ffv[v] = hi[v * L.fy];
           }
-          if ((cc & (1u << 14)) && jl + 1 < tj) {
+          if ((cc & (1u << 14)) && j0 + jl <= n) {
             float ML[5], MR[5];
             states(code_fwd(__ldg(a.codes + go0 + (size_t)p * SS + S), 1), qm + L.pitch, L.pitch,
                    ML, MR);
             face_flux_delta<1>(ML, MR, z.ef, z.rho0, z.P0, Ffv, dummy);
           }
 #pragma unroll
-          for (int v = 0; v < 5; ++v) {
-            const float t = (Ffv[v] - Fbv[v]) * inv;
-            acc[v] = acc[v] + t;
-          }
+          for (int v = 0; v < 5; ++v) acc[v] = __fmaf_rn(Ffv[v] - Fbv[v], inv, acc[v]);
         }
         {
           const float *const lo = g + 5 * L.fy + jl * (n + 1) + kl, *const hi = lo + 1;
@@ -400,10 +449,7 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
             face_flux_delta<2>(ML, MR, z.ef, z.rho0, z.P0, Ffv, Ffv[5]);
           }
 #pragma unroll
-          for (int v = 0; v < 5; ++v) {
-            const float t = (Ffv[v] - Fbv[v]) * inv;
-            acc[v] = acc[v] + t;
-          }
+          for (int v = 0; v < 5; ++v) acc[v] = __fmaf_rn(Ffv[v] - Fbv[v], inv, acc[v]);
           dPdz = Ffv[5] - Fbv[5];
         }
         const PrimF *const q0 = prims + ((p - 1) & (kPrimRing - 1)) * L.prim_plane + prow;
@@ -421,7 +467,7 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
             pushI = 5 * ((ptrdiff_t)(d - cube) * ((ptrdiff_t)SS * S) +
                          (ptrdiff_t)(p <= 3 ? n : -n) * SS);
         }
-        split_cell<VISCOUS>(a, z, cube, inv, P, qm, acc, dPdx, dPdz, go, (cc & 1u) != 0, Mw, s5,
+        split_cell<VISCOUS, NORMS>(a, z, cube, inv, P, qm, acc, lv.x, src, dPdx, dPdz, go, (cc & 1u) != 0, Mw, s5,
                             [&](auto *U, const auto *un) {
                               auto *u = U + 5 * go;
                               if (pushI) {
@@ -437,6 +483,12 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
                                 for (int r = 0; r < 5; ++r) u[pushK + r] = un[r];
                               }
                             });
+        if (NORMS && NN == 8 && q == 0) {
+          norm_exchange(s5, tid & 31);
+          s8 = s5[0];
+#pragma unroll
+          for (int v = 0; v < 8; ++v) s5[v] = 0;
+        }
 #pragma unroll
         for (int v = 0; v < 6; ++v) {
           Fx[v] = Fa[v];
@@ -444,42 +496,44 @@ __global__ void __launch_bounds__(NN == 32 ? 576 : 288, NN == 32 ? 1 : 2)
         }
       }
     }
-    // Norm and force partial sums of a chunk of planes (stage 3), through
-    // the flux area.
-    if (a.RK == 3 && (i - 2) % kChunk == kChunk - 2) {
+    // Norm and force partial sums of the step's planes (stage 3), through the
+    // flux area: each warp's sums, then the warps' in order.  For n = 8 each
+    // warp adds the two planes' sums, as the tile kernel's warps do.
+    if (NORMS) {
       __syncthreads();  // the cells have read the fluxes
       double *red = reinterpret_cast<double *>(flux);
-#pragma unroll
-      for (int m = 0; m < 7; ++m) {
-        double v = s5[m];
-        s5[m] = 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((tid & 31) == 0) red[(tid >> 5) * 7 + m] = v;
-      }
+      const int m = norm_exchange(s5, tid & 31);
+      if ((tid & 31) < 8 && m < 7) red[(tid >> 5) * 7 + m] = NN == 8 ? s8 + s5[0] : s5[0];
       __syncthreads();
       if (tid < 7) {
         double v = 0;
-        for (int w = 0; w < ncol32 / 32; ++w) v += red[w * 7 + tid];
-        const int block = ((cube - a.cube0) * tiles + (j0 - 2) / tj) * (n / kChunk) + (i - 2) / kChunk;
-        a.partials[(size_t)block * 7 + tid] = v;
+        for (int w = 0; w < NT / 32; ++w) v += red[w * 7 + tid];
+        a.partials[(size_t)(tile * per_tile + (i - 2) / kChunk) * 7 + tid] = v;
       }
+#pragma unroll
+      for (int v = 0; v < 8; ++v) s5[v] = 0;
     }
+    c0 = c2;
+    c1 = c3;
+    c2 = c4;
     cp_async_wait_all();
     __syncthreads();  // planes i+5, i+6 have arrived; fluxes may be written again
   }
+  }  // march segments of this CTA
 }
 
 // Rows of a tile: the whole cross-section where two CTAs fit an SM, else the
 // widest divisor of n that leaves room for two (one of 16 rows for n = 32,
 // whose eight rows are a little too wide for two); 0: none fits.
+static int march_threads(int n, int tj) { return (tj * n + 31) & ~31; }
+
 static int march_tj(int n) {
   if (n < 8) return 0;
   if (n == 32) return 16;
+
   for (int tj = n; tj >= 1; --tj) {
     if (n % tj) continue;
-    const int threads = ((tj * n + 31) & ~31) + ((tj + n + 31) & ~31);
-    if (threads <= 288 && MarchLayout(n, tj).bytes() <= 112 * 1024) return tj;
+    if (march_threads(n, tj) <= 256 && march_threads(n, tj) >= n + tj && MarchLayout(n, tj).bytes() <= 112 * 1024) return tj;
   }
   return 0;
 }
@@ -488,28 +542,24 @@ bool flux_march_fits(int n) { return march_tj(n) > 0; }
 
 int flux_march_blocks(int n, int ncubes) { return ncubes * (n / march_tj(n)) * (n / kChunk); }
 
-template <int NN, bool VISCOUS, bool PACK>
+template <int NN, bool VISCOUS, bool PACK, bool NORMS>
 static cudaError_t launch_march_k(const FluxSplitArgs &a, const MarchShape &sh, unsigned grid,
                                   unsigned threads, size_t smem, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(
-      k_flux_march<NN, VISCOUS, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      k_flux_march<NN, VISCOUS, PACK, NORMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_flux_march<NN, VISCOUS, PACK><<<grid, threads, smem, s>>>(a, sh);
+  k_flux_march<NN, VISCOUS, PACK, NORMS><<<grid, threads, smem, s>>>(a, sh);
   return cudaGetLastError();
 }
 
-template <int NN>
+template <int NN, bool PACK>
 static cudaError_t launch_march_n(const FluxSplitArgs &a, const MarchShape &sh, unsigned grid,
                                   unsigned threads, size_t smem, cudaStream_t s) {
-  const bool visc = a.ph.mu_L != 0.0;
-  // one face at a time where the tile kernel's 4^3 form evaluated them so
-  // (edges that are no multiple of 8) or on request
-  const bool pack = a.form == 1 && a.ph.n % 8 == 0;
-  if (visc)
-    return pack ? launch_march_k<NN, true, true>(a, sh, grid, threads, smem, s)
-                : launch_march_k<NN, true, false>(a, sh, grid, threads, smem, s);
-  return pack ? launch_march_k<NN, false, true>(a, sh, grid, threads, smem, s)
-              : launch_march_k<NN, false, false>(a, sh, grid, threads, smem, s);
+  if (a.ph.mu_L != 0.0)
+    return a.RK == 3 ? launch_march_k<NN, true, PACK, true>(a, sh, grid, threads, smem, s)
+                     : launch_march_k<NN, true, PACK, false>(a, sh, grid, threads, smem, s);
+  return a.RK == 3 ? launch_march_k<NN, false, PACK, true>(a, sh, grid, threads, smem, s)
+                   : launch_march_k<NN, false, PACK, false>(a, sh, grid, threads, smem, s);
 }
 
 cudaError_t launch_flux_march(const FluxSplitArgs &a, int ncubes, cudaStream_t s) {
@@ -517,28 +567,28 @@ cudaError_t launch_flux_march(const FluxSplitArgs &a, int ncubes, cudaStream_t s
   if (tj == 0) return cudaErrorInvalidValue;
   if (ncubes <= 0) return cudaSuccess;
   const MarchLayout L(n, tj);
-  const unsigned threads = ((tj * n + 31) & ~31) + ((tj + n + 31) & ~31);
-  // Segment length: the march pays about three planes for its start, and
-  // whole waves of CTAs should fill the machine.
-  const int per_sm = std::max<int>(1, std::min<int>(576 / threads, (int)(227 * 1024 / (L.bytes() + 1024))));
-  const long long slots = 152LL * per_sm;
-  MarchShape sh{tj, n};
-  double best = 0;
-  for (int len = n; len >= kChunk; len -= kChunk) {
-    if (n % len) continue;
-    const long long ctas = (long long)ncubes * (n / tj) * (n / len);
-    const double t = (double)((ctas + slots - 1) / slots) * (len + 3);
-    if (best == 0 || t < best * 0.97) {
-      best = t;
-      sh.len = len;
-    }
+  const unsigned threads = march_threads(n, tj);
+  const int per_sm = std::max<int>(
+      1, std::min<int>(512 / threads, (int)(227 * 1024 / (L.bytes() + 1024))));
+  const long long total = (long long)ncubes * (n / tj) * (n / kChunk), slots = 152LL * per_sm;
+  if (total > INT32_MAX - slots) return cudaErrorInvalidValue;
+  const int each = (int)((total + slots - 1) / slots);
+  const MarchShape sh{tj, each, (int)total};
+  const unsigned grid = (unsigned)((total + each - 1) / each);
+  // Faces in packed pairs where 8 divides n, one at a time elsewhere (where
+  // the 4^3 tiles evaluated them so) or on request.
+  if (a.form == 1 && n % 8 == 0) {
+    if (n == 8) return launch_march_n<8, true>(a, sh, grid, threads, L.bytes(), s);
+    if (n == 16) return launch_march_n<16, true>(a, sh, grid, threads, L.bytes(), s);
+    if (n == 24) return launch_march_n<24, true>(a, sh, grid, threads, L.bytes(), s);
+    if (n == 32) return launch_march_n<32, true>(a, sh, grid, threads, L.bytes(), s);
+    return launch_march_n<0, true>(a, sh, grid, threads, L.bytes(), s);
   }
-  const unsigned grid = (unsigned)((long long)ncubes * (n / tj) * (n / sh.len));
-  if (n == 8) return launch_march_n<8>(a, sh, grid, threads, L.bytes(), s);
-  if (n == 16) return launch_march_n<16>(a, sh, grid, threads, L.bytes(), s);
-  if (n == 24) return launch_march_n<24>(a, sh, grid, threads, L.bytes(), s);
-  if (n == 32) return launch_march_n<32>(a, sh, grid, threads, L.bytes(), s);
-  return launch_march_n<0>(a, sh, grid, threads, L.bytes(), s);
+  if (n == 12) return launch_march_n<12, false>(a, sh, grid, threads, L.bytes(), s);
+  if (n == 20) return launch_march_n<20, false>(a, sh, grid, threads, L.bytes(), s);
+  if (n == 28) return launch_march_n<28, false>(a, sh, grid, threads, L.bytes(), s);
+  if (n == 32) return launch_march_n<32, false>(a, sh, grid, threads, L.bytes(), s);
+  return launch_march_n<0, false>(a, sh, grid, threads, L.bytes(), s);
 }
 
 }  // namespace bcmg

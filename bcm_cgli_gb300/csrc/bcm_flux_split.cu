@@ -356,7 +356,8 @@ __global__ void __launch_bounds__(split_threads<T>(), split_ctas_per_sm<T>())
   __syncthreads();
   // Norm / force partial sums of this CTA (stage 3), reduced below by all
   // threads.
-  double s5[7] = {0, 0, 0, 0, 0, 0, 0};
+  double s5[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  __shared__ double red8[T == 8 ? 16 * 7 : 1];  // n = 8: each warp turn's sums
   // Not unrolled: with the packed face pass, two cells' tails interleaved
   // measured 2.5% slower per launch (n = 16; 1.9% at n = 24, same bits).
 #pragma unroll 1
@@ -408,12 +409,33 @@ __global__ void __launch_bounds__(split_threads<T>(), split_ctas_per_sm<T>())
     return prim[((mi + 1 + di) * B + (mj + 1 + dj)) * B + (mk + 1 + dk)];
   };
   const size_t go = cb + ((size_t)(bi + mi) * S + (bj + mj)) * S + (bk + mk);
-  split_cell<VISCOUS>(a, z, cube, inv, P, BX(mi, mj, mk), acc, dPdx, dPdz, go,
+  SplitLevels lv;
+  float src[5];
+  split_load(a, go, lv);
+  split_source(lv, src);
+  split_cell<VISCOUS, true>(a, z, cube, inv, P, BX(mi, mj, mk), acc, lv.x, src, dPdx, dPdz, go,
                       FL(mi, mj, mk) == kFluid, Mw, s5, [&](auto *U, const auto *un) {
                         if (a.push) push_same_level(U, a.push, n, cube, bi + mi, bj + mj, bk + mk, un);
                       });
+  if (T == 8 && nt == 1 && a.RK == 3) {  // (whole warps: 288 and 224 cells)
+    const int m = norm_exchange(s5, tid & 31);
+    if ((tid & 31) < 8 && m < 7) red8[(cl >> 5) * 7 + m] = s5[0];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) s5[v] = 0;
+  }
   }  // cells of this thread
   if (a.RK != 3) return;
+  if (T == 8 && nt == 1) {
+    // n = 8: the march's partial sums (two planes each: a plane is two warp
+    // turns), so that either kernel gives a case the same norms
+    __syncthreads();
+    if (tid < 28) {
+      const int c = tid / 7, m = tid - 7 * c;
+      const double *r = red8 + 28 * c + m;
+      a.partials[(size_t)blockIdx.x * 28 + tid] = 0 + (r[0] + r[14]) + (r[7] + r[21]);
+    }
+    return;
+  }
   __syncthreads();  // the face buffers are reused for the block reduction
   double *red = reinterpret_cast<double *>(Fb);  // [NW][7]
   constexpr int NWR = NT / 32;
@@ -460,7 +482,14 @@ int flux_tile(int n, int tile) {
   return n % 8 == 0 ? 8 : 4;
 }
 
+// The march serves every cube edge from 12 on that fits its shared memory.
+// For n = 8 a whole cube is one tile: the march wins while its two-plane
+// units spread few cubes over the SMs (8 cubes 26 -> 20 us, 216 cubes 34 ->
+// 28 us); the tile kernel's 18 warps per SM against 12 win from about 700
+// cubes on (1000 cubes: 101 against 109 us).  Both leave the same bits,
+// norms included.
 static bool use_march(int n, int tile) { return tile != 4 && flux_march_fits(n); }
+constexpr int kMarchCubes8 = 700;
 
 int flux_split_blocks(int n, int ncubes, int tile) {
   if (use_march(n, tile)) return flux_march_blocks(n, ncubes);
@@ -471,7 +500,8 @@ int flux_split_blocks(int n, int ncubes, int tile) {
 
 cudaError_t launch_flux_split(const FluxSplitArgs &a, int ncubes, cudaStream_t s) {
   if (a.ph.n % 4 != 0) return cudaErrorInvalidValue;
-  if (use_march(a.ph.n, a.tile)) return launch_flux_march(a, ncubes, s);
+  if (use_march(a.ph.n, a.tile) && !(a.ph.n == 8 && ncubes >= kMarchCubes8))
+    return launch_flux_march(a, ncubes, s);
   if (flux_tile(a.ph.n, a.tile) == 8) return launch_split_t<8>(a, ncubes, s);
   return launch_split_t<4>(a, ncubes, s);
 }

@@ -305,14 +305,42 @@ __device__ __forceinline__ PrimF prim_split(const SplitConst &z, const float *q)
   return pr;
 }
 
-// The rest of a cell's stage, given its inviscid balance acc: viscous
-// balance (P(di, dj, dk) are the primitives around it), source,
+// A cell's FP64 state, the previous level and the level difference, as
+// loaded; split_source forms the BDF2 source (times -2 dT) from the FP64
+// time-level differences, then FP32.  The FP64 <-> FP32 conversions of the cell's stage
+// are the hardware's (IEEE round to nearest): here the FP64 pipe has room and
+// the integer pipes do not (measured: the integer-pipe routines of k_mirror
+// made the launch 7-8% longer).
+struct SplitLevels {
+  double x[5], y[5];
+  float d2[5];
+};
+__device__ __forceinline__ void split_load(const FluxSplitArgs &a, size_t go, SplitLevels &l) {
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    l.x[v] = a.U1_[5 * go + v];  // only this thread reads or writes these cells
+    l.y[v] = __ldg(a.U1 + 5 * go + v);
+    l.d2[v] = __ldg(a.D2 + 5 * go + v);
+  }
+}
+// (fused operations written out where the operands come from different
+// places in the kernels, so that both round alike)
+__device__ __forceinline__ void split_source(const SplitLevels &l, float *src) {
+#pragma unroll
+  for (int v = 0; v < 5; ++v)
+    src[v] = __fmaf_rn(3.0f, __double2float_rn(l.x[v] - l.y[v]), -l.d2[v]);
+}
+
+// The rest of a cell's stage, given its inviscid balance acc, state xq and
+// source src: viscous balance (P(di, dj, dk) are the primitives around it),
 // preconditioner, state update, norm terms, next mirror value.  qm are the
 // cell's deltas, go its offset; push(array, values) copies a new value into
-// the same-level neighbours' ghost layers.
-template <bool VISCOUS, typename Prims, typename Push>
+// the same-level neighbours' ghost layers.  NORMS: stage 3 (the sums take 14
+// registers).
+template <bool VISCOUS, bool NORMS, typename Prims, typename Push>
 __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitConst &z, int cube,
                                            float inv, Prims P, const float *qm, const float *acc,
+                                           const double *xq, const float *src,
                                            float dPdx, float dPdz, size_t go, bool fluid,
                                            float *Mw, double *s5, Push push) {
   const PrimF &c = P(0, 0, 0);
@@ -338,25 +366,11 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
       vF[v] = ((Lf[v - 1] - Lb[v - 1]) + (Mf[v - 1] - Mb[v - 1]) + (Nf[v - 1] - Nb[v - 1])) * inv;
   }
 
-  // BDF2 source from FP64 time-level differences, then FP32.  The FP64 <->
-  // FP32 conversions of this tail are the hardware's (IEEE round to
-  // nearest): here the FP64 pipe has room and the integer pipes do not
-  // (measured: the integer-pipe routines of k_mirror made the launch 7-8%
-  // longer).
-  double *u = a.U1_ + 5 * go;  // only this thread reads or writes these cells
-  const double *uu = a.U1 + 5 * go;
-  const float *d2p = a.D2 + 5 * go;
-  const float i2dt = z.i2dt;
+  double *u = a.U1_ + 5 * go;
   float Rk[5];
-  double xq[5], un[5];
+  double un[5];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    const double x = u[v], y = __ldg(uu + v);
-    xq[v] = x;
-    const float d1 = __double2float_rn(x - y), d2 = __ldg(d2p + v);
-    const float Rp = -(3.0f * d1 - d2) * i2dt;
-    Rk[v] = Rp - acc[v] + vF[v];
-  }
+  for (int v = 0; v < 5; ++v) Rk[v] = __fmaf_rn(-src[v], z.i2dt, -acc[v]) + vF[v];
   if (fluid && a.RK == 0) {
     // residual only: the LU-SGS right-hand side
 #pragma unroll
@@ -420,7 +434,7 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
     // FP64 state of another cell during the stage, so the write races with
     // nothing.
     push(a.U1_, un);
-    if (a.RK == 3) {
+    if (NORMS && a.RK == 3) {
       // Change norms of p, u, v, w, T from the increment, in FP32; summed
       // in FP64 (BCM_Flux...cpp:2530-2566).
       const float rf = rho, m1 = __double2float_rn(xq[1]), m2 = __double2float_rn(xq[2]),
@@ -450,8 +464,10 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
     const double r1 = -((double)(-dPdz * inv) + (double)vF[3]) * dV;
     a.Residual1[5 * go + 0] = r0;
     a.Residual1[5 * go + 1] = r1;
-    s5[5] += r0;
-    s5[6] += r1;
+    if (NORMS) {
+      s5[5] += r0;
+      s5[6] += r1;
+    }
   }
   if (Mw) {
     // The cell's mirror value after the stage into the next buffer (the
@@ -476,6 +492,23 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
     for (int v = 0; v < 5; ++v) mw[v] = m5[v];
     push(Mw, m5);
   }
+}
+
+// Sums of s[0..7] over the warp: lane l < 8 ends with value bit-reversed(l) in
+// s[0]; returns that value's number.
+__device__ __forceinline__ int norm_exchange(double *s, int lane) {
+#pragma unroll
+  for (int h = 4, b = 1; h >= 1; h >>= 1, b <<= 1) {
+    const bool up = lane & b;
+#pragma unroll
+    for (int m = 0; m < h; ++m) {
+      const double give = up ? s[m] : s[m + h], keep = up ? s[m + h] : s[m];
+      s[m] = keep + __shfl_xor_sync(0xffffffffu, give, b);
+    }
+  }
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 8);
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 16);
+  return 4 * (lane & 1) + 2 * ((lane >> 1) & 1) + ((lane >> 2) & 1);
 }
 
 }  // namespace bcmg
