@@ -589,7 +589,7 @@ LusgsSplitArgs lusgs_split_args(bcmg_case *c) {
   l.inv_dx = c->inv_dx;
   l.mir = c->mir();
   l.U1_ = c->U1_;
-  l.R32 = reinterpret_cast<const float *>(c->Rku1);
+  l.R32 = reinterpret_cast<float *>(c->Rku1);
   l.scr = c->lu_scr;
   l.Residual1 = c->Residual1;
   l.partials = c->partials;
@@ -617,12 +617,18 @@ int case_norms(bcmg_case *c, int nb) {
   return BCMG_OK;
 }
 
+// Norm partial sums per cube of an LU-SGS sub-iteration.
+int case_lu_blocks(const bcmg_case *c) {
+  return c->precision == BCMG_PRECISION_SPLIT ? lusgs_split_blocks(c->ph.n) : 1;
+}
+
 int case_lusgs(bcmg_case *c, bool full = true) {
   int r;
   if ((r = case_prologue(c, full))) return r;
   if ((r = case_flux(c, 0))) return r;
   if (c->precision == BCMG_PRECISION_SPLIT) {
     CK(launch_lusgs_split(lusgs_split_args(c), c->nreal, c->stream));
+    c->launches += lusgs_split_launches() - 1;
   } else {
     LusgsArgs l;
     l.ph = c->ph;
@@ -645,7 +651,7 @@ int case_lusgs(bcmg_case *c, bool full = true) {
   if (c->batched)
     CK(launch_norms_batch(c->ph.n, c->cases, c->case_blk_cube, c->ncase, c->partials, c->er,
                           c->stream, c->bt().active));
-  else if ((r = case_norms(c, c->nreal)))
+  else if ((r = case_norms(c, c->nreal * case_lu_blocks(c))))
     return r;
   if (c->batched) ++c->launches;
   // the split sweep made the same-level copies of the updated cells
@@ -1159,7 +1165,7 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
   c->nparts = rk_partial_blocks(probe);
   if (d->precision == BCMG_PRECISION_SPLIT)  // room for either tile edge
     c->nparts = std::max(c->nparts, flux_split_blocks(d->n, d->ncube - 1, 4));
-  c->nparts = std::max(c->nparts, d->ncube - 1);  // LU-SGS: one block per cube
+  c->nparts = std::max(c->nparts, (d->ncube - 1) * case_lu_blocks(c));
   if (c->batched) {
     // Stage-update blocks of about equal size that never straddle two cases
     // (per-case norms), the flux kernel's per-case block ranges (one block
@@ -1172,7 +1178,7 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
     std::vector<long long> blk;
     std::vector<int> cbr(c->ncase + 1), cbf(c->ncase + 1), cbc(c->ncase + 1),
         cube_case(d->ncube, 0);
-    for (int q = 0; q <= c->ncase; ++q) cbc[q] = c->case_cube0[q] - 1;
+    for (int q = 0; q <= c->ncase; ++q) cbc[q] = (c->case_cube0[q] - 1) * case_lu_blocks(c);
     for (int q = 0; q < c->ncase; ++q) {
       cbr[q] = (int)blk.size();
       cbf[q] = (c->case_cube0[q] - 1) * tiles;

@@ -198,15 +198,18 @@ struct LusgsSplitArgs {
   const float *inv_dx;     // [ncube] n / cube_size
   Mirror mir;              // FP32 deltas of the state: read and updated in place
   double *U1_;             // updated in place on fluid cells
-  const float *R32;        // residual (FP32) of every cell
-  float *scr;              // [ncube-1][11][n^3] sweep scratch (lusgs_split_scratch)
-  int threads = 0;         // threads per cube (0: the widest plane, in whole warps)
+  float *R32;              // in: residual (FP32) of every cell; out: increment
+  float *scr;              // [ncube-1][16][n^3] sweep scratch (lusgs_split_scratch)
+  int threads = 0;         // most threads per sweeping CTA (0: its widest plane)
   const double *Residual1;
-  double *partials;        // [ncube-1][7]
+  double *partials;        // [ncube-1][lusgs_split_blocks][7]
   Batch bt;
   const int *push = nullptr;  // same-level push table (FluxSplitArgs::push)
 };
 cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t s);
+// Norm partial sums per cube and kernels of one launch_lusgs_split call.
+int lusgs_split_blocks(int n);
+int lusgs_split_launches();
 // Floats of that scratch per cube.
 size_t lusgs_split_scratch(int n);
 // Default threads per cube of the split LU-SGS kernel (the widest plane).

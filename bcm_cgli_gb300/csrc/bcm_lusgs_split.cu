@@ -1,27 +1,40 @@
 // Split-precision LU-SGS sub-iteration: the sweeps in FP32, the update and
-// norm sums in FP64.  Same scheme and parallel form as the FP64 kernel
-// (bcm_lusgs.cu): per cube, forward and backward sweeps over the planes
-// i+j+k = const, the previous plane's values double-buffered in shared memory.  The cube's
-// inputs are first packed into a scratch in plane order, so the cells of a
-// plane are consecutive: they go to consecutive threads (full warps) and the
-// sequential sweeps read and write consecutive words; the update runs
-// afterwards slab by slab in memory order.  The sweep
-// is a preconditioner of the dual-time iteration (the FP32 residual it is
-// fed decides the converged state), so its coefficients come from the FP32
-// mirror of the state: deltas from the case's reference state (rho0, 0, 0,
-// 0, P0/(K-1)), pressure p = P0 + p'.  The increment is added to the FP64
+// norm sums in FP64.  Same scheme and parallel form as the FP64 kernels
+// (bcm_lusgs.cu): coefficients first, then forward and backward sweeps over
+// the planes i+j+k = const by a cluster of CTAs per cube, then the update.
+// The sweep is a preconditioner of the dual-time iteration (the FP32 residual
+// it is fed decides the converged state), so its coefficients come from the
+// FP32 mirror of the state: deltas from the case's reference state (rho0, 0,
+// 0, 0, P0/(K-1)), pressure p = P0 + p'.  The increment is added to the FP64
 // state and the change norms are formed from the FP32 increments and summed
 // in FP64, as in the split RK path.
+//
+// Plane order.  Between the kernels a cube's values lie value-major in the
+// order of the sweep (the cells of plane h, i then j ascending), so the
+// threads of a plane read and write consecutive words; k_lus_pack and
+// k_lus_update change between that order and the memory order slab by slab
+// (i fixed) through shared memory, where the cells of an anti-diagonal j + k
+// of the slab are a run of the plane order.
+//
+// A sub-iteration less its flux stage (ms), against one kernel that packed,
+// swept and updated a cube in one CTA and formed the coefficients in the chain
+// of planes: 216 cubes of 24^3 0.88 -> 0.63, 8 of 24^3 0.53 -> 0.29, 512 of
+// 32^3 5.20 -> 3.32, 512 of 16^3 0.53 -> 0.44 and 512 of 12^3 0.29 -> 0.28.  (512
+// of 8^3, where the three launches are most of it, 0.14 -> 0.15.)
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
-#include <atomic>
+#include <algorithm>
 
 #include "bcm_common.cuh"
 #include "bcm_kernels.h"
+#include "bcm_split_cell.cuh"
 
 namespace bcmg {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 // Cell coefficients U, V, W, VV, H, r_x, r_y, r_z, nu, dg from the FP32
 // deltas m (rho' = m0, rho u = m1.., E' = m4).
@@ -47,385 +60,432 @@ __device__ __forceinline__ void luf_coef(const float *m, float rho0, float P0, f
   k[5] = r0; k[6] = r1; k[7] = r2; k[8] = nu; k[9] = dg;
 }
 
-template <int D, bool LOWER>
-__device__ __forceinline__ void luf_off(const float *k, float idx, float omega, const float *dq,
-                                        float *s) {
+// Off-diagonal terms of a cell (coefficients k, increment dq) for its
+// neighbours across the faces of the three directions; LOWER: the A+ parts
+// (forward sweep), else A-.
+template <bool LOWER, typename Store>
+__device__ __forceinline__ void luf_terms(const float *k, float idx, float omega, const float *dq,
+                                          Store store) {
   const float U = k[0], V = k[1], W = k[2], VV = k[3], H = k[4];
-  const float un = D == 0 ? U : (D == 1 ? V : W);
-  const float dp = 0.4f * (dq[4] - (U * dq[1] + V * dq[2] + W * dq[3]) + 0.5f * VV * dq[0]);
-  const float t = dq[1 + D] - un * dq[0];
-  float a[5];
-  a[0] = dq[1 + D];
-  a[1] = un * dq[1] + U * t;
-  a[2] = un * dq[2] + V * t;
-  a[3] = un * dq[3] + W * t;
-  a[1 + D] += dp;
-  a[4] = un * (dq[4] + dp) + H * t;
-  const float h = 0.5f * idx, w = omega * k[5 + D], v = k[8] * idx * idx;
 #pragma unroll
-  for (int m = 0; m < 5; ++m)
-    s[m] += LOWER ? h * (a[m] + w * dq[m]) + v * dq[m] : h * (a[m] - w * dq[m]) - v * dq[m];
+  for (int D = 0; D < 3; ++D) {
+    const float un = D == 0 ? U : (D == 1 ? V : W);
+    const float dp =
+        0.4f * (dq[4] - (U * dq[1] + V * dq[2] + W * dq[3]) + 0.5f * VV * dq[0]);
+    const float t = dq[1 + D] - un * dq[0];
+    float a[5];
+    a[0] = dq[1 + D];
+    a[1] = un * dq[1] + U * t;
+    a[2] = un * dq[2] + V * t;
+    a[3] = un * dq[3] + W * t;
+    a[1 + D] += dp;
+    a[4] = un * (dq[4] + dp) + H * t;
+    const float h = 0.5f * idx, w = omega * k[5 + D], v = k[8] * idx * idx;
+#pragma unroll
+    for (int m = 0; m < 5; ++m)
+      store(D, m, LOWER ? h * (a[m] + w * dq[m]) + v * dq[m] : h * (a[m] - w * dq[m]) - v * dq[m]);
+  }
 }
 
-// Per-cube scratch in plane order: the cells of plane h = i+j+k, i then j
-// ascending, at positions pos = P[h] + Q[h][i] + (j - jlo(h, i)), one array
-// per value (mirror 0..4, residual / increment 5..9, fluid flag 10).  The
-// threads of a sweep plane (consecutive columns) and of a packing pass
-// (consecutive cells of a slab's anti-diagonal) touch consecutive words, so
-// every global access of the kernel is coalesced.
-constexpr int kScr = 11;
-// Shared slots of the previous plane, value-major [kSlot][n*n]: coefficients
-// 0..9, increment 10..14, fluid flag 15.
-constexpr int kSlot = 16;
+// Scratch of a cube, value-major [kScr][n^3] in plane order: coefficients
+// 0..9, residual / increment 10..14, flags 15 (bit 0 fluid; bits 1..3 the
+// lower x, y, z neighbour inside the cube is fluid, bits 4..6 the upper).
+constexpr int kScr = 16;
+constexpr int kSlabThreads = 256;
 
+// Position of the first cell of row i in plane h, and the row's first j.
 __device__ __forceinline__ int jlo_of(int h, int i, int n) {
   const int x = h - i - (n - 1);
   return x > 0 ? x : 0;
 }
+// cells of planes 0 .. h-1
+__device__ __forceinline__ int plane_start(int h, int n) {
+  // planes up to n-1 are triangles, the last n-1 too, between them the cube's
+  // count less both
+  auto tet = [](int x) { return x * (x + 1) * (x + 2) / 6; };  // sum of x triangles
+  int c = tet(h);
+  if (h > n) c -= 3 * tet(h - n);
+  if (h > 2 * n) c += 3 * tet(h - 2 * n);
+  return c;
+}
+// cells of rows 0 .. i-1 of plane h
+__device__ __forceinline__ int row_start(int h, int i, int n) {
+  // row l has max(0, min(n, h-l+1) - max(0, h-l-n+1)) cells: the counts of
+  // x = h - l + 1 summed over x = h-i+2 .. h+1, x clipped to [0, n], less the
+  // same of x - n
+  auto upto = [&](int x) {  // sum over y <= x of min(max(y, 0), n)
+    if (x <= 0) return 0;
+    return x <= n ? x * (x + 1) / 2 : n * (n + 1) / 2 + (x - n) * n;
+  };
+  return (upto(h + 1) - upto(h + 1 - i)) - (upto(h + 1 - n) - upto(h + 1 - n - i));
+}
 
-template <int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 448 ? 2 : 1) k_lusgs_split(LusgsSplitArgs a) {
-  extern __shared__ __align__(16) float fbuf[];
-  const int n = a.ph.n, S = n + 4, nn = n * n, n3 = nn * n, np = 3 * n - 2;
-  const int cube = 1 + blockIdx.x;
-  if (!case_active(a.bt, cube)) return;  // converged case
-  float dT = a.dTf, mu_L = a.mu_Lf, rho0 = a.rho0f, P0 = a.P0f, T0 = a.T0f;
-  double rho0d = a.mir.rho0, E0d = a.mir.E0;  // mirror reference state (FP64)
+// Cell t of a slab in anti-diagonal order: d = j + k ascending, then j.
+__device__ __forceinline__ void slab_cell(const unsigned short *start, int n, int t, int &j,
+                                          int &k) {
+  int lo = 0, hi = 2 * n - 1;  // the last diagonal that starts at or before t
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (start[mid] <= t) lo = mid; else hi = mid;
+  }
+  j = max(0, lo - (n - 1)) + t - start[lo];
+  k = lo - j;
+}
+__device__ __forceinline__ void slab_starts(unsigned short *start, int n) {
+  for (int d = threadIdx.x; d < 2 * n - 1; d += blockDim.x)
+    start[d] = (unsigned short)(d <= n ? d * (d + 1) / 2
+                                       : n * n - (2 * n - 1 - d) * (2 * n - d) / 2);
+}
+
+// The constants of a cube's case.
+struct LusConst {
+  float dT, mu_L, rho0, P0, T0;
+  double rho0d, E0d;  // mirror reference state (FP64)
+};
+__device__ __forceinline__ LusConst lus_const(const LusgsSplitArgs &a, int cube) {
+  LusConst z = {a.dTf, a.mu_Lf, a.rho0f, a.P0f, a.T0f, a.mir.rho0, a.mir.E0};
   if (a.bt.cube_case) {
     const CaseConst *q = a.bt.cases + a.bt.cube_case[cube];
-    dT = q->dTf; mu_L = q->mu_Lf; rho0 = q->rho0f; P0 = q->P0f; T0 = q->T0f;
-    rho0d = q->rho0; E0d = q->E0;
+    z = {q->dTf, q->mu_Lf, q->rho0f, q->P0f, q->T0f, q->rho0, q->E0};
   }
-  // The mirror of the state, read by the pack and updated in place with the
-  // state: this block reads only its own cube's interior cells of it, and
-  // writes those and (same-level pushes) other cubes' ghost cells, which no
-  // block of this launch reads.
-  float *const Mc = mirror_current(a.mir);
-  const float omega = a.omegaf, cfl = a.cflf;
+  return z;
+}
+
+// One slab (cube, i) per CTA: coefficients, residual and flags into plane
+// order.  (The mirror is read here and updated in k_lus_update: its interior
+// cells belong to one cube each.)
+__global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a) {
+  extern __shared__ __align__(16) float stage[];  // [kScr][n^2]
+  __shared__ unsigned short start[64];
+  const int n = a.ph.n, S = n + 4, nn = n * n;
+  const int cube = 1 + blockIdx.x / n, i = blockIdx.x % n;
+  if (!case_active(a.bt, cube)) return;  // converged case
+  const LusConst z = lus_const(a, cube);
   const float idx = a.inv_dx[cube];
-  const size_t cb = cell_index(S, cube, 0, 0, 0);
-  float *scr = a.scr + (size_t)blockIdx.x * kScr * n3;
-
-  // Shared memory: slots (also the slab staging area), then the tables.
-  float *slots = fbuf;                                   // [2][kSlot][nn]
-  int *Pt = reinterpret_cast<int *>(fbuf + 2 * kSlot * nn);  // [np + 1]
-  int *Qt = Pt + np + 1;                                 // [np][n]
-  int *At = Qt + np * n;                                 // [2n] anti-diagonal starts
-  int *sorder = At + 2 * n;                              // [nn] slab cells by anti-diagonal
-  unsigned short *dec = reinterpret_cast<unsigned short *>(sorder + nn);  // [n3] column of a position
-  const int tid = threadIdx.x, NT = blockDim.x;
-  for (int h = tid; h < np; h += NT) {
-    const int ilo = h - 2 * (n - 1) > 0 ? h - 2 * (n - 1) : 0, ihi = h < n - 1 ? h : n - 1;
-    int acc = 0;
-    for (int i = 0; i < n; ++i) {
-      Qt[h * n + i] = acc;
-      if (i >= ilo && i <= ihi) acc += (h - i < n - 1 ? h - i : n - 1) - jlo_of(h, i, n) + 1;
-    }
-  }
-  if (tid == 0) {
-    int acc = 0;
-    for (int h = 0; h < np; ++h) {
-      Pt[h] = acc;
-      const int ilo = h - 2 * (n - 1) > 0 ? h - 2 * (n - 1) : 0, ihi = h < n - 1 ? h : n - 1;
-      for (int i = ilo; i <= ihi; ++i)
-        acc += (h - i < n - 1 ? h - i : n - 1) - jlo_of(h, i, n) + 1;
-    }
-    Pt[np] = acc;
-    int d0 = 0;
-    for (int d = 0; d <= 2 * n - 2; ++d) {
-      At[d] = d0;
-      d0 += (d < 2 * n - 2 - d ? d : 2 * n - 2 - d) + 1;
-    }
+  const float *const Mc = mirror_current(a.mir);
+  slab_starts(start, n);
+  for (int jk = threadIdx.x; jk < nn; jk += kSlabThreads) {
+    const int j = jk / n, k = jk - j * n;
+    const size_t o = cell_index(S, cube, i + 2, j + 2, k + 2);
+    float m[5], kc[10];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) m[v] = Mc[5 * o + v];
+    luf_coef(m, z.rho0, z.P0, z.T0, z.mu_L, idx, z.dT, a.cflf, a.omegaf, kc);
+#pragma unroll
+    for (int v = 0; v < 10; ++v) stage[v * nn + jk] = kc[v];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) stage[(10 + v) * nn + jk] = a.R32[5 * o + v];
+    const int *F = a.FWS + o;
+    int f = F[0] == kFluid ? 1 : 0;
+    if (i > 0 && F[-S * S] == kFluid) f |= 2;
+    if (j > 0 && F[-S] == kFluid) f |= 4;
+    if (k > 0 && F[-1] == kFluid) f |= 8;
+    if (i + 1 < n && F[S * S] == kFluid) f |= 16;
+    if (j + 1 < n && F[S] == kFluid) f |= 32;
+    if (k + 1 < n && F[1] == kFluid) f |= 64;
+    stage[15 * nn + jk] = __int_as_float(f);
   }
   __syncthreads();
+  float *const scr = a.scr + (size_t)(cube - 1) * kScr * nn * n;
+  for (int t = threadIdx.x; t < nn; t += kSlabThreads) {
+    int j, k;
+    slab_cell(start, n, t, j, k);
+    const int h = i + j + k;
+    float *dst = scr + plane_start(h, n) + row_start(h, i, n) + (j - jlo_of(h, i, n));
+#pragma unroll
+    for (int v = 0; v < kScr; ++v) dst[(size_t)v * nn * n] = stage[v * nn + j * n + k];
+  }
+}
+
+// Shared memory of a sweeping CTA: the terms its cells add, value-major
+// [2 planes][3 directions][5][rows * n], then per plane the first cell of each
+// of its rows (its part of the plane counted from 0) and where the row lies
+// in the plane order.
+__host__ __device__ inline int lus_rows(int n, int size) { return (n + size - 1) / size; }
+__host__ __device__ inline size_t lus_smem(int n, int size) {
+  const size_t rows = lus_rows(n, size), np = 3 * n - 2;
+  return sizeof(float) * 30 * rows * n + sizeof(int) * np * rows +
+         sizeof(unsigned short) * np * (rows + 1);
+}
+
+// Two CTAs on an SM hide each other's barriers (65536 registers / 896).
+constexpr int kSweepThreads = 448;
+
+struct LusCell {
+  int i, j, pos;  // pos < 0: none
+  int k;
+  int fl;
+  float r[5], c[10];
+};
+
+template <bool LOWER>
+__device__ __forceinline__ void lus_sweep(const LusgsSplitArgs &a, cg::cluster_group cl,
+                                          float *slots, const int *where,
+                                          const unsigned short *first, float *scr, float *inc,
+                                          float idx) {
+  const int n = a.ph.n, S = n + 4, n3 = n * n * n, np = 3 * n - 2;
+  const int size = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int rows = lus_rows(n, size), cols = rows * n;
+  // cell t of the CTA's part of plane p
+  auto load = [&](int p, int t, LusCell &z) {
+    z.pos = -1;
+    if (p < 0 || p >= np) return;
+    const unsigned short *f = first + p * (rows + 1);
+    if (t >= f[rows]) return;
+    int lo = 0, hi = rows;  // the last row that starts at or before t
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (f[mid] <= t) lo = mid; else hi = mid;
+    }
+    z.i = lo * size + rank;
+    z.j = jlo_of(p, z.i, n) + t - f[lo];
+    z.k = p - z.i - z.j;
+    z.pos = where[p * rows + lo] + t - f[lo];
+    const float *q = scr + z.pos;
+#pragma unroll
+    for (int m = 0; m < 10; ++m) z.c[m] = q[(size_t)m * n3];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) z.r[m] = q[(size_t)(10 + m) * n3];
+    z.fl = __float_as_int(q[(size_t)15 * n3]);
+  };
+  auto cell = [&](int p, const LusCell &z) {
+    if (z.pos < 0 || !(z.fl & 1)) return;
+    const int col = (z.i / size) * n + z.j;
+    const float *in = slots + (p & 1) * 15 * cols + col;
+    const int nb = LOWER ? z.fl >> 1 : z.fl >> 4;
+    float s[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) s[m] = LOWER ? z.r[m] : 0.f;
+#pragma unroll
+    for (int D = 0; D < 3; ++D)
+      if (nb & (1 << D)) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) s[m] += in[(5 * D + m) * cols];
+      }
+    const float idg = 1.0f / z.c[9];
+    float dq[5];
+    float *q = scr + z.pos;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      dq[m] = LOWER ? s[m] * idg : z.r[m] - s[m] * idg;
+      if (LOWER) q[(size_t)(10 + m) * n3] = dq[m];
+      else inc[5 * (((z.i + 2) * S + (z.j + 2)) * S + z.k + 2) + m] = dq[m];
+    }
+    const int d = LOWER ? 1 : -1;
+    const bool wi = LOWER ? z.i + 1 < n : z.i > 0, wj = LOWER ? z.j + 1 < n : z.j > 0,
+               wk = LOWER ? z.k + 1 < n : z.k > 0;
+    float *const out = slots + ((p + d) & 1) * 15 * cols;
+    float *oi = out;
+    if (wi && size > 1) oi = cl.map_shared_rank(out, (z.i + d) % size);
+    oi += wi ? ((z.i + d) / size) * n + z.j : 0;
+    luf_terms<LOWER>(z.c, idx, a.omegaf, dq, [&](int D, int m, float x) {
+      if (D == 0) { if (wi) oi[m * cols] = x; }
+      else if (D == 1) { if (wj) out[(5 + m) * cols + col + d] = x; }
+      else { if (wk) out[(10 + m) * cols + col] = x; }
+    });
+  };
+  LusCell cur, nxt;
+  const int p0 = LOWER ? 0 : np - 1, d = LOWER ? 1 : -1;
+  load(p0, threadIdx.x, nxt);
+  for (int s = 0, p = p0; s < np; ++s, p += d) {
+    cur = nxt;
+    load(p + d, threadIdx.x, nxt);
+    cell(p, cur);
+    for (int t = threadIdx.x + blockDim.x; t < first[p * (rows + 1) + rows]; t += blockDim.x) {
+      load(p, t, cur);
+      cell(p, cur);
+    }
+    if (size == 1) __syncthreads(); else cl.sync();
+  }
+}
+
+__global__ void __launch_bounds__(kSweepThreads, 2) k_lus_sweep(LusgsSplitArgs a) {
+  extern __shared__ __align__(16) float slots[];
+  const cg::cluster_group cl = cg::this_cluster();
+  const int n = a.ph.n, np = 3 * n - 2;
+  const int size = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int cube = 1 + blockIdx.x / size;
+  if (!case_active(a.bt, cube)) return;  // converged case (the whole cluster)
+  const int rows = lus_rows(n, size);
+  int *where = reinterpret_cast<int *>(slots + 30 * rows * n);
+  unsigned short *first = reinterpret_cast<unsigned short *>(where + np * rows);
+  for (int p = threadIdx.x; p < np; p += blockDim.x) {
+    int sum = 0;
+    const int base = plane_start(p, n);
+    for (int l = 0; l < rows; ++l) {
+      const int i = l * size + rank;
+      first[p * (rows + 1) + l] = (unsigned short)sum;
+      where[p * rows + l] = base + row_start(p, i, n);
+      const int jlo = jlo_of(p, i, n), jhi = min(n - 1, p - i);
+      if (i < n && jhi >= jlo) sum += jhi - jlo + 1;
+    }
+    first[p * (rows + 1) + rows] = (unsigned short)sum;
+  }
+  // every CTA of the cluster has started before any writes into its memory
+  if (size == 1) __syncthreads(); else cl.sync();
+  float *const scr = a.scr + (size_t)(cube - 1) * kScr * n * n * n;
+  float *const inc = a.R32 + 5 * cell_index(n + 4, cube, 0, 0, 0);
+  const float idx = a.inv_dx[cube];
+  lus_sweep<true>(a, cl, slots, where, first, scr, inc, idx);   // dq* = (R + sum of lower A+ terms) / dg
+  lus_sweep<false>(a, cl, slots, where, first, scr, inc, idx);  // dq = dq* - (sum of upper A- terms) / dg
+}
+
+// Q += dq on fluid cells (FP64), one slab (i fixed) per CTA; change norms of
+// p, u, v, w, T from the FP32 increment (the split RK path's third-stage
+// formulas) and the force integrands of the non-fluid cells (fluid cells
+// have none).  The FP64 pipe bounds it (12 additions per cell and the warps'
+// sums), so the ten conversions go to the integer pipes: 216 cubes of 24^3
+// 232 -> 170 us.
+struct LusState {
+  size_t o;
+  bool fluid;
+  double u[5];
+  float m[5], dq[5];
+};
+
+constexpr int kUpdThreads = 256;
+
+__global__ void __launch_bounds__(kUpdThreads, 3) k_lus_update(LusgsSplitArgs a) {
+  __shared__ double red[kUpdThreads / 32][7];
+  const int n = a.ph.n, S = n + 4, nn = n * n, NT = blockDim.x, tid = threadIdx.x;
+  const int cube = 1 + blockIdx.x / n, i = blockIdx.x % n;
+  if (!case_active(a.bt, cube)) return;  // converged case
+  const LusConst z = lus_const(a, cube);
+  // The mirror of the state is updated in place with it: this block writes
+  // its own cells of it and (same-level pushes) other cubes' ghost cells,
+  // which no block of this launch reads.
+  float *const Mc = mirror_current(a.mir);
+  auto load = [&](int jk, LusState &s) {
+    if (jk >= nn) return;
+    const int j = jk / n, k = jk - j * n;
+    s.o = cell_index(S, cube, i + 2, j + 2, k + 2);
+    s.fluid = a.FWS[s.o] == kFluid;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      s.u[v] = a.U1_[5 * s.o + v];
+      s.m[v] = Mc[5 * s.o + v];
+      s.dq[v] = a.R32[5 * s.o + v];
+    }
+  };
+  LusState s;
+  double e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (int jk = tid; jk < nn; jk += NT) {
-    const int j = jk / n, k = jk - j * n, d = j + k;
-    sorder[At[d] + j - (d - (n - 1) > 0 ? d - (n - 1) : 0)] = jk;
-  }
-  auto pos = [&](int h, int i, int j) { return Pt[h] + Qt[h * n + i] + (j - jlo_of(h, i, n)); };
-  auto SV = [&](int v, int p) -> float & { return scr[(size_t)v * n3 + p]; };
-  __syncthreads();
-  for (int c = tid; c < n3; c += NT) {
-    const int i = c / nn, j = (c / n) % n, k = c % n;
-    dec[pos(i + j + k, i, j)] = (unsigned short)(i * n + j);
-  }
-  __syncthreads();
-
-  // Pack, slab by slab (i fixed): coalesced loads in memory order into
-  // shared memory, coalesced stores in plane order.
-  float *stage = slots;  // [kScr][nn]
-  for (int i = 0; i < n; ++i) {
-    for (int jk = tid; jk < nn; jk += NT) {
-      const int j = jk / n, k = jk - j * n;
-      const size_t o = cb + ((size_t)(i + 2) * S + (j + 2)) * S + (k + 2);
-#pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        stage[v * nn + jk] = Mc[5 * o + v];
-        stage[(5 + v) * nn + jk] = a.R32[5 * o + v];
-      }
-      stage[10 * nn + jk] = a.FWS[o] == kFluid ? 1.f : 0.f;
+    load(jk, s);
+    if (!s.fluid) {
+      e[5] += a.Residual1[5 * s.o + 0];
+      e[6] += a.Residual1[5 * s.o + 1];
+      continue;
     }
-    __syncthreads();
-    for (int t = tid; t < nn; t += NT) {
-      const int jk = sorder[t], j = jk / n, k = jk - j * n;
-      const int p = pos(i + j + k, i, j);
-#pragma unroll
-      for (int v = 0; v < kScr; ++v) SV(v, p) = stage[v * nn + jk];
-    }
-    __syncthreads();
-  }
-
-  // Sweeps: the cells of plane h (positions Pt[h] .. Pt[h+1]) go to
-  // consecutive threads, so every active warp is full; each cell finds its
-  // neighbours' previous-plane values in the shared slot of their column.
-  auto nb = [&](const float *prv, int c, float *kk, float *dd) {
-#pragma unroll
-    for (int v = 0; v < 10; ++v) kk[v] = prv[v * nn + c];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) dd[v] = prv[(10 + v) * nn + c];
-  };
-  float m[5], r[5], fl = 0.f;     // this plane's cell
-  float m2[5], r2[5], fl2 = 0.f;  // the next plane's, loaded a plane ahead
-  auto fetch = [&](int pp) {
+    const int j = jk / n, k = jk - j * n;
+    const float *const dq = s.dq;
+    const float rf = z.rho0 + s.m[0];
+    const float m1 = s.m[1], m2 = s.m[2], m3 = s.m[3];
+    const float mm = m1 * m1 + m2 * m2 + m3 * m3;
+    const float Pc = z.P0 + (s.m[4] - 0.5f * mm / rf) * 0.4f;
+    double un[5];
+    float mn[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      m[v] = SV(v, pp);
-      r[v] = SV(5 + v, pp);
+      un[v] = s.u[v] + to_double_int(dq[v]);
+      a.U1_[5 * s.o + v] = un[v];
+      mn[v] = to_float_int(v == 0 ? un[v] - z.rho0d : (v == 4 ? un[v] - z.E0d : un[v]));
+      Mc[5 * s.o + v] = mn[v];
     }
-    fl = SV(10, pp);
-  };
-  auto fetch2 = [&](int pp) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      m2[v] = SV(v, pp);
-      r2[v] = SV(5 + v, pp);
+    // Same-level interface copy of this cell (state and mirror), done
+    // here: no block reads another cube's cells during the sweep.
+    if (a.push && (i < 2 || i >= n - 2 || j < 2 || j >= n - 2 || k < 2 || k >= n - 2)) {
+      push_same_level(a.U1_, a.push, n, cube, i + 2, j + 2, k + 2, un);
+      push_same_level(Mc, a.push, n, cube, i + 2, j + 2, k + 2, mn);
     }
-    fl2 = SV(10, pp);
-  };
-  auto take2 = [&]() {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      m[v] = m2[v];
-      r[v] = r2[v];
-    }
-    fl = fl2;
-  };
-
-  // Forward sweep: dq* = (R + sum of lower A+ terms) / dg.
-  if (tid < Pt[1] - Pt[0]) fetch2(Pt[0] + tid);
-  for (int h = 0; h < np; ++h) {
-    float *cur = slots + (size_t)(h & 1) * kSlot * nn;
-    const float *prv = slots + (size_t)((h + 1) & 1) * kSlot * nn;
-    const int cnt = Pt[h + 1] - Pt[h];
-    take2();
-    if (h + 1 < np && tid < Pt[h + 2] - Pt[h + 1]) fetch2(Pt[h + 1] + tid);  // next plane
-    for (int t = tid; t < cnt; t += NT) {
-      const int pp = Pt[h] + t;
-      if (t != tid) fetch(pp);  // further cells of a wide plane
-      const int col = dec[pp], ci = col / n, cj = col - ci * n, k = h - ci - cj;
-      cur[15 * nn + col] = fl;
-      if (fl != 0.f) {
-        float kc[10], kk[10], dd[5];
-        luf_coef(m, rho0, P0, T0, mu_L, idx, dT, cfl, omega, kc);
-        if (ci > 0 && prv[15 * nn + col - n] != 0.f) {
-          nb(prv, col - n, kk, dd);
-          luf_off<0, true>(kk, idx, omega, dd, r);
-        }
-        if (cj > 0 && prv[15 * nn + col - 1] != 0.f) {
-          nb(prv, col - 1, kk, dd);
-          luf_off<1, true>(kk, idx, omega, dd, r);
-        }
-        if (k > 0 && prv[15 * nn + col] != 0.f) {  // the column's previous cell
-          nb(prv, col, kk, dd);
-          luf_off<2, true>(kk, idx, omega, dd, r);
-        }
-        const float idg = 1.0f / kc[9];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) {
-          const float x = r[v] * idg;
-          SV(5 + v, pp) = x;
-          cur[(10 + v) * nn + col] = x;
-        }
-#pragma unroll
-        for (int v = 0; v < 10; ++v) cur[v * nn + col] = kc[v];
-      }
-    }
-    __syncthreads();
+    const float dr = dq[0], e1 = dq[1], e2 = dq[2], e3 = dq[3], dE = dq[4];
+    const float den = 1.0f / (rf * (rf + dr));
+    const float dU = (e1 * rf - m1 * dr) * den;
+    const float dVv = (e2 * rf - m2 * dr) * den;
+    const float dW = (e3 * rf - m3 * dr) * den;
+    const float dKE =
+        0.5f * ((2.f * (m1 * e1 + m2 * e2 + m3 * e3) + e1 * e1 + e2 * e2 + e3 * e3) * rf - mm * dr) * den;
+    const float dP = 0.4f * (dE - dKE);
+    const float dTt = (dP * rf - Pc * dr) * den;
+    e[0] += to_double_int(dP * dP);
+    e[1] += to_double_int(dU * dU);
+    e[2] += to_double_int(dVv * dVv);
+    e[3] += to_double_int(dW * dW);
+    e[4] += to_double_int(dTt * dTt);
   }
-
-  // Backward sweep: dq = dq* - (sum of upper A- terms) / dg.
-  if (tid < Pt[np] - Pt[np - 1]) fetch2(Pt[np - 1] + tid);
-  for (int h = np - 1; h >= 0; --h) {
-    float *cur = slots + (size_t)(h & 1) * kSlot * nn;
-    const float *prv = slots + (size_t)((h + 1) & 1) * kSlot * nn;
-    const int cnt = Pt[h + 1] - Pt[h];
-    take2();
-    if (h > 0 && tid < Pt[h] - Pt[h - 1]) fetch2(Pt[h - 1] + tid);
-    for (int t = tid; t < cnt; t += NT) {
-      const int pp = Pt[h] + t;
-      if (t != tid) fetch(pp);
-      const int col = dec[pp], ci = col / n, cj = col - ci * n, k = h - ci - cj;
-      cur[15 * nn + col] = fl;
-      if (fl != 0.f) {
-        float kc[10], kk[10], dd[5], s[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        luf_coef(m, rho0, P0, T0, mu_L, idx, dT, cfl, omega, kc);
-        if (ci + 1 < n && prv[15 * nn + col + n] != 0.f) {
-          nb(prv, col + n, kk, dd);
-          luf_off<0, false>(kk, idx, omega, dd, s);
-        }
-        if (cj + 1 < n && prv[15 * nn + col + 1] != 0.f) {
-          nb(prv, col + 1, kk, dd);
-          luf_off<1, false>(kk, idx, omega, dd, s);
-        }
-        if (k + 1 < n && prv[15 * nn + col] != 0.f) {
-          nb(prv, col, kk, dd);
-          luf_off<2, false>(kk, idx, omega, dd, s);
-        }
-        const float idg = 1.0f / kc[9];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) {
-          const float x = r[v] - s[v] * idg;
-          SV(5 + v, pp) = x;
-          cur[(10 + v) * nn + col] = x;
-        }
-#pragma unroll
-        for (int v = 0; v < 10; ++v) cur[v * nn + col] = kc[v];
-      }
-    }
-    __syncthreads();
-  }
-
-  // Update, slab by slab: increments gathered in plane order (coalesced)
-  // into shared memory, then Q += dq on fluid cells in memory order (FP64),
-  // change norms of p, u, v, w, T from the FP32 increment (the split RK
-  // path's third-stage formulas) and the force integrands of every cell.
-  double e[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int i = 0; i < n; ++i) {
-    for (int t = tid; t < nn; t += NT) {
-      const int jk = sorder[t], j = jk / n, k = jk - j * n;
-      const int pp = pos(i + j + k, i, j);
-#pragma unroll
-      for (int v = 0; v < 5; ++v) stage[v * nn + jk] = SV(5 + v, pp);
-    }
-    __syncthreads();
-    for (int jk = tid; jk < nn; jk += NT) {
-      const int j = jk / n, k = jk - j * n;
-      const size_t o = cb + ((size_t)(i + 2) * S + (j + 2)) * S + (k + 2);
-      e[5] += a.Residual1[5 * o + 0];
-      e[6] += a.Residual1[5 * o + 1];
-      if (a.FWS[o] != kFluid) continue;
-      float dq[5];
-#pragma unroll
-      for (int v = 0; v < 5; ++v) dq[v] = stage[v * nn + jk];
-      float *mm_ = Mc + 5 * o;
-      const float rf = rho0 + mm_[0];
-      const float m1 = mm_[1], m2 = mm_[2], m3 = mm_[3];
-      const float mm = m1 * m1 + m2 * m2 + m3 * m3;
-      const float Pc = P0 + (mm_[4] - 0.5f * mm / rf) * 0.4f;
-      double un[5];
-      float mn[5];
-#pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        un[v] = a.U1_[5 * o + v] + (double)dq[v];
-        a.U1_[5 * o + v] = un[v];
-        mn[v] = mirror_value_hw(un[v], v, rho0d, E0d);
-        mm_[v] = mn[v];
-      }
-      // Same-level interface copy of this cell (state and mirror), done
-      // here: no block reads another cube's cells during the sweep.
-      if (a.push) {
-        push_same_level(a.U1_, a.push, n, cube, i + 2, j + 2, k + 2, un);
-        push_same_level(Mc, a.push, n, cube, i + 2, j + 2, k + 2, mn);
-      }
-      const float dr = dq[0], e1 = dq[1], e2 = dq[2], e3 = dq[3], dE = dq[4];
-      const float den = 1.0f / (rf * (rf + dr));
-      const float dU = (e1 * rf - m1 * dr) * den;
-      const float dVv = (e2 * rf - m2 * dr) * den;
-      const float dW = (e3 * rf - m3 * dr) * den;
-      const float dKE =
-          0.5f * ((2.f * (m1 * e1 + m2 * e2 + m3 * e3) + e1 * e1 + e2 * e2 + e3 * e3) * rf - mm * dr) * den;
-      const float dP = 0.4f * (dE - dKE);
-      const float dTt = (dP * rf - Pc * dr) * den;
-      e[0] += (double)(dP * dP);
-      e[1] += (double)(dU * dU);
-      e[2] += (double)(dVv * dVv);
-      e[3] += (double)(dW * dW);
-      e[4] += (double)(dTt * dTt);
-    }
-    __syncthreads();
-  }
-
-  double *red = reinterpret_cast<double *>(fbuf);  // [warps][7]
-  const int nw = (NT + 31) / 32;
-#pragma unroll
-  for (int v = 0; v < 7; ++v) {
-    double x = e[v];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-    if ((tid & 31) == 0) red[(tid >> 5) * 7 + v] = x;
-  }
+  const int m = norm_exchange(e, tid & 31);
+  if ((tid & 31) < 8 && m < 7) red[tid >> 5][m] = e[0];
   __syncthreads();
   if (tid < 7) {
     double x = 0;
-    for (int w = 0; w < nw; ++w) x += red[w * 7 + tid];
+    for (int w = 0; w < NT / 32; ++w) x += red[w][tid];
     a.partials[(size_t)blockIdx.x * 7 + tid] = x;
   }
+}
+
+// The most cells of a plane in one CTA of a cluster.
+int lus_plane_cells(int n, int size) {
+  int most = 0;
+  for (int p = 0; p <= 3 * n - 3; ++p)
+    for (int r = 0; r < size; ++r) {
+      int c = 0;
+      for (int i = r; i < n; i += size) {
+        const int lo = std::max(0, p - i - (n - 1)), hi = std::min(n - 1, p - i);
+        if (hi >= lo) c += hi - lo + 1;
+      }
+      most = std::max(most, c);
+    }
+  return most;
 }
 
 }  // namespace
 
 size_t lusgs_split_scratch(int n) { return (size_t)kScr * n * n * n; }
+int lusgs_split_blocks(int n) { return n; }
+int lusgs_split_launches() { return 3; }
 
-// Threads of the split LU-SGS kernel: the widest plane of a cube, in whole
-// warps (every plane then takes one pass).
-static int lusgs_split_threads(int n) {
-  int mx = 0;
-  for (int h = 0; h <= 3 * n - 3; ++h) {
-    int c = 0;
-    for (int i = 0; i < n; ++i)
-      for (int j = 0; j < n; ++j) {
-        const int k = h - i - j;
-        c += k >= 0 && k < n;
-      }
-    mx = c > mx ? c : mx;
-  }
-  return (mx + 31) / 32 * 32;
-}
-
-int lusgs_split_default_threads(int n) { return lusgs_split_threads(n); }
+// Threads for the widest plane of a cube, in whole warps.
+int lusgs_split_default_threads(int n) { return (lus_plane_cells(n, 1) + 31) / 32 * 32; }
 
 cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t s) {
   if (ncubes <= 0) return cudaSuccess;
-  const int n = a.ph.n;
-  if (n * n > 1024) return cudaErrorInvalidValue;  // columns are 16-bit shared indices
-  static std::atomic<int> cache[33];  // widest plane per n (0: not yet computed)
-  int threads = cache[n].load(std::memory_order_relaxed);
-  if (threads == 0) {
-    threads = lusgs_split_threads(n);
-    cache[n].store(threads, std::memory_order_relaxed);
-  }
-  if (a.threads > 0) {
-    if (a.threads % 32 != 0 || a.threads > threads) return cudaErrorInvalidValue;
-    threads = a.threads;  // fewer threads: wide planes take several passes
-  }
-  const int np = 3 * n - 2;
-  size_t smem = (size_t)2 * n * n * kSlot * sizeof(float) +
-                (size_t)(np + 1 + np * n + 2 * n + n * n) * sizeof(int) +
-                (size_t)n * n * n * sizeof(unsigned short);
-  const size_t red = (size_t)(threads / 32) * 7 * sizeof(double);
-  if (smem < red) smem = red;
+  const int n = a.ph.n, nn = n * n;
+  if (nn > 1024) return cudaErrorInvalidValue;
+  if (a.threads > 0 && (a.threads % 32 != 0 || a.threads > lusgs_split_default_threads(n)))
+    return cudaErrorInvalidValue;
   cudaError_t e;
-  if (threads <= 448) {
-    e = cudaFuncSetAttribute(k_lusgs_split<448>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return e;
-    k_lusgs_split<448><<<ncubes, threads, smem, s>>>(a);
-  } else {
-    e = cudaFuncSetAttribute(k_lusgs_split<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return e;
-    k_lusgs_split<1024><<<ncubes, threads, smem, s>>>(a);
-  }
+  const size_t pack = sizeof(float) * kScr * nn;
+  e = cudaFuncSetAttribute(k_lus_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pack);
+  if (e != cudaSuccess) return e;
+  k_lus_pack<<<ncubes * n, kSlabThreads, pack, s>>>(a);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  // One CTA per cube while the widest plane fits it (up to edge 24): the planes
+  // are a chain, and a barrier of the CTA is cheaper than one of a cluster (216
+  // cubes of 24^3, the rest of a sub-iteration as above: 0.63 ms, by clusters
+  // of two 0.69; 8 cubes 0.29 and 0.30).  Wider planes go to clusters of four:
+  // 64 cubes of 32^3 0.62 ms, by one CTA of 768 threads 0.74; 512 the same.
+  const int size = lus_plane_cells(n, 1) <= kSweepThreads ? 1 : 4;
+  int threads = (lus_plane_cells(n, size) + 31) / 32 * 32;
+  if (a.threads > 0) threads = std::min(threads, a.threads);  // wide planes take several passes
+  const size_t smem = lus_smem(n, size);
+  e = cudaFuncSetAttribute(k_lus_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncubes * size);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = size;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if ((e = cudaLaunchKernelEx(&cfg, k_lus_sweep, a)) != cudaSuccess) return e;
+  // Three cells per thread or so: a warp's norm sums take 9 FP64 additions a
+  // turn on top of the 12 of each cell (two and four: the same within 1%).
+  const int ut = std::min(kUpdThreads, (nn / 3 + 31) / 32 * 32);
+  k_lus_update<<<ncubes * n, ut, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -47,6 +47,30 @@ __device__ __forceinline__ double to_double_exact(float f) {
   return __hiloint2double((int)hi, (int)(b << 29));
 }
 
+// The same two conversions with one rare branch and no shortcut for zero: for
+// kernels whose integer pipes idle while the FP64 pipe is the busiest (12 and
+// 8 integer instructions against a slot of 64 cycles).  The rare operands go
+// through calls: inlined, the hardware conversion is predicated instead of
+// branched around and takes its FP64 slot every time.
+static __device__ __noinline__ float to_float_rare(double x) { return __double2float_rn(x); }
+static __device__ __noinline__ double to_double_rare(float f) { return (double)f; }
+__device__ __forceinline__ float to_float_int(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const bool zero = ((hi << 1) | lo) == 0;
+  const int e = (int)((hi >> 20) & 0x7FF) - 896;  // float exponent field
+  if (!zero && (unsigned)(e - 1) >= 254u) return to_float_rare(x);
+  const unsigned m = __funnelshift_l(lo, hi & 0xFFFFFu, 3);  // top 23 fraction bits
+  const unsigned up = ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (m & 1u)) >> 29;
+  const unsigned r = ((unsigned)e << 23) + m + up;  // a carry may raise the exponent
+  return __uint_as_float((hi & 0x80000000u) | (zero ? 0u : r));
+}
+__device__ __forceinline__ double to_double_int(float f) {
+  const unsigned b = __float_as_uint(f), a = b & 0x7FFFFFFFu;
+  if (a - 1u < 0x007FFFFFu || a >= 0x7F800000u) return to_double_rare(f);  // subnormal, inf, nan
+  const unsigned hi = a == 0 ? 0u : (a >> 3) + (896u << 20);
+  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(b << 29));
+}
+
 // (float)(x - r) without FP64 arithmetic when x and r have the same sign and
 // binade: their difference is then exact in FP64 (Sterbenz), so the integer
 // difference of the 53-bit significands, rounded once to nearest even, is
