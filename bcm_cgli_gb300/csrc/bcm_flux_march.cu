@@ -18,18 +18,17 @@
 // pairs (PACK), like the tile kernel's two faces per thread.
 //
 // One RK-stage launch, tile kernel -> march (ms): 2,744 cubes of 16^3 1.726 ->
-// 1.367, 512 of 16^3 0.336 -> 0.276, 512 of 24^3 1.094 -> 0.929, 216 of 32^3
-// 1.096 -> 0.855; edges that 8 does not divide took 4^3 tiles: 512 cubes of
-// 12^3 0.361 -> 0.152, 216 of 20^3 0.696 -> 0.277, 125 of 28^3 1.104 -> 0.439.
+// 1.301, 512 of 16^3 0.336 -> 0.269, 512 of 24^3 1.094 -> 0.887, 216 of 32^3
+// 1.096 -> 0.764; edges that 8 does not divide took 4^3 tiles: 512 cubes of
+// 12^3 0.361 -> 0.152, 216 of 20^3 0.696 -> 0.264, 125 of 28^3 1.104 -> 0.427.
 // 39% fewer instructions than the tiles at n = 16.  What bounds it now (ncu, n =
 // 16): instruction latency with four warps per scheduler (issue slots 42%
-// active; 128 registers and 107 KB a CTA allow no more), the FP64 pipe 48%
-// busy with the cells' FP64 sums and conversions.  Tried and left out: nine
-// warps of 96 registers with a warp for the far faces (spills: 1.69 ms at
-// 2,744 cubes), loading the next cell's FP64 levels ahead into registers
-// (spills: 1.63), conversions on the integer pipes (1.40), whole cubes per
-// CTA instead of equal shares (1.34 there, but 0.294 at 512 cubes), one CTA
-// of 576 threads for n = 24 (1.11).
+// active; 128 registers and 107 KB a CTA allow no more), the FP64 pipe busy
+// with the cells' FP64 sums.  Tried and left out: nine warps of 96 registers
+// with a warp for the far faces (spills: 1.69 ms at 2,744 cubes), loading the
+// next cell's FP64 levels ahead into registers (spills: 1.63), whole cubes per
+// CTA instead of equal shares (1.34 there, but 0.294 at 512 cubes), one CTA of
+// 576 threads for n = 24 (1.11).
 #include <algorithm>
 #include <type_traits>
 
@@ -130,6 +129,7 @@ struct MarchShape {
 template <int NN, bool VISCOUS, bool PACK, bool NORMS>
 __global__ void __launch_bounds__(NN == 32 ? 512 : 256, NN == 32 ? 1 : 2)
     k_flux_march(FluxSplitArgs a, MarchShape sh) {
+  constexpr int CVT = NN == 24 || NN == 32 ? 3 : (NN >= 16 ? 1 : 0);  // measured there
   extern __shared__ __align__(16) float smem[];
   const int n = NN ? NN : a.ph.n, S = n + 4;
   const int tj = NN ? march_rows<NN>() : sh.tj;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(NN == 32 ? 512 : 256, NN == 32 ? 1 : 2)
         SplitLevels lv;
         float src[5];
         split_load(a, go0 + (size_t)(i + q) * SS, lv);
-        split_source(lv, src);
+        split_source<CVT>(lv, src);
 
         const int p = i + q;
         const unsigned cc = q == 0 ? c0 : c1;
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(NN == 32 ? 512 : 256, NN == 32 ? 1 : 2)
             pushI = 5 * ((ptrdiff_t)(d - cube) * ((ptrdiff_t)SS * S) +
                          (ptrdiff_t)(p <= 3 ? n : -n) * SS);
         }
-        split_cell<VISCOUS, NORMS>(a, z, cube, inv, P, qm, acc, lv.x, src, dPdx, dPdz, go, (cc & 1u) != 0, Mw, s5,
+        split_cell<VISCOUS, NORMS, CVT>(a, z, cube, inv, P, qm, acc, lv.x, src, dPdx, dPdz, go, (cc & 1u) != 0, Mw, s5,
                             [&](auto *U, const auto *un) {
                               auto *u = U + 5 * go;
                               if (pushI) {

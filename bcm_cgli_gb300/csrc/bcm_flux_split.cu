@@ -412,8 +412,9 @@ __global__ void __launch_bounds__(split_threads<T>(), split_ctas_per_sm<T>())
   SplitLevels lv;
   float src[5];
   split_load(a, go, lv);
-  split_source(lv, src);
-  split_cell<VISCOUS, true>(a, z, cube, inv, P, BX(mi, mj, mk), acc, lv.x, src, dPdx, dPdz, go,
+  constexpr int CVT = T == 4 ? 3 : 0;
+  split_source<CVT>(lv, src);
+  split_cell<VISCOUS, true, CVT>(a, z, cube, inv, P, BX(mi, mj, mk), acc, lv.x, src, dPdx, dPdz, go,
                       FL(mi, mj, mk) == kFluid, Mw, s5, [&](auto *U, const auto *un) {
                         if (a.push) push_same_level(U, a.push, n, cube, bi + mi, bj + mj, bk + mk, un);
                       });

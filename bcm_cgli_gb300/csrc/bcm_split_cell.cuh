@@ -307,10 +307,25 @@ __device__ __forceinline__ PrimF prim_split(const SplitConst &z, const float *q)
 
 // A cell's FP64 state, the previous level and the level difference, as
 // loaded; split_source forms the BDF2 source (times -2 dT) from the FP64
-// time-level differences, then FP32.  The FP64 <-> FP32 conversions of the cell's stage
-// are the hardware's (IEEE round to nearest): here the FP64 pipe has room and
-// the integer pipes do not (measured: the integer-pipe routines of k_mirror
-// made the launch 7-8% longer).
+// time-level differences, then FP32.
+//
+// CVT: which conversions of a cell's stage go to the integer pipes (bit 0: FP64
+// to FP32, bit 1: FP32 to FP64; the same bits as the hardware's, which take a
+// slot of the FP64 pipe each).  Per stage of a 30-stage step, ns a cell, CVT 0,
+// 1, 3: march n = 16 (2,744 cubes) 0.152 0.142 0.142, n = 20 0.208 0.199 0.203,
+// n = 24 0.162 0.154 0.153, n = 28 0.201 0.192 0.198, n = 32 0.152 0.136 0.133;
+// tiles of 4^3 (4,096) 0.73 0.66 0.66.  Left to the hardware where the longer chain
+// of instructions costs more than the slot: march n = 8 0.376 0.381 0.385, n =
+// 12 (1,728) 0.204 0.220 0.224, edges without a kernel of their own (36) 0.202
+// 0.205 0.210, tiles of 8^3 (4,096) 0.227 0.233 0.233.
+template <int CVT>
+__device__ __forceinline__ float split_f(double x) {
+  return (CVT & 1) ? to_float_int(x) : __double2float_rn(x);
+}
+template <int CVT>
+__device__ __forceinline__ double split_d(float x) {
+  return (CVT & 2) ? to_double_int(x) : (double)x;
+}
 struct SplitLevels {
   double x[5], y[5];
   float d2[5];
@@ -325,10 +340,11 @@ __device__ __forceinline__ void split_load(const FluxSplitArgs &a, size_t go, Sp
 }
 // (fused operations written out where the operands come from different
 // places in the kernels, so that both round alike)
+template <int CVT>
 __device__ __forceinline__ void split_source(const SplitLevels &l, float *src) {
 #pragma unroll
   for (int v = 0; v < 5; ++v)
-    src[v] = __fmaf_rn(3.0f, __double2float_rn(l.x[v] - l.y[v]), -l.d2[v]);
+    src[v] = __fmaf_rn(3.0f, split_f<CVT>(l.x[v] - l.y[v]), -l.d2[v]);
 }
 
 // The rest of a cell's stage, given its inviscid balance acc, state xq and
@@ -337,7 +353,7 @@ __device__ __forceinline__ void split_source(const SplitLevels &l, float *src) {
 // cell's deltas, go its offset; push(array, values) copies a new value into
 // the same-level neighbours' ghost layers.  NORMS: stage 3 (the sums take 14
 // registers).
-template <bool VISCOUS, bool NORMS, typename Prims, typename Push>
+template <bool VISCOUS, bool NORMS, int CVT, typename Prims, typename Push>
 __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitConst &z, int cube,
                                            float inv, Prims P, const float *qm, const float *acc,
                                            const double *xq, const float *src,
@@ -427,7 +443,7 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
     for (int r = 0; r < 5; ++r) {
       dq[r] = w * dTau * (d[r][0] * Rk[0] + d[r][1] * Rk[1] + d[r][2] * Rk[2] +
                           d[r][3] * Rk[3] + d[r][4] * Rk[4]);
-      un[r] = xq[r] + (double)dq[r];
+      un[r] = xq[r] + split_d<CVT>(dq[r]);
       u[r] = un[r];
     }
     // Same-level interface copy of this cell, done here.  No CTA reads the
@@ -437,8 +453,8 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
     if (NORMS && a.RK == 3) {
       // Change norms of p, u, v, w, T from the increment, in FP32; summed
       // in FP64 (BCM_Flux...cpp:2530-2566).
-      const float rf = rho, m1 = __double2float_rn(xq[1]), m2 = __double2float_rn(xq[2]),
-                  m3 = __double2float_rn(xq[3]);
+      // (the momentum's deltas are the rounded values of xq)
+      const float rf = rho, m1 = qm[1], m2 = qm[2], m3 = qm[3];
       const float dr = dq[0], e1 = dq[1], e2 = dq[2], e3 = dq[3], dE = dq[4];
       const float den = 1.0f / (rf * (rf + dr));
       const float dU = (e1 * rf - m1 * dr) * den;
@@ -449,11 +465,11 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
           0.5f * ((2.f * (m1 * e1 + m2 * e2 + m3 * e3) + e1 * e1 + e2 * e2 + e3 * e3) * rf - mm * dr) * den;
       const float dP = Km1 * (dE - dKE);
       const float dTt = (dP * rf - Pc * dr) * den;
-      s5[0] += (double)(dP * dP);
-      s5[1] += (double)(dU * dU);
-      s5[2] += (double)(dVv * dVv);
-      s5[3] += (double)(dW * dW);
-      s5[4] += (double)(dTt * dTt);
+      s5[0] += split_d<CVT>(dP * dP);
+      s5[1] += split_d<CVT>(dU * dU);
+      s5[2] += split_d<CVT>(dVv * dVv);
+      s5[3] += split_d<CVT>(dW * dW);
+      s5[4] += split_d<CVT>(dTt * dTt);
     }
   } else {
     // Force integrands on non-fluid cells (:2395-2398); their sum over the
@@ -474,15 +490,11 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
     // staged value where the cell did not change), and into the same-level
     // neighbour's ghost layers: every cell of those layers pushes, since the
     // next buffer's ghost layers hold values two stages old.
-    // The conversion is the hardware's (IEEE round to nearest, the same bits
-    // as the integer-pipe routine of the other writers): this kernel's FP64
-    // pipe has room, its integer pipes do not (measured: the integer routine
-    // made the launch 17% longer, this form 9%).
     float m5[5];
     if (fluid) {
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        m5[v] = __double2float_rn(v == 0 ? un[v] - z.rho0d : (v == 4 ? un[v] - z.E0d : un[v]));
+        m5[v] = split_f<CVT>(v == 0 ? un[v] - z.rho0d : (v == 4 ? un[v] - z.E0d : un[v]));
     } else {
   #pragma unroll
       for (int v = 0; v < 5; ++v) m5[v] = qm[v];
