@@ -88,20 +88,6 @@ __global__ void k_copy_fluid(int n, int ncubes, const double *__restrict__ U1_,
   }
 }
 
-__global__ void k_emax(double *er, double *emax, const int *active) {
-  // main.cpp:1249-1259: E_k = max(E_k, er_k); er_k /= E_k.  One block per
-  // case: er[8q..], emax[6q..]; converged cases keep theirs.
-  if (active && !active[blockIdx.x]) return;
-  er += 8 * (size_t)blockIdx.x;
-  emax += 6 * (size_t)blockIdx.x;
-  const int v = threadIdx.x + 1;
-  if (v <= 5) {
-    double E = emax[v] > er[v] ? emax[v] : er[v];
-    emax[v] = E;
-    er[v] = er[v] / E;
-  }
-}
-
 // Convergence-driven sub-iterations (main.cpp:1249-1271): before a step
 // every case is active with zero sub-iterations; after each sub-iteration
 // (and its E normalisation) a case whose normalised change norms er[1..5]
@@ -242,6 +228,7 @@ struct bcmg_case {
       m.buf[0] = M;
       m.buf[1] = M2;
       m.parity = mpar;
+      m.phase = phase;
       m.rho0 = ph.rho0;
       m.E0 = ph.P0 / (BCMG_K - 1);
     }
@@ -252,9 +239,15 @@ struct bcmg_case {
   uint16_t *codes = nullptr;             // split precision: cell codes of FWS
   int *FWS = nullptr;
   double *cube_size = nullptr;
-  int *task_cube = nullptr;  // destination cube of each face task
-  FaceTask *tasks = nullptr;
-  int ntasks = 0;
+  // Face tasks by destination cube: those of cube c are tasks[off[c] ..
+  // off[c+1]).
+  struct FaceList {
+    int *off = nullptr;  // device [ncube+1]
+    FaceTask *tasks = nullptr;
+    int ntasks = 0;
+    void free() { dfree(off); dfree(tasks); }
+  };
+  FaceList faces;  // all of them
   // The face tasks a stage's first interface call must repeat after the
   // previous stage's last one (main.cpp:1161-1204 runs the interface before
   // and after every update): level jumps, faces the boundary fill writes and
@@ -262,9 +255,11 @@ struct bcmg_case {
   // other copies would write the values already there: between the two
   // calls only the boundary fill (its own ghost faces) and the IBM ghost
   // fill (its listed cells) write the state.
-  int *task_cube_p = nullptr;
-  FaceTask *tasks_p = nullptr;
-  int ntasks_p = 0;
+  FaceList faces_p;
+  // The same where no IBM ghost fill and no exchange lies between the two
+  // calls: the boundary fill then leaves out the faces that same-level tasks
+  // fill (LayerArgs::cover), so only the level jumps remain.
+  FaceList faces_j;
   // Split-precision RK stages and LU-SGS sweeps make the same-level face
   // copies of the cells they update inside the updating kernel (push table,
   // see FluxSplitArgs::push); their closing interface call then runs only
@@ -273,17 +268,21 @@ struct bcmg_case {
   int *push = nullptr;
   bool push_on = true;  // bcmg_case_set_face_copies
   const int *push_table() const { return push_on ? push : nullptr; }
-  int *task_cube_q = nullptr;
-  FaceTask *tasks_q = nullptr;
-  int ntasks_q = 0;
+  FaceList faces_q;
   // the closing call of split RK stages 1 and 2: the level jumps and edge
   // fills read before the next stage's opening call rewrites them
-  int *task_cube_r = nullptr, *edge_r = nullptr;
-  FaceTask *tasks_r = nullptr;
-  int ntasks_r = 0, nedge_r = 0;
+  FaceList faces_r;
   bool closing_reduced = false;
-  int *bc_cubes = nullptr, *bc_masks = nullptr;
+  // per cube: boundary faces (bits 0..5), kLayerEdge where the reduced
+  // closing call fills edges, faces with same-level tasks (kLayerCover); the cubes with boundary faces and their flags
+  int *flags = nullptr, *bc_cubes = nullptr, *bc_flags = nullptr;
   int nbc = 0;
+  // A stage's closing interface call waits here for the next stage's opening
+  // one (case_prologue runs both in one launch) or for case_settle.
+  LayerArgs closing;
+  bool has_closing = false;
+  int phase = 0;            // Mirror::phase of the next launch
+  bool fold_emax = false;   // the norms' launch also does the E normalisation
   // The IBM ghost fill on a side stream beside the boundary fill: allowed
   // when no cube holds both an IBM entry's cells (ghost or stencil) and a
   // boundary face, so neither reads or writes a cell of the other; the
@@ -387,10 +386,9 @@ struct bcmg_case {
     ev.clear();
     dfree(U1_); dfree(U1); dfree(U1q); dfree(U1p1); dfree(U1p2); dfree(Rku1); dfree(Residual1);
     dfree(M); dfree(M2); dfree(mpar); dfree(D2); dfree(inv_dx); dfree(codes);
-    dfree(FWS); dfree(cube_size); dfree(task_cube); dfree(tasks); dfree(task_cube_p);
-    dfree(tasks_p); dfree(push); dfree(task_cube_q); dfree(tasks_q); dfree(bc_cubes);
-    dfree(task_cube_r); dfree(tasks_r); dfree(edge_r);
-    dfree(bc_masks); dfree(partials); dfree(er); dfree(emax);
+    dfree(FWS); dfree(cube_size); dfree(push); dfree(flags); dfree(bc_cubes);
+    faces.free(); faces_p.free(); faces_j.free(); faces_q.free(); faces_r.free();
+    dfree(bc_flags); dfree(partials); dfree(er); dfree(emax);
     dfree(cases); dfree(cube_case); dfree(rk_blk); dfree(case_blk_rk); dfree(case_blk_flux);
     dfree(case_blk_cube);
     dfree(nsum);
@@ -487,60 +485,98 @@ int case_flux(bcmg_case *c, int RK) {
   }
   if (c->profile) CK(cudaEventRecord(e1, c->stream));
   ++c->launches;
-  if (c->precision == BCMG_PRECISION_SPLIT && RK >= 1) {
-    // the flux kernel wrote the stage's mirror into the other buffer
+  // the flux kernel wrote the stage's mirror into the other buffer
+  if (c->precision == BCMG_PRECISION_SPLIT && RK >= 1) c->phase ^= 1;
+  return BCMG_OK;
+}
+
+// Which face tasks an interface call runs.
+enum IfaceList { kIfaceFull, kIfacePrologue, kIfaceJumps, kIfaceClosing, kIfaceClosingReduced };
+
+int case_layers(bcmg_case *c, LayerArgs &a, int ncubes) {
+  a.n = c->ph.n;
+  a.U1_ = c->U1_;
+  a.bt = c->bt();
+  a.mir = c->mir();
+  a.Uin = c->ph.Uin;
+  CK(launch_layers(a, ncubes, c->stream));
+  if (ncubes > 0) ++c->launches;
+  return BCMG_OK;
+}
+
+void interface_round(const bcmg_case *c, LayerArgs &a, int round, IfaceList list) {
+  const bcmg_case::FaceList &f = list == kIfacePrologue ? c->faces_p
+                                 : list == kIfaceJumps ? c->faces_j
+                                 : list == kIfaceClosing ? c->faces_q
+                                 : list == kIfaceClosingReduced ? c->faces_r : c->faces;
+  a.off[round] = f.ntasks > 0 ? f.off : nullptr;
+  a.tasks[round] = f.tasks;
+  a.edges[round] = list == kIfaceClosingReduced ? 2 : 1;
+  a.flags = c->flags;
+}
+
+int case_exchange(bcmg_case *c) {  // sharded: the proxies' face bands
+  if (c->xchg && c->xchg(c->xchg_user, BCMG_XCHG_HALO, c->stream) != 0) {
+    set_err("exchange hook failed (halo)");
+    return BCMG_ERR_CUDA;
+  }
+  return BCMG_OK;
+}
+
+// The closing interface call of a stage or sweep: kept for the next opening
+// one (sharded contexts run it at once, after the exchange).
+int case_closing(bcmg_case *c, IfaceList list = kIfaceFull) {
+  c->closing = LayerArgs();
+  interface_round(c, c->closing, 0, list);
+  c->has_closing = true;
+  if (!c->xchg) return BCMG_OK;
+  int r;
+  if ((r = case_exchange(c))) return r;
+  c->has_closing = false;
+  return case_layers(c, c->closing, c->ncube - 1);
+}
+
+// The closing call that still waits, and the mirror flag brought up to date:
+// at the end of a step or single stage, and before a convergence check.
+int case_settle(bcmg_case *c) {
+  int r;
+  if (c->has_closing) {
+    c->has_closing = false;
+    if ((r = case_layers(c, c->closing, c->ncube - 1))) return r;
+  }
+  if (c->phase) {
+    c->phase = 0;
     CK(launch_mirror_flip(c->mpar, c->stream));
     ++c->launches;
   }
   return BCMG_OK;
 }
 
-// Which face tasks an interface call runs.
-enum IfaceList { kIfaceFull, kIfacePrologue, kIfaceClosing, kIfaceClosingReduced };
-
-int case_interface(bcmg_case *c, IfaceList list = kIfaceFull) {
-  if (c->xchg) {  // sharded: the proxies' face bands first
-    if (c->xchg(c->xchg_user, BCMG_XCHG_HALO, c->stream) != 0) {
-      set_err("exchange hook failed (halo)");
-      return BCMG_ERR_CUDA;
-    }
-  }
-  InterfaceArgs ia;
-  ia.n = c->ph.n;
-  ia.ntasks = c->ntasks;
-  ia.task_cube = c->task_cube;
-  ia.tasks = c->tasks;
-  if (list == kIfacePrologue) {
-    ia.ntasks = c->ntasks_p;
-    ia.task_cube = c->task_cube_p;
-    ia.tasks = c->tasks_p;
-  } else if (list == kIfaceClosing) {
-    ia.ntasks = c->ntasks_q;
-    ia.task_cube = c->task_cube_q;
-    ia.tasks = c->tasks_q;
-  } else if (list == kIfaceClosingReduced) {
-    ia.ntasks = c->ntasks_r;
-    ia.task_cube = c->task_cube_r;
-    ia.tasks = c->tasks_r;
-    ia.edge_list = true;
-    ia.edge_cubes = c->edge_r;
-    ia.nedge = c->nedge_r;
-  }
-  ia.U1_ = c->U1_;
-  ia.bt = c->bt();
-  ia.mir = c->mir();
-  CK(launch_interface(ia, c->ncube, c->stream));
-  c->launches += (ia.ntasks > 0 ? 1 : 0) + (ia.edge_list && ia.nedge == 0 ? 0 : 1);
-  return BCMG_OK;
-}
-
 // Boundary conditions, IBM ghost cells and interface ahead of each update
 // (main.cpp:1161-1204).  full == false: the stage follows another stage's
 // closing interface call, so only the face copies that can change run.
+// Without ghost cells and exchange all of it, and the closing call before
+// it, is one launch.
 int case_prologue(bcmg_case *c, bool full = true) {
   int r;
+  const IfaceList open = full ? kIfaceFull : kIfacePrologue;
+  LayerArgs a;
+  if (c->has_closing) a = c->closing;
+  const bool ghosts = c->ibm.nbc > 0 || c->ibm_side.nbc > 0;
+  if (!ghosts && !c->xchg) {
+    c->has_closing = false;
+    a.axes = 7;
+    a.cover = true;
+    interface_round(c, a, 1, full ? kIfaceFull : kIfaceJumps);
+    return case_layers(c, a, c->ncube - 1);
+  }
   const bool beside = c->ghost_beside_bc && c->ghost_side_on;
   if (beside) {  // fork: the side table's ghost levels on the side stream
+    if (c->has_closing) {
+      c->has_closing = false;
+      if ((r = case_layers(c, a, c->ncube - 1))) return r;
+      a = LayerArgs();
+    }
     CK(cudaEventRecord(c->ev_fork, c->stream));
     CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
     if ((r = ibm_run(c->ibm_side, c->ph.n, c->ph.rho0, c->ph.P0, c->U1_, c->side, &c->launches,
@@ -548,18 +584,17 @@ int case_prologue(bcmg_case *c, bool full = true) {
       return r;
     CK(cudaEventRecord(c->ev_join, c->side));
   }
-  if (c->nbc > 0) {
-    BcArgs b;
-    b.n = c->ph.n;
-    b.Uin = c->ph.Uin;
-    b.cubes = c->bc_cubes;
-    b.masks = c->bc_masks;
-    b.axes = 7;
-    b.U1_ = c->U1_;
-    b.bt = c->bt();
-    b.mir = c->mir();
-    CK(launch_bc(b, c->nbc, c->stream));
-    ++c->launches;
+  if (c->has_closing || c->nbc > 0) {
+    a.axes = 7;
+    if (c->has_closing) {
+      c->has_closing = false;
+      r = case_layers(c, a, c->ncube - 1);
+    } else {
+      a.cubes = c->bc_cubes;
+      a.flags = c->bc_flags;
+      r = case_layers(c, a, c->nbc);
+    }
+    if (r) return r;
   }
   if (beside) {  // join; the other cases' entries after the boundary fill
     CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
@@ -570,7 +605,10 @@ int case_prologue(bcmg_case *c, bool full = true) {
   if ((r = ibm_run(c->ibm, c->ph.n, c->ph.rho0, c->ph.P0, c->U1_, c->stream, &c->launches,
                    c->bt(), c->mir())))
     return r;
-  return case_interface(c, full ? kIfaceFull : kIfacePrologue);
+  if ((r = case_exchange(c))) return r;
+  LayerArgs o;
+  interface_round(c, o, 1, open);
+  return case_layers(c, o, c->ncube - 1);
 }
 
 // One LU-SGS sub-iteration: prologue, residual, sweeps with the update and
@@ -603,7 +641,8 @@ LusgsSplitArgs lusgs_split_args(bcmg_case *c) {
 // sums to the exchange hook, which adds them over the ranks.
 int case_norms(bcmg_case *c, int nb) {
   if (!c->xchg) {
-    CK(launch_norms(c->ph, c->partials, nb, c->er, c->stream, c->bt().active));
+    CK(launch_norms(c->ph, c->partials, nb, c->er, c->stream, c->bt().active,
+                    c->fold_emax ? c->emax : nullptr));
     ++c->launches;
     return BCMG_OK;
   }
@@ -612,7 +651,8 @@ int case_norms(bcmg_case *c, int nb) {
     set_err("exchange hook failed (norms)");
     return BCMG_ERR_CUDA;
   }
-  CK(launch_norm_final(c->ph, c->nsum, c->er, c->stream, c->bt().active));
+  CK(launch_norm_final(c->ph, c->nsum, c->er, c->stream, c->bt().active,
+                       c->fold_emax ? c->emax : nullptr));
   c->launches += 2;
   return BCMG_OK;
 }
@@ -650,12 +690,12 @@ int case_lusgs(bcmg_case *c, bool full = true) {
   ++c->launches;
   if (c->batched)
     CK(launch_norms_batch(c->ph.n, c->cases, c->case_blk_cube, c->ncase, c->partials, c->er,
-                          c->stream, c->bt().active));
+                          c->stream, c->bt().active, c->fold_emax ? c->emax : nullptr));
   else if ((r = case_norms(c, c->nreal * case_lu_blocks(c))))
     return r;
   if (c->batched) ++c->launches;
   // the split sweep made the same-level copies of the updated cells
-  return case_interface(c, c->precision == BCMG_PRECISION_SPLIT && c->push_table()
+  return case_closing(c, c->precision == BCMG_PRECISION_SPLIT && c->push_table()
                                ? kIfaceClosing
                                : kIfaceFull);
 }
@@ -674,15 +714,15 @@ int case_stage(bcmg_case *c, int RK, bool full = true, bool reduced = false) {
     if (RK == 3) {
       if (c->batched) {
         CK(launch_norms_batch(c->ph.n, c->cases, c->case_blk_flux, c->ncase, c->partials, c->er,
-                              c->stream, c->bt().active));
+                          c->stream, c->bt().active, c->fold_emax ? c->emax : nullptr));
         ++c->launches;
       } else if ((r = case_norms(c, nb))) {
         return r;
       }
     }
     // the flux kernel made the same-level copies of the updated cells
-    if (!c->push_table()) return case_interface(c, kIfaceFull);
-    return case_interface(c, reduced && c->closing_reduced && !c->xchg ? kIfaceClosingReduced
+    if (!c->push_table()) return case_closing(c);
+    return case_closing(c, reduced && c->closing_reduced && !c->xchg ? kIfaceClosingReduced
                                                                       : kIfaceClosing);
   }
   RkArgs k;
@@ -707,30 +747,29 @@ int case_stage(bcmg_case *c, int RK, bool full = true, bool reduced = false) {
   if (RK == 3) {
     if (c->batched) {
       CK(launch_norms_batch(c->ph.n, c->cases, c->case_blk_rk, c->ncase, c->partials, c->er,
-                            c->stream, c->bt().active));
+                          c->stream, c->bt().active, c->fold_emax ? c->emax : nullptr));
       ++c->launches;
     } else {
       int r = case_norms(c, nb);
       if (r) return r;
     }
   }
-  return case_interface(c);
+  return case_closing(c);
 }
 
 // One sub-iteration (three RK stages or one LU-SGS update) and the E
 // normalisation of its norms (main.cpp:1249-1259).
+// Ends with the closing interface call waiting (case_settle).
 int case_subiter(bcmg_case *c, bool full = true) {
-  int r;
+  int r = BCMG_OK;
+  c->fold_emax = true;
   if (c->method == BCMG_METHOD_LUSGS) {
-    if ((r = case_lusgs(c, full))) return r;
+    r = case_lusgs(c, full);
   } else {
-    for (int RK = 1; RK <= 3; ++RK)
-      if ((r = case_stage(c, RK, full && RK == 1, RK < 3))) return r;
+    for (int RK = 1; RK <= 3 && !r; ++RK) r = case_stage(c, RK, full && RK == 1, RK < 3);
   }
-  k_emax<<<c->ncase, 32, 0, c->stream>>>(c->er, c->emax, c->bt().active);
-  CK(cudaGetLastError());
-  ++c->launches;
-  return BCMG_OK;
+  c->fold_emax = false;
+  return r;
 }
 
 // Time-level shift at the end of a dual-time step (main.cpp:1292-1315).
@@ -768,9 +807,12 @@ int case_mirror_all(bcmg_case *c) {
 
 int case_step(bcmg_case *c, int subiters) {
   int r;
+  c->has_closing = false;
+  c->phase = 0;
   if ((r = case_mirror_all(c))) return r;
   for (int it = 0; it < subiters; ++it)  // the step's first stage runs every face copy
     if ((r = case_subiter(c, it == 0))) return r;
+  if ((r = case_settle(c))) return r;
   return case_shift(c);
 }
 
@@ -819,7 +861,10 @@ int build_conv_graph(bcmg_case *c, int max_subiters, double tol) {
   cudaGraph_t body = p.conditional.phGraph_out[0];
   CK(cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, mode));
   const long long l0 = c->launches;
+  c->has_closing = false;
+  c->phase = 0;
   int r = case_subiter(c);
+  if (!r) r = case_settle(c);
   if (!r) {
     k_conv_check<<<1, 32, 0, c->stream>>>(c->er, c->active, c->iters, c->ncase, tol,
                                           max_subiters, c->cont, h, 1);
@@ -1109,7 +1154,6 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
     tasks.swap(kt);
     task_cube.swap(kc);
   }
-  c->ntasks = (int)tasks.size();
   const int *lists[6] = {d->xl, d->xu, d->yl, d->yu, d->zl, d->zu};
   const int counts[6] = {d->nxl, d->nxu, d->nyl, d->nyu, d->nzl, d->nzu};
   for (int l = 0; l < 6; ++l)
@@ -1134,10 +1178,9 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
             ck(dalloc(&c->U1p2, nd), "alloc") && ck(dalloc(&c->Rku1, nd), "alloc") &&
             ck(dalloc(&c->Residual1, nd), "alloc") && ck(dalloc(&c->FWS, c->ncell), "alloc") &&
             ck(dalloc(&c->cube_size, (size_t)d->ncube), "alloc") &&
-            ck(dalloc(&c->task_cube, tasks.size()), "alloc") &&
-            ck(dalloc(&c->tasks, tasks.size()), "alloc") &&
+            ck(dalloc(&c->flags, (size_t)d->ncube), "alloc") &&
             ck(dalloc(&c->bc_cubes, bcc.size()), "alloc") &&
-            ck(dalloc(&c->bc_masks, bcm.size()), "alloc") &&
+            ck(dalloc(&c->bc_flags, bcm.size()), "alloc") &&
             ck(dalloc(&c->er, 8 * (size_t)c->ncase), "alloc") &&
             ck(dalloc(&c->nsum, 7), "alloc") &&
             ck(dalloc(&c->emax, 6 * (size_t)c->ncase), "alloc");
@@ -1226,14 +1269,9 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
           "copy") &&
        ck(cudaMemcpyAsync(c->cube_size, d->cube_size, sizeof(double) * d->ncube,
                           cudaMemcpyHostToDevice, s), "copy") &&
-       (tasks.empty() || ck(cudaMemcpyAsync(c->task_cube, task_cube.data(),
-                                            sizeof(int) * task_cube.size(),
-                                            cudaMemcpyHostToDevice, s), "copy")) &&
-       (tasks.empty() || ck(cudaMemcpyAsync(c->tasks, tasks.data(), sizeof(FaceTask) * tasks.size(),
-                                            cudaMemcpyHostToDevice, s), "copy")) &&
        (bcc.empty() || (ck(cudaMemcpyAsync(c->bc_cubes, bcc.data(), sizeof(int) * bcc.size(),
                                            cudaMemcpyHostToDevice, s), "copy") &&
-                        ck(cudaMemcpyAsync(c->bc_masks, bcm.data(), sizeof(int) * bcm.size(),
+                        ck(cudaMemcpyAsync(c->bc_flags, bcm.data(), sizeof(int) * bcm.size(),
                                            cudaMemcpyHostToDevice, s), "copy"))) &&
        (!c->codes || ck(launch_cell_codes(c->FWS, c->codes, d->n, d->ncube, s), "cell codes")) &&
        ck(cudaStreamSynchronize(s), "sync");
@@ -1317,6 +1355,30 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
       c->ghost_beside_bc = true;
     }
   }
+  // A list of the tasks with keep[t] set (they are in order of their cube).
+  auto face_list = [&](const std::vector<char> &keep, bcmg_case::FaceList &l) {
+    std::vector<FaceTask> kt;
+    std::vector<int> o((size_t)d->ncube + 1, 0);
+    for (size_t t = 0; t < tasks.size(); ++t)
+      if (keep[t]) {
+        kt.push_back(tasks[t]);
+        ++o[(size_t)task_cube[t] + 1];
+      }
+    for (int cb = 0; cb < d->ncube; ++cb) o[(size_t)cb + 1] += o[cb];
+    l.ntasks = (int)kt.size();
+    return kt.empty() ||
+           (ck(dalloc(&l.tasks, kt.size()), "alloc") && ck(dalloc(&l.off, o.size()), "alloc") &&
+            ck(cudaMemcpy(l.tasks, kt.data(), sizeof(FaceTask) * kt.size(),
+                          cudaMemcpyHostToDevice), "copy") &&
+            ck(cudaMemcpy(l.off, o.data(), sizeof(int) * o.size(), cudaMemcpyHostToDevice),
+               "copy"));
+  };
+  if (!face_list(std::vector<char>(tasks.size(), 1), c->faces)) return fail(BCMG_ERR_CUDA);
+  std::vector<int> flags((size_t)d->ncube, 0);
+  for (size_t q = 0; q < bcc.size(); ++q) flags[bcc[q]] |= bcm[q];
+  for (size_t t = 0; t < tasks.size(); ++t)
+    if (tasks[t].kind == 0)
+      flags[task_cube[t]] |= 1 << (kLayerCover + 2 * tasks[t].axis + tasks[t].side);
   // Reduced face-task list of the prologue interface calls.
   {
     std::vector<char> keep;
@@ -1325,48 +1387,22 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
     // a proxy's bands are refilled by the exchange before every call
     for (size_t t = 0; t < tasks.size(); ++t)
       if (tasks[t].src > c->nreal) keep[t] = 1;
-    std::vector<FaceTask> tp;
-    std::vector<int> cp;
-    for (size_t t = 0; t < tasks.size(); ++t)
-      if (keep[t]) {
-        tp.push_back(tasks[t]);
-        cp.push_back(task_cube[t]);
-      }
-    c->ntasks_p = (int)tp.size();
-    if (!tp.empty() &&
-        !(ck(dalloc(&c->tasks_p, tp.size()), "alloc") &&
-          ck(dalloc(&c->task_cube_p, cp.size()), "alloc") &&
-          ck(cudaMemcpy(c->tasks_p, tp.data(), sizeof(FaceTask) * tp.size(),
-                        cudaMemcpyHostToDevice), "copy") &&
-          ck(cudaMemcpy(c->task_cube_p, cp.data(), sizeof(int) * cp.size(),
-                        cudaMemcpyHostToDevice), "copy")))
-      return fail(BCMG_ERR_CUDA);
+    if (!face_list(keep, c->faces_p)) return fail(BCMG_ERR_CUDA);
+    for (size_t t = 0; t < tasks.size(); ++t) keep[t] = tasks[t].kind != 0;
+    if (!face_list(keep, c->faces_j)) return fail(BCMG_ERR_CUDA);
   }
   // Push table of the split-precision flux kernel and the closing list that
   // goes with it (level-jump tasks only).
   if (d->precision == BCMG_PRECISION_SPLIT) {
     std::vector<int> push;
-    const bool ok_push = build_push_table(d->ncube, tasks, task_cube, push);
-    std::vector<FaceTask> tq;
-    std::vector<int> cq;
-    for (size_t t = 0; t < tasks.size(); ++t)
-      if (tasks[t].kind != 0 || tasks[t].src > c->nreal) {  // proxies push nothing
-        tq.push_back(tasks[t]);
-        cq.push_back(task_cube[t]);
-      }
-    if (ok_push) {
-      c->ntasks_q = (int)tq.size();
+    if (build_push_table(d->ncube, tasks, task_cube, push)) {
+      std::vector<char> keep(tasks.size());
+      for (size_t t = 0; t < tasks.size(); ++t)  // proxies push nothing
+        keep[t] = tasks[t].kind != 0 || tasks[t].src > c->nreal;
       if (!(ck(dalloc(&c->push, push.size()), "alloc") &&
             ck(cudaMemcpy(c->push, push.data(), sizeof(int) * push.size(),
-                          cudaMemcpyHostToDevice), "copy")))
-        return fail(BCMG_ERR_CUDA);
-      if (!tq.empty() &&
-          !(ck(dalloc(&c->tasks_q, tq.size()), "alloc") &&
-            ck(dalloc(&c->task_cube_q, cq.size()), "alloc") &&
-            ck(cudaMemcpy(c->tasks_q, tq.data(), sizeof(FaceTask) * tq.size(),
                           cudaMemcpyHostToDevice), "copy") &&
-            ck(cudaMemcpy(c->task_cube_q, cq.data(), sizeof(int) * cq.size(),
-                          cudaMemcpyHostToDevice), "copy")))
+            face_list(keep, c->faces_q)))
         return fail(BCMG_ERR_CUDA);
       // the closing call of RK stages 1 and 2 (not for sharded contexts,
       // whose proxies are refilled by each call's exchange)
@@ -1374,33 +1410,16 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
         std::vector<char> keep_r, edge;
         closing_plan(d->n, d->ncube, tasks, task_cube, bcc, bcm, d->ip_minus, nm, d->ip_plus,
                      np, keep_r, edge);
-        std::vector<FaceTask> tr;
-        std::vector<int> cr, er_;
-        for (size_t t = 0; t < tasks.size(); ++t)
-          if (keep_r[t]) {
-            tr.push_back(tasks[t]);
-            cr.push_back(task_cube[t]);
-          }
+        if (!face_list(keep_r, c->faces_r)) return fail(BCMG_ERR_CUDA);
         for (int cb = 1; cb < d->ncube; ++cb)
-          if (edge[cb]) er_.push_back(cb);
-        c->ntasks_r = (int)tr.size();
-        c->nedge_r = (int)er_.size();
-        if ((!tr.empty() &&
-             !(ck(dalloc(&c->tasks_r, tr.size()), "alloc") &&
-               ck(dalloc(&c->task_cube_r, cr.size()), "alloc") &&
-               ck(cudaMemcpy(c->tasks_r, tr.data(), sizeof(FaceTask) * tr.size(),
-                             cudaMemcpyHostToDevice), "copy") &&
-               ck(cudaMemcpy(c->task_cube_r, cr.data(), sizeof(int) * cr.size(),
-                             cudaMemcpyHostToDevice), "copy"))) ||
-            (!er_.empty() &&
-             !(ck(dalloc(&c->edge_r, er_.size()), "alloc") &&
-               ck(cudaMemcpy(c->edge_r, er_.data(), sizeof(int) * er_.size(),
-                             cudaMemcpyHostToDevice), "copy"))))
-          return fail(BCMG_ERR_CUDA);
+          if (edge[cb]) flags[cb] |= kLayerEdge;
         c->closing_reduced = true;
       }
     }
   }
+  if (!ck(cudaMemcpy(c->flags, flags.data(), sizeof(int) * flags.size(), cudaMemcpyHostToDevice),
+          "copy"))
+    return fail(BCMG_ERR_CUDA);
   *out = c;
   return BCMG_OK;
 }
@@ -1461,8 +1480,11 @@ int bcmg_case_stage(bcmg_case *c, int RK) {
   clear_err();
   if (!c || RK < 1 || RK > 3) { set_err("bad context or RK"); return BCMG_ERR_ARG; }
   c->launches = 0;
+  c->has_closing = false;
+  c->phase = 0;
   int r = case_mirror_all(c);
   if (!r) r = case_stage(c, RK);
+  if (!r) r = case_settle(c);
   if (r) return r;
   CK(cudaStreamSynchronize(c->stream));
   return BCMG_OK;
@@ -1615,6 +1637,7 @@ int bcmg_case_time_flux(bcmg_case *c, int reps, double *ms) {
     for (int i = 0; i < reps && !r; ++i) r = case_flux(c, 1);
     cudaEventRecord(b, c->stream);
   }
+  if (!r) r = case_settle(c);
   if (c->precision == BCMG_PRECISION_SPLIT) {
     CK(cudaMemcpyAsync(c->U1_, c->U1p1, bytes, cudaMemcpyDeviceToDevice, c->stream));
     if (!r) r = case_mirror_all(c);
@@ -1862,11 +1885,13 @@ int bcmg_case_advance_converged(bcmg_case *c, int steps, int max_subiters, doubl
       CK(cudaGetLastError());
     }
   } else {
+    c->has_closing = false;
+    c->phase = 0;
     for (int st = 0; st < steps; ++st) {
       k_conv_reset<<<1, 128, 0, c->stream>>>(c->active, c->iters, c->ncase);
       CK(cudaGetLastError());
       for (int it = 0; it < max_subiters; ++it) {
-        if ((r = case_subiter(c))) return r;
+        if ((r = case_subiter(c)) || (r = case_settle(c))) return r;
         k_conv_check<<<1, 32, 0, c->stream>>>(c->er, c->active, c->iters, c->ncase, tol,
                                               max_subiters, c->cont, 0, 0);
         CK(cudaGetLastError());
@@ -2565,14 +2590,14 @@ int compat_bc(int axis, int nl, int nu, const int *lo, const int *up, double *U)
   CK(cudaMemcpyAsync(C.ibuf, cubes.data(), sizeof(int) * cubes.size(), cudaMemcpyHostToDevice, C.s));
   CK(cudaMemcpyAsync(C.ibuf + cubes.size(), masks.data(), sizeof(int) * masks.size(),
                      cudaMemcpyHostToDevice, C.s));
-  BcArgs b;
+  LayerArgs b;
   b.n = C.cfg.ncube_x;
   b.Uin = C.cfg.Uin;
   b.cubes = C.ibuf;
-  b.masks = C.ibuf + cubes.size();
+  b.flags = C.ibuf + cubes.size();
   b.axes = 1 << axis;
   b.U1_ = C.cubes;
-  CK(launch_bc(b, (int)cubes.size(), C.s));
+  CK(launch_layers(b, (int)cubes.size(), C.s));
   return scatter_cubes(C, uniq, U);
 }
 
@@ -2912,27 +2937,23 @@ void BCM_Interface(int myid, int ncube, int mPI_Nadj, int ncpu_bs, int ncpu_eq, 
       return BCMG_ERR_ARG;
     }
     if ((r = C.ensure_full(ncube))) return r;
-    std::vector<int> task_cube(tasks.size());
-    for (int cc = 1; cc < ncube; ++cc)
-      for (int t = off[cc]; t < off[cc + 1]; ++t) task_cube[t] = cc;
-    if ((r = C.grow(&C.ibuf, C.ibuf_cap, task_cube.size()))) return r;
+    if ((r = C.grow(&C.ibuf, C.ibuf_cap, off.size()))) return r;
     if ((r = C.grow(&C.tasks, C.tasks_cap, tasks.size()))) return r;
     const size_t b = C.ncell * 5 * sizeof(double);
-    if (!task_cube.empty())
-      CK(cudaMemcpyAsync(C.ibuf, task_cube.data(), sizeof(int) * task_cube.size(),
-                         cudaMemcpyHostToDevice, C.s));
+    CK(cudaMemcpyAsync(C.ibuf, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice,
+                       C.s));
     if (!tasks.empty())
       CK(cudaMemcpyAsync(C.tasks, tasks.data(), sizeof(FaceTask) * tasks.size(),
                          cudaMemcpyHostToDevice, C.s));
     g_pins.pin(U1_, b);
     CK(host_copy(C.U1_, U1_, b, cudaMemcpyHostToDevice, C.s));
-    InterfaceArgs ia;
+    LayerArgs ia;
     ia.n = C.cfg.ncube_x;
-    ia.ntasks = (int)tasks.size();
-    ia.task_cube = C.ibuf;
-    ia.tasks = C.tasks;
+    ia.off[0] = C.ibuf;
+    ia.tasks[0] = C.tasks;
+    ia.edges[0] = 1;
     ia.U1_ = C.U1_;
-    CK(launch_interface(ia, ncube, C.s));
+    CK(launch_layers(ia, ncube - 1, C.s));
     CK(host_copy(U1_, C.U1_, b, cudaMemcpyDeviceToHost, C.s));
     CK(cudaStreamSynchronize(C.s));
     return BCMG_OK;

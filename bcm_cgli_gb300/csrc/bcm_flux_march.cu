@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(NN == 32 ? 512 : 256, NN == 32 ? 1 : 2)
   const SplitConst z = split_const(a, cube);
   const float inv = a.inv_dx[cube];
   // Mirror buffers: read the current one; stages 1..3 write the other one.
-  const int par = *a.mir.parity;
+  const int par = mirror_index(a.mir);
   const float *__restrict__ M = a.mir.buf[par];
   float *const Mw = a.RK >= 1 ? a.mir.buf[par ^ 1] : nullptr;
   const size_t cb = cell_index(S, cube, 0, 0, 0);

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(split_threads<T>(), split_ctas_per_sm<T>())
   const int bi = 2 + (tl / (nt * nt)) * T, bj = 2 + ((tl / nt) % nt) * T, bk = 2 + (tl % nt) * T;
   // Mirror buffers: read the current one; stages 1..3 write the deltas of
   // the tile's cells into the other one.
-  const int par = *a.mir.parity;
+  const int par = mirror_index(a.mir);
   const float *__restrict__ M = a.mir.buf[par];
   float *const Mw = a.RK >= 1 ? a.mir.buf[par ^ 1] : nullptr;
   const int *__restrict__ F = a.FWS;

@@ -2,9 +2,10 @@
 // boundary conditions and the immersed-boundary ghost cells.
 //
 // All three are pure data movement plus a little FP64 arithmetic; each is
-// organised so one CTA owns the cells it writes and only reads cells nobody
-// writes during the launch, which makes every launch race-free and gives the
-// reference's results exactly.
+// organised so one CTA or cluster owns the cells it writes and only reads cells
+// that no other writes during the launch, which makes every launch race-free and
+// gives the reference's results exactly.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -14,14 +15,26 @@
 
 namespace bcmg {
 
-constexpr int kHaloThreads = 256;
+namespace cg = cooperative_groups;
+
+constexpr int kHaloThreads = 256, kLayerThreads = 256;
+
+// The cube a cluster of k_layers works on: its arrays (and the offset of its
+// first value in the flat ones), the mirror's reference state, the inflow
+// velocity.
+struct LayerCube {
+  double *U;
+  float *M;  // current mirror, nullptr: none
+  ptrdiff_t base;
+  double r0, e0, Uin;
+};
 
 // ---------------------------------------------------------------------------
 // Interface (BCM_Interface.cpp).  Same-level faces (:1745-1783 x, :2608-2642
 // y, :3478-3512 z) copy the neighbour's two interior layers into this cube's
 // two ghost layers over the n x n face; every read is an interior cell, every
 // write a ghost cell of the task's destination cube, so all face tasks run in
-// parallel.  A second launch then averages the edge ghosts in the
+// parallel.  A pass after them averages the edge ghosts in the
 // reference's three ordered phases (:5640-5732): i-edges, then j-edges, then
 // k-edges.
 // ---------------------------------------------------------------------------
@@ -36,134 +49,102 @@ constexpr int kHaloThreads = 256;
 //    summed in the reference's order (000,100,010,001,110,101,011,111 in i,j,k).
 // With a mirror (split precision) every written value's mirror value is
 // written too: injections copy the source's, averages are converted.
-__device__ __forceinline__ void level_face(const InterfaceArgs &a, int c, const FaceTask &ft) {
-  const int n = a.n, S = n + 4, h = n / 2;
-  const int ax = ft.axis;
-  const int t0 = ax == 0 ? 1 : 0, t1 = ax == 2 ? 1 : 2;
+__device__ __forceinline__ void level_face(const LayerArgs &a, const LayerCube &z,
+                                           const FaceTask &ft) {
+  const int n = a.n, S = n + 4, h = n / 2, ax = ft.axis;
+  // strides (values) along the face's axis and the in-face axes, x<y<z order
+  const int sx = ax == 0 ? 5 * S * S : (ax == 1 ? 5 * S : 5);
+  const int s0 = ax == 0 ? 5 * S : 5 * S * S, s1 = ax == 2 ? 5 * S : 5;
   const int o0 = (ft.slot == 2 || ft.slot == 4) ? h : 0;
   const int o1 = (ft.slot == 3 || ft.slot == 4) ? h : 0;
-  double *U = a.U1_;
-  float *M = mirror_current(a.mir);
-  double r0 = 0, e0 = 0;
-  if (M) mirror_base(a.mir, a.bt, c, r0, e0);
+  const ptrdiff_t other = cell_index(S, ft.src, 0, 0, 0) * 5;  // the neighbour
+  const double *B = a.U1_ + other;
+  const float *MB = z.M ? z.M + (other - z.base) : nullptr;
   if (ft.kind == 1) {
-    const int gs = ft.side == 0 ? n + 1 : 2;
-    for (int w = threadIdx.x; w < 2 * n * n * 5; w += blockDim.x) {
+    const int gs = (ft.side == 0 ? n + 1 : 2) * sx;
+    for (int w = threadIdx.x; w < 2 * n * n * 5; w += kLayerThreads) {
       const int v = w % 5, cell = w / 5;
-      const int l = cell / (n * n), p = 2 + (cell / n) % n, q = 2 + cell % n;
-      int d[3], sr[3];
-      d[ax] = ft.side == 0 ? l : n + 2 + l;
-      d[t0] = p;
-      d[t1] = q;
-      sr[ax] = gs;
-      sr[t0] = p / 2 + 1 + o0;
-      sr[t1] = q / 2 + 1 + o1;
-      const size_t od = 5 * cell_index(S, c, d[0], d[1], d[2]) + v;
-      const size_t os = 5 * cell_index(S, ft.src, sr[0], sr[1], sr[2]) + v;
-      U[od] = U[os];
-      if (M) M[od] = M[os];
+      const int row = cell / n, q = cell - row * n, l = row >= n, p = row - l * n;
+      const int os = gs + (p / 2 + 2 + o0) * s0 + (q / 2 + 2 + o1) * s1 + v;
+      const int od = (ft.side == 0 ? l : n + 2 + l) * sx + (p + 2) * s0 + (q + 2) * s1 + v;
+      z.U[od] = B[os];
+      if (z.M) z.M[od] = MB[os];
     }
   } else {
-    for (int w = threadIdx.x; w < 2 * h * h * 5; w += blockDim.x) {
+    for (int w = threadIdx.x; w < 2 * h * h * 5; w += kLayerThreads) {
       const int v = w % 5, cell = w / 5;
-      const int l = cell / (h * h), p = 2 + (cell / h) % h, q = 2 + cell % h;
-      int d[3], b[3];
-      d[ax] = ft.side == 1 ? n + 2 + l : l;
-      d[t0] = p + o0;
-      d[t1] = q + o1;
-      b[ax] = ft.side == 1 ? 2 * (l + 1) : n - 2 + 2 * l;
-      b[t0] = (p - 1) * 2;
-      b[t1] = (q - 1) * 2;
-      const double *B = U + 5 * cell_index(S, ft.src, b[0], b[1], b[2]) + v;
-      const size_t si = (size_t)S * S * 5, sj = (size_t)S * 5, sk = 5;
-      double sum = B[0];
-      sum = sum + B[si];
-      sum = sum + B[sj];
-      sum = sum + B[sk];
-      sum = sum + B[si + sj];
-      sum = sum + B[si + sk];
-      sum = sum + B[sj + sk];
-      sum = sum + B[si + sj + sk];
-      const size_t od = 5 * cell_index(S, c, d[0], d[1], d[2]) + v;
-      U[od] = 0.125 * sum;
-      if (M) M[od] = mirror_value_hw(0.125 * sum, v, r0, e0);
+      const int row = cell / h, q = cell - row * h, l = row >= h, p = row - l * h;
+      const double *x = B + (ft.side == 1 ? 2 * (l + 1) : n - 2 + 2 * l) * sx + (2 * p + 2) * s0 +
+                        (2 * q + 2) * s1 + v;
+      const int si = 5 * S * S, sj = 5 * S, sk = 5;
+      double sum = x[0];
+      sum = sum + x[si];
+      sum = sum + x[sj];
+      sum = sum + x[sk];
+      sum = sum + x[si + sj];
+      sum = sum + x[si + sk];
+      sum = sum + x[sj + sk];
+      sum = sum + x[si + sj + sk];
+      const int od = (ft.side == 1 ? n + 2 + l : l) * sx + (p + 2 + o0) * s0 + (q + 2 + o1) * s1 + v;
+      z.U[od] = 0.125 * sum;
+      if (z.M) z.M[od] = mirror_value_hw(0.125 * sum, v, z.r0, z.e0);
     }
   }
 }
 
-// Face copies: one CTA per (destination cube, face task).  Work items are
-// (layer, row) pairs; a row is the n cells along the innermost index that
-// both source and destination store contiguously (k for x and y faces), so
-// lanes move consecutive doubles.  For z faces a row is one (i, j) column of
-// the two ghost layers.
-__global__ void __launch_bounds__(kHaloThreads) k_iface_faces(InterfaceArgs a) {
-  const int n = a.n, S = n + 4;
-  const int t = blockIdx.x;
-  const int c = a.task_cube[t];
-  if (!case_active(a.bt, c)) return;
-  const FaceTask ft = a.tasks[t];
-  const int ax = ft.axis;
-  const int dbase = ft.side == 0 ? 0 : n + 2;
-  const int sbase = ft.side == 0 ? n : 2;
-  double *U = a.U1_;
-  if (ft.kind != 0) {
-    level_face(a, c, ft);
-    return;
-  }
-  // Copies move pairs of values (16-byte pairs of doubles, 8-byte pairs of
-  // mirror floats): S is even, so every row below starts at an even cell
-  // index (an even value index) and is 5n or 10 values long (n is a multiple
-  // of 4).  The mirror (split precision) is copied like the state: an exact
-  // copy of a value has the same rounding.
-  double2 *U2 = reinterpret_cast<double2 *>(U);
-  float2 *M2 = reinterpret_cast<float2 *>(mirror_current(a.mir));
-  // Source (the neighbour's interior) and destination (this cube's ghost
-  // layers) never overlap: each thread issues its loads for kBatch items
-  // before storing them, so the copies are not a chain of round trips.
-  constexpr int kBatch = 4;
-  auto copy = [&](int total, auto index) {
-    for (int w0 = threadIdx.x; w0 < total; w0 += kBatch * kHaloThreads) {
-      double2 u[kBatch];
-      float2 m[kBatch];
-      size_t od[kBatch];
+// One same-level face task by the threads of a CTA.  Copies move pairs of
+// values (16-byte pairs of doubles, 8-byte pairs of mirror floats): S is even,
+// so every row below starts at an even value and is 5n or 10 values long (n is
+// a multiple of 4).  Rows are the n cells along the innermost index that both
+// source and destination store contiguously (k for x and y faces); for z faces
+// a row is one (i, j) column of the two ghost layers.  The mirror (split
+// precision) is copied like the state: an exact copy of a value has the same
+// rounding.  Source (the neighbour's interior) and destination (this cube's
+// ghost layers) never overlap: a thread issues its loads for kCopyBatch items
+// before storing them, so the copies are not a chain of round trips.
+constexpr int kCopyBatch = 4;
+
+__device__ __forceinline__ void face_copy(const LayerArgs &a, const LayerCube &z,
+                                          const FaceTask &ft) {
+  const int n = a.n, S = n + 4, ax = ft.axis;
+  double2 *const D = reinterpret_cast<double2 *>(z.U);
+  float2 *const DM = reinterpret_cast<float2 *>(z.M);
+  const ptrdiff_t other = (ptrdiff_t)cell_index(S, ft.src, 0, 0, 0) * 5;
+  // everything in pairs; source minus destination is one constant: the cubes
+  // and n layers
+  const int len = ax < 2 ? 5 * n / 2 : 5, rows = ax < 2 ? n : n * n;
+  const int srow = ax == 0 ? 5 * S / 2 : 5 * S * S / 2;  // next row of a layer
+  const int layer = ax == 0 ? 5 * S * S / 2 : 5 * S / 2;
+  const int g = ft.side == 0 ? 0 : n + 2;
+  const ptrdiff_t shift =
+      (other - z.base) / 2 + (ft.side == 0 ? n : -n) * (ax == 0 ? 5 * S * S : (ax == 1 ? 5 * S : 5)) / 2;
+  const int total = len * rows * (ax < 2 ? 2 : 1);
+  auto dest = [&](int w) {
+    const int row = w / len, e = w - row * len;
+    if (ax == 2) {
+      const int i = row / n, j = row - i * n;
+      return ((i + 2) * S + j + 2) * (5 * S / 2) + 5 * g / 2 + e;
+    }
+    const int l = row >= n, p = row - l * n;
+    return (g + l) * layer + (p + 2) * srow + 5 + e;
+  };
+  for (int w0 = threadIdx.x; w0 < total; w0 += kCopyBatch * kLayerThreads) {
+    double2 u[kCopyBatch];
+    float2 m[kCopyBatch];
+    int d[kCopyBatch];
 #pragma unroll
-      for (int b = 0; b < kBatch; ++b) {
-        const int w = w0 + b * kHaloThreads;
-        if (w < total) {
-          size_t os;
-          index(w, od[b], os);
-          u[b] = U2[os];
-          if (M2) m[b] = M2[os];
-        }
+    for (int b = 0; b < kCopyBatch; ++b)
+      if (w0 + b * kLayerThreads < total) {
+        d[b] = dest(w0 + b * kLayerThreads);
+        u[b] = D[d[b] + shift];
+        if (DM) m[b] = DM[d[b] + shift];
       }
 #pragma unroll
-      for (int b = 0; b < kBatch; ++b)
-        if (w0 + b * kHaloThreads < total) {
-          U2[od[b]] = u[b];
-          if (M2) M2[od[b]] = m[b];
-        }
-    }
-  };
-  if (ax < 2) {
-    // rows: (layer l, transverse index p); each row = 5n doubles along k
-    const int rowlen = 5 * n / 2;
-    copy(2 * n * rowlen, [&](int w, size_t &od, size_t &os) {
-      const int row = w / rowlen, e = w - row * rowlen;
-      const int l = row / n, p = 2 + (row - l * n);
-      int di, dj, si, sj;
-      if (ax == 0) { di = dbase + l; si = sbase + l; dj = sj = p; }
-      else { dj = dbase + l; sj = sbase + l; di = si = p; }
-      od = 5 * cell_index(S, c, di, dj, 2) / 2 + e;
-      os = 5 * cell_index(S, ft.src, si, sj, 2) / 2 + e;
-    });
-  } else {
-    // z faces: per (i, j) the two layers are 10 contiguous doubles
-    copy(n * n * 5, [&](int w, size_t &od, size_t &os) {
-      const int col = w / 5, e = w - col * 5;
-      const int i = 2 + col / n, j = 2 + (col - (col / n) * n);
-      od = 5 * cell_index(S, c, i, j, dbase) / 2 + e;
-      os = 5 * cell_index(S, ft.src, i, j, sbase) / 2 + e;
-    });
+    for (int b = 0; b < kCopyBatch; ++b)
+      if (w0 + b * kLayerThreads < total) {
+        D[d[b]] = u[b];
+        if (DM) DM[d[b]] = m[b];
+      }
   }
 }
 
@@ -178,69 +159,37 @@ __global__ void __launch_bounds__(kHaloThreads) k_iface_faces(InterfaceArgs a) {
 // averages of face ghosts.  So one pass computes each edge cell from two
 // face ghosts and each corner from the two edge values it averages (formed
 // from four face ghosts in registers): the reference's operations, the same
-// bits, one round trip to memory instead of three dependent ones.  A thread
-// issues the loads of kEdgeBatch items before their stores.
-constexpr int kEdgeThreads = 256, kEdgeBatch = 4;
-
-__global__ void __launch_bounds__(kEdgeThreads) k_iface_edges(InterfaceArgs a) {
-  const int n = a.n, S = n + 4, nx = n + 1, nyy = n + 2;
-  const int c = a.edge_list ? a.edge_cubes[blockIdx.x] : blockIdx.x + 1;
-  if (!case_active(a.bt, c)) return;
-  double *U = a.U1_;
-  float *M = mirror_current(a.mir);
-  double r0 = 0, e0 = 0;
-  if (M) mirror_base(a.mir, a.bt, c, r0, e0);
-  auto at = [&](int i, int j, int k, int v) { return 5 * cell_index(S, c, i, j, k) + v; };
-  auto ghost = [&](int x) { return x == 1 || x == nyy; };
-  auto in = [&](int x) { return x == 1 ? 2 : nx; };
-  // an edge cell (two ghost coordinates): the average of its two inward
-  // neighbours across its ghost axes, both face ghosts
-  auto edge = [&](int i, int j, int k, int v) -> double {
-    double p, q;
-    if (!ghost(i)) { p = U[at(i, in(j), k, v)]; q = U[at(i, j, in(k), v)]; }
-    else if (!ghost(j)) { p = U[at(in(i), j, k, v)]; q = U[at(i, j, in(k), v)]; }
-    else { p = U[at(in(i), j, k, v)]; q = U[at(i, in(j), k, v)]; }
-    return 0.5 * (p + q);
-  };
+// bits, one round trip to memory instead of three dependent ones.
+__device__ __forceinline__ void edge_fill(const LayerArgs &a, const LayerCube &z, int first,
+                                          int stride) {
+  const int n = a.n, S = n + 4, s0 = 5 * S * S, s1 = 5 * S, s2 = 5;
+  // an edge cell at offset o: its inward neighbours across its ghost axes
+  auto edge = [&](int o, int da, int db) { return 0.5 * (z.U[o + da] + z.U[o + db]); };
   const int nedge = 12 * n, items = 5 * (nedge + 8);
-  // the value and destination of item w
-  auto item = [&](int w, double &r, size_t &d, int &v) {
-    v = w % 5;
-    const int cell = w / 5;
-    int ci, cj, ck;
+#pragma unroll 2
+  for (int w = first; w < items; w += stride) {
+    const int v = w % 5, cell = w / 5;
+    double r;
+    int o;
     if (cell < nedge) {
-      // edge family f (free coordinate i, j or k = 2..nx) and its two ghost
-      // coordinates
-      const int f = cell / (4 * n), rem = cell - f * 4 * n;
-      const int pos = 2 + (rem >> 2), g1 = (rem & 1) ? nyy : 1, g2 = (rem & 2) ? nyy : 1;
-      if (f == 0) { ci = pos; cj = g1; ck = g2; }
-      else if (f == 1) { ci = g1; cj = pos; ck = g2; }
-      else { ci = g1; cj = g2; ck = pos; }
-      r = edge(ci, cj, ck, v);
+      // edge family f (free coordinate i, j or k = 2..nx), its two ghost axes
+      // a, b (a < b) and their sides
+      const int f = cell / (4 * n), rem = cell - f * 4 * n, pos = 2 + (rem >> 2);
+      const int sa = f == 0 ? s1 : s0, sb = f == 2 ? s1 : s2, sf = f == 0 ? s0 : (f == 1 ? s1 : s2);
+      const int ua = rem & 1, ub = rem >> 1 & 1;
+      o = pos * sf + (ua ? n + 2 : 1) * sa + (ub ? n + 2 : 1) * sb + v;
+      r = edge(o, ua ? -sa : sa, ub ? -sb : sb);
     } else {
       // corner: the k-edge phase's average of the j-edge cell and the i-edge
       // cell next to it
-      const int q = cell - nedge;
-      ci = (q & 1) ? nyy : 1; cj = (q & 2) ? nyy : 1; ck = (q & 4) ? nyy : 1;
-      const double xj = edge(ci, in(cj), ck, v), yi = edge(in(ci), cj, ck, v);
+      const int q = cell - nedge, d0 = q & 1 ? -s0 : s0, d1 = q & 2 ? -s1 : s1,
+                d2 = q & 4 ? -s2 : s2;
+      o = (q & 1 ? n + 2 : 1) * s0 + (q & 2 ? n + 2 : 1) * s1 + (q & 4 ? n + 2 : 1) * s2 + v;
+      const double xj = edge(o + d1, d0, d2), yi = edge(o + d0, d1, d2);
       r = 0.5 * (xj + yi);
     }
-    d = at(ci, cj, ck, v);
-  };
-  for (int w0 = threadIdx.x; w0 < items; w0 += kEdgeBatch * kEdgeThreads) {
-    double r0v = 0, r1v = 0, r2v = 0, r3v = 0;
-    size_t d0 = 0, d1 = 0, d2 = 0, d3 = 0;
-    int v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-    const int w1 = w0 + kEdgeThreads, w2 = w0 + 2 * kEdgeThreads, w3 = w0 + 3 * kEdgeThreads;
-    item(w0, r0v, d0, v0);
-    if (w1 < items) item(w1, r1v, d1, v1);
-    if (w2 < items) item(w2, r2v, d2, v2);
-    if (w3 < items) item(w3, r3v, d3, v3);
-    U[d0] = r0v;
-    if (M) M[d0] = mirror_value_hw(r0v, v0, r0, e0);
-    if (w1 < items) { U[d1] = r1v; if (M) M[d1] = mirror_value_hw(r1v, v1, r0, e0); }
-    if (w2 < items) { U[d2] = r2v; if (M) M[d2] = mirror_value_hw(r2v, v2, r0, e0); }
-    if (w3 < items) { U[d3] = r3v; if (M) M[d3] = mirror_value_hw(r3v, v3, r0, e0); }
+    z.U[o] = r;
+    if (z.M) z.M[o] = mirror_value_hw(r, v, z.r0, z.e0);
   }
 }
 
@@ -293,18 +242,6 @@ cudaError_t launch_halo(double *U, const Mirror &mir, const int *bands, const lo
   return cudaGetLastError();
 }
 
-cudaError_t launch_interface(const InterfaceArgs &a, int ncubes_total, cudaStream_t s) {
-  if (ncubes_total <= 1) return cudaSuccess;
-  if (a.ntasks > 0) {
-    k_iface_faces<<<a.ntasks, kHaloThreads, 0, s>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  const int ne = a.edge_list ? a.nedge : ncubes_total - 1;
-  if (ne > 0) k_iface_edges<<<ne, kEdgeThreads, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------------------
 // Boundary conditions (BCM_X/Y/Z_boundary_condition.cpp) in one pass.  The
 // reference fills the x faces (j, k interior: inflow from cell 2, zero
@@ -321,134 +258,211 @@ cudaError_t launch_interface(const InterfaceArgs &a, int ncubes_total, cudaStrea
 // pass to the faces of one twin call (the others' ghosts are then read as
 // they are).
 // ---------------------------------------------------------------------------
-constexpr int kBcThreads = 256, kBcChunks = 8, kBcBatch = 4;
+// The inflow's total energy: pressure of the cell next to it, velocity (Uin, 0,
+// 0).  A call: inlined at each of a thread's items its three divisions made
+// the kernel wait for instructions.
+__device__ __noinline__ double inflow_energy(const double *q, double Uin) {
+  const double rho = q[0];
+  const double Uu = Uin, Vv = 0., Ww = 0;
+  const double U0 = q[1] / rho, V0 = q[2] / rho, W0 = q[3] / rho;
+  double VV = U0 * U0 + V0 * V0 + W0 * W0;
+  const double P = (q[4] - 0.5 * rho * VV) * (BCMG_K - 1);
+  VV = Uu * Uu + Vv * Vv + Ww * Ww;
+  return P / (BCMG_K - 1) + 0.5 * rho * VV;
+}
 
-__global__ void __launch_bounds__(kBcThreads) k_bc(BcArgs a) {
-  const int n = a.n, S = n + 4, nx = n + 1, nxx = n + 2, nxxx = n + 3;
-  const int c = a.cubes[blockIdx.x];
-  if (!case_active(a.bt, c)) return;
-  const int m = a.masks[blockIdx.x];
+constexpr int kBcBatch = 2;
+
+// cover: boundary faces (bits as in m) that a same-level face task also fills
+// (a periodic box's boundary lists name such faces): over their interior n x n
+// positions the opening interface call would put the neighbour's cells back
+// before anything reads them, so nothing is written there and the layers stay
+// as the last interface call, or this launch's full one, leaves them.
+__device__ __forceinline__ void bc_fill(const LayerArgs &a, const LayerCube &z, int m, int cover,
+                                        int first, int stride) {
+  const int n = a.n, S = n + 4, nx = n + 1, nxx = n + 2;
   const int mx = (a.axes & 1) ? (m & 3) : 0, my = (a.axes & 2) ? ((m >> 2) & 3) : 0,
             mz = (a.axes & 4) ? ((m >> 4) & 3) : 0;
-  double *U = a.U1_;
+  double *const U = z.U;
   // Split precision: the mirror values of every write, into both mirror
   // buffers.  The flux kernel writes the next buffer's interior cells and
   // same-level ghost layers, and the interface call after it the level-jump
   // layers and edges; the boundary layers are written here only, so the
   // next buffer takes them now and equals the state's rounding in every
   // cell once it becomes current.
-  float *M = mirror_current(a.mir);
-  float *Mo = M ? (M == a.mir.buf[0] ? a.mir.buf[1] : a.mir.buf[0]) : nullptr;
-  double r0 = 0, e0 = 0;
-  if (M) mirror_base(a.mir, a.bt, c, r0, e0);
-  const double Uin = a.bt.cube_case ? a.bt.cases[a.bt.cube_case[c]].Uin : a.Uin;
-  auto Q = [&](int i, int j, int k) { return U + 5 * cell_index(S, c, i, j, k); };
-  auto interior = [&](int x) { return x >= 2 && x <= nx; };
-  // component v of the inflow state (:43-80): rho and p from the cell,
-  // u = Uin, v = w = 0
-  auto inflow = [&](const double *q, int v) -> double {
-    const double rho = q[0];
-    if (v == 0) return rho;
-    const double Uu = Uin, Vv = 0., Ww = 0;
-    if (v == 1) return rho * Uu;
-    if (v == 2) return rho * Vv;
-    if (v == 3) return rho * Ww;
-    const double U0 = q[1] / rho, V0 = q[2] / rho, W0 = q[3] / rho;
-    double VV = U0 * U0 + V0 * V0 + W0 * W0;
-    const double P = (q[4] - 0.5 * rho * VV) * (BCMG_K - 1);
-    VV = Uu * Uu + Vv * Vv + Ww * Ww;
-    return P / (BCMG_K - 1) + 0.5 * rho * VV;
+  float *const M = z.M;
+  float *const Mo = M ? (mirror_index(a.mir) ? a.mir.buf[0] : a.mir.buf[1]) + z.base : nullptr;
+  const double Uin = z.Uin;
+  // ghost positions: x faces n^2 each, y faces S n each, z faces S^2 each
+  // (covered faces: none, the 4 n and the 8 n + 16 outside n x n); each
+  // position fills both ghost layers with one value.  Items are (position,
+  // component), component fastest, so a warp's loads and stores run over
+  // whole cells in a row.
+  auto count = [&](int f) -> int {  // positions of face f
+    if (!((f < 2 ? mx : (f < 4 ? my : mz)) >> (f & 1) & 1)) return 0;
+    const bool cov = cover >> f & 1;
+    return f < 2 ? (cov ? 0 : n * n) : (f < 4 ? (cov ? 4 : S) * n : (cov ? 8 * n + 16 : S * S));
   };
-  // component v of cell (i, j, k) as the reference's order leaves it after
-  // the x phase (upto 1) or after the x and y phases (upto 2)
-  auto read = [&](int i, int j, int k, int upto, int v) -> double {
-    if (upto >= 2 && my && interior(k)) {
+  int end[6];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) end[f] = count(f) + (f ? end[f ? f - 1 : 0] : 0);
+  const int items = 5 * end[5];
+  auto ghost = [&](int g) { return g < 2 ? g : n + g; };
+  // Item w: the cell its value comes from as the reference's order of phases
+  // leaves it there (offset in the cube), whether that is the inflow formula
+  // of the cell, and its first destination (the second is `step` further).
+  auto item = [&](int w, int &src, int &v, bool &infl, bool &neg, int &dst, int &step) {
+    v = w % 5;
+    int q = w / 5, f = 0, before = 0;
+#pragma unroll
+    for (int g = 0; g < 5; ++g)
+      if (q >= end[g]) { f = g + 1; before = end[g]; }
+    q -= before;
+    const int ax = f >> 1, up = f & 1;
+    const bool cov = cover >> f & 1;
+    // (p, r): the position's in-face indices, x<y<z order
+    int p, r;
+    if (ax < 2) {
+      p = q / n;
+      r = 2 + q - p * n;
+      p = ax == 0 ? p + 2 : (cov ? ghost(p) : p);
+    } else if (!cov || q < 4 * S) {
+      p = q / S;
+      r = q - p * S;
+      if (cov) p = ghost(p);
+    } else {
+      q -= 4 * S;
+      p = 2 + (q >> 2);
+      r = ghost(q & 3);
+    }
+    const int in = up ? nx : 2;
+    int i = ax == 0 ? in : p, j = ax == 0 ? p : (ax == 1 ? in : r), k = ax == 2 ? in : r;
+    const int g = up ? nxx : 1;
+    dst = ax == 0 ? (g * S + j) * S + k : (ax == 1 ? (i * S + g) * S + k : (i * S + j) * S + g);
+    step = (ax == 0 ? S * S : (ax == 1 ? S : 1)) * (up ? 1 : -1);
+    infl = ax == 0 && !up;
+    neg = ax == 2 && !up;  // slip wall: rho*w negated (:42-65)
+    if (ax == 2) {  // rows the y phase wrote
       if ((my & 1) && j <= 1) j = 2;
       else if ((my & 2) && j >= nxx) j = nx;
     }
-    if (mx && interior(j) && interior(k)) {
-      if ((mx & 1) && i <= 1) return inflow(Q(2, j, k), v);
-      if ((mx & 2) && i >= nxx) i = nx;
+    if (ax > 0 && mx && j >= 2 && j <= nx) {  // and the x phase
+      if ((mx & 1) && i <= 1) { i = 2; infl = true; }
+      else if ((mx & 2) && i >= nxx) i = nx;
     }
-    return Q(i, j, k)[v];
-  };
-  // ghost positions: x faces n^2 each, y faces S n each, z faces S^2 each;
-  // each position fills both ghost layers with one value.  Items are
-  // (position, component), component fastest, so a warp's loads and stores
-  // run over whole cells in a row.
-  const int cx = n * n, cy = S * n, cz = S * S;
-  const int nxl = (mx & 1) ? cx : 0, nxu = (mx & 2) ? cx : 0, nyl = (my & 1) ? cy : 0,
-            nyu = (my & 2) ? cy : 0, nzl = (mz & 1) ? cz : 0, nzu = (mz & 2) ? cz : 0;
-  const int items = 5 * (nxl + nxu + nyl + nyu + nzl + nzu);
-  // item w: its value and the offsets of its two destinations
-  auto item = [&](int w, double &x, size_t &d1, size_t &d0) {
-    const int v = w % 5;
-    int q = w / 5;
-    if (q < nxl) {
-      const int j = 2 + q / n, k = 2 + q % n;
-      x = inflow(Q(2, j, k), v);
-      d1 = 5 * cell_index(S, c, 1, j, k) + v; d0 = 5 * cell_index(S, c, 0, j, k) + v;
-      return;
-    }
-    q -= nxl;
-    if (q < nxu) {
-      const int j = 2 + q / n, k = 2 + q % n;
-      x = Q(nx, j, k)[v];
-      d1 = 5 * cell_index(S, c, nxx, j, k) + v; d0 = 5 * cell_index(S, c, nxxx, j, k) + v;
-      return;
-    }
-    q -= nxu;
-    if (q < nyl) {
-      const int i = q / n, k = 2 + q % n;
-      x = read(i, 2, k, 1, v);
-      d1 = 5 * cell_index(S, c, i, 1, k) + v; d0 = 5 * cell_index(S, c, i, 0, k) + v;
-      return;
-    }
-    q -= nyl;
-    if (q < nyu) {
-      const int i = q / n, k = 2 + q % n;
-      x = read(i, nx, k, 1, v);
-      d1 = 5 * cell_index(S, c, i, nxx, k) + v; d0 = 5 * cell_index(S, c, i, nxxx, k) + v;
-      return;
-    }
-    q -= nyu;
-    if (q < nzl) {  // slip wall: rho*w negated (:42-65)
-      const int i = q / S, j = q % S;
-      x = read(i, j, 2, 2, v);
-      if (v == 3) x = -x;
-      d1 = 5 * cell_index(S, c, i, j, 1) + v; d0 = 5 * cell_index(S, c, i, j, 0) + v;
-      return;
-    }
-    q -= nzl;
-    const int i = q / S, j = q % S;
-    x = read(i, j, nx, 2, v);
-    d1 = 5 * cell_index(S, c, i, j, nxx) + v; d0 = 5 * cell_index(S, c, i, j, nxxx) + v;
+    src = (i * S + j) * S + k;
   };
   // kBcBatch items per round, all loaded before any is stored
-  const int stride = gridDim.y * kBcThreads;
-  for (int w0 = blockIdx.y * kBcThreads + threadIdx.x; w0 < items; w0 += kBcBatch * stride) {
+  for (int w0 = first; w0 < items; w0 += kBcBatch * stride) {
     double x[kBcBatch];
-    size_t d1[kBcBatch], d0[kBcBatch];
-#pragma unroll
-    for (int b = 0; b < kBcBatch; ++b)
-      if (w0 + b * stride < items) item(w0 + b * stride, x[b], d1[b], d0[b]);
+    int src[kBcBatch], v[kBcBatch], dst[kBcBatch], step[kBcBatch];
+    bool infl[kBcBatch], neg[kBcBatch];
 #pragma unroll
     for (int b = 0; b < kBcBatch; ++b)
       if (w0 + b * stride < items) {
-        U[d1[b]] = x[b];
-        U[d0[b]] = x[b];
+        item(w0 + b * stride, src[b], v[b], infl[b], neg[b], dst[b], step[b]);
+        x[b] = U[5 * src[b] + (infl[b] && v[b] < 4 ? 0 : v[b])];
+      }
+#pragma unroll
+    for (int b = 0; b < kBcBatch; ++b)
+      if (w0 + b * stride < items) {
+        if (infl[b]) {  // rho and p from the cell, u = Uin, v = w = 0 (:43-80)
+          if (v[b] == 1) x[b] = x[b] * Uin;
+          else if (v[b] == 2 || v[b] == 3) x[b] = x[b] * 0.0;
+          else if (v[b] == 4) x[b] = inflow_energy(U + 5 * src[b], Uin);
+        }
+        if (neg[b] && v[b] == 3) x[b] = -x[b];
+        const int d1 = 5 * dst[b] + v[b], d0 = d1 + 5 * step[b];
+        U[d1] = x[b];
+        U[d0] = x[b];
         if (M) {
-          const float mv = mirror_value_hw(x[b], (int)(d1[b] % 5), r0, e0);
-          M[d1[b]] = mv; M[d0[b]] = mv; Mo[d1[b]] = mv; Mo[d0[b]] = mv;
+          const float mv = mirror_value_hw(x[b], v[b], z.r0, z.e0);
+          M[d1] = mv; M[d0] = mv; Mo[d1] = mv; Mo[d0] = mv;
         }
       }
   }
 }
 
-cudaError_t launch_bc(const BcArgs &a, int ncubes, cudaStream_t s) {
+// ---------------------------------------------------------------------------
+// The ghost layers of a cube by a cluster of CTAs.  Each of the up to five
+// passes writes ghost cells of its cube only and reads the cube's own cells
+// and other cubes' interior cells, which no pass writes: so passes depend on
+// each other within a cube only, and barriers of its cluster order them.
+// That replaces four or five launches a stage (closing faces, closing edges,
+// boundary conditions, opening faces, opening edges), each of 8 to 45 us, most
+// of it launch and dependent round trips, whatever the number of cubes: 512
+// periodic cubes of 24^3 about 110 -> 34 us a stage, and with the mirror flag's
+// and E normalisation's launches gone too, a step of 10 sub-iterations of 8
+// cubes of 8^3 1.21 -> 0.80 ms.  What bounds it now: the passes' dependent
+// loads (4 CTAs of 64 registers on an SM).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kLayerThreads, 4) k_layers(LayerArgs a) {
+  const cg::cluster_group cl = cg::this_cluster();
+  const int size = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int q = blockIdx.x / size;
+  const int c = a.cubes ? a.cubes[q] : q + 1;
+  if (!case_active(a.bt, c)) return;  // converged case (the whole cluster)
+  const int flags = a.flags ? a.flags[a.cubes ? q : c] : 0;
+  const int first = rank * kLayerThreads + threadIdx.x, stride = size * kLayerThreads;
+  LayerCube z;
+  z.base = (ptrdiff_t)cell_index(a.n + 4, c, 0, 0, 0) * 5;
+  z.U = a.U1_ + z.base;
+  z.M = mirror_current(a.mir);
+  z.r0 = z.e0 = 0;
+  if (z.M) {
+    mirror_base(a.mir, a.bt, c, z.r0, z.e0);
+    z.M += z.base;
+  }
+  z.Uin = a.bt.cube_case ? a.bt.cases[a.bt.cube_case[c]].Uin : a.Uin;
+  bool wrote = false;
+  auto order = [&]() {  // after the passes so far (uniform over the cluster)
+    if (wrote) {
+      if (size == 1) __syncthreads(); else cl.sync();
+    }
+    wrote = true;
+  };
+#pragma unroll 1
+  for (int r = 0; r < 2; ++r) {
+    if (r == 1 && a.axes && (flags & 63)) {
+      order();
+      bc_fill(a, z, flags, a.cover ? flags >> kLayerCover : 0, first, stride);
+    }
+    const int *off = r ? a.off[1] : a.off[0];
+    if (off && off[c + 1] > off[c]) {
+      order();
+      const FaceTask *tasks = r ? a.tasks[1] : a.tasks[0];
+      for (int t = off[c] + rank; t < off[c + 1]; t += size) {
+        const FaceTask ft = tasks[t];
+        if (ft.kind == 0) face_copy(a, z, ft); else level_face(a, z, ft);
+      }
+    }
+    const int e = r ? a.edges[1] : a.edges[0];
+    if (e == 1 || (e == 2 && (flags & kLayerEdge))) {
+      order();
+      edge_fill(a, z, first, stride);
+    }
+  }
+}
+
+cudaError_t launch_layers(const LayerArgs &a, int ncubes, cudaStream_t s) {
   if (ncubes <= 0) return cudaSuccess;
-  k_bc<<<dim3(ncubes, kBcChunks), kBcThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  // Four CTAs a cube while that leaves the chip room, else two (a step's stage,
+  // us, by clusters of 1, 2 and 4: 8 cubes of 8^3 31.4 29.6 26.8, 64 of 16^3 in
+  // FP64 535 528 525, 216 of 24^3 473 467 467, 216 of 12^3 87.9 84.9 87.2, 512
+  // of 24^3 1026 1020 1024, 2,744 of 16^3 1516 1523 1541).
+  const int size = ncubes <= 64 || (ncubes <= 304 && a.n >= 16) ? 4 : 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncubes * size);
+  cfg.blockDim = dim3(kLayerThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = size;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_layers, a);
 }
 
 // ---------------------------------------------------------------------------

@@ -152,20 +152,22 @@ cudaError_t launch_rk(const RkArgs &a, int *nblocks_out, cudaStream_t s);
 int rk_partial_blocks(const RkArgs &a);
 // Same combination with an explicit chunk (cells per block) and block count.
 cudaError_t launch_rk_chunked(const RkArgs &a, long long chunk, int nblocks, cudaStream_t s);
-// Deterministic final reduction of partials -> er[1..7] (device, 8 doubles).
+// Deterministic final reduction of partials -> er[1..7] (device, 8 doubles);
+// with emax (device, 6 doubles) the end of a sub-iteration: E_k = max(E_k,
+// er_k), er_k /= E_k.
 cudaError_t launch_norms(const Phys &ph, const double *partials, int nblocks, double *er,
-                         cudaStream_t s, const int *active = nullptr);
+                         cudaStream_t s, const int *active = nullptr, double *emax = nullptr);
 // Cube-sharded runs: raw sums of the partial blocks (sums[7]), and the norms
 // er[1..7] from sums added over the ranks.
 cudaError_t launch_norm_sums(const double *partials, int nblocks, double *sums, cudaStream_t s,
                              const int *active = nullptr);
 cudaError_t launch_norm_final(const Phys &ph, const double *sums, double *er, cudaStream_t s,
-                              const int *active = nullptr);
+                              const int *active = nullptr, double *emax = nullptr);
 // Batches: case q reduces partial blocks [case_blk[q], case_blk[q+1]) into
 // er[8q .. 8q+7] with its own normalisers.
 cudaError_t launch_norms_batch(int n, const CaseConst *cases, const int *case_blk, int ncase,
                                const double *partials, double *er, cudaStream_t s,
-                               const int *active = nullptr);
+                               const int *active = nullptr, double *emax = nullptr);
 // Batch form of launch_rk over an explicit block table (nblocks blocks).
 cudaError_t launch_rk_table(const RkArgs &a, int nblocks, cudaStream_t s);
 
@@ -223,8 +225,8 @@ cudaError_t launch_plot3d_q(const double *U, double *out, int n, int cube0, int 
 cudaError_t launch_plot3d_x(const double *cube_size, const double *origin, double *out, int n,
                             int cube0, int ncubes, cudaStream_t s);
 
-// Interface: face-copy tasks (destination cube, source cube, axis, side) built
-// on the host, then the ordered three-phase edge fill of every cube.
+// Interface: face-copy tasks (source cube, axis, side) of each destination cube,
+// built on the host.
 struct FaceTask {
   int32_t src;   // source cube
   int8_t axis;   // 0 x, 1 y, 2 z
@@ -232,19 +234,35 @@ struct FaceTask {
   int8_t kind;   // 0 same-level copy, 1 coarse->fine injection, 2 fine->coarse average
   int8_t slot;   // kinds 1, 2: sub-face slot 1..4 of the small cube on the big face
 };
-struct InterfaceArgs {
+// Ghost layers around an update, one launch (k_layers): up to two rounds of
+// interface calls with the boundary conditions between them, in the order
+// closing faces, closing edges, boundary conditions, opening faces, opening
+// edges; any of the five may be absent.
+struct LayerArgs {
   int n;
-  int ntasks;             // face tasks (all destination cubes)
-  const int *task_cube;   // [ntasks] destination cube of each task
-  const FaceTask *tasks;  // [ntasks]
   double *U1_;
   Batch bt;
   Mirror mir;  // split precision: every written cell's mirror value too
-  bool edge_list = false;           // the edge fill over edge_cubes only (else all)
-  const int *edge_cubes = nullptr;  // [nedge] cube numbers
-  int nedge = 0;
+  // face tasks of the closing [0] and opening [1] call: those of cube c are
+  // tasks[r][off[r][c] .. off[r][c+1]); off[r] == nullptr: none
+  const int *off[2] = {nullptr, nullptr};
+  const FaceTask *tasks[2] = {nullptr, nullptr};
+  // edge fill of the two calls: 0 none, 1 every cube, 2 cubes whose flags
+  // have kLayerEdge set
+  int edges[2] = {0, 0};
+  // X/Y/Z boundary conditions: flags bits 0..5 = x lower, x upper, y lower, y
+  // upper, z lower, z upper; axes selects the phases (bit 0 x, 1 y, 2 z; 0:
+  // none)
+  int axes = 0;
+  bool cover = false;  // leave out what same-level face tasks fill (kLayerCover)
+  double Uin = 0;
+  // cubes == nullptr: cubes 1.. with flags[cube]; else cubes[q] with flags[q]
+  const int *cubes = nullptr;
+  const int *flags = nullptr;
 };
-cudaError_t launch_interface(const InterfaceArgs &a, int ndst, cudaStream_t s);
+constexpr int kLayerEdge = 64;
+constexpr int kLayerCover = 8;  // flags bits 8..13: faces with a same-level face task
+cudaError_t launch_layers(const LayerArgs &a, int ncubes, cudaStream_t s);
 
 // Halo exchange of cube-sharded runs: band b = bands[4b..4b+3] = (cube slot,
 // axis, side 1 high / 0 low face, layers); its cells are the `layers`
@@ -256,21 +274,6 @@ cudaError_t launch_interface(const InterfaceArgs &a, int ndst, cudaStream_t s);
 cudaError_t launch_halo(double *U, const Mirror &mir, const int *bands, const long long *offs,
                         int nband, long long total_cells, int n, void *buf, int unpack,
                         cudaStream_t s);
-
-// X/Y/Z boundary conditions for a list of (cube, mask) pairs; mask bits
-// 0..5 = x lower, x upper, y lower, y upper, z lower, z upper.  axes selects
-// which of the three phases run (bit 0 x, 1 y, 2 z).
-struct BcArgs {
-  int n;
-  double Uin;
-  const int *cubes;
-  const int *masks;
-  int axes;
-  double *U1_;
-  Batch bt;  // batches: Uin of the cube's case
-  Mirror mir;  // split precision: every written cell's mirror value too
-};
-cudaError_t launch_bc(const BcArgs &a, int ncubes, cudaStream_t s);
 
 // IBM ghost-cell fill for one dependency level of the combined entry list.
 struct GhostArgs {

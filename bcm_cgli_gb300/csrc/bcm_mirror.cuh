@@ -131,15 +131,17 @@ __device__ __forceinline__ float mirror_value_hw(double x, int v, double rho0, d
 // buf[0] == nullptr: no mirror (the FP64 path); kernels then skip it.
 struct Mirror {
   float *buf[2] = {nullptr, nullptr};
-  const int *parity = nullptr;  // device [1]: index of the current buffer
+  const int *parity = nullptr;  // device [1]: index of the current buffer ...
+  int phase = 0;                // ... at the last launch of k_mirror_flip; 1: the other one now
   double rho0 = 0, E0 = 0;
 };
 
 #ifdef __CUDACC__
-// (a select, not m.buf[*m.parity]: indexing a kernel argument's array with
+__device__ __forceinline__ int mirror_index(const Mirror &m) { return *m.parity ^ m.phase; }
+// (a select, not m.buf[mirror_index(m)]: indexing a kernel argument's array with
 // a run-time value would copy the argument to local memory)
 __device__ __forceinline__ float *mirror_current(const Mirror &m) {
-  return m.buf[0] ? (*m.parity ? m.buf[1] : m.buf[0]) : nullptr;
+  return m.buf[0] ? (mirror_index(m) ? m.buf[1] : m.buf[0]) : nullptr;
 }
 #endif
 

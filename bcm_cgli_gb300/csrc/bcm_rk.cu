@@ -4,15 +4,18 @@
 // updated; at stage 3 the L2 change norms of p, u, v, w, T over fluid cells
 // and the force sums over all interior cells are formed.  The reference sums
 // serially (its OpenMP accumulation at :2523 is unsynchronised); here each
-// block sums a fixed contiguous range of cells in a fixed tree order and a
-// single block adds the block sums in order, so the result is run-to-run
+// block sums a fixed contiguous range of cells in a fixed tree order and one
+// cluster adds the block sums in a fixed order, so the result is run-to-run
 // reproducible and equal to the serial sum within rounding.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "bcm_common.cuh"
 #include "bcm_kernels.h"
 
 namespace bcmg {
+
+namespace cg = cooperative_groups;
 
 constexpr int kRkThreads = 256;
 
@@ -101,15 +104,22 @@ __global__ void __launch_bounds__(kRkThreads) k_rk(RkArgs a, long long total, lo
 }
 
 // Deterministic sum of partials[b][0..6] over blocks [b0, b1) into tot[7]
-// (shared).  kNormWarps warps per quantity; lane l of warp w takes blocks
-// b0 + 32 w + l, then every 32 kNormWarps-th, into four accumulators in turn
-// (loads in flight), combined as (v0 + v1) + (v2 + v3); a fixed shuffle tree
-// per warp and the warps' results in warp order.  The order depends only on
-// b1 - b0, never on timing, so a batch's case and the same case alone sum
-// identically.  Launch with 7 * kNormWarps warps.
-constexpr int kNormWarps = 4;
+// (shared) of the cluster's first CTA.  CTA r of the cluster takes the r-th of
+// kNormCtas equal ranges; in it kNormWarps warps per quantity; lane l of warp w
+// takes blocks 32 w + l, then every 32 kNormWarps-th, into four accumulators in
+// turn (loads in flight), combined as (v0 + v1) + (v2 + v3); a fixed shuffle
+// tree per warp, the warps' results in warp order and the CTAs' in theirs.
+// The order depends only on b1 - b0, never on timing, so a batch's case and
+// the same case alone sum identically.  Launch with 7 * kNormWarps warps.
+// One CTA alone is bound by what it can keep in flight (7,776 blocks: 24 us;
+// the cluster takes 13 for 18,432).
+constexpr int kNormWarps = 4, kNormCtas = 8;
 __device__ void sum_partials(const double *partials, int b0, int b1, double *tot) {
   __shared__ double part[7][kNormWarps];
+  const cg::cluster_group cl = cg::this_cluster();
+  const int each = (b1 - b0 + kNormCtas - 1) / kNormCtas;
+  b0 += (int)cl.block_rank() * each;
+  b1 = min(b1, b0 + each);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m = w / kNormWarps, sub = w % kNormWarps;
   constexpr int kStride = 32 * kNormWarps;
@@ -134,26 +144,43 @@ __device__ void sum_partials(const double *partials, int b0, int b1, double *tot
     for (int q = 1; q < kNormWarps; ++q) t += part[threadIdx.x][q];
     tot[threadIdx.x] = t;
   }
-  __syncthreads();
+  cl.sync();
+  if (cl.block_rank() == 0 && threadIdx.x < 7) {
+    double t = tot[threadIdx.x];
+    for (int r = 1; r < kNormCtas; ++r) t += *cl.map_shared_rank(tot + threadIdx.x, r);
+    tot[threadIdx.x] = t;
+  }
+  cl.sync();  // no CTA leaves while its sums are read
 }
 
 // er[1..5] = L2 change norms / (MPI_Ncube n^3), er[6], er[7] = force sums /
-// (0.5 rho0 U0^2 2.602) (BCM_Flux...cpp:2628-2650).
+// (0.5 rho0 U0^2 2.602) (BCM_Flux...cpp:2628-2650); thread m forms the m-th.
+// With emax (the end of a sub-iteration, main.cpp:1249-1259): E_k = max(E_k,
+// er_k); er_k /= E_k.
 __device__ void write_norms(int n, int mpi_ncube, double rho0, double U0, const double *tot,
-                            double *er) {
-  double DN = 1. / (mpi_ncube * n * n * n);
-  er[0] = 0;
-  for (int m = 0; m < 5; ++m) er[1 + m] = sqrt(tot[m]) * DN;
-  er[6] = tot[5] / (0.5 * rho0 * U0 * U0 * 2.602);
-  er[7] = tot[6] / (0.5 * rho0 * U0 * U0 * 2.602);
+                            double *er, double *emax) {
+  const int m = threadIdx.x;
+  if (m == 0) er[0] = 0;
+  if (m < 5) {
+    double DN = 1. / (mpi_ncube * n * n * n);
+    double x = sqrt(tot[m]) * DN;
+    if (emax) {
+      const double E = emax[1 + m] > x ? emax[1 + m] : x;
+      emax[1 + m] = E;
+      x = x / E;
+    }
+    er[1 + m] = x;
+  } else if (m < 7) {
+    er[1 + m] = tot[m] / (0.5 * rho0 * U0 * U0 * 2.602);
+  }
 }
 
 __global__ void k_norms(Phys ph, const double *partials, int nblocks, double *er,
-                        const int *active) {
-  if (active && !active[0]) return;
+                        const int *active, double *emax) {
+  if (active && !active[0]) return;  // the whole cluster
   __shared__ double tot[7];
   sum_partials(partials, 0, nblocks, tot);
-  if (threadIdx.x == 0) write_norms(ph.n, ph.mpi_ncube, ph.rho0, ph.U0, tot, er);
+  if (blockIdx.x == 0) write_norms(ph.n, ph.mpi_ncube, ph.rho0, ph.U0, tot, er, emax);
 }
 
 // Cube-sharded runs: the raw sums of this rank's blocks (the ranks' sums are
@@ -164,24 +191,27 @@ __global__ void k_norm_sums(const double *partials, int nblocks, double *sums,
   if (active && !active[0]) return;
   __shared__ double tot[7];
   sum_partials(partials, 0, nblocks, tot);
-  if (threadIdx.x < 7) sums[threadIdx.x] = tot[threadIdx.x];
+  if (blockIdx.x == 0 && threadIdx.x < 7) sums[threadIdx.x] = tot[threadIdx.x];
 }
 
-__global__ void k_norm_final(Phys ph, const double *sums, double *er, const int *active) {
+__global__ void k_norm_final(Phys ph, const double *sums, double *er, const int *active,
+                             double *emax) {
   if (active && !active[0]) return;
-  write_norms(ph.n, ph.mpi_ncube, ph.rho0, ph.U0, sums, er);
+  write_norms(ph.n, ph.mpi_ncube, ph.rho0, ph.U0, sums, er, emax);
 }
 
-// One CTA per case of a batch.
+// One cluster per case of a batch.
 __global__ void k_norms_batch(int n, const CaseConst *cases, const int *case_blk,
-                              const double *partials, double *er, const int *active) {
+                              const double *partials, double *er, const int *active,
+                              double *emax) {
   __shared__ double tot[7];
-  const int q = blockIdx.x;
+  const int q = blockIdx.x / kNormCtas;
   if (active && !active[q]) return;
   sum_partials(partials, case_blk[q], case_blk[q + 1], tot);
-  if (threadIdx.x == 0) {
+  if (blockIdx.x % kNormCtas == 0) {
     const CaseConst &c = cases[q];
-    write_norms(n, c.mpi_ncube, c.rho0, c.U0, tot, er + 8 * (size_t)q);
+    write_norms(n, c.mpi_ncube, c.rho0, c.U0, tot, er + 8 * (size_t)q,
+                emax ? emax + 6 * (size_t)q : nullptr);
   }
 }
 
@@ -211,30 +241,43 @@ cudaError_t launch_rk(const RkArgs &a, int *nblocks_out, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+template <typename... P, typename... A>
+static cudaError_t launch_sums(void (*k)(P...), int clusters, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(clusters * kNormCtas);
+  cfg.blockDim = dim3(7 * 32 * kNormWarps);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kNormCtas;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
 cudaError_t launch_norms(const Phys &ph, const double *partials, int nblocks, double *er,
-                         cudaStream_t s, const int *active) {
-  k_norms<<<1, 7 * 32 * kNormWarps, 0, s>>>(ph, partials, nblocks, er, active);
-  return cudaGetLastError();
+                         cudaStream_t s, const int *active, double *emax) {
+  return launch_sums(k_norms, 1, s, ph, partials, nblocks, er, active, emax);
 }
 
 cudaError_t launch_norm_sums(const double *partials, int nblocks, double *sums, cudaStream_t s,
                              const int *active) {
-  k_norm_sums<<<1, 7 * 32 * kNormWarps, 0, s>>>(partials, nblocks, sums, active);
-  return cudaGetLastError();
+  return launch_sums(k_norm_sums, 1, s, partials, nblocks, sums, active);
 }
 
 cudaError_t launch_norm_final(const Phys &ph, const double *sums, double *er, cudaStream_t s,
-                              const int *active) {
-  k_norm_final<<<1, 1, 0, s>>>(ph, sums, er, active);
+                              const int *active, double *emax) {
+  k_norm_final<<<1, 32, 0, s>>>(ph, sums, er, active, emax);
   return cudaGetLastError();
 }
 
 cudaError_t launch_norms_batch(int n, const CaseConst *cases, const int *case_blk, int ncase,
                                const double *partials, double *er, cudaStream_t s,
-                               const int *active) {
+                               const int *active, double *emax) {
   if (ncase <= 0) return cudaSuccess;
-  k_norms_batch<<<ncase, 7 * 32 * kNormWarps, 0, s>>>(n, cases, case_blk, partials, er, active);
-  return cudaGetLastError();
+  return launch_sums(k_norms_batch, ncase, s, n, cases, case_blk, partials, er, active, emax);
 }
 
 cudaError_t launch_rk_table(const RkArgs &a, int nblocks, cudaStream_t s) {
