@@ -126,39 +126,66 @@ __global__ void k_store_iters(const int *iters, int *dst, int ncase) {
 
 struct Ibm {
   int nbc = 0;
+  GhostEntry *entries = nullptr;
   double *w = nullptr;
-  int *gc = nullptr, *ip = nullptr, *order = nullptr;
-  std::vector<int> level_off;
+  int *levels = nullptr, *groups = nullptr;
+  std::vector<int> launches;
   void release() {
+    dfree(entries);
     dfree(w);
-    dfree(gc);
-    dfree(ip);
-    dfree(order);
+    dfree(levels);
+    dfree(groups);
     nbc = 0;
-    level_off.clear();
+    launches.clear();
   }
 };
 
-// Upload one IBM table (1-based packed) and its dependency levels.
+// Upload one IBM table (1-based packed), arranged for the ghost fill.
 int ibm_upload(Ibm &t, int nbc, const double *w, const int *gc, const int *ip, int n, int ncube,
                cudaStream_t s) {
   t.release();
   if (nbc <= 0) return BCMG_OK;
-  std::vector<int> order;
+  std::vector<int> order, level_off;
   std::string err;
-  if (!build_ibm_levels(nbc, gc, ip, n, ncube, order, t.level_off, err)) {
+  if (!build_ibm_levels(nbc, gc, ip, n, ncube, order, level_off, err)) {
     set_err(err);
     return BCMG_ERR_ARG;
   }
+  GhostPlan plan;
+  build_ghost_plan(gc, ip, ncube, order, level_off, plan);
+  std::vector<GhostEntry> entries((size_t)nbc);
+  std::vector<double> ws(8 * (size_t)nbc);
+  for (int t0 = 0; t0 < nbc; ++t0) {
+    const size_t e = (size_t)plan.order[t0] - 1;
+    const int *G = gc + 1 + 4 * e, *I = ip + 1 + 4 * e;
+    GhostEntry &x = entries[t0];
+    x.stencil = (unsigned)cell_index(n + 4, I[0], I[1], I[2], I[3]);
+    x.ghost = (unsigned)cell_index(n + 4, G[0], G[1], G[2], G[3]);
+    x.cube = I[0];
+    x.ghost_cube = G[0];
+    // Ghost inside its own stencil (:192-449); like the reference, only the
+    // local indices are compared, not the cube.  The slot in the stencil's
+    // 000,100,010,001,... order (bit patterns 3 and 4 swap).
+    const int d[3] = {G[1] - I[1], G[2] - I[2], G[3] - I[3]};
+    const int b = d[0] + 2 * d[1] + 4 * d[2];
+    bool self = true;
+    for (int a = 0; a < 3; ++a) self &= d[a] == 0 || d[a] == 1;
+    x.self = !self ? 8 : (b == 3 ? 4 : (b == 4 ? 3 : b));
+    std::copy(w + 1 + 8 * e, w + 9 + 8 * e, ws.begin() + 8 * (size_t)t0);
+  }
   t.nbc = nbc;
-  CK(dalloc(&t.w, (size_t)8 * nbc + 1));
-  CK(dalloc(&t.gc, (size_t)4 * nbc + 1));
-  CK(dalloc(&t.ip, (size_t)4 * nbc + 1));
-  CK(dalloc(&t.order, (size_t)nbc));
-  CK(cudaMemcpyAsync(t.w, w, sizeof(double) * (8 * (size_t)nbc + 1), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(t.gc, gc, sizeof(int) * (4 * (size_t)nbc + 1), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(t.ip, ip, sizeof(int) * (4 * (size_t)nbc + 1), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(t.order, order.data(), sizeof(int) * nbc, cudaMemcpyHostToDevice, s));
+  t.launches = plan.launches;
+  CK(dalloc(&t.entries, entries.size()));
+  CK(dalloc(&t.w, ws.size()));
+  CK(dalloc(&t.levels, plan.levels.size()));
+  CK(dalloc(&t.groups, plan.groups.size()));
+  CK(cudaMemcpyAsync(t.entries, entries.data(), sizeof(GhostEntry) * entries.size(),
+                     cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(t.w, ws.data(), sizeof(double) * ws.size(), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(t.levels, plan.levels.data(), sizeof(int) * plan.levels.size(),
+                     cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(t.groups, plan.groups.data(), sizeof(int) * plan.groups.size(),
+                     cudaMemcpyHostToDevice, s));
   CK(cudaStreamSynchronize(s));
   return BCMG_OK;
 }
@@ -166,19 +193,19 @@ int ibm_upload(Ibm &t, int nbc, const double *w, const int *gc, const int *ip, i
 int ibm_run(const Ibm &t, int n, double rho0, double P0, double *U, cudaStream_t s,
             long long *launches, const Batch &bt = Batch(), const Mirror &mir = Mirror(),
             int priority = 0) {
-  for (size_t l = 1; l < t.level_off.size(); ++l) {
+  for (size_t l = 1; l < t.launches.size(); ++l) {
     GhostArgs g;
     g.n = n;
     g.rho0 = rho0;
     g.P0 = P0;
-    g.entries = t.order + t.level_off[l - 1];
-    g.weight = t.w;
-    g.GCindex = t.gc;
-    g.IPsur = t.ip;
+    g.entries = t.entries;
+    g.weights = t.w;
+    g.levels = t.levels;
+    g.groups = t.groups + t.launches[l - 1];
     g.U1_ = U;
     g.bt = bt;
     g.mir = mir;
-    CK(launch_ghost(g, t.level_off[l] - t.level_off[l - 1], s, priority));
+    CK(launch_ghost(g, t.launches[l] - t.launches[l - 1], s, priority));
     if (launches) ++*launches;
   }
   return BCMG_OK;

@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "bcm_common.cuh"
+#include "bcm_fp64_int.cuh"
 #include "bcm_kernels.h"
 
 namespace bcmg {
@@ -466,168 +467,164 @@ cudaError_t launch_layers(const LayerArgs &a, int ncubes, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// IBM ghost cells (BCM_Ghostcell_minus.cpp:72-489; _plus is identical).  One
-// dependency level per launch: within a level no entry reads a cell another
-// entry of the level writes, and the host orders the levels so every read
-// sees exactly the value the reference's serial loop sees.
+// IBM ghost cells (BCM_Ghostcell_minus.cpp:72-489; _plus is identical).  The
+// host orders the entries in dependency levels: within a level no entry reads
+// a cell another entry of the level writes, and every read sees exactly the
+// value the reference's serial loop sees.  A CTA runs the levels of one group
+// of entries, a barrier between them; groups share no cube.  A sphere of
+// 2,792 entries in 32 cubes takes 21 levels, the later ones of some 40
+// entries: launches of a level each took 230 us (under ncu; 21 x 10.9), the
+// group's levels 74.  A stage of a step of that sphere among 400 cubes of 16^3,
+// split: 490 -> 374 us, among 96 cubes in FP64: 1057 -> 952.
 //
-// Eight lanes per entry, one stencil cell each: a cell's primitives take
-// three FP64 divisions, which on this part's narrow FP64 pipe dominate an
-// entry's latency, so the eight cells run side by side; their weighted terms
-// go through shared memory to the group's first lane, which sums them in
-// the reference's order (000,100,010,001,110,101,011,111) and writes the
-// ghost cell.  The levels are short, so the launch is latency-bound and
-// this parallelism is what shortens it.
+// Eight lanes per entry, one stencil cell each, the next entry's indices and
+// weights loaded ahead.  The FP64 pipe (64 cycles an instruction of a warp)
+// bounds a level's chain: the cells' divisions go to the integer pipes, each
+// lane forms its cell's weighted terms, and lanes 0..4 sum one quantity each
+// in the reference's order (000,100,010,001,110,101,011,111) and form one
+// component of the ghost cell each: 34 FP64 instructions in a row.
 // ---------------------------------------------------------------------------
-constexpr int kGhostThreads = 128, kGhostPer = kGhostThreads / 8;  // entries per CTA
+__device__ __noinline__ double ghost_quotient(double x, double y) { return x / y; }
 
-__global__ void __launch_bounds__(kGhostThreads) k_ghost(GhostArgs a, int count) {
-  // per entry and stencil cell: rho, p, u, v, w and the weighted density and
-  // pressure deltas
-  __shared__ double sh[kGhostPer][8][7];
+constexpr int kGhostThreads = 8 * kGhostPer;
+
+__global__ void __launch_bounds__(kGhostThreads) k_ghost(GhostArgs a) {
+  // per entry: the stencil cells' weighted terms, the results; of a ghost
+  // inside its own stencil that cell's density and pressure
+  __shared__ double term[kGhostPer][8][5], val[kGhostPer][5], raw[kGhostPer][2];
   const int g = threadIdx.x >> 3, m = threadIdx.x & 7;
-  const int t = blockIdx.x * kGhostPer + g;
-  const bool live = t < count;
-  const int e = live ? a.entries[t] : 0;
   const int S = a.n + 4;
-  const int b = (e - 1) * 4;
-  int c = 0, i = 0, j = 0, k = 0;
-  bool act = false;
-  if (live) {
-    c = a.IPsur[b + 1]; i = a.IPsur[b + 2]; j = a.IPsur[b + 3]; k = a.IPsur[b + 4];
-    act = case_active(a.bt, c);
-  }
-  double rho0 = a.rho0, P0 = a.P0;
-  if (act && a.bt.cube_case) {  // the case of the stencil's cube
-    const CaseConst &cq = a.bt.cases[a.bt.cube_case[c]];
-    rho0 = cq.rho0;
-    P0 = cq.P0;
-  }
-  if (act) {
-    // cell m of the stencil, order 000,100,010,001,110,101,011,111 (:81-145)
-    const int oi = (m == 1 || m == 4 || m == 5 || m == 7);
-    const int oj = (m == 2 || m == 4 || m == 6 || m == 7);
-    const int ok = (m == 3 || m == 5 || m == 6 || m == 7);
-    const double *q = a.U1_ + 5 * cell_index(S, c, i + oi, j + oj, k + ok);
-    const double rh = q[0];
-    const double Uu = q[1] / rh, Vv = q[2] / rh, Ww = q[3] / rh;
-    const double VV = Uu * Uu + Vv * Vv + Ww * Ww;
-    const double Pp = (q[4] - 0.5 * rh * VV) * (BCMG_K - 1);
-    double *o = sh[g][m];
-    o[0] = rh; o[1] = Pp; o[2] = Uu; o[3] = Vv; o[4] = Ww;
-  }
-  __syncwarp();
-  if (!act) return;
-  const double(*X)[7] = sh[g];
-  const int gc = a.GCindex[b + 1], gi = a.GCindex[b + 2], gj = a.GCindex[b + 3],
-            gk = a.GCindex[b + 4];
-  // Ghost inside its own stencil (:192-449); like the reference, only the
-  // local indices are compared, not the cube.
-  const int s = (gi - i) + 2 * (gj - j) + 4 * (gk - k);
-  const bool self = (gi - i == 0 || gi - i == 1) && (gj - j == 0 || gj - j == 1) &&
-                    (gk - k == 0 || gk - k == 1);
-  // bit pattern (di,dj,dk) -> stencil slot in the 000,100,010,001,...
-  // order (patterns 3 and 4 swap)
-  const int sl = s == 3 ? 4 : (s == 4 ? 3 : s);
-  // Lanes 0..4 form the weighted sums of one quantity each (density, p, u,
-  // v, w), every sum in the reference's term order, into sh[g][q][5] (all
-  // eight terms) and sh[g][q][6] (the seven terms without the ghost's own
-  // slot, for a ghost inside its stencil).  On this part's narrow FP64 pipe
-  // the five chains side by side take a fifth of the issue slots of one lane
-  // forming all five.
-  if (m < 5) {
-    const double *w = a.weight + (size_t)(e - 1) * 8 + 1;
-    double wl[8];
-#pragma unroll
-    for (int l = 0; l < 8; ++l) wl[l] = w[l];
-    const double base = m == 0 ? rho0 : (m == 1 ? P0 : 0.0);
-    auto term = [&](int l) { return m < 2 ? wl[l] * (X[l][m] - base) : wl[l] * X[l][m]; };
-    double acc = term(0);
-#pragma unroll
-    for (int l = 1; l < 8; ++l) acc = acc + term(l);
-    if (m < 2) acc = acc + base;
-    sh[g][m][5] = acc;
-    if (self) {
-      const double wsl = wl[sl];
-      double r;
-      if (m < 2) {
-        if (wsl > 0.9999) {
-          r = X[sl][m];
-        } else {
-          double ar = 0;
-          bool first = true;
-          for (int l = 0; l < 8; ++l) {
-            if (l == sl) continue;
-            const double t = term(l);
-            if (first) { ar = t; first = false; }
-            else { ar = ar + t; }
-          }
-          r = ar / (1 - wsl) + base;
-        }
-      } else {
-        double su = 0;
-        bool first = true;
-        for (int l = 0; l < 8; ++l) {
-          if (l == sl) continue;
-          const double t = term(l);
-          if (first) { su = t; first = false; }
-          else { su = su + t; }
-        }
-        r = su / (2 - wsl);
-      }
-      sh[g][m][6] = r;
+  // cell m of the stencil, order 000,100,010,001,110,101,011,111 (:81-145)
+  const int oi = (m == 1 || m == 4 || m == 5 || m == 7), oj = (m == 2 || m == 4 || m == 6 || m == 7),
+            ok = (m == 3 || m == 5 || m == 6 || m == 7);
+  const unsigned cell = (oi * S + oj) * S + ok;
+  float *const M = mirror_current(a.mir);
+  int l = a.groups[blockIdx.x];
+  const int l1 = a.groups[blockIdx.x + 1];
+  if (l >= l1) return;
+  int e0 = a.levels[l], e1 = a.levels[l + 1], e2 = l + 1 < l1 ? a.levels[l + 2] : e1;
+  GhostEntry nxt;
+  double wn = 0;
+  auto load = [&]() {
+    nxt.cube = 0;  // none
+    if (e0 + g < e1) {
+      nxt = a.entries[e0 + g];
+      wn = a.weights[8 * (size_t)(e0 + g) + m];
+      if (!case_active(a.bt, nxt.cube)) nxt.cube = 0;
     }
-  }
-  __syncwarp();
-  if (m != 0) return;
-  double o[5];
-  if (!self) {
-    const double rho = X[0][5], P = X[1][5], U = X[2][5], V = X[3][5], W = X[4][5];
-    const double VV = U * U + V * V + W * W;
-    o[0] = rho;
-    o[1] = 0.5 * rho * U;
-    o[2] = 0.5 * rho * V;
-    o[3] = 0.5 * rho * W;
-    o[4] = P / (BCMG_K - 1) + 0.5 * rho * 0.25 * VV;
-  } else {
-    const double r2 = X[0][6], p2 = X[1][6], U2 = X[2][6], V2 = X[3][6], W2 = X[4][6];
-    const double VV2 = U2 * U2 + V2 * V2 + W2 * W2;
-    o[0] = r2;
-    o[1] = r2 * U2;
-    o[2] = r2 * V2;
-    o[3] = r2 * W2;
-    o[4] = p2 / (BCMG_K - 1) + 0.5 * r2 * VV2;
-  }
-  const size_t go = 5 * cell_index(S, gc, gi, gj, gk);
-  double *gp = a.U1_ + go;
+  };
+  load();
+  for (bool more = true; more;) {
+    const GhostEntry e = nxt;
+    const double w = wn;
+    bool level_ends = false;
+    e0 += kGhostPer;
+    if (e0 >= e1) {
+      level_ends = true;
+      more = ++l < l1;
+      e0 = e1;
+      e1 = e2;
+      if (l + 1 < l1) e2 = a.levels[l + 2];  // in time for the level after this
+    }
+    if (more) load();
+    const bool act = e.cube != 0, self = e.self < 8;
+    double rho0 = a.rho0, P0 = a.P0, ws = 0;
+    IntFp os;
+    Recip ks = {};
+    if (act) {
+      if (a.bt.cube_case) {  // the case of the stencil's cube
+        const CaseConst &cq = a.bt.cases[a.bt.cube_case[e.cube]];
+        rho0 = cq.rho0;
+        P0 = cq.P0;
+      }
+      const double *q = a.U1_ + 5 * (size_t)(e.stencil + cell);
+      const double rh = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4];
+      // (while the loads are on their way) the divisor of a ghost in its stencil
+      if (self) {
+        ws = __shfl_sync(0xffu << (threadIdx.x & 24), w, (threadIdx.x & 24) + e.self);
+        ks = os.recip((m < 2 ? 1. : 2.) - ws);
+      }
+      IntFp o;
+      const Recip k = o.recip(rh);
+      double Uu = o.div(q1, k), Vv = o.div(q2, k), Ww = o.div(q3, k);
+      if (!o.ok) {
+        Uu = ghost_quotient(q1, rh);
+        Vv = ghost_quotient(q2, rh);
+        Ww = ghost_quotient(q3, rh);
+      }
+      const double VV = Uu * Uu + Vv * Vv + Ww * Ww;
+      const double Pp = (q4 - 0.5 * rh * VV) * (BCMG_K - 1);
+      double *t = term[g][m];
+      t[0] = w * (rh - rho0);
+      t[1] = w * (Pp - P0);
+      t[2] = w * Uu;
+      t[3] = w * Vv;
+      t[4] = w * Ww;
+      if (m == e.self) {
+        double *r = raw[g];
+        r[0] = rh; r[1] = Pp;
+      }
+    }
+    __syncwarp();
+    if (act && m < 5) {
+      const double base = m == 0 ? rho0 : P0;
+      double acc = -0.0;  // -0 + t is t
 #pragma unroll
-  for (int v = 0; v < 5; ++v) gp[v] = o[v];
-  if (float *M = mirror_current(a.mir)) {
-    double r0, e0;
-    mirror_base(a.mir, a.bt, gc, r0, e0);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) M[go + v] = mirror_value_hw(o[v], v, r0, e0);
+      for (int c = 0; c < 8; ++c)
+        if (c != e.self) acc = acc + term[g][c][m];
+      if (self) {
+        if (m < 2 && ws > 0.9999) {
+          acc = raw[g][m];
+        } else {
+          const double q = os.div(acc, ks);
+          acc = os.ok ? q : ghost_quotient(acc, (m < 2 ? 1. : 2.) - ws);
+          if (m < 2) acc = acc + base;
+        }
+      } else if (m < 2) {
+        acc = acc + base;
+      }
+      val[g][m] = acc;
+    }
+    __syncwarp();
+    if (act && m < 5) {
+      const double rho = val[g][0], hr = 0.5 * rho;
+      double o;
+      if (m == 0) {
+        o = rho;
+      } else if (m < 4) {
+        o = (self ? rho : hr) * val[g][m + 1];
+      } else {
+        const double P = val[g][1], U = val[g][2], V = val[g][3], W = val[g][4];
+        const double VV = U * U + V * V + W * W;
+        IntFp op;
+        double p = op.div(P, RecipConst<__builtin_bit_cast(uint64_t, (double)(BCMG_K - 1))>::get());
+        if (!op.ok) p = ghost_quotient(P, BCMG_K - 1);
+        o = p + (self ? hr : hr * 0.25) * VV;
+      }
+      const size_t go = 5 * (size_t)e.ghost + m;
+      a.U1_[go] = o;
+      if (M) {
+        double r0, e0_;
+        mirror_base(a.mir, a.bt, e.ghost_cube, r0, e0_);
+        M[go] = mirror_value_hw(o, m, r0, e0_);
+      }
+    }
+    if (level_ends && more) __syncthreads(); else __syncwarp();
   }
 }
 
-cudaError_t launch_ghost(const GhostArgs &a, int count, cudaStream_t s, int priority) {
-  if (count <= 0) return cudaSuccess;
-  const unsigned grid = (count + kGhostPer - 1) / kGhostPer;
-  if (priority == 0) {
-    k_ghost<<<grid, kGhostThreads, 0, s>>>(a, count);
-    return cudaGetLastError();
-  }
+cudaError_t launch_ghost(const GhostArgs &a, int groups, cudaStream_t s, int priority) {
+  if (groups <= 0) return cudaSuccess;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = dim3(groups);
   cfg.blockDim = dim3(kGhostThreads);
-  cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributePriority;
   at[0].val.priority = priority;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_ghost, a, count);
+  cfg.numAttrs = priority != 0;
+  return cudaLaunchKernelEx(&cfg, k_ghost, a);
 }
 
 }  // namespace bcmg

@@ -275,21 +275,29 @@ cudaError_t launch_halo(double *U, const Mirror &mir, const int *bands, const lo
                         int nband, long long total_cells, int n, void *buf, int unpack,
                         cudaStream_t s);
 
-// IBM ghost-cell fill for one dependency level of the combined entry list.
+// IBM ghost-cell fill.  The entries stand in the order of groups, in a group
+// in that of its dependency levels: group b has levels groups[b] ..
+// groups[b+1], level l the entries levels[l] .. levels[l+1].  Groups of one
+// launch write and read no common cell (but what all only read).
+struct GhostEntry {
+  unsigned stencil, ghost;  // first stencil cell, ghost cell (flat)
+  int cube, ghost_cube;
+  int self;  // the stencil cell that is the ghost itself (local indices), 8: none
+};
+constexpr int kGhostPer = 32;  // entries a CTA works on at a time
 struct GhostArgs {
   int n;
   double rho0, P0;
-  const int *entries;      // entry numbers (1-based) of this level
-  const double *weight;    // 1-based packed [8*nbc+1]
-  const int *GCindex;      // 1-based packed [4*nbc+1]
-  const int *IPsur;        // 1-based packed [4*nbc+1]
+  const GhostEntry *entries;
+  const double *weights;  // 8 per entry, stencil order 000,100,010,001,110,...
+  const int *levels, *groups;
   double *U1_;
-  Batch bt;  // batches: rho0, P0 of the ghost cell's case
+  Batch bt;  // batches: rho0, P0 of the stencil cube's case
   Mirror mir;  // split precision: the ghost cell's mirror value too
 };
 // priority != 0: launched with that scheduling priority (a launch
 // attribute, kept by stream capture), so its blocks go ahead of pending
 // blocks of lower-priority kernels running beside it
-cudaError_t launch_ghost(const GhostArgs &a, int count, cudaStream_t s, int priority = 0);
+cudaError_t launch_ghost(const GhostArgs &a, int groups, cudaStream_t s, int priority = 0);
 
 }  // namespace bcmg

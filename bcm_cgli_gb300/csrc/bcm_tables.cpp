@@ -275,6 +275,73 @@ bool build_ibm_levels(int nbc, const int *GC, const int *IP, int n, int ncube,
   return true;
 }
 
+// Entries whose cubes (ghost or stencil) are linked form a component; entries
+// of different components touch no common cell.  One launch runs a component
+// per CTA, all its levels in turn.  Where a component takes many passes
+// of kGhostPer entries (few CTAs for many entries, such as a table that links
+// all cubes), a launch per level spreads the level over CTAs instead: a pass
+// takes about 2 us, a launch of a level about 5.
+void build_ghost_plan(const int *GC, const int *IP, int ncube, const std::vector<int> &order,
+                      const std::vector<int> &level_off, GhostPlan &plan) {
+  std::vector<int> root((size_t)ncube);
+  for (int c = 0; c < ncube; ++c) root[c] = c;
+  auto find = [&](int c) {
+    while (root[c] != c) c = root[c] = root[root[c]];
+    return c;
+  };
+  auto gcube = [&](int e) { return GC[4 * (e - 1) + 1]; };
+  for (int e : order) root[find(gcube(e))] = find(IP[4 * (e - 1) + 1]);
+  const int nlev = (int)level_off.size() - 1;
+  // entries of each component, level by level
+  std::vector<std::vector<int>> entries, bounds;
+  std::vector<int> comp((size_t)ncube, -1);
+  for (int l = 1; l <= nlev; ++l) {
+    for (int t = level_off[l - 1]; t < level_off[l]; ++t) {
+      int &q = comp[find(gcube(order[t]))];
+      if (q < 0) {
+        q = (int)entries.size();
+        entries.emplace_back();
+        bounds.emplace_back();
+      }
+      entries[q].push_back(order[t]);
+    }
+    for (size_t q = 0; q < entries.size(); ++q)
+      if ((int)entries[q].size() > (bounds[q].empty() ? 0 : bounds[q].back()))
+        bounds[q].push_back((int)entries[q].size());
+  }
+  int passes = 0;
+  for (const auto &b : bounds) {
+    int sum = 0, from = 0;
+    for (int to : b) {
+      sum += (to - from + kGhostPer - 1) / kGhostPer;
+      from = to;
+    }
+    passes = std::max(passes, sum);
+  }
+  plan = GhostPlan();
+  plan.levels.push_back(0);
+  plan.groups.push_back(0);
+  plan.launches.push_back(0);
+  if (2 * passes <= 5 * nlev) {
+    for (size_t q = 0; q < entries.size(); ++q) {
+      const int base = (int)plan.order.size();
+      plan.order.insert(plan.order.end(), entries[q].begin(), entries[q].end());
+      for (int to : bounds[q]) plan.levels.push_back(base + to);
+      plan.groups.push_back((int)plan.levels.size() - 1);
+    }
+    plan.launches.push_back((int)plan.groups.size() - 1);
+    return;
+  }
+  plan.order = order;
+  for (int l = 1; l <= nlev; ++l) {
+    for (int t = level_off[l - 1]; t < level_off[l]; t += kGhostPer) {
+      plan.levels.push_back(std::min(t + kGhostPer, level_off[l]));
+      plan.groups.push_back((int)plan.levels.size() - 1);
+    }
+    plan.launches.push_back((int)plan.groups.size() - 1);
+  }
+}
+
 void prologue_task_mask(int n, int ncube, const std::vector<FaceTask> &tasks,
                         const std::vector<int> &task_cube, const std::vector<int> &bc_cubes,
                         const std::vector<int> &bc_masks, const int *gc_minus, int nminus,

@@ -20,6 +20,14 @@ bool build_bc_entries(int ncube, const int *const lists[6], const int counts[6],
                       std::vector<int> &cubes, std::vector<int> &masks, std::string &err);
 bool build_ibm_levels(int nbc, const int *GC, const int *IP, int n, int ncube,
                       std::vector<int> &order, std::vector<int> &level_off, std::string &err);
+// The levels arranged for k_ghost: entry numbers in the order of the table, the
+// levels and groups of GhostArgs, and the groups of each launch (launches[q] ..
+// launches[q+1]).
+struct GhostPlan {
+  std::vector<int> order, levels, groups, launches;
+};
+void build_ghost_plan(const int *GC, const int *IP, int ncube, const std::vector<int> &order,
+                      const std::vector<int> &level_off, GhostPlan &plan);
 // Which face tasks the interface call ahead of a stage must repeat right
 // after the previous stage's closing call: keep[t] = 1 for level-jump tasks,
 // for faces the boundary fill writes (bc cubes/masks as build_bc_entries
