@@ -17,15 +17,19 @@
 //  * the side test of a cell uses the dotp of the last hit cell at or before
 //    it in the reference's (cube, i, j, k) order, because the reference never
 //    resets it; that carry is a short sequential pass on the host;
-//  * k_ibm_weights: one thread per ghost cell forms the boundary and image
-//    points, the distance test, the image point's base cell, the inverse of
-//    the 8x8 Vandermonde matrix (Gauss-Jordan with partial pivoting) and the
-//    eight weights (:759-1040).
+//  * both searches leave out the pairs that an FP32 filter with a rigorous
+//    margin shows to miss, so the FP64 tests, and with them every result, are
+//    those of the full search;
+//  * k_ibm_place: one thread per ghost cell forms the boundary and image
+//    points, the distance test and the image point's base cell;
+//    k_ibm_weights: 16 lanes per cell the inverse of the 8x8 Vandermonde matrix
+//    (Gauss-Jordan with partial pivoting) and the eight weights (:759-1040).
 // Every step keeps the reference's operation order and the translation unit
 // is built with --fmad=false, so the tables equal the reference's.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -58,31 +62,48 @@ __global__ void k_ibm_cube_box(int ncube, int n, const double *__restrict__ cube
   b[4] = Z[c] - 1.5 * dx; b[5] = Z[c] + cube_size[c] + 1.5 * dx;
 }
 
+// The order of the doubles as integers (NaN excluded, -0 as 0): comparisons
+// on the integer pipes instead of 64 cycles a warp each on the FP64 pipe.
+__device__ __forceinline__ long long sort_key(double x) {
+  const long long b = __double_as_longlong(x == 0.0 ? 0.0 : x);
+  return b < 0 ? b ^ 0x7fffffffffffffffll : b;
+}
+
 // keep[t] = 1 when a vertex of triangle t lies in some cube's widened box
 // (cubes 1..ncube-1, staged through shared memory).
-constexpr int kBoxChunk = 512;
-__global__ void __launch_bounds__(256) k_ibm_keep(int ntri, const double *__restrict__ tri,
-                                                  int ncube, const double *__restrict__ box,
-                                                  int *__restrict__ keep) {
-  __shared__ double sb[kBoxChunk * 6];
+constexpr int kBoxChunk = 512, kKeepThreads = 128;
+__global__ void __launch_bounds__(kKeepThreads) k_ibm_keep(int ntri,
+                                                           const double *__restrict__ tri,
+                                                           int ncube,
+                                                           const double *__restrict__ box,
+                                                           int *__restrict__ keep) {
+  __shared__ long long sb[kBoxChunk * 6];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  double v[9];
-  for (int e = 0; e < 9; ++e) v[e] = t < ntri ? tri[9 * (size_t)t + e] : 0.0;
+  long long v[9];
+  bool num[3] = {true, true, true};
+  for (int e = 0; e < 9; ++e) {
+    const double x = t < ntri ? tri[9 * (size_t)t + e] : 0.0;
+    v[e] = sort_key(x);
+    num[e / 3] &= x == x;
+  }
   int k = 0;
   for (int c0 = 1; c0 < ncube; c0 += kBoxChunk) {
     const int cnt = min(kBoxChunk, ncube - c0);
     __syncthreads();
-    for (int e = threadIdx.x; e < cnt * 6; e += blockDim.x) sb[e] = box[6 * (size_t)c0 + e];
+    for (int e = threadIdx.x; e < cnt * 6; e += blockDim.x) {
+      const double x = box[6 * (size_t)c0 + e];
+      // no number lies above a NaN lower or below a NaN upper bound
+      sb[e] = x == x ? sort_key(x) : (e & 1 ? LLONG_MIN : LLONG_MAX);
+    }
     __syncthreads();
     if (k || t >= ntri) continue;
     for (int c = 0; c < cnt && !k; ++c) {
-      const double *b = sb + 6 * c;
+      const long long *b = sb + 6 * c;
+#pragma unroll
       for (int q = 0; q < 3; ++q)
-        if (v[3 * q] >= b[0] && v[3 * q] <= b[1] && v[3 * q + 1] >= b[2] &&
-            v[3 * q + 1] <= b[3] && v[3 * q + 2] >= b[4] && v[3 * q + 2] <= b[5]) {
+        if (num[q] && v[3 * q] >= b[0] && v[3 * q] <= b[1] && v[3 * q + 1] >= b[2] &&
+            v[3 * q + 1] <= b[3] && v[3 * q + 2] >= b[4] && v[3 * q + 2] <= b[5])
           k = 1;
-          break;
-        }
     }
   }
   if (t < ntri) keep[t] = k;
@@ -90,7 +111,7 @@ __global__ void __launch_bounds__(256) k_ibm_keep(int ntri, const double *__rest
 
 // Closest point of a triangle (:1290-1405), with the interior weight formed
 // as the reference forms it.
-__device__ __forceinline__ void closest(const double *v, double x, double y, double z,
+__device__ __noinline__ void closest(const double *v, double x, double y, double z,
                                         double *p) {
   const double *a = v, *b = v + 3, *c = v + 6;
   const double ab[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
@@ -138,9 +159,23 @@ __device__ __forceinline__ void closest(const double *v, double x, double y, dou
 // reference recomputes for every ghost cell): v0, e1 = v1 - v0, e2 = v2 - v0,
 // the normal nu = e1 x e2, dir = -nu / |nu|, p = dir x e2, det = e1 . p,
 // 1 / det and dir . dir.
+//
+// And an FP32 filter: the search tests every ghost cell against every
+// triangle, and nearly all pairs miss by far.  In coordinates o' = o - org
+// relative to the ghost cells' box (centre org, half extents ext), f[0] and
+// f[1] give u / det and w / det of the ray test as affine functions, each
+// raised by a bound m on the error of evaluating it in FP32 (at most 8 roundings
+// of 2^-24 of A = |p|.ext + |c| + 1; m = 2^-18 A also covers the FP64 test's own
+// rounding) and scaled so that a hit has f0 >= 0, f1 >= 0 and f0 + f1 <= 1
+// for certain.  f[2] is a sphere around the triangle (centre, radius widened
+// in the same way).  Where m is not small (thin or far triangles, NaN), every
+// pair passes.
 constexpr int kRec = 22;
-__global__ void k_ibm_tri_prep(int ntri, const double *__restrict__ tri,
-                               double *__restrict__ rec) {
+struct GhostBox {
+  double org[3], ext[3];
+};
+__global__ void k_ibm_tri_prep(int ntri, const double *__restrict__ tri, GhostBox gb,
+                               double *__restrict__ rec, float4 *__restrict__ filter) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ntri) return;
   const double *v = tri + 9 * (size_t)t;
@@ -166,12 +201,50 @@ __global__ void k_ibm_tri_prep(int ntri, const double *__restrict__ tri,
   r[19] = 1.0 / det;
   r[20] = dir[0] * dir[0] + dir[1] * dir[1] + dir[2] * dir[2];
   r[21] = 0.0;
+  const double ed[3] = {e1[1] * dir[2] - e1[2] * dir[1], e1[2] * dir[0] - e1[0] * dir[2],
+                        e1[0] * dir[1] - e1[1] * dir[0]};
+  double cu = 0, cw = 0, au = 1, aw = 1, ctr[3], far = 0, reach = 0;
+  for (int q = 0; q < 3; ++q) {
+    cu += (gb.org[q] - v[q]) * pp[q] / det;
+    cw += (gb.org[q] - v[q]) * ed[q] / det;
+    au += fabs(pp[q] / det) * gb.ext[q];
+    aw += fabs(ed[q] / det) * gb.ext[q];
+    ctr[q] = (v[q] + v[3 + q] + v[6 + q]) / 3.0;
+    reach += gb.ext[q] + fabs(ctr[q] - gb.org[q]);
+  }
+  const double m = ldexp(fmax(au + fabs(cu), aw + fabs(cw)), -18), sc = 1.0 / (1.0 + 3.0 * m);
+  // (a NaN in a term fails the comparison or shows in the sum)
+  const bool use = m < 0.25 && au + aw + cu + cw < 1e30;
+  float4 *f = filter + 3 * (size_t)t;
+  f[0] = f[1] = make_float4(0.f, 0.f, 0.f, 0.25f);
+  if (use) {
+    const double ku = sc / det;
+    f[0] = make_float4((float)(pp[0] * ku), (float)(pp[1] * ku), (float)(pp[2] * ku),
+                       (float)((cu + m) * sc));
+    f[1] = make_float4((float)(ed[0] * ku), (float)(ed[1] * ku), (float)(ed[2] * ku),
+                       (float)((cw + m) * sc));
+  }
+  for (int e = 0; e < 3; ++e) {
+    double d2 = 0;
+    for (int q = 0; q < 3; ++q) d2 += (v[3 * e + q] - ctr[q]) * (v[3 * e + q] - ctr[q]);
+    far = d2 > far || !(d2 == d2) ? d2 : far;
+  }
+  f[2] = make_float4((float)(ctr[0] - gb.org[0]), (float)(ctr[1] - gb.org[1]),
+                     (float)(ctr[2] - gb.org[2]),
+                     (float)(sqrt(far) * (1 + 1e-6) + ldexp(reach, -20)));
+}
+
+// False where the pair surely misses: o' outside the triangle's prism.
+__device__ __forceinline__ bool may_hit(const float *o, float4 a, float4 b) {
+  const float u = __fmaf_rn(o[0], a.x, __fmaf_rn(o[1], a.y, __fmaf_rn(o[2], a.z, a.w)));
+  const float w = __fmaf_rn(o[0], b.x, __fmaf_rn(o[1], b.y, __fmaf_rn(o[2], b.z, b.w)));
+  return !(fminf(fminf(u, w), 1.0f - u - w) < 0.f);
 }
 
 // Ray test of ghost centre o against triangle record r (Moller-Trumbore,
 // :1409-1450: det below 1e-7 rejected, both directions accepted); on a hit
 // returns 1 with tt = t.
-__device__ __forceinline__ int ray_hit(const double *o, const double *r, double *tt) {
+__device__ __noinline__ int ray_hit(const double *o, const double *r, double *tt) {
   if (r[18] < kMinimum) return 0;
   const double tv[3] = {o[0] - r[0], o[1] - r[1], o[2] - r[2]};
   const double u = tv[0] * r[12] + tv[1] * r[13] + tv[2] * r[14];
@@ -190,30 +263,40 @@ __device__ __forceinline__ int ray_hit(const double *o, const double *r, double 
 // smallest |t| (dir . dir), the reference's strict `<` over its serial loop.
 // Cells are a list (cell < 0: skipped) so the closest-point pass below can
 // reuse the layout.
+// The FP32 filter leaves one or two triangles a cell for the FP64 test: 5,984
+// cells by 20,480 triangles took 1,996 us with the FP64 test on every pair (its
+// first dot product alone takes six slots of 64 cycles a warp), 57 with the
+// filter.
 constexpr int kGhostBlock = 128;
 __global__ void __launch_bounds__(kGhostBlock)
-    k_ibm_ray_part(int ng, const double *__restrict__ cen, int ntri, int per,
-                   const double *__restrict__ rec, int *__restrict__ hits_p,
-                   int *__restrict__ best_p, double *__restrict__ nd_p) {
-  __shared__ double st[kTriChunk * kRec];
+    k_ibm_ray_part(int ng, const double *__restrict__ cen, GhostBox gb, int ntri, int per,
+                   const double *__restrict__ rec, const float4 *__restrict__ filter,
+                   int *__restrict__ hits_p, int *__restrict__ best_p,
+                   double *__restrict__ nd_p) {
+  __shared__ float4 sf[kTriChunk][2];
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const bool has = g < ng;
   double o[3] = {0, 0, 0};
   if (has) { o[0] = cen[3 * g]; o[1] = cen[3 * g + 1]; o[2] = cen[3 * g + 2]; }
+  float of[3];
+  for (int q = 0; q < 3; ++q) of[q] = (float)(o[q] - gb.org[q]);
   const int t0 = blockIdx.y * per, t1 = min(ntri, t0 + per);
   int hits = 0, best = -1;
   double dmin = kBig;
   for (int base = t0; base < t1; base += kTriChunk) {
     const int cnt = min(kTriChunk, t1 - base);
     __syncthreads();
-    for (int e = threadIdx.x; e < cnt * kRec; e += blockDim.x)
-      st[e] = rec[kRec * (size_t)base + e];
+    for (int e = threadIdx.x; e < cnt * 2; e += blockDim.x)
+      sf[e >> 1][e & 1] = filter[3 * ((size_t)base + (e >> 1)) + (e & 1)];
     __syncthreads();
     if (!has) continue;
+#pragma unroll 4
     for (int t = 0; t < cnt; ++t) {
+      if (!may_hit(of, sf[t][0], sf[t][1])) continue;
+      const double *r = rec + kRec * ((size_t)base + t);
       double tt;
-      if (!ray_hit(o, st + kRec * t, &tt)) continue;
-      const double nd = fabs(tt) * st[kRec * t + 20];
+      if (!ray_hit(o, r, &tt)) continue;
+      const double nd = fabs(tt) * r[20];
       ++hits;
       if (nd < dmin) { dmin = nd; best = base + t; }
     }
@@ -229,19 +312,32 @@ __global__ void __launch_bounds__(kGhostBlock)
 // lowest triangle on ties) |t|, direction and dotp = nu . (v0 - centre),
 // recomputed from that triangle with the same arithmetic.  out[g*8 + 0..5] =
 // hits, |t|, d0, d1, d2, dotp.
+// One warp per cell: its lanes take the ranges in turn.
 __global__ void k_ibm_ray_combine(int ng, int nsplit, const double *__restrict__ cen,
                                   const double *__restrict__ rec,
                                   const int *__restrict__ hits_p, const int *__restrict__ best_p,
                                   const double *__restrict__ nd_p, double *__restrict__ out) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (g >= ng) return;
-  int hits = 0, best = -1;
+  int hits = 0, best = INT_MAX;
   double dmin = kBig;
-  for (int sp = 0; sp < nsplit; ++sp) {
+  for (int sp = lane; sp < nsplit; sp += 32) {
     const size_t at = (size_t)sp * ng + g;
     hits += hits_p[at];
-    if (best_p[at] >= 0 && nd_p[at] < dmin) { dmin = nd_p[at]; best = best_p[at]; }
+    const int b = best_p[at];
+    if (b >= 0 && nd_p[at] < dmin) { dmin = nd_p[at]; best = b; }
   }
+  for (int d = 16; d > 0; d >>= 1) {
+    hits += __shfl_xor_sync(0xffffffffu, hits, d);
+    const double nd = __shfl_xor_sync(0xffffffffu, dmin, d);
+    const int b = __shfl_xor_sync(0xffffffffu, best, d);
+    if (b != INT_MAX && (best == INT_MAX || nd < dmin || (nd == dmin && b < best))) {
+      dmin = nd;
+      best = b;
+    }
+  }
+  if (lane) return;
+  if (best == INT_MAX) best = -1;
   double tmin = kBig, d0 = 0, d1 = 0, d2 = 0, dotp = 0;
   if (best >= 0) {
     const double o[3] = {cen[3 * g], cen[3 * g + 1], cen[3 * g + 2]};
@@ -259,12 +355,17 @@ __global__ void k_ibm_ray_combine(int ng, int nsplit, const double *__restrict__
 // Closest-point search for the ghost cells without any hit (list[m] ghost
 // numbers), split like the ray search: per (range, cell) the LAST triangle
 // with the smallest squared distance (the reference's `<=`).
-constexpr int kRawChunk = kTriChunk * kRec / 9;
+// The closest point lies in the triangle, so a triangle whose sphere is
+// farther than the best so far is left out, unless the cell may lie in the
+// triangle's prism: there the interior weight (as the reference forms it) puts
+// the point anywhere.  5,874 cells: 455 us with every pair in FP64, 193 with each
+// range's own best, 65 with a first pass for an upper bound.
 __global__ void __launch_bounds__(kGhostBlock)
     k_ibm_closest_part(int m, const int *__restrict__ list, const double *__restrict__ cen,
-                       int ntri, int per, const double *__restrict__ tri,
+                       GhostBox gb, int ntri, int per, const double *__restrict__ tri,
+                       const float4 *__restrict__ filter, unsigned *__restrict__ bound,
                        int *__restrict__ best_p, double *__restrict__ nd_p) {
-  __shared__ double sv[kRawChunk * 9];
+  __shared__ float4 sf[kTriChunk][3];
   const int e0 = blockIdx.x * blockDim.x + threadIdx.x;
   const bool has = e0 < m;
   double o[3] = {0, 0, 0};
@@ -272,21 +373,49 @@ __global__ void __launch_bounds__(kGhostBlock)
     const int g = list[e0];
     o[0] = cen[3 * g]; o[1] = cen[3 * g + 1]; o[2] = cen[3 * g + 2];
   }
+  float of[3];
+  for (int q = 0; q < 3; ++q) of[q] = (float)(o[q] - gb.org[q]);
   const int t0 = blockIdx.y * per, t1 = min(ntri, t0 + per);
   int best = -1;
   double dmin = kBig;
-  for (int base = t0; base < t1; base += kRawChunk) {
-    const int cnt = min(kRawChunk, t1 - base);
-    __syncthreads();
-    for (int e = threadIdx.x; e < cnt * 9; e += blockDim.x) sv[e] = tri[9 * (size_t)base + e];
-    __syncthreads();
-    if (!has) continue;
-    for (int t = 0; t < cnt; ++t) {
-      double p[3];
-      closest(sv + 9 * t, o[0], o[1], o[2], p);
-      const double nd = (p[0] - o[0]) * (p[0] - o[0]) + (p[1] - o[1]) * (p[1] - o[1]) +
-                        (p[2] - o[2]) * (p[2] - o[2]);
-      if (nd <= dmin) { dmin = nd; best = base + t; }
+  float rmin = 1e4f * (1 + 1e-6f);  // no less than the closest point's distance
+  // first pass: the smallest upper bound of the range, shared by all ranges
+  // (whichever of them a range sees, it leaves out only triangles that are
+  // farther than some other's point)
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int base = t0; base < t1; base += kTriChunk) {
+      const int cnt = min(kTriChunk, t1 - base);
+      __syncthreads();
+      for (int e = threadIdx.x; e < cnt * 3; e += blockDim.x)
+        sf[e / 3][e % 3] = filter[3 * (size_t)base + e];
+      __syncthreads();
+      if (!has) continue;
+      for (int t = 0; t < cnt; ++t) {
+        const float4 c = sf[t][2];
+        const float x = of[0] - c.x, y = of[1] - c.y, z = of[2] - c.z;
+        const float d2 = __fmaf_rn(x, x, __fmaf_rn(y, y, z * z));
+        if (pass == 0) {
+          const float far = sqrtf(d2) * (1 + 1e-6f) + c.w;
+          if (far < rmin && !may_hit(of, sf[t][0], sf[t][1])) rmin = far;
+          continue;
+        }
+        const float r = c.w + rmin;
+        if (d2 > r * r * (1 + 1e-6f) && !may_hit(of, sf[t][0], sf[t][1])) continue;
+        double p[3];
+        closest(tri + 9 * ((size_t)base + t), o[0], o[1], o[2], p);
+        const double nd = (p[0] - o[0]) * (p[0] - o[0]) + (p[1] - o[1]) * (p[1] - o[1]) +
+                          (p[2] - o[2]) * (p[2] - o[2]);
+        if (nd <= dmin) {
+          dmin = nd;
+          best = base + t;
+          rmin = fminf(rmin, sqrtf((float)nd) * (1 + 1e-6f) + 1e-18f);
+        }
+      }
+    }
+    if (pass == 0 && has) {
+      const unsigned mine = __float_as_uint(rmin);  // positive: ordered as integers
+      rmin = __uint_as_float(min(mine, atomicMin(bound + e0, mine)));
     }
   }
   if (!has) return;
@@ -296,20 +425,31 @@ __global__ void __launch_bounds__(kGhostBlock)
 }
 
 // The closest point of those cells (the highest triangle on ties) into
-// out[g*8 + 2..4]; 0 when no triangle is within the search distance.
+// out[g*8 + 2..4]; 0 when no triangle is within the search distance.  One warp
+// per cell.
 __global__ void k_ibm_closest_combine(int m, int nsplit, const int *__restrict__ list,
                                       const double *__restrict__ cen,
                                       const double *__restrict__ tri,
                                       const int *__restrict__ best_p,
                                       const double *__restrict__ nd_p, double *__restrict__ out) {
-  const int e0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int e0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (e0 >= m) return;
   int best = -1;
   double dmin = kBig;
-  for (int sp = 0; sp < nsplit; ++sp) {
+  for (int sp = lane; sp < nsplit; sp += 32) {
     const size_t at = (size_t)sp * m + e0;
-    if (best_p[at] >= 0 && nd_p[at] <= dmin) { dmin = nd_p[at]; best = best_p[at]; }
+    const int b = best_p[at];
+    if (b >= 0 && nd_p[at] <= dmin) { dmin = nd_p[at]; best = b; }
   }
+  for (int d = 16; d > 0; d >>= 1) {
+    const double nd = __shfl_xor_sync(0xffffffffu, dmin, d);
+    const int b = __shfl_xor_sync(0xffffffffu, best, d);
+    if (b >= 0 && (best < 0 || nd < dmin || (nd == dmin && b > best))) {
+      dmin = nd;
+      best = b;
+    }
+  }
+  if (lane) return;
   const int g = list[e0];
   double p[3] = {0, 0, 0};
   if (best >= 0) closest(tri + 9 * (size_t)best, cen[3 * g], cen[3 * g + 1], cen[3 * g + 2], p);
@@ -328,49 +468,48 @@ int ibm_splits(int nblocks, int ntri) {
   return std::max(1, std::min(want, most));
 }
 
-// In-place inverse of the 8x8 row-major matrix m (:1504-1576).
-__device__ void invert8(double *m) {
-  double a[8][8], b[8][8];
-  for (int j = 0; j < 8; ++j)
-    for (int i = 0; i < 8; ++i) {
-      a[j][i] = m[i + 8 * j];
-      b[j][i] = i == j ? 1.0 : 0.0;
-    }
+__device__ __noinline__ double plain_quotient(double x, double y) { return x / y; }
+
+// The inverse of an 8x8 matrix (:1504-1576) by 16 lanes: lane l < 8 brings
+// column l of the matrix in a, lane 8 + l the unit matrix's and ends with
+// column l of the inverse.  The reference's Gauss-Jordan steps with row pivots
+// treat columns alike, so each lane keeps one, and lane k shows its own (pivot
+// row, pivot, factors) to the others at step k.
+__device__ __forceinline__ void invert8(double *a, unsigned group, int lane0) {
+#pragma unroll
   for (int k = 0; k < 8; ++k) {
+    double col[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) col[j] = __shfl_sync(group, a[j], lane0 + k);
     int mx = k;
+    double big = fabs(col[k]);
+#pragma unroll
     for (int j = k + 1; j < 8; ++j)
-      if (fabs(a[j][k]) > fabs(a[mx][k])) mx = j;
-    if (mx != k)
-      for (int i = 0; i < 8; ++i) {
-        double t = a[mx][i]; a[mx][i] = a[k][i]; a[k][i] = t;
-        t = b[mx][i]; b[mx][i] = b[k][i]; b[k][i] = t;
+      if (fabs(col[j]) > big) { mx = j; big = fabs(col[j]); }
+#pragma unroll
+    for (int j = k + 1; j < 8; ++j)
+      if (mx == j) {  // swap rows k and mx
+        double t = a[j]; a[j] = a[k]; a[k] = t;
+        t = col[j]; col[j] = col[k]; col[k] = t;
       }
-    const double t = a[k][k];
-    for (int i = 0; i < 8; ++i) { a[k][i] /= t; b[k][i] /= t; }
+    const double t = col[k];
+    a[k] = plain_quotient(a[k], t);
+    const double one = t == t && t != 0 && fabs(t) < INFINITY ? 1.0 : plain_quotient(t, t);
+#pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (j != k) {
-        const double f = a[j][k] / a[k][k];
-        for (int i = 0; i < 8; ++i) {
-          a[j][i] = a[j][i] - a[k][i] * f;
-          b[j][i] = b[j][i] - b[k][i] * f;
-        }
-      }
+      if (j != k) a[j] = a[j] - a[k] * (one == 1.0 ? col[j] : plain_quotient(col[j], one));
   }
-  for (int j = 0; j < 8; ++j)
-    for (int i = 0; i < 8; ++i) m[i + 8 * j] = b[j][i];
 }
 
 // Per ghost cell: status (0 dropped, 1 turned fluid, 2 minus entry, 3 plus
-// entry), the image point's base cell and the eight weights.
-__global__ void __launch_bounds__(128) k_ibm_weights(int ng, int n, const int *__restrict__ gidx,
-                                                     const double *__restrict__ cen,
-                                                     const double *__restrict__ srch,
-                                                     const double *__restrict__ dotp_eff,
-                                                     const double *__restrict__ cube_size,
-                                                     int ncube, const double *__restrict__ ctr,
-                                                     int *__restrict__ status,
-                                                     int *__restrict__ base,
-                                                     double *__restrict__ weight) {
+// entry, these two if k_ibm_weights agrees), the image point's base cell, its
+// offsets s1..s3 in it and the cell's edges (weight[0..5]).
+constexpr int kPlaceThreads = 32;
+__global__ void __launch_bounds__(kPlaceThreads)
+    k_ibm_place(int ng, int n, const int *__restrict__ gidx, const double *__restrict__ cen,
+                const double *__restrict__ srch, const double *__restrict__ dotp_eff,
+                const double *__restrict__ cube_size, int ncube, const double *__restrict__ ctr,
+                int *__restrict__ status, int *__restrict__ base, double *__restrict__ weight) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= ng) return;
   const int c = gidx[4 * g];
@@ -425,38 +564,46 @@ __global__ void __launch_bounds__(128) k_ibm_weights(int ng, int n, const int *_
   const double hx = cx[ii + 1] - cx[ii];
   const double hy = cy[jj + 1] - cy[jj];
   const double hz = cz[kk + 1] - cz[kk];
-  // corners 000, 100, 010, 001, 110, 101, 011, 111
-  const int ox[8] = {0, 1, 0, 0, 1, 1, 0, 1}, oy[8] = {0, 0, 1, 0, 1, 0, 1, 1},
-            oz[8] = {0, 0, 0, 1, 0, 1, 1, 1};
-  double V[64];
-  for (int q = 0; q < 8; ++q) {
-    const double sx = ox[q] ? hx : 0, sy = oy[q] ? hy : 0, sz = oz[q] ? hz : 0;
-    V[q * 8 + 7] = 1;
-    V[q * 8 + 6] = sz;
-    V[q * 8 + 5] = sy;
-    V[q * 8 + 4] = sx;
-    V[q * 8 + 3] = sy * sz;
-    V[q * 8 + 2] = sx * sz;
-    V[q * 8 + 1] = sx * sy;
-    V[q * 8 + 0] = sx * sy * sz;
-  }
-  invert8(V);
-  bool ok = true;
-  double w[8];
-  for (int q = 0; q < 8; ++q) {
-    w[q] = V[q] * s1 * s2 * s3 + V[q + 8] * s1 * s2 + V[q + 16] * s1 * s3 + V[q + 24] * s2 * s3 +
-           V[q + 32] * s1 + V[q + 40] * s2 + V[q + 48] * s3 + V[q + 56];
-    if (!(w[q] >= (-kMinimum) && w[q] <= (1 + kMinimum))) ok = false;
-  }
-  if (!ok) {
-    status[g] = 0;
-    return;
-  }
   status[g] = dotp >= 0 ? 2 : 3;
   base[3 * g] = ii;
   base[3 * g + 1] = jj;
   base[3 * g + 2] = kk;
-  for (int q = 0; q < 8; ++q) weight[8 * (size_t)g + q] = w[q];
+  const double mid[6] = {s1, s2, s3, hx, hy, hz};
+  for (int q = 0; q < 6; ++q) weight[8 * (size_t)g + q] = mid[q];
+}
+
+// The eight trilinear weights of the cells k_ibm_place kept, 16 lanes a cell;
+// status 0 where one lies outside [0, 1].  A thread per cell with both
+// matrices in local memory took 214 us for 5,984 cells (47 CTAs); this, with
+// k_ibm_place, 62.
+constexpr int kWeightThreads = 128;
+__global__ void __launch_bounds__(kWeightThreads)
+    k_ibm_weights(int ng, int *__restrict__ status, double *__restrict__ weight) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  if (g >= ng || status[g] < 2) return;  // all 16 lanes
+  const int l = threadIdx.x & 15, lane0 = threadIdx.x & 16;
+  const unsigned group = 0xffffu << lane0;
+  double *const w = weight + 8 * (size_t)g;
+  const double s1 = w[0], s2 = w[1], s3 = w[2], hx = w[3], hy = w[4], hz = w[5];
+  double a[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {  // corners 000, 100, 010, 001, 110, 101, 011, 111
+    const double sx = q == 1 || q == 4 || q == 5 || q == 7 ? hx : 0,
+                 sy = q == 2 || q == 4 || q == 6 || q == 7 ? hy : 0,
+                 sz = q == 3 || q == 5 || q == 6 || q == 7 ? hz : 0;
+    a[q] = l == 7 ? 1.0 : l == 6 ? sz : l == 5 ? sy : l == 4 ? sx : l == 3 ? sy * sz
+         : l == 2 ? sx * sz : l == 1 ? sx * sy : l == 0 ? sx * sy * sz : (l - 8 == q ? 1.0 : 0.0);
+  }
+  invert8(a, group, lane0);
+  const double x = a[0] * s1 * s2 * s3 + a[1] * s1 * s2 + a[2] * s1 * s3 + a[3] * s2 * s3 +
+                   a[4] * s1 + a[5] * s2 + a[6] * s3 + a[7];
+  const bool in = x >= (-kMinimum) && x <= (1 + kMinimum);
+  const unsigned all = __ballot_sync(group, l < 8 || in);
+  if ((all & group) != group) {
+    if (l == 0) status[g] = 0;
+  } else if (l >= 8) {
+    w[l - 8] = x;
+  }
 }
 
 template <typename T>
@@ -515,6 +662,7 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
   if (ng == 0 || ntri == 0) return BCMG_OK;  // nothing to do
   DevBuf<double> dtri, dsize, dX, dY, dZ, dctr, dcen, drec, dsrch, ddot, dw;
   DevBuf<int> dkeep, dg, dstat, dbase;
+  DevBuf<float4> dfilter;
   CKI(dtri.alloc((size_t)ntri * 9));
   CKI(dsize.alloc(ncube));
   CKI(dX.alloc(ncube));
@@ -531,7 +679,7 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
     CKI(dbox.alloc((size_t)6 * ncube));
     k_ibm_cube_box<<<(ncube + 127) / 128, 128>>>(ncube, n, dsize.p, dX.p, dY.p, dZ.p, dbox.p);
     CKI(cudaGetLastError());
-    k_ibm_keep<<<(ntri + 255) / 256, 256>>>(ntri, dtri.p, ncube, dbox.p, dkeep.p);
+    k_ibm_keep<<<(ntri + kKeepThreads - 1) / kKeepThreads, kKeepThreads>>>(ntri, dtri.p, ncube, dbox.p, dkeep.p);
     CKI(cudaGetLastError());
   }
   std::vector<int> keep(ntri);
@@ -543,7 +691,18 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
   if (nk == 0) return BCMG_OK;  // no triangle near any cube
   CKI(cudaMemcpy(dtri.p, kept.data(), sizeof(double) * kept.size(), cudaMemcpyHostToDevice));
   CKI(drec.alloc((size_t)nk * kRec));
-  k_ibm_tri_prep<<<(nk + 127) / 128, 128>>>(nk, dtri.p, drec.p);
+  CKI(dfilter.alloc((size_t)nk * 3));
+  GhostBox box;
+  for (int q = 0; q < 3; ++q) {
+    double lo = cen[q], hi = cen[q];
+    for (int g = 1; g < ng; ++g) {
+      lo = std::min(lo, cen[3 * (size_t)g + q]);
+      hi = std::max(hi, cen[3 * (size_t)g + q]);
+    }
+    box.org[q] = 0.5 * (lo + hi);
+    box.ext[q] = 0.5 * (hi - lo) * (1 + 1e-9) + 1e-300;
+  }
+  k_ibm_tri_prep<<<(nk + 127) / 128, 128>>>(nk, dtri.p, box, drec.p, dfilter.p);
   CKI(cudaGetLastError());
   CKI(dcen.alloc(cen.size()));
   CKI(dg.alloc(gidx.size()));
@@ -558,10 +717,10 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
     CKI(hp.alloc((size_t)ns * ng));
     CKI(bp.alloc((size_t)ns * ng));
     CKI(np_.alloc((size_t)ns * ng));
-    k_ibm_ray_part<<<dim3(gb, ns), kGhostBlock>>>(ng, dcen.p, nk, per, drec.p, hp.p, bp.p,
-                                                  np_.p);
+    k_ibm_ray_part<<<dim3(gb, ns), kGhostBlock>>>(ng, dcen.p, box, nk, per, drec.p, dfilter.p,
+                                                  hp.p, bp.p, np_.p);
     CKI(cudaGetLastError());
-    k_ibm_ray_combine<<<(ng + 127) / 128, 128>>>(ng, ns, dcen.p, drec.p, hp.p, bp.p, np_.p,
+    k_ibm_ray_combine<<<(ng + 3) / 4, 128>>>(ng, ns, dcen.p, drec.p, hp.p, bp.p, np_.p,
                                                  dsrch.p);
     CKI(cudaGetLastError());
   }
@@ -583,15 +742,18 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
     const int gb = (m + kGhostBlock - 1) / kGhostBlock;
     const int ns = ibm_splits(gb, nk), per = (nk + ns - 1) / ns;
     DevBuf<int> dl, bp;
+    DevBuf<unsigned> db;
     DevBuf<double> np_;
     CKI(dl.alloc(m));
+    CKI(db.alloc(m));
+    CKI(cudaMemsetAsync(db.p, 0x7f, sizeof(unsigned) * m, nullptr));
     CKI(bp.alloc((size_t)ns * m));
     CKI(np_.alloc((size_t)ns * m));
     CKI(cudaMemcpy(dl.p, nohit.data(), sizeof(int) * m, cudaMemcpyHostToDevice));
-    k_ibm_closest_part<<<dim3(gb, ns), kGhostBlock>>>(m, dl.p, dcen.p, nk, per, dtri.p, bp.p,
-                                                      np_.p);
+    k_ibm_closest_part<<<dim3(gb, ns), kGhostBlock>>>(m, dl.p, dcen.p, box, nk, per, dtri.p,
+                                                      dfilter.p, db.p, bp.p, np_.p);
     CKI(cudaGetLastError());
-    k_ibm_closest_combine<<<(m + 127) / 128, 128>>>(m, ns, dl.p, dcen.p, dtri.p, bp.p, np_.p,
+    k_ibm_closest_combine<<<(m + 3) / 4, 128>>>(m, ns, dl.p, dcen.p, dtri.p, bp.p, np_.p,
                                                     dsrch.p);
     CKI(cudaGetLastError());
   }
@@ -602,8 +764,11 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
   CKI(dw.alloc((size_t)ng * 8));
   CKI(cudaMemcpy(dctr.p, ctr, sizeof(double) * 3 * (size_t)ncube * S, cudaMemcpyHostToDevice));
   CKI(cudaMemcpy(ddot.p, deff.data(), sizeof(double) * ng, cudaMemcpyHostToDevice));
-  k_ibm_weights<<<(ng + 127) / 128, 128>>>(ng, n, dg.p, dcen.p, dsrch.p, ddot.p, dsize.p, ncube,
-                                           dctr.p, dstat.p, dbase.p, dw.p);
+  k_ibm_place<<<(ng + kPlaceThreads - 1) / kPlaceThreads, kPlaceThreads>>>(
+      ng, n, dg.p, dcen.p, dsrch.p, ddot.p, dsize.p, ncube, dctr.p, dstat.p, dbase.p, dw.p);
+  CKI(cudaGetLastError());
+  k_ibm_weights<<<(16 * (long long)ng + kWeightThreads - 1) / kWeightThreads, kWeightThreads>>>(
+      ng, dstat.p, dw.p);
   CKI(cudaGetLastError());
   std::vector<int> stat(ng), base((size_t)ng * 3);
   std::vector<double> w((size_t)ng * 8);
