@@ -164,7 +164,7 @@ def ibm_preprocess(case, tris, fws=None):
     IPsur[m,4], weight[m,8]) with 0-based rows and unrounded weights."""
     fws = _fws_inplace(case.fws if fws is None else fws)
     tri = np.ascontiguousarray(np.asarray(tris, np.float64).reshape(-1, 9))
-    cap = int((fws == 0).sum()) + 1
+    cap = fws.size - np.count_nonzero(fws) + 1
     o = np.ascontiguousarray(case.origin, dtype=np.float64)
     out = [np.zeros(4 * cap, np.int32), np.zeros(4 * cap, np.int32), np.zeros(8 * cap),
            np.zeros(4 * cap, np.int32), np.zeros(4 * cap, np.int32), np.zeros(8 * cap)]
@@ -185,23 +185,18 @@ def interface_lists(case):
     """The 15 neighbour lists of BCM_Interface_table.cpp:96-308 (1-based
     arrays): per axis x, y, z the same-level, big->small (+), small->big (+),
     big->small (-) and small->big (-) lists."""
-    adj, csl = case.adj, case.csl
+    n = case.ncube
+    c, csl = np.arange(1, n), np.asarray(case.csl)
     out = []
     for ax in range(3):
-        eq, bsp, sbp, bsm, sbm = [], [], [], [], []
-        for c in range(1, case.ncube):
-            plus = adj[c, 1:5, 2 + 2 * ax]
-            if (plus > 0).any():
-                a = plus.max()
-                (eq if csl[c] == csl[a] else (sbp if csl[c] < csl[a] else bsp)).append(c)
-            minus = adj[c, 1:5, 1 + 2 * ax]
-            if (minus > 0).any():
-                a = minus.max()
-                if csl[c] < csl[a]:
-                    sbm.append(c)
-                elif csl[c] > csl[a]:
-                    bsm.append(c)
-        out.append([_one_based(x) for x in (eq, bsp, sbp, bsm, sbm)])
+        plus = case.adj[1:n, 1:5, 2 + 2 * ax].max(axis=1)
+        minus = case.adj[1:n, 1:5, 1 + 2 * ax].max(axis=1)
+        # by the level difference to the neighbour, where there is one
+        p, m = plus > 0, minus > 0
+        dp = csl[1:n] - csl[np.where(p, plus, 0)]
+        dm = csl[1:n] - csl[np.where(m, minus, 0)]
+        out.append([_one_based(c[q]) for q in (p & (dp == 0), p & (dp > 0), p & (dp < 0),
+                                               m & (dm > 0), m & (dm < 0))])
     return out
 
 

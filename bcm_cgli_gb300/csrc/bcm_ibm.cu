@@ -459,11 +459,14 @@ __global__ void k_ibm_closest_combine(int m, int nsplit, const int *__restrict__
 
 // Triangle ranges per ghost block so that a search launch fills the GPU
 // (about 8 CTAs per SM), each range at least 64 triangles.
-int ibm_splits(int nblocks, int ntri) {
+int sm_count() {
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int want = (8 * sms + nblocks - 1) / nblocks;
+  return sms;
+}
+int ibm_splits(int nblocks, int ntri) {
+  const int want = (8 * sm_count() + nblocks - 1) / nblocks;
   const int most = (ntri + 63) / 64;
   return std::max(1, std::min(want, most));
 }
@@ -606,11 +609,27 @@ __global__ void __launch_bounds__(kWeightThreads)
   }
 }
 
+// Device memory of one call: a single allocation, handed out in pieces.
+struct DevArena {
+  char *p = nullptr;
+  size_t cap = 0, used = 0;
+  ~DevArena() { if (p) cudaFree(p); }
+  cudaError_t reserve(size_t bytes) {
+    cap = bytes;
+    return cudaMalloc((void **)&p, bytes);
+  }
+  static size_t padded(size_t bytes) { return (bytes + 255) / 256 * 256; }
+};
 template <typename T>
 struct DevBuf {
   T *p = nullptr;
-  ~DevBuf() { if (p) cudaFree(p); }
-  cudaError_t alloc(size_t count) { return cudaMalloc((void **)&p, sizeof(T) * (count ? count : 1)); }
+  cudaError_t alloc(DevArena &a, size_t count) {
+    const size_t bytes = DevArena::padded(sizeof(T) * count);
+    if (a.used + bytes > a.cap) return cudaErrorMemoryAllocation;
+    p = reinterpret_cast<T *>(a.p + a.used);
+    a.used += bytes;
+    return cudaSuccess;
+  }
 };
 
 }  // namespace
@@ -650,25 +669,42 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
     if (csl[c] != 0) continue;
     if (!(cube_size[c] > 0)) return fail("cube_size must be positive", BCMG_ERR_ARG);
     for (int i = 2; i <= nx; ++i)
-      for (int j = 2; j <= nx; ++j)
+      for (int j = 2; j <= nx; ++j) {
+        const int *row = FWS + cell_index(S, c, i, j, 0);
+        int zeros = 0;
+        for (int k = 2; k <= nx; ++k) zeros += row[k] == 0;
+        if (zeros == 0) continue;
         for (int k = 2; k <= nx; ++k)
-          if (FWS[cell_index(S, c, i, j, k)] == 0) {
+          if (row[k] == 0) {
             gidx.insert(gidx.end(), {c, i, j, k});
             cen.insert(cen.end(), {ctr[(size_t)c * S + i], ctr[((size_t)ncube + c) * S + j],
                                    ctr[(2 * (size_t)ncube + c) * S + k]});
           }
+      }
   }
   const int ng = (int)(gidx.size() / 4);
   if (ng == 0 || ntri == 0) return BCMG_OK;  // nothing to do
   DevBuf<double> dtri, dsize, dX, dY, dZ, dctr, dcen, drec, dsrch, ddot, dw;
   DevBuf<int> dkeep, dg, dstat, dbase;
   DevBuf<float4> dfilter;
-  CKI(dtri.alloc((size_t)ntri * 9));
-  CKI(dsize.alloc(ncube));
-  CKI(dX.alloc(ncube));
-  CKI(dY.alloc(ncube));
-  CKI(dZ.alloc(ncube));
-  CKI(dkeep.alloc(ntri));
+  DevArena mem;
+  {
+    // everything allocated below; a search's split results are at most
+    // (8 SMs + blocks) blocks of cells
+    const size_t blocks = (ng + kGhostBlock - 1) / kGhostBlock;
+    const size_t parts = (ibm_splits((int)blocks, ntri) * blocks + 1) * kGhostBlock;
+    const size_t parts_m = std::max(parts, (8 * (size_t)sm_count() + blocks + 1) * kGhostBlock);
+    CKI(mem.reserve(64 * 256 + (size_t)ntri * (9 * 8 + 4 + kRec * 8 + 3 * 16) +
+                    (size_t)ncube * (4 * 8 + 6 * 8 + 3 * 8 * (size_t)S) +
+                    (size_t)ng * (3 * 8 + 4 * 4 + 8 * 8 + 8 + 4 + 3 * 4 + 8 * 8 + 8) +
+                    (parts + parts_m) * 16));
+  }
+  CKI(dtri.alloc(mem, (size_t)ntri * 9));
+  CKI(dsize.alloc(mem, ncube));
+  CKI(dX.alloc(mem, ncube));
+  CKI(dY.alloc(mem, ncube));
+  CKI(dZ.alloc(mem, ncube));
+  CKI(dkeep.alloc(mem, ntri));
   CKI(cudaMemcpy(dtri.p, tri, sizeof(double) * 9 * (size_t)ntri, cudaMemcpyHostToDevice));
   CKI(cudaMemcpy(dsize.p, cube_size, sizeof(double) * ncube, cudaMemcpyHostToDevice));
   CKI(cudaMemcpy(dX.p, Xcube, sizeof(double) * ncube, cudaMemcpyHostToDevice));
@@ -676,7 +712,7 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
   CKI(cudaMemcpy(dZ.p, Zcube, sizeof(double) * ncube, cudaMemcpyHostToDevice));
   {
     DevBuf<double> dbox;
-    CKI(dbox.alloc((size_t)6 * ncube));
+    CKI(dbox.alloc(mem, (size_t)6 * ncube));
     k_ibm_cube_box<<<(ncube + 127) / 128, 128>>>(ncube, n, dsize.p, dX.p, dY.p, dZ.p, dbox.p);
     CKI(cudaGetLastError());
     k_ibm_keep<<<(ntri + kKeepThreads - 1) / kKeepThreads, kKeepThreads>>>(ntri, dtri.p, ncube, dbox.p, dkeep.p);
@@ -690,8 +726,8 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
   const int nk = (int)(kept.size() / 9);
   if (nk == 0) return BCMG_OK;  // no triangle near any cube
   CKI(cudaMemcpy(dtri.p, kept.data(), sizeof(double) * kept.size(), cudaMemcpyHostToDevice));
-  CKI(drec.alloc((size_t)nk * kRec));
-  CKI(dfilter.alloc((size_t)nk * 3));
+  CKI(drec.alloc(mem, (size_t)nk * kRec));
+  CKI(dfilter.alloc(mem, (size_t)nk * 3));
   GhostBox box;
   for (int q = 0; q < 3; ++q) {
     double lo = cen[q], hi = cen[q];
@@ -704,9 +740,9 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
   }
   k_ibm_tri_prep<<<(nk + 127) / 128, 128>>>(nk, dtri.p, box, drec.p, dfilter.p);
   CKI(cudaGetLastError());
-  CKI(dcen.alloc(cen.size()));
-  CKI(dg.alloc(gidx.size()));
-  CKI(dsrch.alloc((size_t)ng * 8));
+  CKI(dcen.alloc(mem, cen.size()));
+  CKI(dg.alloc(mem, gidx.size()));
+  CKI(dsrch.alloc(mem, (size_t)ng * 8));
   CKI(cudaMemcpy(dcen.p, cen.data(), sizeof(double) * cen.size(), cudaMemcpyHostToDevice));
   CKI(cudaMemcpy(dg.p, gidx.data(), sizeof(int) * gidx.size(), cudaMemcpyHostToDevice));
   {
@@ -714,9 +750,9 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
     const int ns = ibm_splits(gb, nk), per = (nk + ns - 1) / ns;
     DevBuf<int> hp, bp;
     DevBuf<double> np_;
-    CKI(hp.alloc((size_t)ns * ng));
-    CKI(bp.alloc((size_t)ns * ng));
-    CKI(np_.alloc((size_t)ns * ng));
+    CKI(hp.alloc(mem, (size_t)ns * ng));
+    CKI(bp.alloc(mem, (size_t)ns * ng));
+    CKI(np_.alloc(mem, (size_t)ns * ng));
     k_ibm_ray_part<<<dim3(gb, ns), kGhostBlock>>>(ng, dcen.p, box, nk, per, drec.p, dfilter.p,
                                                   hp.p, bp.p, np_.p);
     CKI(cudaGetLastError());
@@ -744,11 +780,11 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
     DevBuf<int> dl, bp;
     DevBuf<unsigned> db;
     DevBuf<double> np_;
-    CKI(dl.alloc(m));
-    CKI(db.alloc(m));
+    CKI(dl.alloc(mem, m));
+    CKI(db.alloc(mem, m));
     CKI(cudaMemsetAsync(db.p, 0x7f, sizeof(unsigned) * m, nullptr));
-    CKI(bp.alloc((size_t)ns * m));
-    CKI(np_.alloc((size_t)ns * m));
+    CKI(bp.alloc(mem, (size_t)ns * m));
+    CKI(np_.alloc(mem, (size_t)ns * m));
     CKI(cudaMemcpy(dl.p, nohit.data(), sizeof(int) * m, cudaMemcpyHostToDevice));
     k_ibm_closest_part<<<dim3(gb, ns), kGhostBlock>>>(m, dl.p, dcen.p, box, nk, per, dtri.p,
                                                       dfilter.p, db.p, bp.p, np_.p);
@@ -757,11 +793,11 @@ int ibm_run(int n, int ncube, const double *cube_size, const int *csl, const dou
                                                     dsrch.p);
     CKI(cudaGetLastError());
   }
-  CKI(dctr.alloc((size_t)3 * ncube * S));
-  CKI(ddot.alloc(ng));
-  CKI(dstat.alloc(ng));
-  CKI(dbase.alloc((size_t)ng * 3));
-  CKI(dw.alloc((size_t)ng * 8));
+  CKI(dctr.alloc(mem, (size_t)3 * ncube * S));
+  CKI(ddot.alloc(mem, ng));
+  CKI(dstat.alloc(mem, ng));
+  CKI(dbase.alloc(mem, (size_t)ng * 3));
+  CKI(dw.alloc(mem, (size_t)ng * 8));
   CKI(cudaMemcpy(dctr.p, ctr, sizeof(double) * 3 * (size_t)ncube * S, cudaMemcpyHostToDevice));
   CKI(cudaMemcpy(ddot.p, deff.data(), sizeof(double) * ng, cudaMemcpyHostToDevice));
   k_ibm_place<<<(ng + kPlaceThreads - 1) / kPlaceThreads, kPlaceThreads>>>(

@@ -9,7 +9,6 @@
 #include <cstdint>
 #include <cstdio>
 #include <map>
-#include <unordered_map>
 
 namespace bcmg {
 
@@ -223,11 +222,21 @@ bool build_ibm_levels(int nbc, const int *GC, const int *IP, int n, int ncube,
                       std::vector<int> &order, std::vector<int> &level_off, std::string &err) {
   const int S = n + 4;
   struct Tag {
-    int write = 0;  // level of the last writer
-    int read = 0;   // highest level of any reader so far
+    long long key = -1;  // cell; -1: free slot
+    int write = 0;       // level of the last writer
+    int read = 0;        // highest level of any reader so far
   };
-  std::unordered_map<long long, Tag> cells;
-  cells.reserve((size_t)nbc * 9 + 16);
+  // The cells touched so far, by open addressing (each entry touches nine
+  // cells at most, so the table stays under 9/16 full).
+  size_t cap = 64;
+  while (cap < 16 * (size_t)nbc) cap *= 2;
+  std::vector<Tag> cells(cap);
+  auto tag = [&](long long key) -> Tag & {
+    size_t q = (size_t)((unsigned long long)key * 0x9e3779b97f4a7c15ull >> 20) & (cap - 1);
+    while (cells[q].key != key && cells[q].key != -1) q = (q + 1) & (cap - 1);
+    cells[q].key = key;
+    return cells[q];
+  };
   std::vector<int> lev((size_t)nbc + 1, 0);
   int maxlev = 0;
   auto key = [&](int c, int i, int j, int k) {
@@ -247,20 +256,17 @@ bool build_ibm_levels(int nbc, const int *GC, const int *IP, int n, int ncube,
       return false;
     }
     int L = 1;
+    Tag *at[8];  // (the table never moves)
     for (int m = 0; m < 8; ++m) {
-      auto it = cells.find(key(c, i + (m & 1), j + ((m >> 1) & 1), k + ((m >> 2) & 1)));
-      if (it != cells.end()) L = std::max(L, it->second.write + 1);
+      at[m] = &tag(key(c, i + (m & 1), j + ((m >> 1) & 1), k + ((m >> 2) & 1)));
+      L = std::max(L, at[m]->write + 1);
     }
-    const long long w = key(gc, gi, gj, gk);
-    auto it = cells.find(w);
-    if (it != cells.end()) L = std::max(L, std::max(it->second.read, it->second.write) + 1);
+    Tag &w = tag(key(gc, gi, gj, gk));
+    L = std::max(L, std::max(w.read, w.write) + 1);
     lev[e] = L;
     maxlev = std::max(maxlev, L);
-    for (int m = 0; m < 8; ++m) {
-      Tag &t = cells[key(c, i + (m & 1), j + ((m >> 1) & 1), k + ((m >> 2) & 1))];
-      t.read = std::max(t.read, L);
-    }
-    cells[w].write = L;
+    for (int m = 0; m < 8; ++m) at[m]->read = std::max(at[m]->read, L);
+    w.write = L;
   }
   level_off.assign((size_t)maxlev + 1, 0);
   for (int e = 1; e <= nbc; ++e) level_off[lev[e]]++;
