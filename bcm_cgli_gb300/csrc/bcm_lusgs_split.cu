@@ -10,7 +10,8 @@
 // in FP64, as in the split RK path.
 //
 // Plane order.  Between the kernels a cube's values lie value-major in the
-// order of the sweep (the cells of plane h, i then j ascending), so the
+// order of the sweep (the cells of plane h, i then j ascending, the rows of a
+// cluster's CTAs one after the other), so the
 // threads of a plane read and write consecutive words; k_lus_pack and
 // k_lus_update change between that order and the memory order slab by slab
 // (i fixed) through shared memory, where the cells of an anti-diagonal j + k
@@ -81,16 +82,20 @@ __device__ __forceinline__ void luf_terms(const float *k, float idx, float omega
     a[1 + D] += dp;
     a[4] = un * (dq[4] + dp) + H * t;
     const float h = 0.5f * idx, w = omega * k[5 + D], v = k[8] * idx * idx;
+    float t5[5];
 #pragma unroll
     for (int m = 0; m < 5; ++m)
-      store(D, m, LOWER ? h * (a[m] + w * dq[m]) + v * dq[m] : h * (a[m] - w * dq[m]) - v * dq[m]);
+      t5[m] = LOWER ? h * (a[m] + w * dq[m]) + v * dq[m] : h * (a[m] - w * dq[m]) - v * dq[m];
+    store(D, t5);
   }
 }
 
-// Scratch of a cube, value-major [kScr][n^3] in plane order: coefficients
-// 0..9, residual / increment 10..14, flags 15 (bit 0 fluid; bits 1..3 the
-// lower x, y, z neighbour inside the cube is fluid, bits 4..6 the upper).
-constexpr int kScr = 16;
+// Scratch of a cube: four words of four values per cell, word-major
+// [kWords][n^3] in plane order: U V W VV, H r_x r_y r_z, nu dg flags R4 and R0 ..
+// R3 (the residual, then the forward sweep's increment).  Flags: bit 0 fluid;
+// bits 1..3 the lower x, y, z neighbour inside the cube is fluid, bits 4..6 the
+// upper; i, j, k from bits 7, 12 and 17.
+constexpr int kWords = 4;
 constexpr int kSlabThreads = 256;
 
 // Position of the first cell of row i in plane h, and the row's first j.
@@ -108,16 +113,17 @@ __device__ __forceinline__ int plane_start(int h, int n) {
   if (h > 2 * n) c += 3 * tet(h - 2 * n);
   return c;
 }
-// cells of rows 0 .. i-1 of plane h
-__device__ __forceinline__ int row_start(int h, int i, int n) {
-  // row l has max(0, min(n, h-l+1) - max(0, h-l-n+1)) cells: the counts of
-  // x = h - l + 1 summed over x = h-i+2 .. h+1, x clipped to [0, n], less the
-  // same of x - n
-  auto upto = [&](int x) {  // sum over y <= x of min(max(y, 0), n)
-    if (x <= 0) return 0;
-    return x <= n ? x * (x + 1) / 2 : n * (n + 1) / 2 + (x - n) * n;
-  };
-  return (upto(h + 1) - upto(h + 1 - i)) - (upto(h + 1 - n) - upto(h + 1 - n - i));
+__device__ __forceinline__ int row_cells(int h, int i, int n) {
+  const int lo = jlo_of(h, i, n), hi = min(n - 1, h - i);
+  return hi >= lo ? hi - lo + 1 : 0;
+}
+// cells of plane h ahead of row i: of its CTA's rows (i mod size alike) the
+// lower ones, and all of the CTAs before
+__device__ __forceinline__ int row_start(int h, int i, int n, int size) {
+  int c = 0;
+  for (int r = 0; r <= i % size; ++r)
+    for (int l = r; l < (r < i % size ? n : i); l += size) c += row_cells(h, l, n);
+  return c;
 }
 
 // Cell t of a slab in anti-diagonal order: d = j + k ascending, then j.
@@ -154,9 +160,10 @@ __device__ __forceinline__ LusConst lus_const(const LusgsSplitArgs &a, int cube)
 // One slab (cube, i) per CTA: coefficients, residual and flags into plane
 // order.  (The mirror is read here and updated in k_lus_update: its interior
 // cells belong to one cube each.)
-__global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a) {
-  extern __shared__ __align__(16) float stage[];  // [kScr][n^2]
+__global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a, int size) {
+  extern __shared__ float4 stage[];  // [kWords][n^2]
   __shared__ unsigned short start[64];
+  __shared__ int place[64];  // of the slab's cells of anti-diagonal d
   const int n = a.ph.n, S = n + 4, nn = n * n;
   const int cube = 1 + blockIdx.x / n, i = blockIdx.x % n;
   if (!case_active(a.bt, cube)) return;  // converged case
@@ -164,6 +171,8 @@ __global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a) {
   const float idx = a.inv_dx[cube];
   const float *const Mc = mirror_current(a.mir);
   slab_starts(start, n);
+  for (int d = threadIdx.x; d < 2 * n - 1; d += kSlabThreads)
+    place[d] = plane_start(i + d, n) + row_start(i + d, i, n, size) - jlo_of(i + d, i, n);
   for (int jk = threadIdx.x; jk < nn; jk += kSlabThreads) {
     const int j = jk / n, k = jk - j * n;
     const size_t o = cell_index(S, cube, i + 2, j + 2, k + 2);
@@ -171,10 +180,9 @@ __global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) m[v] = Mc[5 * o + v];
     luf_coef(m, z.rho0, z.P0, z.T0, z.mu_L, idx, z.dT, a.cflf, a.omegaf, kc);
+    float R[5];
 #pragma unroll
-    for (int v = 0; v < 10; ++v) stage[v * nn + jk] = kc[v];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) stage[(10 + v) * nn + jk] = a.R32[5 * o + v];
+    for (int v = 0; v < 5; ++v) R[v] = a.R32[5 * o + v];
     const int *F = a.FWS + o;
     int f = F[0] == kFluid ? 1 : 0;
     if (i > 0 && F[-S * S] == kFluid) f |= 2;
@@ -183,105 +191,104 @@ __global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a) {
     if (i + 1 < n && F[S * S] == kFluid) f |= 16;
     if (j + 1 < n && F[S] == kFluid) f |= 32;
     if (k + 1 < n && F[1] == kFluid) f |= 64;
-    stage[15 * nn + jk] = __int_as_float(f);
+    f |= i << 7 | j << 12 | k << 17;
+    stage[jk] = make_float4(kc[0], kc[1], kc[2], kc[3]);
+    stage[nn + jk] = make_float4(kc[4], kc[5], kc[6], kc[7]);
+    stage[2 * nn + jk] = make_float4(kc[8], kc[9], __int_as_float(f), R[4]);
+    stage[3 * nn + jk] = make_float4(R[0], R[1], R[2], R[3]);
   }
   __syncthreads();
-  float *const scr = a.scr + (size_t)(cube - 1) * kScr * nn * n;
+  float4 *const scr = reinterpret_cast<float4 *>(a.scr) + (size_t)(cube - 1) * kWords * nn * n;
   for (int t = threadIdx.x; t < nn; t += kSlabThreads) {
     int j, k;
     slab_cell(start, n, t, j, k);
-    const int h = i + j + k;
-    float *dst = scr + plane_start(h, n) + row_start(h, i, n) + (j - jlo_of(h, i, n));
+    float4 *dst = scr + place[j + k] + j;
 #pragma unroll
-    for (int v = 0; v < kScr; ++v) dst[(size_t)v * nn * n] = stage[v * nn + j * n + k];
+    for (int v = 0; v < kWords; ++v) dst[(size_t)v * nn * n] = stage[v * nn + j * n + k];
   }
 }
 
-// Shared memory of a sweeping CTA: the terms its cells add, value-major
-// [2 planes][3 directions][5][rows * n], then per plane the first cell of each
-// of its rows (its part of the plane counted from 0) and where the row lies
-// in the plane order.
+// Shared memory of a sweeping CTA: the terms its cells add, [2 planes][3
+// directions][rows * n] of the first four and after them the fifth, then the
+// place of its part of each plane and its size.
 __host__ __device__ inline int lus_rows(int n, int size) { return (n + size - 1) / size; }
 __host__ __device__ inline size_t lus_smem(int n, int size) {
-  const size_t rows = lus_rows(n, size), np = 3 * n - 2;
-  return sizeof(float) * 30 * rows * n + sizeof(int) * np * rows +
-         sizeof(unsigned short) * np * (rows + 1);
+  return sizeof(float) * 30 * lus_rows(n, size) * n + 2 * sizeof(int) * (3 * n - 2);
 }
 
 // Two CTAs on an SM hide each other's barriers (65536 registers / 896).
 constexpr int kSweepThreads = 448;
 
+// A cell is moved by 16-byte words throughout: four loads and six reads and six
+// writes of shared memory, where single values took 16, 15 and 15, each with
+// its address, and its place comes from its flags, where a search of the row
+// tables took a third of a plane's instructions: 216 cubes of 24^3 325 ->
+// SWEEPNOW us.
 struct LusCell {
-  int i, j, pos;  // pos < 0: none
-  int k;
-  int fl;
-  float r[5], c[10];
+  float4 w[kWords];
+  int pos;  // < 0: none
 };
 
-template <bool LOWER>
+template <bool LOWER, int SIZE>
 __device__ __forceinline__ void lus_sweep(const LusgsSplitArgs &a, cg::cluster_group cl,
-                                          float *slots, const int *where,
-                                          const unsigned short *first, float *scr, float *inc,
-                                          float idx) {
+                                          float4 *slots, const int *place, const int *cells,
+                                          float4 *scr, float *inc, float idx) {
   const int n = a.ph.n, S = n + 4, n3 = n * n * n, np = 3 * n - 2;
-  const int size = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int rows = lus_rows(n, size), cols = rows * n;
-  // cell t of the CTA's part of plane p
+  const int rank = SIZE == 1 ? 0 : (int)cl.block_rank();
+  const int cols = lus_rows(n, SIZE) * n;
+  float *const fifth = reinterpret_cast<float *>(slots + 6 * cols);
   auto load = [&](int p, int t, LusCell &z) {
     z.pos = -1;
-    if (p < 0 || p >= np) return;
-    const unsigned short *f = first + p * (rows + 1);
-    if (t >= f[rows]) return;
-    int lo = 0, hi = rows;  // the last row that starts at or before t
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (f[mid] <= t) lo = mid; else hi = mid;
-    }
-    z.i = lo * size + rank;
-    z.j = jlo_of(p, z.i, n) + t - f[lo];
-    z.k = p - z.i - z.j;
-    z.pos = where[p * rows + lo] + t - f[lo];
-    const float *q = scr + z.pos;
+    if (p < 0 || p >= np || t >= cells[p]) return;
+    z.pos = place[p] + t;
 #pragma unroll
-    for (int m = 0; m < 10; ++m) z.c[m] = q[(size_t)m * n3];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) z.r[m] = q[(size_t)(10 + m) * n3];
-    z.fl = __float_as_int(q[(size_t)15 * n3]);
+    for (int v = 0; v < kWords; ++v) z.w[v] = scr[z.pos + (size_t)v * n3];
   };
   auto cell = [&](int p, const LusCell &z) {
-    if (z.pos < 0 || !(z.fl & 1)) return;
-    const int col = (z.i / size) * n + z.j;
-    const float *in = slots + (p & 1) * 15 * cols + col;
-    const int nb = LOWER ? z.fl >> 1 : z.fl >> 4;
+    const int fl = __float_as_int(z.w[2].z);
+    if (z.pos < 0 || !(fl & 1)) return;
+    const int i = fl >> 7 & 31, j = fl >> 12 & 31, k = fl >> 17 & 31;
+    const int col = (i / SIZE) * n + j, in = (p & 1) * 3 * cols;
+    const int nb = LOWER ? fl >> 1 : fl >> 4;
+    const float r[5] = {z.w[3].x, z.w[3].y, z.w[3].z, z.w[3].w, z.w[2].w};
     float s[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) s[m] = LOWER ? z.r[m] : 0.f;
+    for (int m = 0; m < 5; ++m) s[m] = LOWER ? r[m] : 0.f;
 #pragma unroll
     for (int D = 0; D < 3; ++D)
       if (nb & (1 << D)) {
-#pragma unroll
-        for (int m = 0; m < 5; ++m) s[m] += in[(5 * D + m) * cols];
+        const float4 x = slots[in + D * cols + col];
+        s[0] += x.x; s[1] += x.y; s[2] += x.z; s[3] += x.w;
+        s[4] += fifth[in + D * cols + col];
       }
-    const float idg = 1.0f / z.c[9];
+    const float c[10] = {z.w[0].x, z.w[0].y, z.w[0].z, z.w[0].w, z.w[1].x,
+                         z.w[1].y, z.w[1].z, z.w[1].w, z.w[2].x, z.w[2].y};
+    const float idg = 1.0f / c[9];
     float dq[5];
-    float *q = scr + z.pos;
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      dq[m] = LOWER ? s[m] * idg : z.r[m] - s[m] * idg;
-      if (LOWER) q[(size_t)(10 + m) * n3] = dq[m];
-      else inc[5 * (((z.i + 2) * S + (z.j + 2)) * S + z.k + 2) + m] = dq[m];
+    for (int m = 0; m < 5; ++m) dq[m] = LOWER ? s[m] * idg : r[m] - s[m] * idg;
+    if (LOWER) {
+      scr[z.pos + (size_t)3 * n3] = make_float4(dq[0], dq[1], dq[2], dq[3]);
+      scr[z.pos + (size_t)2 * n3].w = dq[4];
+    } else {
+      float *q = inc + 5 * (((i + 2) * S + (j + 2)) * S + k + 2);
+#pragma unroll
+      for (int m = 0; m < 5; ++m) q[m] = dq[m];
     }
-    const int d = LOWER ? 1 : -1;
-    const bool wi = LOWER ? z.i + 1 < n : z.i > 0, wj = LOWER ? z.j + 1 < n : z.j > 0,
-               wk = LOWER ? z.k + 1 < n : z.k > 0;
-    float *const out = slots + ((p + d) & 1) * 15 * cols;
-    float *oi = out;
-    if (wi && size > 1) oi = cl.map_shared_rank(out, (z.i + d) % size);
-    oi += wi ? ((z.i + d) / size) * n + z.j : 0;
-    luf_terms<LOWER>(z.c, idx, a.omegaf, dq, [&](int D, int m, float x) {
-      if (D == 0) { if (wi) oi[m * cols] = x; }
-      else if (D == 1) { if (wj) out[(5 + m) * cols + col + d] = x; }
-      else { if (wk) out[(10 + m) * cols + col] = x; }
+    const int d = LOWER ? 1 : -1, out = ((p + d) & 1) * 3 * cols;
+    const bool wi = LOWER ? i + 1 < n : i > 0, wj = LOWER ? j + 1 < n : j > 0,
+               wk = LOWER ? k + 1 < n : k > 0;
+    luf_terms<LOWER>(c, idx, a.omegaf, dq, [&](int D, const float *x) {
+      if (!(D == 0 ? wi : (D == 1 ? wj : wk))) return;
+      const int at = out + D * cols + (D == 0 ? ((i + d) / SIZE) * n + j : (D == 1 ? col + d : col));
+      float4 *q = slots + at;
+      float *f = fifth + at;
+      if (SIZE > 1 && D == 0) {
+        q = cl.map_shared_rank(q, (rank + d + SIZE) % SIZE);
+        f = cl.map_shared_rank(f, (rank + d + SIZE) % SIZE);
+      }
+      *q = make_float4(x[0], x[1], x[2], x[3]);
+      *f = x[4];
     });
   };
   LusCell cur, nxt;
@@ -290,44 +297,44 @@ __device__ __forceinline__ void lus_sweep(const LusgsSplitArgs &a, cg::cluster_g
   for (int s = 0, p = p0; s < np; ++s, p += d) {
     cur = nxt;
     load(p + d, threadIdx.x, nxt);
-    cell(p, cur);
-    for (int t = threadIdx.x + blockDim.x; t < first[p * (rows + 1) + rows]; t += blockDim.x) {
-      load(p, t, cur);
+    // (one copy of the cell's code: two may contract their products unlike)
+#pragma unroll 1
+    for (int t = threadIdx.x;;) {
       cell(p, cur);
+      t += blockDim.x;
+      if (t >= cells[p]) break;
+      load(p, t, cur);
     }
-    if (size == 1) __syncthreads(); else cl.sync();
+    if (SIZE == 1) __syncthreads(); else cl.sync();
   }
 }
 
+template <int SIZE>
 __global__ void __launch_bounds__(kSweepThreads, 2) k_lus_sweep(LusgsSplitArgs a) {
-  extern __shared__ __align__(16) float slots[];
+  extern __shared__ float4 slots[];
   const cg::cluster_group cl = cg::this_cluster();
   const int n = a.ph.n, np = 3 * n - 2;
-  const int size = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int cube = 1 + blockIdx.x / size;
+  const int rank = SIZE == 1 ? 0 : (int)cl.block_rank();
+  const int cube = 1 + blockIdx.x / SIZE;
   if (!case_active(a.bt, cube)) return;  // converged case (the whole cluster)
-  const int rows = lus_rows(n, size);
-  int *where = reinterpret_cast<int *>(slots + 30 * rows * n);
-  unsigned short *first = reinterpret_cast<unsigned short *>(where + np * rows);
+  int *place = reinterpret_cast<int *>(reinterpret_cast<float *>(slots) +
+                                       30 * lus_rows(n, SIZE) * n);
+  int *cells = place + np;
   for (int p = threadIdx.x; p < np; p += blockDim.x) {
     int sum = 0;
-    const int base = plane_start(p, n);
-    for (int l = 0; l < rows; ++l) {
-      const int i = l * size + rank;
-      first[p * (rows + 1) + l] = (unsigned short)sum;
-      where[p * rows + l] = base + row_start(p, i, n);
-      const int jlo = jlo_of(p, i, n), jhi = min(n - 1, p - i);
-      if (i < n && jhi >= jlo) sum += jhi - jlo + 1;
-    }
-    first[p * (rows + 1) + rows] = (unsigned short)sum;
+    for (int i = rank; i < n; i += SIZE) sum += row_cells(p, i, n);
+    place[p] = plane_start(p, n) + row_start(p, rank, n, SIZE);
+    cells[p] = sum;
   }
   // every CTA of the cluster has started before any writes into its memory
-  if (size == 1) __syncthreads(); else cl.sync();
-  float *const scr = a.scr + (size_t)(cube - 1) * kScr * n * n * n;
+  if (SIZE == 1) __syncthreads(); else cl.sync();
+  float4 *const scr = reinterpret_cast<float4 *>(a.scr) + (size_t)(cube - 1) * kWords * n * n * n;
   float *const inc = a.R32 + 5 * cell_index(n + 4, cube, 0, 0, 0);
   const float idx = a.inv_dx[cube];
-  lus_sweep<true>(a, cl, slots, where, first, scr, inc, idx);   // dq* = (R + sum of lower A+ terms) / dg
-  lus_sweep<false>(a, cl, slots, where, first, scr, inc, idx);  // dq = dq* - (sum of upper A- terms) / dg
+  // dq* = (R + sum of lower A+ terms) / dg, then dq = dq* - (sum of upper A-
+  // terms) / dg
+  lus_sweep<true, SIZE>(a, cl, slots, place, cells, scr, inc, idx);
+  lus_sweep<false, SIZE>(a, cl, slots, place, cells, scr, inc, idx);
 }
 
 // Q += dq on fluid cells (FP64), one slab (i fixed) per CTA; change norms of
@@ -439,7 +446,7 @@ int lus_plane_cells(int n, int size) {
 
 }  // namespace
 
-size_t lusgs_split_scratch(int n) { return (size_t)kScr * n * n * n; }
+size_t lusgs_split_scratch(int n) { return (size_t)4 * kWords * n * n * n; }
 int lusgs_split_blocks(int n) { return n; }
 int lusgs_split_launches() { return 3; }
 
@@ -453,21 +460,22 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   if (a.threads > 0 && (a.threads % 32 != 0 || a.threads > lusgs_split_default_threads(n)))
     return cudaErrorInvalidValue;
   cudaError_t e;
-  const size_t pack = sizeof(float) * kScr * nn;
+  const size_t pack = sizeof(float4) * kWords * nn;
   e = cudaFuncSetAttribute(k_lus_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pack);
   if (e != cudaSuccess) return e;
-  k_lus_pack<<<ncubes * n, kSlabThreads, pack, s>>>(a);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   // One CTA per cube while the widest plane fits it (up to edge 24): the planes
   // are a chain, and a barrier of the CTA is cheaper than one of a cluster (216
   // cubes of 24^3, the rest of a sub-iteration as above: 0.63 ms, by clusters
   // of two 0.69; 8 cubes 0.29 and 0.30).  Wider planes go to clusters of four:
   // 64 cubes of 32^3 0.62 ms, by one CTA of 768 threads 0.74; 512 the same.
   const int size = lus_plane_cells(n, 1) <= kSweepThreads ? 1 : 4;
+  k_lus_pack<<<ncubes * n, kSlabThreads, pack, s>>>(a, size);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   int threads = (lus_plane_cells(n, size) + 31) / 32 * 32;
   if (a.threads > 0) threads = std::min(threads, a.threads);  // wide planes take several passes
   const size_t smem = lus_smem(n, size);
-  e = cudaFuncSetAttribute(k_lus_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const auto sweep = size == 1 ? k_lus_sweep<1> : k_lus_sweep<4>;
+  e = cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ncubes * size);
@@ -481,7 +489,7 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if ((e = cudaLaunchKernelEx(&cfg, k_lus_sweep, a)) != cudaSuccess) return e;
+  if ((e = cudaLaunchKernelEx(&cfg, sweep, a)) != cudaSuccess) return e;
   // Three cells per thread or so: a warp's norm sums take 9 FP64 additions a
   // turn on top of the 12 of each cell (two and four: the same within 1%).
   const int ut = std::min(kUpdThreads, (nn / 3 + 31) / 32 * 32);
