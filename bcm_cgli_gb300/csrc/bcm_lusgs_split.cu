@@ -19,9 +19,9 @@
 //
 // A sub-iteration less its flux stage (ms), against one kernel that packed,
 // swept and updated a cube in one CTA and formed the coefficients in the chain
-// of planes: 216 cubes of 24^3 0.88 -> 0.63, 8 of 24^3 0.53 -> 0.29, 512 of
-// 32^3 5.20 -> 3.32, 512 of 16^3 0.53 -> 0.44 and 512 of 12^3 0.29 -> 0.28.  (512
-// of 8^3, where the three launches are most of it, 0.14 -> 0.15.)
+// of planes: 216 cubes of 24^3 0.88 -> 0.49, 8 of 24^3 0.53 -> 0.19, 512 of
+// 32^3 5.20 -> 3.18, 512 of 16^3 0.53 -> 0.37, 512 of 12^3 0.29 -> 0.23, 512 of
+// 8^3 0.143 -> 0.115.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -223,7 +223,7 @@ constexpr int kSweepThreads = 448;
 // writes of shared memory, where single values took 16, 15 and 15, each with
 // its address, and its place comes from its flags, where a search of the row
 // tables took a third of a plane's instructions: 216 cubes of 24^3 325 ->
-// SWEEPNOW us.
+// 247 us.
 struct LusCell {
   float4 w[kWords];
   int pos;  // < 0: none
@@ -297,6 +297,16 @@ __device__ __forceinline__ void lus_sweep(const LusgsSplitArgs &a, cg::cluster_g
   for (int s = 0, p = p0; s < np; ++s, p += d) {
     cur = nxt;
     load(p + d, threadIdx.x, nxt);
+    // Clusters have fewer warps an SM to hide the loads: the plane after next
+    // starts towards L2 (512 cubes of 32^3 3.31 -> 3.25 ms of a sub-iteration;
+    // a CTA a cube, 8 of 24^3: 0.187 -> 0.204, so not there).
+    if (SIZE > 1) {
+      const int q = p + 2 * d;
+      if (q >= 0 && q < np && threadIdx.x < cells[q]) {
+#pragma unroll
+        for (int v = 0; v < kWords; ++v) prefetch_l2(scr + place[q] + threadIdx.x + (size_t)v * n3);
+      }
+    }
     // (one copy of the cell's code: two may contract their products unlike)
 #pragma unroll 1
     for (int t = threadIdx.x;;) {
@@ -341,8 +351,8 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_lus_sweep(LusgsSplitArgs a
 // p, u, v, w, T from the FP32 increment (the split RK path's third-stage
 // formulas) and the force integrands of the non-fluid cells (fluid cells
 // have none).  The FP64 pipe bounds it (12 additions per cell and the warps'
-// sums), so the ten conversions go to the integer pipes: 216 cubes of 24^3
-// 232 -> 170 us.
+// sums), so the conversions go to the integer pipes: 216 cubes of 24^3
+// 232 -> 170 us, with four CTAs of 64 registers an SM 165.
 struct LusState {
   size_t o;
   bool fluid;
@@ -352,7 +362,7 @@ struct LusState {
 
 constexpr int kUpdThreads = 256;
 
-__global__ void __launch_bounds__(kUpdThreads, 3) k_lus_update(LusgsSplitArgs a) {
+__global__ void __launch_bounds__(kUpdThreads, 4) k_lus_update(LusgsSplitArgs a) {
   __shared__ double red[kUpdThreads / 32][7];
   const int n = a.ph.n, S = n + 4, nn = n * n, NT = blockDim.x, tid = threadIdx.x;
   const int cube = 1 + blockIdx.x / n, i = blockIdx.x % n;
@@ -465,9 +475,10 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   if (e != cudaSuccess) return e;
   // One CTA per cube while the widest plane fits it (up to edge 24): the planes
   // are a chain, and a barrier of the CTA is cheaper than one of a cluster (216
-  // cubes of 24^3, the rest of a sub-iteration as above: 0.63 ms, by clusters
-  // of two 0.69; 8 cubes 0.29 and 0.30).  Wider planes go to clusters of four:
-  // 64 cubes of 32^3 0.62 ms, by one CTA of 768 threads 0.74; 512 the same.
+  // cubes of 24^3, the rest of a sub-iteration as above, before the words of 16
+  // bytes: 0.63 ms, by clusters of two 0.69; 8 cubes 0.29 and 0.30).  Wider
+  // planes go to clusters of four: 64 cubes of 32^3 0.62 ms, by one CTA of 768
+  // threads 0.74; now by clusters of two, four and eight 0.58, 0.56 and 0.58.
   const int size = lus_plane_cells(n, 1) <= kSweepThreads ? 1 : 4;
   k_lus_pack<<<ncubes * n, kSlabThreads, pack, s>>>(a, size);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -490,9 +501,11 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   cfg.attrs = at;
   cfg.numAttrs = 1;
   if ((e = cudaLaunchKernelEx(&cfg, sweep, a)) != cudaSuccess) return e;
-  // Three cells per thread or so: a warp's norm sums take 9 FP64 additions a
-  // turn on top of the 12 of each cell (two and four: the same within 1%).
-  const int ut = std::min(kUpdThreads, (nn / 3 + 31) / 32 * 32);
+  // Three cells per thread or so, six of large slabs: a warp's norm sums take 9
+  // FP64 additions a turn on top of the 12 of each cell (n = 16, three and six:
+  // 0.369 and 0.379 ms of a sub-iteration of 512 cubes; n = 24 0.503 and 0.494;
+  // n = 32 3.22 and 3.18).
+  const int ut = std::min(kUpdThreads, (nn / (n < 24 ? 3 : 6) + 31) / 32 * 32);
   k_lus_update<<<ncubes * n, ut, 0, s>>>(a);
   return cudaGetLastError();
 }
