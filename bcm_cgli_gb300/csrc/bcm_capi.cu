@@ -56,8 +56,12 @@ void dfree(T *&p) {
 }
 
 __global__ void k_time_shift(int n, int ncubes, const double2 *__restrict__ U1_,
-                             double2 *__restrict__ U1, double2 *__restrict__ U1q) {
-  // main.cpp:1292-1315: U1q <- U1, U1 <- U1_ on interior cells.  An interior
+                             double2 *__restrict__ U1, double2 *__restrict__ U1q,
+                             float2 *__restrict__ D2) {
+  // main.cpp:1292-1315: U1q <- U1, U1 <- U1_ on interior cells; split
+  // precision (D2): the FP32 difference of the two new levels, constant over
+  // the next step, while both are at hand (a pass of its own read them again:
+  // 7.1 M cells 184 + 203 us, now 224).  An interior
   // row (cube, i, j) is 5n contiguous doubles starting at an even cell index
   // (S even), so it moves as 5n/2 aligned 16-byte pairs; cubes on blockIdx.y.
   const int S = n + 4, rl = 5 * n / 2, per = n * n * rl;
@@ -68,6 +72,7 @@ __global__ void k_time_shift(int n, int ncubes, const double2 *__restrict__ U1_,
       const double2 a = U1[o], b = U1_[o];
       U1q[o] = a;
       U1[o] = b;
+      if (D2) D2[o] = make_float2(to_float_int(b.x - a.x), to_float_int(b.y - a.y));
     }
 }
 
@@ -808,13 +813,10 @@ int case_shift(bcmg_case *c) {
     k_time_shift<<<grid, 256, 0, c->stream>>>(n, c->ncube - 1,
                                               reinterpret_cast<const double2 *>(c->U1_),
                                               reinterpret_cast<double2 *>(c->U1),
-                                              reinterpret_cast<double2 *>(c->U1q));
+                                              reinterpret_cast<double2 *>(c->U1q),
+                                              reinterpret_cast<float2 *>(c->D2));
     CK(cudaGetLastError());
     ++c->launches;
-    if (c->precision == BCMG_PRECISION_SPLIT) {
-      CK(launch_level_diff(c->U1, c->U1q, c->D2, c->ph.n, c->ncube, c->stream));
-      ++c->launches;
-    }
   }
   return BCMG_OK;
 }

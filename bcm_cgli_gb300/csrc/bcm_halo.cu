@@ -88,7 +88,7 @@ __device__ __forceinline__ void level_face(const LayerArgs &a, const LayerCube &
       sum = sum + x[si + sj + sk];
       const int od = (ft.side == 1 ? n + 2 + l : l) * sx + (p + 2 + o0) * s0 + (q + 2 + o1) * s1 + v;
       z.U[od] = 0.125 * sum;
-      if (z.M) z.M[od] = mirror_value_hw(0.125 * sum, v, z.r0, z.e0);
+      if (z.M) z.M[od] = mirror_value(0.125 * sum, v, z.r0, z.e0);
     }
   }
 }
@@ -190,7 +190,7 @@ __device__ __forceinline__ void edge_fill(const LayerArgs &a, const LayerCube &z
       r = 0.5 * (xj + yi);
     }
     z.U[o] = r;
-    if (z.M) z.M[o] = mirror_value_hw(r, v, z.r0, z.e0);
+    if (z.M) z.M[o] = mirror_value(r, v, z.r0, z.e0);
   }
 }
 
@@ -377,7 +377,7 @@ __device__ __forceinline__ void bc_fill(const LayerArgs &a, const LayerCube &z, 
         U[d1] = x[b];
         U[d0] = x[b];
         if (M) {
-          const float mv = mirror_value_hw(x[b], v[b], z.r0, z.e0);
+          const float mv = mirror_value(x[b], v[b], z.r0, z.e0);
           M[d1] = mv; M[d0] = mv; Mo[d1] = mv; Mo[d0] = mv;
         }
       }
@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(kGhostThreads) k_ghost(GhostArgs a) {
       if (M) {
         double r0, e0_;
         mirror_base(a.mir, a.bt, e.ghost_cube, r0, e0_);
-        M[go] = mirror_value_hw(o, m, r0, e0_);
+        M[go] = mirror_value(o, m, r0, e0_);
       }
     }
     if (level_ends && more) __syncthreads(); else __syncwarp();
