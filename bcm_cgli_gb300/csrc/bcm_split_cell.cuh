@@ -506,21 +506,4 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
   }
 }
 
-// Sums of s[0..7] over the warp: lane l < 8 ends with value bit-reversed(l) in
-// s[0]; returns that value's number.
-__device__ __forceinline__ int norm_exchange(double *s, int lane) {
-#pragma unroll
-  for (int h = 4, b = 1; h >= 1; h >>= 1, b <<= 1) {
-    const bool up = lane & b;
-#pragma unroll
-    for (int m = 0; m < h; ++m) {
-      const double give = up ? s[m] : s[m + h], keep = up ? s[m + h] : s[m];
-      s[m] = keep + __shfl_xor_sync(0xffffffffu, give, b);
-    }
-  }
-  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 8);
-  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 16);
-  return 4 * (lane & 1) + 2 * ((lane >> 1) & 1) + ((lane >> 2) & 1);
-}
-
 }  // namespace bcmg
