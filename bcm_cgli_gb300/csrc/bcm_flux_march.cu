@@ -129,7 +129,7 @@ struct MarchShape {
 template <int NN, bool VISCOUS, bool PACK, bool NORMS>
 __global__ void __launch_bounds__(NN == 32 ? 512 : 256, NN == 32 ? 1 : 2)
     k_flux_march(FluxSplitArgs a, MarchShape sh) {
-  constexpr int CVT = NN == 24 || NN == 32 ? 3 : (NN >= 16 ? 1 : 0);  // measured there
+  constexpr int CVT = NN == 32 ? 3 : (NN >= 16 ? 1 : 2);  // measured there
   extern __shared__ __align__(16) float smem[];
   const int n = NN ? NN : a.ph.n, S = n + 4;
   const int tj = NN ? march_rows<NN>() : sh.tj;

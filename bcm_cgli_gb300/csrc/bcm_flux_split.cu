@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(split_threads<T>(), split_ctas_per_sm<T>())
   SplitLevels lv;
   float src[5];
   split_load(a, go, lv);
-  constexpr int CVT = T == 4 ? 3 : 0;
+  constexpr int CVT = 2;
   split_source<CVT>(lv, src);
   split_cell<VISCOUS, true, CVT>(a, z, cube, inv, P, BX(mi, mj, mk), acc, lv.x, src, dPdx, dPdz, go,
                       FL(mi, mj, mk) == kFluid, Mw, s5, [&](auto *U, const auto *un) {

@@ -312,12 +312,12 @@ __device__ __forceinline__ PrimF prim_split(const SplitConst &z, const float *q)
 // CVT: which conversions of a cell's stage go to the integer pipes (bit 0: FP64
 // to FP32, bit 1: FP32 to FP64; the same bits as the hardware's, which take a
 // slot of the FP64 pipe each).  Per stage of a 30-stage step, ns a cell, CVT 0,
-// 1, 3: march n = 16 (2,744 cubes) 0.152 0.142 0.142, n = 20 0.208 0.199 0.203,
-// n = 24 0.162 0.154 0.153, n = 28 0.201 0.192 0.198, n = 32 0.152 0.136 0.133;
-// tiles of 4^3 (4,096) 0.73 0.66 0.66.  Left to the hardware where the longer chain
-// of instructions costs more than the slot: march n = 8 0.376 0.381 0.385, n =
-// 12 (1,728) 0.204 0.220 0.224, edges without a kernel of their own (36) 0.202
-// 0.205 0.210, tiles of 8^3 (4,096) 0.227 0.233 0.233.
+// 1, 2, 3: march n = 8 0.314 0.320 0.314 0.323, n = 12 (1,728 cubes) 0.193 0.204
+// 0.193 0.213, n = 16 (2,744) 0.142 0.132 0.136 0.133, n = 20 0.187 0.177 0.180
+// 0.181, n = 24 0.149 0.142 0.145 0.147, n = 28 0.180 0.169 0.173 0.175, n = 32
+// 0.140 0.124 0.130 0.121, edges without a kernel of their own (36) 0.175
+// 0.174 0.171 0.179; tiles of 4^3 (4,096) 0.745 0.671 0.667 0.673, of 8^3 (4,096)
+// 0.215 0.219 0.211 0.220.
 template <int CVT>
 __device__ __forceinline__ float split_f(double x) {
   return (CVT & 1) ? to_float_int(x) : __double2float_rn(x);
@@ -400,49 +400,29 @@ __device__ __forceinline__ void split_cell(const FluxSplitArgs &a, const SplitCo
     const float Pc = z.P0 + (qm[4] - 0.5f * rho * VV) * Km1;
     const float Tt = Pc / rho;  // P/rho (:2302)
     const float C = K * Tt;
-    const float H = 0.5f * VV + C / Km1;
     const float qv = VV / C;
     const float beta = qv > z.ef ? qv : z.ef;
-    const float itemp = 1.0f / (K * Tt * (2 * dT + 3 * dTau) * (2 * dT + 3 * beta * dTau));
-    const float temp2 = Km1 * (beta - 1) * dT * dT;
-    const float temp3 = 0.5f * Km1 * VV;  // == H - H*K - VV + K*(T+VV) since C = K*T
-    const float bm1 = beta - 1;
-    const float a4 = 4 * temp3 * bm1 * dT * dT;
-    const float D = 3 * K * Tt * beta * dTau;
-    float d[5][5];
-    d[0][0] = (2 * dT * (-2 * (-Km1 * (H - VV) - temp3 * beta) * dT + D)) * itemp;
-    d[0][1] = (-4 * Uc * temp2) * itemp;
-    d[0][2] = (-4 * Vc * temp2) * itemp;
-    d[0][3] = (-4 * Wc * temp2) * itemp;
-    d[0][4] = (4 * temp2) * itemp;
-    d[1][0] = Uc * a4 * itemp;
-    d[1][1] = (2 * dT * (2 * K * (Tt - Uc * Uc * bm1) * dT + 2 * Uc * Uc * bm1 * dT + D)) * itemp;
-    d[1][2] = (-4 * Uc * Vc * temp2) * itemp;
-    d[1][3] = (-4 * Uc * Wc * temp2) * itemp;
-    d[1][4] = (4 * Uc * temp2) * itemp;
-    d[2][0] = Vc * a4 * itemp;
-    d[2][1] = d[1][2];
-    d[2][2] = (2 * dT * (2 * K * (Tt - Vc * Vc * bm1) * dT + 2 * Vc * Vc * bm1 * dT + D)) * itemp;
-    d[2][3] = (-4 * Vc * Wc * temp2) * itemp;
-    d[2][4] = (4 * Vc * temp2) * itemp;
-    d[3][0] = Wc * a4 * itemp;
-    d[3][1] = d[1][3];
-    d[3][2] = d[2][3];
-    d[3][3] = (2 * dT * (2 * K * (Tt - Wc * Wc * bm1) * dT + 2 * Wc * Wc * bm1 * dT + D)) * itemp;
-    d[3][4] = (4 * Wc * temp2) * itemp;
-    d[4][0] = H * a4 * itemp;
-    d[4][1] = (-4 * H * Uc * temp2) * itemp;
-    d[4][2] = (-4 * H * Vc * temp2) * itemp;
-    d[4][3] = (-4 * H * Wc * temp2) * itemp;
-    d[4][4] = (2 * dT * (2 * H * Km1 * bm1 * dT + K * Tt * (2 * dT + 3 * beta * dTau))) * itemp;
+    // The inverse preconditioner (:2315-2390) is diagonal plus rank one: with X =
+    // (1, u, v, w, H), Y = (V^2/2, -u, -v, -w, 1) and C = K T it is alpha (I +
+    // g (K-1)/C X Y^T), alpha = 2 dT / (2 dT + 3 dTau), g = 2 dT (beta-1) / (2 dT +
+    // 3 beta dTau).  In the energy, whose terms cancel to a part beta, h = 1 + g
+    // is formed as the product it is.  Its 25 entries written out take some 130
+    // operations more a cell (1 to 4% of the stage) and cancel in FP32.
+    const float iden = 1.0f / (2 * dT + 3 * beta * dTau);
+    const float g = 2 * dT * (beta - 1) * iden, h = beta * (2 * dT + 3 * dTau) * iden;
+    const float alpha = 2 * dT / (2 * dT + 3 * dTau);
     // Stage update Q += w dQ (w = 1, 1/4, 2/3): the reference's RK
     // combinations with Q1 = Q2 = Q on fluid cells at stage entry.
     const float w = a.RK == 1 ? 1.0f : (a.RK == 2 ? 0.25f : 2.0f / 3.0f);
-    float dq[5];
+    const float wa = w * dTau * alpha, VV2 = 0.5f * VV;
+    const float kin =
+        __fmaf_rn(-Uc, Rk[1], __fmaf_rn(-Vc, Rk[2], __fmaf_rn(-Wc, Rk[3], VV2 * Rk[0])));
+    const float gp = g * Km1 * (Rk[4] + kin) / C;
+    const float dq[5] = {wa * (Rk[0] + gp), wa * __fmaf_rn(Uc, gp, Rk[1]),
+                         wa * __fmaf_rn(Vc, gp, Rk[2]), wa * __fmaf_rn(Wc, gp, Rk[3]),
+                         wa * __fmaf_rn(h, Rk[4], __fmaf_rn(g, kin, VV2 * gp))};
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
-      dq[r] = w * dTau * (d[r][0] * Rk[0] + d[r][1] * Rk[1] + d[r][2] * Rk[2] +
-                          d[r][3] * Rk[3] + d[r][4] * Rk[4]);
       un[r] = xq[r] + split_d<CVT>(dq[r]);
       u[r] = un[r];
     }
