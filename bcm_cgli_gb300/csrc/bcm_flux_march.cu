@@ -18,17 +18,17 @@
 // pairs (PACK), like the tile kernel's two faces per thread.
 //
 // One RK-stage launch, tile kernel -> march (ms): 2,744 cubes of 16^3 1.726 ->
-// 1.301, 512 of 16^3 0.336 -> 0.269, 512 of 24^3 1.094 -> 0.887, 216 of 32^3
-// 1.096 -> 0.764; edges that 8 does not divide took 4^3 tiles: 512 cubes of
-// 12^3 0.361 -> 0.152, 216 of 20^3 0.696 -> 0.264, 125 of 28^3 1.104 -> 0.427.
-// 39% fewer instructions than the tiles at n = 16.  What bounds it now (ncu, n =
-// 16): instruction latency with four warps per scheduler (issue slots 42%
-// active; 128 registers and 107 KB a CTA allow no more), the FP64 pipe busy
-// with the cells' FP64 sums.  Tried and left out: nine warps of 96 registers
-// with a warp for the far faces (spills: 1.69 ms at 2,744 cubes), loading the
+// 1.278, 512 of 16^3 0.336 -> 0.259, 512 of 24^3 1.094 -> 0.871, 216 of 32^3
+// 1.096 -> 0.750; edges that 8 does not divide took 4^3 tiles: 512 cubes of
+// 12^3 0.361 -> 0.148, 216 of 20^3 0.696 -> 0.257, 125 of 28^3 1.104 -> 0.412.
+// 44% fewer instructions than the tiles at n = 16.  What bounds it now (ncu, n =
+// 16): instruction latency with four warps per scheduler (issue slots 43%
+// active, no pipe above 26%; 128 registers and 108 KB a CTA allow no more
+// warps).  Tried and left out, against 1.37 ms at 2,744 cubes then: nine warps
+// of 96 registers with a warp for the far faces (spills: 1.69), loading the
 // next cell's FP64 levels ahead into registers (spills: 1.63), whole cubes per
 // CTA instead of equal shares (1.34 there, but 0.294 at 512 cubes), one CTA of
-// 576 threads for n = 24 (1.11).
+// 576 threads for n = 24 (1.11 against 0.93).
 #include <algorithm>
 #include <type_traits>
 

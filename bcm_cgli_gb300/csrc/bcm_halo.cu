@@ -474,8 +474,8 @@ cudaError_t launch_layers(const LayerArgs &a, int ncubes, cudaStream_t s) {
 // of entries, a barrier between them; groups share no cube.  A sphere of
 // 2,792 entries in 32 cubes takes 21 levels, the later ones of some 40
 // entries: launches of a level each took 230 us (under ncu; 21 x 10.9), the
-// group's levels 74.  A stage of a step of that sphere among 400 cubes of 16^3,
-// split: 490 -> 374 us, among 96 cubes in FP64: 1057 -> 952.
+// group's levels 74.  A stage of a step of that sphere among 416 cubes of 16^3,
+// split: 490 -> 374 us, among 92 cubes in FP64: 1057 -> 952.
 //
 // Eight lanes per entry, one stencil cell each, the next entry's indices and
 // weights loaded ahead.  The FP64 pipe (64 cycles an instruction of a warp)
