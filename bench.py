@@ -753,7 +753,7 @@ def run_gpu_arm(args, dist):
                 except Exception:
                     traffic = None
         return {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
-                "frac": achieved / hbm_peak, "traffic": traffic, "kernel": f"k_flux_{prec}",
+                "frac": achieved / hbm_peak, "traffic": traffic, "kernel": "k_flux_march" if prec == "split" else "k_flux_fp64",
                 "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": m["flux_ms_avg"],
                 "launches": m["flux_launches"], "traffic_from": traffic_src,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)"}
