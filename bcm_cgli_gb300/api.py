@@ -191,12 +191,12 @@ def interface_lists(case):
     for ax in range(3):
         plus = case.adj[1:n, 1:5, 2 + 2 * ax].max(axis=1)
         minus = case.adj[1:n, 1:5, 1 + 2 * ax].max(axis=1)
-        # by the level difference to the neighbour, where there is one
+        # by the level of the neighbour, where there is one (compared, not
+        # subtracted: the levels may be of an unsigned type)
         p, m = plus > 0, minus > 0
-        dp = csl[1:n] - csl[np.where(p, plus, 0)]
-        dm = csl[1:n] - csl[np.where(m, minus, 0)]
-        out.append([_one_based(c[q]) for q in (p & (dp == 0), p & (dp > 0), p & (dp < 0),
-                                               m & (dm > 0), m & (dm < 0))])
+        own, lp, lm = csl[1:n], csl[np.where(p, plus, 0)], csl[np.where(m, minus, 0)]
+        out.append([_one_based(c[q]) for q in (p & (own == lp), p & (own > lp), p & (own < lp),
+                                               m & (own > lm), m & (own < lm))])
     return out
 
 
