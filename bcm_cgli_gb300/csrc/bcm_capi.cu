@@ -558,14 +558,23 @@ int case_exchange(bcmg_case *c) {  // sharded: the proxies' face bands
 // The closing interface call of a stage or sweep: kept for the next opening
 // one (sharded contexts run it at once, after the exchange).
 int case_closing(bcmg_case *c, IfaceList list = kIfaceFull) {
-  c->closing = LayerArgs();
-  interface_round(c, c->closing, 0, list);
-  c->has_closing = true;
-  if (!c->xchg) return BCMG_OK;
+  LayerArgs a;
+  interface_round(c, a, 0, list);
+  if (!c->xchg) {
+    c->closing = a;
+    c->has_closing = true;
+    return BCMG_OK;
+  }
   int r;
   if ((r = case_exchange(c))) return r;
+  return case_layers(c, a, c->ncube - 1);
+}
+
+// What a call that stopped on an error (an exchange hook's, say) left waiting
+// belongs to no later call.
+void case_begin(bcmg_case *c) {
   c->has_closing = false;
-  return case_layers(c, c->closing, c->ncube - 1);
+  c->phase = 0;
 }
 
 // The closing call that still waits, and the mirror flag brought up to date:
@@ -836,8 +845,7 @@ int case_mirror_all(bcmg_case *c) {
 
 int case_step(bcmg_case *c, int subiters) {
   int r;
-  c->has_closing = false;
-  c->phase = 0;
+  case_begin(c);
   if ((r = case_mirror_all(c))) return r;
   for (int it = 0; it < subiters; ++it)  // the step's first stage runs every face copy
     if ((r = case_subiter(c, it == 0))) return r;
@@ -890,8 +898,7 @@ int build_conv_graph(bcmg_case *c, int max_subiters, double tol) {
   cudaGraph_t body = p.conditional.phGraph_out[0];
   CK(cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, mode));
   const long long l0 = c->launches;
-  c->has_closing = false;
-  c->phase = 0;
+  case_begin(c);
   int r = case_subiter(c);
   if (!r) r = case_settle(c);
   if (!r) {
@@ -1509,8 +1516,7 @@ int bcmg_case_stage(bcmg_case *c, int RK) {
   clear_err();
   if (!c || RK < 1 || RK > 3) { set_err("bad context or RK"); return BCMG_ERR_ARG; }
   c->launches = 0;
-  c->has_closing = false;
-  c->phase = 0;
+  case_begin(c);
   int r = case_mirror_all(c);
   if (!r) r = case_stage(c, RK);
   if (!r) r = case_settle(c);
@@ -1657,6 +1663,7 @@ int bcmg_case_time_flux(bcmg_case *c, int reps, double *ms) {
   const size_t bytes = c->ncell * 5 * sizeof(double);
   // The split kernel applies its stage update in place: keep a copy of the
   // state in the (split-unused) U1p1 buffer and restore it afterwards.
+  case_begin(c);
   if (c->precision == BCMG_PRECISION_SPLIT)
     CK(cudaMemcpyAsync(c->U1p1, c->U1_, bytes, cudaMemcpyDeviceToDevice, c->stream));
   int r = case_mirror_all(c);
@@ -1914,8 +1921,7 @@ int bcmg_case_advance_converged(bcmg_case *c, int steps, int max_subiters, doubl
       CK(cudaGetLastError());
     }
   } else {
-    c->has_closing = false;
-    c->phase = 0;
+    case_begin(c);
     for (int st = 0; st < steps; ++st) {
       k_conv_reset<<<1, 128, 0, c->stream>>>(c->active, c->iters, c->ncase);
       CK(cudaGetLastError());
