@@ -584,6 +584,7 @@ cudaError_t launch_flux_march(const FluxSplitArgs &a, int ncubes, cudaStream_t s
     if (n == 32) return launch_march_n<32, true>(a, sh, grid, threads, L.bytes(), s);
     return launch_march_n<0, true>(a, sh, grid, threads, L.bytes(), s);
   }
+  if (n == 8) return launch_march_n<8, false>(a, sh, grid, threads, L.bytes(), s);
   if (n == 12) return launch_march_n<12, false>(a, sh, grid, threads, L.bytes(), s);
   if (n == 20) return launch_march_n<20, false>(a, sh, grid, threads, L.bytes(), s);
   if (n == 28) return launch_march_n<28, false>(a, sh, grid, threads, L.bytes(), s);
