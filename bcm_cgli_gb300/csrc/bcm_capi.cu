@@ -268,6 +268,13 @@ struct bcmg_case {
   }
   float *D2 = nullptr;                   // split precision: FP32 of U1 - U1q
   float *inv_dx = nullptr;               // split precision: n / cube_size per cube
+  // Split precision forms no U1p1, U1p2 and Rku1 (its stages update in place), so
+  // what it needs of its own lies there: the copy of a state while a kernel is
+  // timed in U1p1; in U1p2 and Rku1, one allocation of 80 bytes a padded cell, the
+  // LU-SGS scratch (64 bytes an interior cell, at most 45 a padded one: edges up to
+  // 32), from byte 58 the cell codes of FWS and from byte 60 the FP32 residual.
+  float *lu_scr() const { return reinterpret_cast<float *>(U1p2); }
+  float *residual32() const { return reinterpret_cast<float *>(U1p2) + 15 * ncell; }
   uint16_t *codes = nullptr;             // split precision: cell codes of FWS
   int *FWS = nullptr;
   double *cube_size = nullptr;
@@ -355,7 +362,6 @@ struct bcmg_case {
   cudaGraphExec_t cgraph = nullptr;  // step graph with the while node
   int cgraph_max = -1, cgraph_method = -1;
   double cgraph_tol = -1;
-  float *lu_scr = nullptr;  // split LU-SGS sweep scratch
   // PLOT3D output (bcmg_case_output_*): device byte image, a side stream for
   // the copies, two pinned chunks and the writer thread.
   int device = 0;
@@ -413,11 +419,12 @@ struct bcmg_case {
     graph = nullptr;
     if (cgraph) cudaGraphExecDestroy(cgraph);
     cgraph = nullptr;
-    dfree(active); dfree(iters); dfree(cont); dfree(lu_scr);
+    dfree(active); dfree(iters); dfree(cont);
     for (auto x : ev) cudaEventDestroy(x);
     ev.clear();
-    dfree(U1_); dfree(U1); dfree(U1q); dfree(U1p1); dfree(U1p2); dfree(Rku1); dfree(Residual1);
-    dfree(M); dfree(M2); dfree(mpar); dfree(D2); dfree(inv_dx); dfree(codes);
+    dfree(U1_); dfree(U1); dfree(U1q); dfree(U1p1); dfree(U1p2); dfree(Residual1);
+    Rku1 = nullptr;  // (in U1p2's allocation)
+    dfree(M); dfree(M2); dfree(mpar); dfree(D2); dfree(inv_dx);
     dfree(FWS); dfree(cube_size); dfree(push); dfree(flags); dfree(bc_cubes);
     faces.free(); faces_p.free(); faces_j.free(); faces_q.free(); faces_r.free();
     dfree(bc_flags); dfree(partials); dfree(er); dfree(emax);
@@ -501,9 +508,7 @@ int case_flux(bcmg_case *c, int RK) {
     sa.U1q = c->U1q;
     sa.D2 = c->D2;
     sa.RK = RK;
-    // RK 0 (LU-SGS): FP32 residual into the Rku1 buffer, which the split
-    // path does not otherwise use
-    sa.R32 = reinterpret_cast<float *>(c->Rku1);
+    sa.R32 = c->residual32();  // RK 0 (LU-SGS)
     sa.tile = c->tile;
     sa.form = c->form == 2 ? 0 : 1;
     sa.partials = c->partials;
@@ -668,8 +673,8 @@ LusgsSplitArgs lusgs_split_args(bcmg_case *c) {
   l.inv_dx = c->inv_dx;
   l.mir = c->mir();
   l.U1_ = c->U1_;
-  l.R32 = reinterpret_cast<float *>(c->Rku1);
-  l.scr = c->lu_scr;
+  l.R32 = c->residual32();
+  l.scr = c->lu_scr();
   l.Residual1 = c->Residual1;
   l.partials = c->partials;
   l.bt = c->bt();
@@ -1211,7 +1216,7 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
   const size_t nd = c->ncell * 5;
   bool ok = ck(dalloc(&c->U1_, nd), "alloc") && ck(dalloc(&c->U1, nd), "alloc") &&
             ck(dalloc(&c->U1q, nd), "alloc") && ck(dalloc(&c->U1p1, nd), "alloc") &&
-            ck(dalloc(&c->U1p2, nd), "alloc") && ck(dalloc(&c->Rku1, nd), "alloc") &&
+            ck(dalloc(&c->U1p2, 2 * nd), "alloc") &&  // and Rku1 after it
             ck(dalloc(&c->Residual1, nd), "alloc") && ck(dalloc(&c->FWS, c->ncell), "alloc") &&
             ck(dalloc(&c->cube_size, (size_t)d->ncube), "alloc") &&
             ck(dalloc(&c->flags, (size_t)d->ncube), "alloc") &&
@@ -1221,16 +1226,18 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
             ck(dalloc(&c->nsum, 7), "alloc") &&
             ck(dalloc(&c->emax, 6 * (size_t)c->ncase), "alloc");
   if (!ok) return fail(BCMG_ERR_CUDA);
+  c->Rku1 = c->U1p2 + nd;
   if (d->precision == BCMG_PRECISION_SPLIT &&
       !(ck(dalloc(&c->M, nd), "alloc") && ck(dalloc(&c->M2, nd), "alloc") &&
         ck(dalloc(&c->mpar, 1), "alloc") && ck(cudaMemset(c->mpar, 0, sizeof(int)), "memset") &&
         ck(dalloc(&c->D2, nd), "alloc") && ck(cudaMemset(c->D2, 0, nd * sizeof(float)), "memset") &&
         ck(dalloc(&c->inv_dx, (size_t)d->ncube), "alloc") &&
-        ck(dalloc(&c->codes, c->ncell), "alloc") &&
         ck(cudaMemset(c->M, 0, nd * sizeof(float)), "memset") &&
         ck(cudaMemset(c->M2, 0, nd * sizeof(float)), "memset") &&
         true))
     return fail(BCMG_ERR_CUDA);
+  if (d->precision == BCMG_PRECISION_SPLIT)
+    c->codes = reinterpret_cast<uint16_t *>(c->U1p2) + 29 * c->ncell;
   if (c->inv_dx) {
     std::vector<float> inv((size_t)d->ncube, 0.f);
     for (int i = 1; i < d->ncube; ++i) inv[i] = (float)(d->n / d->cube_size[i]);
@@ -1863,8 +1870,6 @@ int bcmg_case_set_method(bcmg_case *c, int method, double cfl, double omega) {
     set_err("LU-SGS needs n <= 32 (one thread per cube column)");
     return BCMG_ERR_ARG;
   }
-  if (method == BCMG_METHOD_LUSGS && c->precision == BCMG_PRECISION_SPLIT && !c->lu_scr)
-    CK(dalloc(&c->lu_scr, lusgs_split_scratch(c->ph.n) * (size_t)(c->ncube - 1)));
   c->method = method;
   c->lu_cfl = cfl;
   c->lu_omega = omega;
@@ -2266,7 +2271,7 @@ int bcmg_case_autotune(bcmg_case *c, int reps, bcmg_tuning *out) {
   // Split LU-SGS sweep: the widest plane's threads or half of them (wide
   // planes then take two passes), timed on the residual of the current
   // state; the state is restored afterwards.
-  if (c->precision == BCMG_PRECISION_SPLIT && c->method == BCMG_METHOD_LUSGS && c->lu_scr) {
+  if (c->precision == BCMG_PRECISION_SPLIT && c->method == BCMG_METHOD_LUSGS) {
     const int full = lusgs_split_default_threads(n);
     const int cand[2] = {full, ((full / 2) + 31) / 32 * 32};
     const size_t bytes = c->ncell * 5 * sizeof(double);
@@ -2389,10 +2394,11 @@ struct Compat {
   FaceTask *tasks = nullptr;
   size_t tasks_cap = 0;
   Ibm ibm;
-  // split-precision flux twin (bcmg_set_reference_precision): mirror
-  // buffers and flag, FP32 level difference, n / cube_size
+  // split-precision flux twin (bcmg_set_reference_precision): mirror buffer
+  // (each call forms it anew, so there is no second one) and flag, FP32 level
+  // difference, n / cube_size
   int precision = BCMG_PRECISION_FP64;
-  float *M = nullptr, *M2 = nullptr, *D2 = nullptr, *inv_dx = nullptr;
+  float *M = nullptr, *D2 = nullptr, *inv_dx = nullptr;
   int *mpar = nullptr;
   uint16_t *codes = nullptr;  // cell codes of the call's flags
 
@@ -2420,7 +2426,7 @@ struct Compat {
     if (nc == ncube && Sx == full_S && U1_) return BCMG_OK;
     dfree(U1_); dfree(U1); dfree(U1q); dfree(U1p1); dfree(U1p2); dfree(Rku1);
     dfree(Residual1); dfree(cube_size); dfree(partials); dfree(er); dfree(FWS);
-    dfree(M); dfree(M2); dfree(D2); dfree(inv_dx); dfree(mpar); dfree(codes);
+    dfree(M); dfree(D2); dfree(inv_dx); dfree(mpar); dfree(codes);
     ncube = nc;
     S = full_S = Sx;
     ncell = (size_t)nc * S * S * S;
@@ -2438,7 +2444,7 @@ struct Compat {
   int ensure_split() {
     if (M) return BCMG_OK;
     const size_t nd = ncell * 5;
-    CK(dalloc(&M, nd)); CK(dalloc(&M2, nd)); CK(dalloc(&D2, nd));
+    CK(dalloc(&M, nd)); CK(dalloc(&D2, nd));
     CK(dalloc(&inv_dx, (size_t)ncube)); CK(dalloc(&mpar, 1)); CK(dalloc(&codes, ncell));
     CK(cudaMemsetAsync(mpar, 0, sizeof(int), s));
     return BCMG_OK;
@@ -2802,7 +2808,7 @@ void BCM_Flux_XYZ_Viscous_Runge_kutta(int myid, int ncube, int RK, double deltaT
       std::vector<float> inv((size_t)ncube, 0.f);
       for (int i = 1; i < ncube; ++i) inv[i] = (float)(ph.n / cube_size[i]);
       CK(cudaMemcpyAsync(C.inv_dx, inv.data(), sizeof(float) * ncube, cudaMemcpyHostToDevice, s));
-      CK(launch_mirror(C.U1_, C.M, C.M2, ph.n, ncube, ph.rho0, ph.P0, Batch(), s));
+      CK(launch_mirror(C.U1_, C.M, nullptr, ph.n, ncube, ph.rho0, ph.P0, Batch(), s));
       CK(launch_level_diff(C.U1, C.U1q, C.D2, ph.n, ncube, s));
       CK(launch_cell_codes(C.FWS, C.codes, ph.n, ncube, s));
       FluxSplitArgs sa;
@@ -2823,7 +2829,6 @@ void BCM_Flux_XYZ_Viscous_Runge_kutta(int myid, int ncube, int RK, double deltaT
       sa.FWS = C.FWS;
       sa.cube_size = C.cube_size;
       sa.mir.buf[0] = C.M;
-      sa.mir.buf[1] = C.M2;
       sa.mir.parity = C.mpar;
       sa.mir.rho0 = ph.rho0;
       sa.mir.E0 = ph.P0 / (BCMG_K - 1);

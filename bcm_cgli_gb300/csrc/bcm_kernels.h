@@ -201,7 +201,7 @@ struct LusgsSplitArgs {
   Mirror mir;              // FP32 deltas of the state: read and updated in place
   double *U1_;             // updated in place on fluid cells
   float *R32;              // in: residual (FP32) of every cell; out: increment
-  float *scr;              // [ncube-1][16][n^3] sweep scratch (lusgs_split_scratch)
+  float *scr;              // [ncube-1][16][n^3] sweep scratch
   int threads = 0;         // most threads per sweeping CTA (0: its widest plane)
   const double *Residual1;
   double *partials;        // [ncube-1][lusgs_split_blocks][7]
@@ -212,8 +212,6 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
 // Norm partial sums per cube and kernels of one launch_lusgs_split call.
 int lusgs_split_blocks(int n);
 int lusgs_split_launches();
-// Floats of that scratch per cube.
-size_t lusgs_split_scratch(int n);
 // Default threads per cube of the split LU-SGS kernel (the widest plane).
 int lusgs_split_default_threads(int n);
 

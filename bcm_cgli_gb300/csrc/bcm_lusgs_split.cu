@@ -456,7 +456,6 @@ int lus_plane_cells(int n, int size) {
 
 }  // namespace
 
-size_t lusgs_split_scratch(int n) { return (size_t)4 * kWords * n * n * n; }
 int lusgs_split_blocks(int n) { return n; }
 int lusgs_split_launches() { return 3; }
 

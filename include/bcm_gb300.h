@@ -259,7 +259,8 @@ void bcmg_case_destroy(bcmg_case *c);
  * pointer may be NULL to skip that array. */
 int bcmg_case_set_state(bcmg_case *c, const double *U1_, const double *U1, const double *U1q);
 int bcmg_case_get_state(bcmg_case *c, double *U1_, double *U1, double *U1q);
-/* Scratch arrays as the reference keeps them (for parity checks). */
+/* Scratch arrays as the reference keeps them (for parity checks; FP64.  The
+ * split path forms no U1p1, U1p2 and Rku1 and keeps values of its own in them). */
 int bcmg_case_get_scratch(bcmg_case *c, double *U1p1, double *U1p2, double *Rku1,
                           double *Residual1);
 
