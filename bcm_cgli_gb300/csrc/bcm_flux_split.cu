@@ -481,13 +481,23 @@ int flux_tile(int n, int tile) {
   return n % 8 == 0 ? 8 : 4;
 }
 
-// The march serves every cube edge from 12 on that fits its shared memory.
+// Which kernel serves a cube edge.  The march holds seven planes of its rows in
+// shared memory, so the larger the edge, the fewer its rows (4 at 48, 2 at 52 to
+// 64, 1 at 68 to 80) and the more often values are loaded and formed, while 8^3
+// tiles cost the same per cell at every edge they divide: 8^3 tiles and march, us a
+// launch, 40 (64 cubes) 643 592, 48 (27) 475 390, 56 (27) 746 927, 64 (27) 1097
+// 1163, 72 (8) 477 825, 80 (27) 2129 3389.  Edges that 8 does not divide would take
+// 4^3 tiles, which the march beats wherever it fits: 52 (27) 1533 923, 60 (27) 2355
+// 1179, 68 (8) 1023 784, 76 (8) 1428 922.
 // For n = 8 a whole cube is one tile: the march wins while its two-plane
 // units spread few cubes over the SMs (8 cubes 26 -> 20 us, 216 cubes 34 ->
 // 28 us); the tile kernel's 18 warps per SM against 12 win from about 700
 // cubes on (1000 cubes: 101 against 109 us).  Both leave the same bits,
 // norms included.
-static bool use_march(int n, int tile) { return tile != 4 && flux_march_fits(n); }
+constexpr int kMarchEdge8 = 48;  // the largest edge divisible by 8 that marches
+static bool use_march(int n, int tile) {
+  return tile != 4 && flux_march_fits(n) && (n % 8 != 0 || n <= kMarchEdge8);
+}
 constexpr int kMarchCubes8 = 700;
 
 int flux_split_blocks(int n, int ncubes, int tile) {
