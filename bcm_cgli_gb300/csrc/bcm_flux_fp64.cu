@@ -810,28 +810,36 @@ __global__ void __launch_bounds__(kFluxThreads, 1) k_flux_fp64(FluxArgs a, Sh sh
   }
 }
 
-// The box of a cube edge that is not a multiple of 8: divisors of n, at most
-// 512 cells in all groups together, with the least time per cell by the
-// measured weights of a turn of the 512 threads over faces (0.36), primitives
-// (0.08) and cells (0.95, however many of the threads have one).
-static ShapeAny flux_shape(int n, int tile) {
+// The boxes of a cube edge that is not a multiple of 8: divisors of n, at most
+// 512 cells in all groups together, with the least waves of CTAs (one to an SM)
+// times the time of a CTA: 28 us, 11 per turn of the 512 threads over its faces,
+// 0.047 per face and 0.006 per primitive (fitted to 186 launches of one wave at
+// edges 4 to 36, within 13%).  Of the groups with the least
+// waves the fewest: where few boxes fill one wave, large CTAs would leave SMs idle
+// (one cube of 20^3 in 16 CTAs of 500 cells 160 us, in 125 of 64 cells 51; eight of
+// 4^3 in two CTAs 139, in eight 51; 64 of 12^3 271, now 257).
+static ShapeAny flux_shape(int n, int tile, int ncubes) {
+  constexpr int kSms = 152;
   ShapeAny best{4, 4, 4, 1};
-  double score = 0;
+  double least = 1e300;
   auto consider = [&](int i, int j, int k) {
     ShapeAny s{i, j, k, 1};
-    if (box_cells(s) > kFluxThreads || flux_smem(s) > 227 * 1024) return;
-    while ((s.groups + 1) * box_cells(s) <= kFluxThreads) {
-      ++s.groups;
-      if (flux_smem(s) > 227 * 1024) {
-        --s.groups;
-        break;
-      }
-    }
+    const int cells = box_cells(s), faces = box_faces(s);
+    if (cells > kFluxThreads || flux_smem(s) > 227 * 1024) return;
+    s.groups = 2;  // shared memory grows by as much with every box
+    const size_t two = flux_smem(s);
+    s.groups = 1;
+    const size_t one = flux_smem(s);
+    const int most = (int)std::min<size_t>(kFluxThreads / cells,
+                                           1 + (227 * 1024 - one) / (two - one));
+    const long long boxes = (long long)ncubes * (n / i) * (n / j) * (n / k);
+    const long long waves = (boxes + (long long)kSms * most - 1) / ((long long)kSms * most);
+    s.groups = (int)((boxes + kSms * waves - 1) / (kSms * waves));
+    const int turns = (s.groups * faces + kFluxThreads - 1) / kFluxThreads;
     const double t =
-        s.groups * (0.36 * box_faces(s) + 0.08 * box_prims(s)) / kFluxThreads + 0.95;
-    const double v = s.groups * box_cells(s) / t;
-    if (v > score * 1.0001) {
-      score = v;
+        waves * (28 + 11 * turns + s.groups * (0.047 * faces + 0.006 * box_prims(s)));
+    if (t < least * 0.9999) {
+      least = t;
       best = s;
     }
   };
@@ -842,6 +850,7 @@ static ShapeAny flux_shape(int n, int tile) {
   int d[64], nd = 0;  // divisors of n (at most 256)
   for (int i = 1; i <= n; ++i)
     if (n % i == 0) d[nd++] = i;
+  // (of a box's turns the one that is longest along k, whose rows are contiguous)
   for (int i = 0; i < nd; ++i)
     for (int j = 0; j < nd; ++j)
       for (int k = 0; k < nd; ++k) consider(d[i], d[j], d[k]);
@@ -870,7 +879,12 @@ cudaError_t launch_flux_fp64(const FluxArgs &a, int ncubes, cudaStream_t s) {
     const Shape888 sh;
     return visc ? launch_shape<true>(a, sh, ncubes, s) : launch_shape<false>(a, sh, ncubes, s);
   }
-  const ShapeAny sh = flux_shape(a.ph.n, a.tile);
+  if (ncubes <= 0) return cudaSuccess;
+  // (a search of a few us: a caller's launches in a row are of one size)
+  thread_local struct { int n = 0, tile, ncubes; ShapeAny sh; } last;
+  if (last.n != a.ph.n || last.tile != a.tile || last.ncubes != ncubes)
+    last = {a.ph.n, a.tile, ncubes, flux_shape(a.ph.n, a.tile, ncubes)};
+  const ShapeAny sh = last.sh;
   return visc ? launch_shape<true>(a, sh, ncubes, s) : launch_shape<false>(a, sh, ncubes, s);
 }
 
