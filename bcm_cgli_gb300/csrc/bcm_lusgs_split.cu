@@ -171,9 +171,9 @@ __global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a, int
   const float idx = a.inv_dx[cube];
   const float *const Mc = mirror_current(a.mir);
   slab_starts(start, n);
-  for (int d = threadIdx.x; d < 2 * n - 1; d += kSlabThreads)
+  for (int d = threadIdx.x; d < 2 * n - 1; d += blockDim.x)
     place[d] = plane_start(i + d, n) + row_start(i + d, i, n, size) - jlo_of(i + d, i, n);
-  for (int jk = threadIdx.x; jk < nn; jk += kSlabThreads) {
+  for (int jk = threadIdx.x; jk < nn; jk += blockDim.x) {
     const int j = jk / n, k = jk - j * n;
     const size_t o = cell_index(S, cube, i + 2, j + 2, k + 2);
     float m[5], kc[10];
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kSlabThreads) k_lus_pack(LusgsSplitArgs a, int
   }
   __syncthreads();
   float4 *const scr = reinterpret_cast<float4 *>(a.scr) + (size_t)(cube - 1) * kWords * nn * n;
-  for (int t = threadIdx.x; t < nn; t += kSlabThreads) {
+  for (int t = threadIdx.x; t < nn; t += blockDim.x) {
     int j, k;
     slab_cell(start, n, t, j, k);
     float4 *dst = scr + place[j + k] + j;
@@ -479,7 +479,9 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   // planes go to clusters of four: 64 cubes of 32^3 0.62 ms, by one CTA of 768
   // threads 0.74; now by clusters of two, four and eight 0.58, 0.56 and 0.58.
   const int size = lus_plane_cells(n, 1) <= kSweepThreads ? 1 : 4;
-  k_lus_pack<<<ncubes * n, kSlabThreads, pack, s>>>(a, size);
+  // (a thread a cell of a slab: 256 whatever the slab took 25 us more for 4,096
+  // cubes of 4^3)
+  k_lus_pack<<<ncubes * n, std::min(kSlabThreads, (nn + 31) / 32 * 32), pack, s>>>(a, size);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   int threads = (lus_plane_cells(n, size) + 31) / 32 * 32;
   if (a.threads > 0) threads = std::min(threads, a.threads);  // wide planes take several passes
@@ -498,7 +500,7 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = size > 1;  // (clusters of one start slowly: 4,096 cubes of 4^3 66 us, now 34)
   if ((e = cudaLaunchKernelEx(&cfg, sweep, a)) != cudaSuccess) return e;
   // Three cells per thread or so, six of large slabs: a warp's norm sums take 9
   // FP64 additions a turn on top of the 12 of each cell (n = 16, three and six:
