@@ -446,9 +446,10 @@ class CaseContext:
                                        o.ctypes.data))
 
     def set_tuning(self, flux_tile=0, lusgs_threads=0, flux_form=0):
-        """Launch shapes: flux tile edge (0, 4 or 8), threads per cube of the
-        split LU-SGS sweep (0: the widest plane) and the split flux form on
-        8^3 tiles (1 packed face pairs, 2 one face at a time, 0 default)."""
+        """Launch shapes: flux shape (0, or 8 where it divides n, the default;
+        4 for 4^3 tiles), most threads of a CTA of the split LU-SGS sweep (0:
+        its widest plane) and the split flux form of edges that 8 divides (1
+        packed face pairs, 2 one face at a time, 0 default)."""
         t = _lib.Tuning(int(flux_tile), int(lusgs_threads), int(flux_form))
         check(lib().bcmg_case_set_tuning(self.h, C.byref(t)))
 
@@ -477,7 +478,9 @@ class CaseContext:
 
     def autotune(self, reps=3):
         """Times the launch-shape candidates on this context's state, applies the
-        fastest and returns the choice with the measured milliseconds."""
+        fastest and returns the choice with the measured milliseconds (of the
+        flux: "8_packed" the default shape, "8_single" the same one face at a
+        time, "4" the 4^3 tiles)."""
         t = _lib.Tuning()
         check(lib().bcmg_case_autotune(self.h, int(reps), C.byref(t)))
         return {"flux_tile": t.flux_tile, "lusgs_threads": t.lusgs_threads,

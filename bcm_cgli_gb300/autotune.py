@@ -8,10 +8,11 @@ path (FP64 / split precision, RK / LU-SGS sub-iterations) it builds a
 Taylor-Green case of 2-3 million cells (8^3 cubes of 16^3, 6^3 of 24^3, 4^3
 of 32^3: many waves of CTAs, as in the benchmark workloads; a case of a
 wave or two favours the smaller tile through its tail alone), lets
-bcmg_case_autotune time the flux tile edges (8, 4) and, for split LU-SGS,
-the sweep's thread counts (widest plane, half of it), and records the
-fastest shape with the measured times.  The shapes change how work is
-spread over the GPU, never a cell's arithmetic.
+bcmg_case_autotune time the flux shapes (the default, on the split path also
+with one face at a time, and 4^3 tiles) and, for split LU-SGS, the sweep's
+thread counts (widest plane, half of it), and records the fastest shape with
+the measured times.  The shapes change how work is spread over the GPU, not the
+FP64 path's arithmetic.
 """
 from __future__ import annotations
 

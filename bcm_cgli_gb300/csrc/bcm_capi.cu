@@ -2150,11 +2150,11 @@ int bcmg_case_mirror_current(bcmg_case *c, float *M) {
 }
 
 // ---------------------------------------------------------------------------
-// Launch-shape tuning.  The choices change how work is split across CTAs,
-// never the arithmetic of a cell: the FP64 path stays bit-identical to the
-// reference with either tile edge (each cell's operations are the same), the
-// split path's results change only by where a CTA boundary falls in its
-// fixed-order norm sums.
+// Launch-shape tuning.  The choices change how work is split across CTAs.  The
+// FP64 path stays bit-identical to the reference with every shape (each cell's
+// operations are the same).  On the split path the forms round differently,
+// march and tiles may differ in the last place next to non-fluid cells, and
+// the norm sums' order follows the shape.
 // ---------------------------------------------------------------------------
 int bcmg_case_set_tuning(bcmg_case *c, const bcmg_tuning *t) {
   clear_err();
@@ -2242,14 +2242,15 @@ int bcmg_case_autotune(bcmg_case *c, int reps, bcmg_tuning *out) {
   best.flux_tile = c->tile;
   best.lusgs_threads = c->lu_threads;
   best.flux_form = c->form;
-  // Flux: tile 8 with packed face pairs, tile 8 one face at a time (the two
-  // forms differ on the split path only), tile 4; each timed on the
-  // context's own state (bcmg_case_time_flux restores it).
-  const int tiles[3] = {8, 8, 4}, forms[3] = {1, 2, 0};
+  // Flux: the default shape (edges that 8 divides: flux_tile 8, in packed face
+  // pairs and one face at a time, which differ on the split path only; other
+  // edges: flux_tile 0), tile 4; each timed on the context's own state
+  // (bcmg_case_time_flux restores it).
+  const bool by8 = n % 8 == 0;
+  const int tiles[3] = {by8 ? 8 : 0, 8, 4}, forms[3] = {by8 ? 1 : 0, 2, 0};
   double best_ms = 1e300;
   for (int v = 0; v < 3; ++v) {
-    if (n % tiles[v] != 0) continue;
-    if (v == 1 && c->precision != BCMG_PRECISION_SPLIT) continue;
+    if (v == 1 && (!by8 || c->precision != BCMG_PRECISION_SPLIT)) continue;
     bcmg_tuning t = best;
     t.flux_tile = tiles[v];
     t.flux_form = forms[v];

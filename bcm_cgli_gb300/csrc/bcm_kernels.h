@@ -95,7 +95,7 @@ struct FluxSplitArgs {
   int RK;              // stage 1..3: the kernel applies the stage update;
                        // 0: it writes the FP32 residual to R32 instead
   float *R32 = nullptr;  // [ncell][5] (RK == 0)
-  int tile = 0;          // 4: 4^3 tiles; else the march where it serves n, or
+  int tile = 0;          // 4: 4^3 tiles; else the march where it is faster, or
                          // 8^3 tiles (4^3 where 8 does not divide n)
   int form = 0;          // 0 faces one at a time, 1 in packed FP32 pairs
   double *partials;    // [blocks][7] norm/force partial sums (stage 3)

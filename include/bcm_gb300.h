@@ -321,22 +321,29 @@ int bcmg_case_mirror(bcmg_case *c, float *M);
  * in every cell. */
 int bcmg_case_mirror_current(bcmg_case *c, float *M);
 
-/* Launch shapes.  flux_tile: edge of the cube tile one flux CTA works on,
- * 8 or 4 (0: 8 when it divides n, else 4); flux_form (split precision, 8^3
- * tiles): 1 each thread evaluates its two faces of an axis together in
- * packed FP32 pairs (Blackwell FFMA2/FADD2/FMUL2), 2 one after the other, 0
- * the default (1); lusgs_threads: threads per cube of the split-precision
- * LU-SGS sweep, a multiple of 32 up to the widest plane of a cube (0: the
- * widest plane; fewer threads take wide planes in several passes).  The
- * shapes change how work is spread over the GPU, not the FP64 path's
- * arithmetic (it stays bit-identical to the reference); the two split flux
- * forms round differently (both within the split path's error bound).
+/* Launch shapes.  flux_tile: 0, or 8 where it divides n, the default: on the
+ * split path a march along i through a cube's planes where that is faster
+ * (edges 12 to 48 and larger ones that 8 does not divide, as far as the planes
+ * fit; 8^3 cubes while they are fewer than 700), elsewhere 8^3 tiles; in FP64 8^3
+ * boxes, for edges that 8 does not divide boxes by the edge and the number of
+ * cubes.  4: 4^3 tiles.  flux_form (split precision, edges that 8 divides): 1 two
+ * faces together in packed FP32 pairs (Blackwell FFMA2/FADD2/FMUL2), 2 one after
+ * the other, 0 the default (1); 4^3 tiles and other edges take one after the
+ * other.  lusgs_threads: most threads of a CTA of the split-precision LU-SGS
+ * sweep, a multiple of 32 up to the widest plane of a cube (0: the widest
+ * plane of a CTA; one CTA sweeps a cube, four a cube of edge 28 or 32; fewer
+ * threads take wide planes in several passes).  The shapes change how work is
+ * spread over the GPU, not the FP64 path's arithmetic (it stays bit-identical to
+ * the reference); on the split path the two forms round differently, and march
+ * and tiles may differ in the last place next to non-fluid cells (all within the
+ * split path's error bound).
  * bcmg_case_autotune times the candidates on the context's own state with
  * CUDA events (`reps` launches each, state restored), applies the fastest
- * and reports every time in `out` (flux_ms: tile 8 packed, tile 8 one face
- * at a time, tile 4; lusgs_ms: widest plane, half of it; 0 where not
- * measured).  The LU-SGS candidates are timed only on the split path with
- * LU-SGS selected. */
+ * and reports every time in `out` (flux_ms: the default shape, the default with
+ * one face at a time, 4^3 tiles; lusgs_ms: widest plane, half of it; 0 where not
+ * measured).  The default shape is reported as flux_tile 8 where 8 divides n, else
+ * as 0.  The LU-SGS candidates are timed only on the split path with LU-SGS
+ * selected. */
 typedef struct bcmg_tuning {
   int flux_tile;
   int lusgs_threads;
