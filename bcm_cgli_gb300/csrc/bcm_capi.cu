@@ -2166,7 +2166,7 @@ int bcmg_case_set_tuning(bcmg_case *c, const bcmg_tuning *t) {
   }
   if (t->lusgs_threads != 0 &&
       (n * n > 1024 || t->lusgs_threads % 32 != 0 || t->lusgs_threads < 32 ||
-       t->lusgs_threads > lusgs_split_default_threads(n))) {
+       t->lusgs_threads > lusgs_split_most_threads(n))) {
     set_err("lusgs_threads must be 0 or a multiple of 32 up to the widest plane of a cube");
     return BCMG_ERR_ARG;
   }
@@ -2269,47 +2269,49 @@ int bcmg_case_autotune(bcmg_case *c, int reps, bcmg_tuning *out) {
     int r = bcmg_case_set_tuning(c, &best);  // the LU-SGS candidates run on the chosen flux
     if (r) return r;
   }
-  // Split LU-SGS sweep: the widest plane's threads or half of them (wide
-  // planes then take two passes), timed on the residual of the current
-  // state; the state is restored afterwards.
+  // Split LU-SGS: a sweeping CTA's widest plane in threads or half of them (wide
+  // planes then take two passes).  Each timed launch starts from the context's own
+  // state and its residual: the sweep leaves its increment in the residual's place.
   if (c->precision == BCMG_PRECISION_SPLIT && c->method == BCMG_METHOD_LUSGS) {
-    const int full = lusgs_split_default_threads(n);
+    const int full = lusgs_split_plane_threads(n);
     const int cand[2] = {full, ((full / 2) + 31) / 32 * 32};
     const size_t bytes = c->ncell * 5 * sizeof(double);
     CK(cudaMemcpyAsync(c->U1p1, c->U1_, bytes, cudaMemcpyDeviceToDevice, c->stream));
-    int r = case_mirror_all(c);
-    if (!r) r = case_flux(c, 0);  // residual of the current state
-    if (r) return r;
-    cudaEvent_t e0, e1;
-    CK(cudaEventCreate(&e0));
-    CK(cudaEventCreate(&e1));
+    struct Events {
+      cudaEvent_t a = nullptr, b = nullptr;
+      ~Events() {
+        if (a) cudaEventDestroy(a);
+        if (b) cudaEventDestroy(b);
+      }
+    } ev;
+    CK(cudaEventCreate(&ev.a));
+    CK(cudaEventCreate(&ev.b));
     double lbest = 1e300;
-    for (int v = 0; v < 2; ++v) {
+    for (int v = 0; v < (cand[1] < full ? 2 : 1); ++v) {
       c->lu_threads = cand[v];
-      LusgsSplitArgs l = lusgs_split_args(c);
-      cudaError_t e = launch_lusgs_split(l, c->ncube - 1, c->stream);  // warm-up
-      if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
-      for (int i = 0; i < reps && e == cudaSuccess; ++i)
-        e = launch_lusgs_split(l, c->ncube - 1, c->stream);
-      if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
-      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-      float ms = 0;
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-      if (e != cudaSuccess) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        CK(e);
+      double ms = 0;
+      for (int i = -1; i < reps; ++i) {  // (the first a warm-up)
+        CK(cudaMemcpyAsync(c->U1_, c->U1p1, bytes, cudaMemcpyDeviceToDevice, c->stream));
+        int r = case_mirror_all(c);
+        if (!r) r = case_flux(c, 0);
+        if (r) return r;
+        CK(cudaEventRecord(ev.a, c->stream));
+        CK(launch_lusgs_split(lusgs_split_args(c), c->nreal, c->stream));
+        CK(cudaEventRecord(ev.b, c->stream));
+        CK(cudaEventSynchronize(ev.b));
+        float t = 0;
+        CK(cudaEventElapsedTime(&t, ev.a, ev.b));
+        if (i >= 0) ms += t;
       }
       best.lusgs_ms[v] = ms / reps;
-      if (ms / reps < lbest) {
-        lbest = ms / reps;
+      if (best.lusgs_ms[v] < lbest) {
+        lbest = best.lusgs_ms[v];
         best.lusgs_threads = v == 0 ? 0 : cand[v];
       }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     CK(cudaMemcpyAsync(c->U1_, c->U1p1, bytes, cudaMemcpyDeviceToDevice, c->stream));
-    if ((r = case_mirror_all(c))) return r;  // the sweeps updated the mirror in place
+    int r = case_mirror_all(c);  // the sweeps updated the mirror in place
+    if (r) return r;
     CK(cudaStreamSynchronize(c->stream));
   }
   int r = bcmg_case_set_tuning(c, &best);

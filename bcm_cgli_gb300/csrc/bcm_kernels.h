@@ -212,8 +212,10 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
 // Norm partial sums per cube and kernels of one launch_lusgs_split call.
 int lusgs_split_blocks(int n);
 int lusgs_split_launches();
-// Default threads per cube of the split LU-SGS kernel (the widest plane).
-int lusgs_split_default_threads(int n);
+// Threads for the widest plane of a cube (the most that may be asked for) and of
+// one of the CTAs that sweep it (the default).
+int lusgs_split_most_threads(int n);
+int lusgs_split_plane_threads(int n);
 
 // PLOT3D byte images of BCM_Output (bcm_output.cu) for cubes
 // [cube0, cube0 + ncubes): solution (4 + 5 (n+2)^3 doubles per cube) and

@@ -459,14 +459,20 @@ int lus_plane_cells(int n, int size) {
 int lusgs_split_blocks(int n) { return n; }
 int lusgs_split_launches() { return 3; }
 
-// Threads for the widest plane of a cube, in whole warps.
-int lusgs_split_default_threads(int n) { return (lus_plane_cells(n, 1) + 31) / 32 * 32; }
+// CTAs that sweep a cube.
+static int lus_size(int n) { return lus_plane_cells(n, 1) <= kSweepThreads ? 1 : 4; }
+
+// Threads for the widest plane of a cube, and of a sweeping CTA, in whole warps.
+int lusgs_split_most_threads(int n) { return (lus_plane_cells(n, 1) + 31) / 32 * 32; }
+int lusgs_split_plane_threads(int n) {
+  return (lus_plane_cells(n, lus_size(n)) + 31) / 32 * 32;
+}
 
 cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t s) {
   if (ncubes <= 0) return cudaSuccess;
   const int n = a.ph.n, nn = n * n;
   if (nn > 1024) return cudaErrorInvalidValue;
-  if (a.threads > 0 && (a.threads % 32 != 0 || a.threads > lusgs_split_default_threads(n)))
+  if (a.threads > 0 && (a.threads % 32 != 0 || a.threads > lusgs_split_most_threads(n)))
     return cudaErrorInvalidValue;
   cudaError_t e;
   const size_t pack = sizeof(float4) * kWords * nn;
@@ -478,12 +484,12 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   // bytes: 0.63 ms, by clusters of two 0.69; 8 cubes 0.29 and 0.30).  Wider
   // planes go to clusters of four: 64 cubes of 32^3 0.62 ms, by one CTA of 768
   // threads 0.74; now by clusters of two, four and eight 0.58, 0.56 and 0.58.
-  const int size = lus_plane_cells(n, 1) <= kSweepThreads ? 1 : 4;
+  const int size = lus_size(n);
   // (a thread a cell of a slab: 256 whatever the slab took 25 us more for 4,096
   // cubes of 4^3)
   k_lus_pack<<<ncubes * n, std::min(kSlabThreads, (nn + 31) / 32 * 32), pack, s>>>(a, size);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  int threads = (lus_plane_cells(n, size) + 31) / 32 * 32;
+  int threads = lusgs_split_plane_threads(n);
   if (a.threads > 0) threads = std::min(threads, a.threads);  // wide planes take several passes
   const size_t smem = lus_smem(n, size);
   const auto sweep = size == 1 ? k_lus_sweep<1> : k_lus_sweep<4>;
