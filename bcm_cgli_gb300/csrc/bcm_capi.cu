@@ -1930,6 +1930,7 @@ int bcmg_case_advance_converged(bcmg_case *c, int steps, int max_subiters, doubl
     for (int st = 0; st < steps; ++st) {
       k_conv_reset<<<1, 128, 0, c->stream>>>(c->active, c->iters, c->ncase);
       CK(cudaGetLastError());
+      if ((r = case_mirror_all(c))) return r;
       for (int it = 0; it < max_subiters; ++it) {
         if ((r = case_subiter(c)) || (r = case_settle(c))) return r;
         k_conv_check<<<1, 32, 0, c->stream>>>(c->er, c->active, c->iters, c->ncase, tol,
