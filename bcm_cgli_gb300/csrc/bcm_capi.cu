@@ -1873,9 +1873,11 @@ int bcmg_case_set_method(bcmg_case *c, int method, double cfl, double omega) {
   c->method = method;
   c->lu_cfl = cfl;
   c->lu_omega = omega;
-  if (c->graph) cudaGraphExecDestroy(c->graph);  // the captured step changes
+  if (c->graph) cudaGraphExecDestroy(c->graph);  // the captured steps change
   c->graph = nullptr;
   c->graph_subiters = -1;
+  if (c->cgraph) cudaGraphExecDestroy(c->cgraph);
+  c->cgraph = nullptr;
   return BCMG_OK;
 }
 

@@ -1,4 +1,5 @@
-"""Convergence-driven stepping on the split path: eager and as a graph."""
+"""Convergence-driven stepping: eager and as a graph on the split path, and
+after a change of the LU-SGS parameters."""
 import numpy as np
 import pytest
 
@@ -24,3 +25,22 @@ def test_eager_steps_equal_graph_steps(method):
         b.close()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", [api.PRECISION_FP64, api.PRECISION_SPLIT])
+def test_new_lusgs_parameters_reach_the_captured_step(precision):
+    case = cases.taylor_green(ncx=2, n=8)
+    out = []
+    for before in (True, False):
+        ctx = api.CaseContext(case, precision=precision)
+        if before:  # a step graph with other parameters
+            ctx.set_method(api.METHOD_LUSGS, cfl=0.0, omega=1.5)
+            ctx.set_state(case.U, case.U, case.U)
+            ctx.advance_converged(1, 4, 1e-3)
+        ctx.set_method(api.METHOD_LUSGS, cfl=2.0, omega=1.1)
+        ctx.set_state(case.U, case.U, case.U)
+        ctx.emax[:] = 0
+        ctx.advance_converged(1, 4, 1e-3)
+        out.append(ctx.get_state()[0])
+        ctx.close()
+    assert np.array_equal(*out)
