@@ -825,13 +825,13 @@ static ShapeAny flux_shape(int n, int tile, int ncubes) {
   auto consider = [&](int i, int j, int k) {
     ShapeAny s{i, j, k, 1};
     const int cells = box_cells(s), faces = box_faces(s);
-    if (cells > kFluxThreads || flux_smem(s) > 227 * 1024) return;
+    if (cells > kFluxThreads || flux_smem(s) > kMaxSmem) return;
     s.groups = 2;  // shared memory grows by as much with every box
     const size_t two = flux_smem(s);
     s.groups = 1;
     const size_t one = flux_smem(s);
     const int most = (int)std::min<size_t>(kFluxThreads / cells,
-                                           1 + (227 * 1024 - one) / (two - one));
+                                           1 + (kMaxSmem - one) / (two - one));
     const long long boxes = (long long)ncubes * (n / i) * (n / j) * (n / k);
     const long long waves = (boxes + (long long)kSms * most - 1) / ((long long)kSms * most);
     s.groups = (int)((boxes + kSms * waves - 1) / (kSms * waves));
@@ -864,7 +864,7 @@ static cudaError_t launch_shape(const FluxArgs &a, const Sh &sh, int ncubes, cud
   const int nboxes = ncubes * (n / sh.ti) * (n / sh.tj) * (n / sh.tk);
   if (nboxes == 0) return cudaSuccess;
   const cudaError_t e = cudaFuncSetAttribute(
-      k_flux_fp64<VISCOUS, Sh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      k_flux_fp64<VISCOUS, Sh>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)((nboxes + sh.groups - 1) / sh.groups);
   k_flux_fp64<VISCOUS, Sh><<<grid, kFluxThreads, smem, s>>>(a, sh, nboxes);

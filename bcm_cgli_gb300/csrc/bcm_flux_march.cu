@@ -546,7 +546,7 @@ template <int NN, bool VISCOUS, bool PACK, bool NORMS>
 static cudaError_t launch_march_k(const FluxSplitArgs &a, const MarchShape &sh, unsigned grid,
                                   unsigned threads, size_t smem, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(
-      k_flux_march<NN, VISCOUS, PACK, NORMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      k_flux_march<NN, VISCOUS, PACK, NORMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return e;
   k_flux_march<NN, VISCOUS, PACK, NORMS><<<grid, threads, smem, s>>>(a, sh);
   return cudaGetLastError();
@@ -569,7 +569,7 @@ cudaError_t launch_flux_march(const FluxSplitArgs &a, int ncubes, cudaStream_t s
   const MarchLayout L(n, tj);
   const unsigned threads = march_threads(n, tj);
   const int per_sm = std::max<int>(
-      1, std::min<int>(512 / threads, (int)(227 * 1024 / (L.bytes() + 1024))));
+      1, std::min<int>(512 / threads, (int)(kMaxSmem / (L.bytes() + 1024))));
   const long long total = (long long)ncubes * (n / tj) * (n / kChunk), slots = 152LL * per_sm;
   if (total > INT32_MAX - slots) return cudaErrorInvalidValue;
   const int each = (int)((total + slots - 1) / slots);

@@ -12,6 +12,11 @@ extern "C" void bcmg_internal_set_error(const char *msg);
 
 namespace bcmg {
 
+// The most dynamic shared memory a CTA may ask for.  Kernels whose need varies with
+// the launch are allowed all of it whatever the launch: the allowance belongs to the
+// function, so another thread's may come between setting it and the launch.
+constexpr int kMaxSmem = 227 * 1024;
+
 // Constants of one case in a batch: several independent cases laid end to
 // end in one flat cube list (same n), each with the values the reference
 // takes from its own prm.h / Resolution.h and its own time steps.  FP32

@@ -401,7 +401,7 @@ cudaError_t launch_lusgs(const LusgsArgs &a, int ncubes, cudaStream_t s) {
   while (size < 8 && ncubes * size * 2 <= 152 && lu_plane_cells(n, size) > 96) size *= 2;
   const size_t smem = lu_smem(n, size);
   const int threads = std::min(kLuThreads, (lu_plane_cells(n, size) + 31) / 32 * 32);
-  e = cudaFuncSetAttribute(k_lu_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = cudaFuncSetAttribute(k_lu_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ncubes * size);

@@ -476,7 +476,8 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
     return cudaErrorInvalidValue;
   cudaError_t e;
   const size_t pack = sizeof(float4) * kWords * nn;
-  e = cudaFuncSetAttribute(k_lus_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pack);
+  e = cudaFuncSetAttribute(k_lus_pack, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(float4) * kWords * 1024);  // the largest edge's
   if (e != cudaSuccess) return e;
   // One CTA per cube while the widest plane fits it (up to edge 24): the planes
   // are a chain, and a barrier of the CTA is cheaper than one of a cluster (216
@@ -493,7 +494,7 @@ cudaError_t launch_lusgs_split(const LusgsSplitArgs &a, int ncubes, cudaStream_t
   if (a.threads > 0) threads = std::min(threads, a.threads);  // wide planes take several passes
   const size_t smem = lus_smem(n, size);
   const auto sweep = size == 1 ? k_lus_sweep<1> : k_lus_sweep<4>;
-  e = cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ncubes * size);
