@@ -545,8 +545,9 @@ int flux_march_blocks(int n, int ncubes) { return ncubes * (n / march_tj(n)) * (
 template <int NN, bool VISCOUS, bool PACK, bool NORMS>
 static cudaError_t launch_march_k(const FluxSplitArgs &a, const MarchShape &sh, unsigned grid,
                                   unsigned threads, size_t smem, cudaStream_t s) {
-  const cudaError_t e = cudaFuncSetAttribute(
-      k_flux_march<NN, VISCOUS, PACK, NORMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  const cudaError_t e = cudaFuncSetAttribute(  // (a compile-time edge has one need)
+      k_flux_march<NN, VISCOUS, PACK, NORMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      NN ? (int)smem : kMaxSmem);
   if (e != cudaSuccess) return e;
   k_flux_march<NN, VISCOUS, PACK, NORMS><<<grid, threads, smem, s>>>(a, sh);
   return cudaGetLastError();
