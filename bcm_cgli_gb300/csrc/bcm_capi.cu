@@ -268,13 +268,17 @@ struct bcmg_case {
   }
   float *D2 = nullptr;                   // split precision: FP32 of U1 - U1q
   float *inv_dx = nullptr;               // split precision: n / cube_size per cube
-  // Split precision forms no U1p1, U1p2 and Rku1 (its stages update in place), so
-  // what it needs of its own lies there: the copy of a state while a kernel is
-  // timed in U1p1; in U1p2 and Rku1, one allocation of 80 bytes a padded cell, the
-  // LU-SGS scratch (64 bytes an interior cell, at most 45 a padded one: edges up to
-  // 32), from byte 58 the cell codes of FWS and from byte 60 the FP32 residual.
+  // U1p2 and Rku1 are one allocation (U1p2's).  Split precision forms no U1p1, U1p2
+  // and Rku1 (its stages update in place), so what it needs of its own lies there: the
+  // copy of a state while a kernel is timed in U1p1; in U1p2 and Rku1, 78 bytes a
+  // padded cell, the LU-SGS scratch (64 bytes an interior cell, at most 45 a padded
+  // one: edges up to 32) and from byte 58 the FP32 residual.  The two bytes that a
+  // whole Rku1 would take more are the cell codes'.
+  size_t update_bytes() const { return (precision == BCMG_PRECISION_SPLIT ? 78 : 80) * ncell; }
   float *lu_scr() const { return reinterpret_cast<float *>(U1p2); }
-  float *residual32() const { return reinterpret_cast<float *>(U1p2) + 15 * ncell; }
+  float *residual32() const {
+    return reinterpret_cast<float *>(U1p2) + 58 * ncell / sizeof(float);
+  }
   uint16_t *codes = nullptr;             // split precision: cell codes of FWS
   int *FWS = nullptr;
   double *cube_size = nullptr;
@@ -424,7 +428,7 @@ struct bcmg_case {
     ev.clear();
     dfree(U1_); dfree(U1); dfree(U1q); dfree(U1p1); dfree(U1p2); dfree(Residual1);
     Rku1 = nullptr;  // (in U1p2's allocation)
-    dfree(M); dfree(M2); dfree(mpar); dfree(D2); dfree(inv_dx);
+    dfree(M); dfree(M2); dfree(mpar); dfree(D2); dfree(inv_dx); dfree(codes);
     dfree(FWS); dfree(cube_size); dfree(push); dfree(flags); dfree(bc_cubes);
     faces.free(); faces_p.free(); faces_j.free(); faces_q.free(); faces_r.free();
     dfree(bc_flags); dfree(partials); dfree(er); dfree(emax);
@@ -1216,7 +1220,7 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
   const size_t nd = c->ncell * 5;
   bool ok = ck(dalloc(&c->U1_, nd), "alloc") && ck(dalloc(&c->U1, nd), "alloc") &&
             ck(dalloc(&c->U1q, nd), "alloc") && ck(dalloc(&c->U1p1, nd), "alloc") &&
-            ck(dalloc(&c->U1p2, 2 * nd), "alloc") &&  // and Rku1 after it
+            ck(dalloc(&c->U1p2, c->update_bytes() / sizeof(double)), "alloc") &&
             ck(dalloc(&c->Residual1, nd), "alloc") && ck(dalloc(&c->FWS, c->ncell), "alloc") &&
             ck(dalloc(&c->cube_size, (size_t)d->ncube), "alloc") &&
             ck(dalloc(&c->flags, (size_t)d->ncube), "alloc") &&
@@ -1226,18 +1230,17 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
             ck(dalloc(&c->nsum, 7), "alloc") &&
             ck(dalloc(&c->emax, 6 * (size_t)c->ncase), "alloc");
   if (!ok) return fail(BCMG_ERR_CUDA);
-  c->Rku1 = c->U1p2 + nd;
+  c->Rku1 = c->U1p2 + c->update_bytes() / sizeof(double) - nd;
   if (d->precision == BCMG_PRECISION_SPLIT &&
       !(ck(dalloc(&c->M, nd), "alloc") && ck(dalloc(&c->M2, nd), "alloc") &&
         ck(dalloc(&c->mpar, 1), "alloc") && ck(cudaMemset(c->mpar, 0, sizeof(int)), "memset") &&
         ck(dalloc(&c->D2, nd), "alloc") && ck(cudaMemset(c->D2, 0, nd * sizeof(float)), "memset") &&
         ck(dalloc(&c->inv_dx, (size_t)d->ncube), "alloc") &&
+        ck(dalloc(&c->codes, c->ncell), "alloc") &&
         ck(cudaMemset(c->M, 0, nd * sizeof(float)), "memset") &&
         ck(cudaMemset(c->M2, 0, nd * sizeof(float)), "memset") &&
         true))
     return fail(BCMG_ERR_CUDA);
-  if (d->precision == BCMG_PRECISION_SPLIT)
-    c->codes = reinterpret_cast<uint16_t *>(c->U1p2) + 29 * c->ncell;
   if (c->inv_dx) {
     std::vector<float> inv((size_t)d->ncube, 0.f);
     for (int i = 1; i < d->ncube; ++i) inv[i] = (float)(d->n / d->cube_size[i]);
@@ -1303,8 +1306,7 @@ int create_common(const bcmg_case_desc *d, const BatchInit *bi, bcmg_case **out,
        ck(cudaMemsetAsync(c->U1, 0, nd * 8, s), "memset") &&
        ck(cudaMemsetAsync(c->U1q, 0, nd * 8, s), "memset") &&
        ck(cudaMemsetAsync(c->U1p1, 0, nd * 8, s), "memset") &&
-       ck(cudaMemsetAsync(c->U1p2, 0, nd * 8, s), "memset") &&
-       ck(cudaMemsetAsync(c->Rku1, 0, nd * 8, s), "memset") &&
+       ck(cudaMemsetAsync(c->U1p2, 0, c->update_bytes(), s), "memset") &&
        ck(cudaMemsetAsync(c->Residual1, 0, nd * 8, s), "memset") &&
        ck(cudaMemsetAsync(c->er, 0, 8 * 8 * (size_t)c->ncase, s), "memset") &&
        ck(cudaMemsetAsync(c->emax, 0, 6 * 8 * (size_t)c->ncase, s), "memset") &&
