@@ -814,10 +814,11 @@ __global__ void __launch_bounds__(kFluxThreads, 1) k_flux_fp64(FluxArgs a, Sh sh
 // 512 cells in all groups together, with the least waves of CTAs (one to an SM)
 // times the time of a CTA: 28 us, 11 per turn of the 512 threads over its faces,
 // 0.047 per face and 0.006 per primitive (fitted to 186 launches of one wave at
-// edges 4 to 36, within 13%).  Of the groups with the least
-// waves the fewest: where few boxes fill one wave, large CTAs would leave SMs idle
-// (one cube of 20^3 in 16 CTAs of 500 cells 160 us, in 125 of 64 cells 51; eight of
-// 4^3 in two CTAs 139, in eight 51; 64 of 12^3 271, now 257).
+// edges 4 to 36, within 13%).  Of the groups with the least waves the fewest: where
+// few boxes fill one wave, large CTAs would leave SMs idle (one cube of 20^3 in 16
+// CTAs of 500 cells 160 us, in 125 of 64 cells 51, with solids 318 and 66; eight
+// of 4^3 in two CTAs 139, in 128 of four cells 49).  Many cubes take the largest
+// boxes (512 of 12^3 1.88 ms in boxes of 432 cells).
 static ShapeAny flux_shape(int n, int tile, int ncubes) {
   constexpr int kSms = 152;
   ShapeAny best{4, 4, 4, 1};

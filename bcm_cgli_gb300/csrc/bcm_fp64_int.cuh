@@ -1,9 +1,9 @@
 // Correctly rounded FP64 division, square root and multiplication on the
 // integer pipes.
 //
-// This part issues an FP64 instruction once in 64 issue slots of an SM
-// sub-partition (73 cycles measured at 1.92 GHz); a division is eight of them (584
-// cycles) and a square root as many.  The same results from 32-bit integer
+// A warp's FP64 instruction takes 73 cycles of an SM sub-partition's FP64 pipe
+// (measured at 1.92 GHz; two lanes an SM and cycle would be 64), a division eight
+// of them (584) and a square root as many.  The same results from 32-bit integer
 // instructions cost 72 cycles per division that shares its divisor's
 // reciprocal (48 more for the reciprocal) and 54 per multiplication, and run
 // beside the FP64 pipe: a multiplication here and an FP64 addition side by

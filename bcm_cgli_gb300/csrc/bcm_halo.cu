@@ -478,7 +478,7 @@ cudaError_t launch_layers(const LayerArgs &a, int ncubes, cudaStream_t s) {
 // split: 490 -> 374 us, among 92 cubes in FP64: 1057 -> 952.
 //
 // Eight lanes per entry, one stencil cell each, the next entry's indices and
-// weights loaded ahead.  The FP64 pipe (64 cycles an instruction of a warp)
+// weights loaded ahead.  The FP64 pipe (73 cycles an instruction of a warp)
 // bounds a level's chain: the cells' divisions go to the integer pipes, each
 // lane forms its cell's weighted terms, and lanes 0..4 sum one quantity each
 // in the reference's order (000,100,010,001,110,101,011,111) and form one

@@ -63,7 +63,7 @@ __global__ void k_ibm_cube_box(int ncube, int n, const double *__restrict__ cube
 }
 
 // The order of the doubles as integers (NaN excluded, -0 as 0): comparisons
-// on the integer pipes instead of 64 cycles a warp each on the FP64 pipe.
+// on the integer pipes instead of 73 cycles a warp each on the FP64 pipe.
 __device__ __forceinline__ long long sort_key(double x) {
   const long long b = __double_as_longlong(x == 0.0 ? 0.0 : x);
   return b < 0 ? b ^ 0x7fffffffffffffffll : b;
@@ -265,7 +265,7 @@ __device__ __noinline__ int ray_hit(const double *o, const double *r, double *tt
 // reuse the layout.
 // The FP32 filter leaves one or two triangles a cell for the FP64 test: 5,984
 // cells by 20,480 triangles took 1,996 us with the FP64 test on every pair (its
-// first dot product alone takes six slots of 64 cycles a warp), 57 with the
+// first dot product alone takes six slots of 73 cycles a warp), 57 with the
 // filter.
 constexpr int kGhostBlock = 128;
 __global__ void __launch_bounds__(kGhostBlock)

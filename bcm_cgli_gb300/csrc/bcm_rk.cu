@@ -37,7 +37,7 @@ __device__ __noinline__ void third_stage_ref(const double *q, const double *p2, 
     x[v] = 1.0 / 3.0 * q[v] + 2.0 / 3.0 * p2[v] + 2.0 / 3.0 * rk[v];
 }
 
-// Bound by the FP64 pipe at stage 3 (64 cycles an operation of a warp, a
+// Bound by the FP64 pipe at stage 3 (73 cycles an operation of a warp, a
 // division 584): the eight divisions and the fifteen products of the
 // combination go to the integer pipes, and a warp's sums take 9 additions
 // instead of 35: 262,144 cells of stage 3 94 -> 39 us, 393,216 with ghost and
